@@ -1,4 +1,6 @@
 // C ABI: argument checks, workspace layout, tensor-map encoding and the launch sequence.
+#include <unistd.h>
+
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -661,6 +663,12 @@ void note_launch(const char* name) {
 extern "C" {
 
 int b200moe_version(void) { return B200MOE_VERSION; }
+
+int b200moe_env_set(void) {
+  for (char** v = environ; v != nullptr && *v != nullptr; ++v)
+    if ((*v)[0] == 'B' && std::strncmp(*v, "B200MOE_", 8) == 0) return 1;
+  return 0;
+}
 
 const char* b200moe_status_string(int code) {
   switch (code) {

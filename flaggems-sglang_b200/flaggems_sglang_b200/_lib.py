@@ -60,6 +60,7 @@ class Router(C.Structure):
 # name -> (restype, argtypes); every symbol include/b200moe.h declares
 SYMBOLS = {
     "b200moe_version": (C.c_int, []),
+    "b200moe_env_set": (C.c_int, []),
     "b200moe_status_string": (C.c_char_p, [C.c_int]),
     "b200moe_pick_block_tokens": (C.c_int, [C.POINTER(Cfg)]),
     "b200moe_uses_matrix_vector_path": (C.c_int, [C.POINTER(Cfg)]),
@@ -108,13 +109,20 @@ SYMBOLS = {
 _lib = None
 
 
+def env_set() -> int:
+    """Is any B200MOE_* environment variable set?  Bound by ``lib()``, called with the interpreter
+    lock held (``os.environ`` cannot change underneath)."""
+    lib()
+    return env_set()
+
+
 class ExtensionMissing(RuntimeError):
     pass
 
 
 def lib() -> C.CDLL:
     """Load the shared object; there is no fallback when it is missing."""
-    global _lib
+    global _lib, env_set
     if _lib is None:
         path = Path(os.environ.get("B200MOE_LIB", LIB_PATH))   # override: development builds
         if not path.exists():
@@ -129,6 +137,7 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         if handle.b200moe_version() != VERSION:
             raise ExtensionMissing(f"{path} has ABI version {handle.b200moe_version()}, expected {VERSION}")
+        env_set = C.PyDLL(str(path)).b200moe_env_set
         _lib = handle
     return _lib
 

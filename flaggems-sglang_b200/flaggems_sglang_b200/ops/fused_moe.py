@@ -7,9 +7,11 @@ library instead of Triton.  Python here only validates, allocates and launches.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import logging
 import os
+import sys
 from types import SimpleNamespace
 from typing import Optional
 
@@ -27,7 +29,18 @@ _DTYPES = {torch.bfloat16: _lib.DTYPE_BF16, torch.float16: _lib.DTYPE_FP16}
 _ACTS = {"silu": _lib.ACT_SILU, "gelu": _lib.ACT_GELU, "swiglu_oai": _lib.ACT_SWIGLU_OAI}
 
 # ---------------------------------------------------------------------------- state
-_workspaces: dict = {}     # (device index, stream handle) -> uint8 tensor
+# A decode call is two to five launches of a few microseconds each, so what the host does around them is
+# kept short: problem descriptions are looked up instead of rebuilt (_plan), the stream, device and
+# capture state come from torch's C functions (the torch.cuda wrappers build a Python object per call),
+# and the environment is read only when it holds one of this library's variables.  One token of the
+# 128-expert layer: 35 us of host time per call before, 16 us now (137 -> 20 us through the plug-in hook,
+# most of it a failing import per call).
+_raw_stream = torch._C._cuda_getCurrentRawStream     # stream handle of a device index
+_current_device = torch._C._cuda_getDevice
+_capturing = torch._C._cuda_isCurrentStreamCapturing
+_SAME_DEVICE = contextlib.nullcontext()
+
+_workspaces: dict = {}     # (device index, stream handle) -> (uint8 tensor, aligned address, usable bytes)
 _status: dict = {}         # device index -> int32[1]
 # re-laid-out weights, keyed by the identity of the caller's tensor object (a dictionary keyed by
 # tensor *value* would compare two tensors with ==, which has no truth value)
@@ -38,22 +51,25 @@ MAX_CACHED_WORKSPACES = 8     # (device, stream) pairs that keep a scratch buffe
 _captured: list = []          # buffers a CUDA graph under capture was given: a replay writes to them
 
 
-def _workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
+def _workspace(dev: torch.device, stream: int, nbytes: int):
     """Scratch buffer of the calling (device, stream), kept between calls so that the hot path
     does not allocate; it grows to the largest call seen on that stream.  At most
     MAX_CACHED_WORKSPACES pairs keep one (the least recently used goes first) and
     ``release_workspaces`` drops them all.  A buffer handed out while the stream is being
-    captured into a CUDA graph is never dropped: replays of the graph keep using it."""
-    key = (dev.index, torch.cuda.current_stream(dev).cuda_stream)
-    ws = _workspaces.pop(key, None)
-    if ws is None or ws.numel() < nbytes:
+    captured into a CUDA graph is never dropped: replays of the graph keep using it.
+    Returns (tensor, 256-byte aligned address, bytes from there on)."""
+    key = (dev.index, stream)
+    ent = _workspaces.pop(key, None)
+    if ent is None or ent[2] < nbytes:
         ws = torch.empty(int(nbytes * 1.25) + 4096, dtype=torch.uint8, device=dev)
-    _workspaces[key] = ws                     # re-inserted last: dict order is the LRU order
+        base = (ws.data_ptr() + 255) & ~255
+        ent = (ws, base, ws.numel() - (base - ws.data_ptr()))
+    _workspaces[key] = ent                    # re-inserted last: dict order is the LRU order
     while len(_workspaces) > MAX_CACHED_WORKSPACES:
         _workspaces.pop(next(iter(_workspaces)))
-    if torch.cuda.is_current_stream_capturing() and not any(ws is c for c in _captured):
-        _captured.append(ws)
-    return ws
+    if _capturing() and not any(ent[0] is c for c in _captured):
+        _captured.append(ent[0])
+    return ent
 
 
 def release_workspaces(device=None) -> None:
@@ -73,7 +89,7 @@ def _status_word(dev: torch.device) -> torch.Tensor:
     return st
 
 
-_status_host: dict = {}    # device index -> pinned int32[1] that trails the device word
+_status_host: dict = {}    # device index -> (pinned int32[1] that trails the device word, the same as a C int)
 _status_calls: dict = {}
 STATUS_COPY_EVERY = 16     # calls between two asynchronous copies of the status word to the host
 
@@ -84,23 +100,21 @@ def _deferred_status_check(dev: torch.device, status: torch.Tensor) -> None:
     host memory, and every call looks at the host copy first.  A time-out therefore surfaces a
     few calls after the kernels that hit it have finished, even in a host that never calls
     ``check_status()``.  ``B200MOE_DEFERRED_STATUS=0`` switches it off."""
-    if os.environ.get("B200MOE_DEFERRED_STATUS", "1") == "0":
-        return
-    host = _status_host.get(dev.index)
+    idx = dev.index
+    host = _status_host.get(idx)
     if host is None:
-        host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _status_host[dev.index] = host
-        _status_calls[dev.index] = 0
-    elif not torch.cuda.is_current_stream_capturing():
-        code = int(host[0])          # plain host read: whatever an earlier copy has delivered
-        if code != 0:
-            host.zero_()
-            status.zero_()
-            raise RuntimeError(f"b200moe: a device-side wait timed out (code {code}) in an earlier call on "
-                               f"cuda:{dev.index}; that call's output is invalid")
-    _status_calls[dev.index] += 1
-    if _status_calls[dev.index] % STATUS_COPY_EVERY == 1 and not torch.cuda.is_current_stream_capturing():
-        host.copy_(status, non_blocking=True)
+        pinned = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _status_host[idx] = host = (pinned, C.c_int.from_address(pinned.data_ptr()))
+        _status_calls[idx] = 0
+    elif host[1].value != 0 and not _capturing():   # plain host read: whatever an earlier copy has delivered
+        code = host[1].value
+        host[0].zero_()
+        status.zero_()
+        raise RuntimeError(f"b200moe: a device-side wait timed out (code {code}) in an earlier call on "
+                           f"cuda:{idx}; that call's output is invalid")
+    calls = _status_calls[idx] = _status_calls[idx] + 1
+    if calls % STATUS_COPY_EVERY == 1 and not _capturing():
+        host[0].copy_(status, non_blocking=True)
 
 
 def check_status(device=None) -> None:
@@ -115,7 +129,7 @@ def check_status(device=None) -> None:
         if code != 0:
             st.zero_()
             if idx in _status_host:
-                _status_host[idx].zero_()
+                _status_host[idx][0].zero_()
             raise RuntimeError(f"b200moe: device-side wait timed out (code {code}) on cuda:{idx}")
 
 
@@ -155,6 +169,25 @@ def _make_cfg(m, h, i, e, k, dtype, wmode, activation, flags, block_tokens, rout
               n_global_experts=0) -> _lib.Cfg:
     return _lib.Cfg(C.sizeof(_lib.Cfg), m, h, i, e, k, dtype, wmode, _lib.LAYOUT_LAYER, activation, flags,
                     block_tokens, routed_scaling, 0, n_global_experts)
+
+
+_plans: dict = {}      # problem description -> (Cfg, reference to it, workspace bytes)
+MAX_PLANS = 512
+
+
+def _plan(key: tuple):
+    """The ``Cfg`` block and the workspace size of one problem: arguments of ``_make_cfg`` and the
+    device index (the kernel choice depends on its number of SMs)."""
+    plan = _plans.get(key)
+    if plan is None:
+        cfg = _make_cfg(*key[:-1])
+        with torch.cuda.device(key[-1]):
+            nbytes = _lib.lib().b200moe_workspace_bytes(C.byref(cfg))
+        plan = (cfg, C.byref(cfg), nbytes)
+        if len(_plans) >= MAX_PLANS:
+            _plans.clear()
+        _plans[key] = plan
+    return plan
 
 
 def _env_flags() -> int:
@@ -236,10 +269,13 @@ def fused_experts(
     ``routing=(hist [E], topk_indx [P], gate_scal [P])`` taken from the
     reference's routing triple.  Returns a new ``[M, H]`` tensor.
     """
-    if activation not in _ACTS:
+    act = _ACTS.get(activation)
+    if act is None:
         raise ValueError(f"Unsupported FusedMoe activation: {activation}")
     if not hidden_states.is_cuda:
         raise RuntimeError("hidden_states must be a CUDA tensor: this package has no CPU path")
+    lib = _lib.lib()
+    env = _lib.env_set()         # is any B200MOE_* variable set?
     x = hidden_states.contiguous()
     dev = x.device
     m, h = x.shape
@@ -247,12 +283,13 @@ def fused_experts(
     i = two_i // 2
     pack = 8 if use_int4_w4a16 else 1
     assert hw * pack == h, "hidden size mismatch"
-    assert w2.shape[0] == e and w2.shape[1] == h and w2.shape[2] * pack == i, "intermediate size mismatch"
+    e2, h2, iw = w2.shape
+    assert e2 == e and h2 == h and iw * pack == i, "intermediate size mismatch"
     assert w13.is_contiguous() and w2.is_contiguous(), "weights must be contiguous"
-    flags = _env_flags()
-    odt = x.dtype
+    flags = _env_flags() if env else 0
+    odt = xdt = x.dtype
     xs_keep = None
-    if x.dtype == torch.float8_e4m3fn:
+    if xdt == torch.float8_e4m3fn:
         assert use_fp8_w8a8 and x_scale is not None, "FP8 activations need FP8 weights and x_scale"
         assert h % 128 == 0 and x_scale.shape == (m, h // 128), "x_scale must be [M, H/128]"
         odt = out_dtype or torch.bfloat16
@@ -282,7 +319,7 @@ def fused_experts(
             quant.x_scale = xs_keep.data_ptr()
     elif use_int4_w4a16:
         wmode = _lib.W_INT4_AWQ
-        assert x.dtype == torch.float16, "int4 w4a16 takes fp16 activations"
+        assert xdt == torch.float16, "int4 w4a16 takes fp16 activations"
         assert w13.dtype == torch.int32 and w2.dtype == torch.int32, "packed int4 weights must be int32"
         assert w13_sz is not None and w2_sz is not None, "scale/zero tables are required"
         assert w13_sz.dtype == torch.int32 and w13_sz.shape == (e, h // 128, 2 * i), "w13_sz must be [E, H/128, 2I] int32"
@@ -291,7 +328,7 @@ def fused_experts(
         keep += [z1, z2]
         quant = _lib.Quant(None, None, z1.data_ptr(), z2.data_ptr())
     else:
-        assert w13.dtype == x.dtype and w2.dtype == x.dtype, "weights must have the activation dtype"
+        assert w13.dtype == xdt and w2.dtype == xdt, "weights must have the activation dtype"
     if b13 is not None or b2 is not None or activation == "swiglu_oai":
         # per-expert biases and the clamped swiglu, for every weight mode
         bias1 = b13.to(torch.float32).contiguous() if b13 is not None else None
@@ -308,7 +345,6 @@ def fused_experts(
         quant.swiglu_alpha = float(swiglu_alpha)
         quant.swiglu_limit = float(swiglu_limit) if swiglu_limit else 0.0
 
-    lib = _lib.lib()
     if router is not None:
         assert routing is None and topk_weights is None and topk_ids is None, "router excludes other routing inputs"
         (rt, logits, _bias_keepalive), k = router
@@ -317,9 +353,10 @@ def fused_experts(
         assert topk_weights is not None and topk_ids is not None, "routing or (topk_weights, topk_ids) required"
         k = topk_ids.shape[1]
         ids = topk_ids.contiguous()
-        assert ids.dtype in (torch.int32, torch.int64), "topk_ids must be int32 or int64"
         if ids.dtype == torch.int64:
             flags |= _lib.FLAG_IDS_I64
+        else:
+            assert ids.dtype == torch.int32, "topk_ids must be int32 or int64"
         tw = topk_weights.to(torch.float32).contiguous()
     else:
         hist, topk_indx, gate_scal, k = routing
@@ -329,49 +366,45 @@ def fused_experts(
 
     if no_combine:
         flags |= _lib.FLAG_NO_COMBINE
+    n_global, emap, emap_ptr = 0, None, None
     if expert_map is not None:
         assert expert_map.ndim == 1 and expert_map.numel() >= e, "expert_map must list every global expert"
-    cfg = _make_cfg(m, h, i, e, k, dtype, wmode, _ACTS[activation], flags,
-                    block_tokens or _block_tokens_env(), float(routed_scaling_factor),
-                    expert_map.numel() if expert_map is not None else 0)
+        n_global = expert_map.numel()
+        emap = expert_map.to(device=dev, dtype=torch.int32).contiguous()
+        emap_ptr = emap.data_ptr()
+    if env and not block_tokens:
+        block_tokens = _block_tokens_env()
+    cfg, cfg_ref, nbytes = _plan((m, h, i, e, k, dtype, wmode, act, flags, block_tokens, float(routed_scaling_factor),
+                                  n_global, dev.index))
     out = torch.empty((m, k, h) if no_combine else (m, h), dtype=odt, device=dev)
     if m == 0:
         return out
-    nbytes = lib.b200moe_workspace_bytes(C.byref(cfg))
     if nbytes == 0:
-        rc = lib.b200moe_pick_block_tokens(C.byref(cfg))
+        rc = lib.b200moe_pick_block_tokens(cfg_ref)
         _lib.check(rc if rc < 0 else _lib.ERR_UNSUPPORTED, "fused_experts")
-    ws = _workspace(dev, nbytes)
-    base = (ws.data_ptr() + 255) & ~255
-    avail = ws.numel() - (base - ws.data_ptr())
+    stream = _raw_stream(dev.index)
+    _, base, avail = _workspace(dev, stream, nbytes)
     status = _status_word(dev)
-    stream = torch.cuda.current_stream(dev).cuda_stream
     qref = C.byref(quant) if quant is not None else None
-    with torch.cuda.device(dev):
+    with _SAME_DEVICE if _current_device() == dev.index else torch.cuda.device(dev):
         if router is not None:
-            emap = None
-            if expert_map is not None:
-                emap = expert_map.to(device=dev, dtype=torch.int32).contiguous()
             rc = lib.b200moe_forward_logits(
-                C.byref(cfg), C.byref(rt), x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, logits.data_ptr(),
-                emap.data_ptr() if emap is not None else None, base, avail, out.data_ptr(),
-                status.data_ptr(), stream)
+                cfg_ref, C.byref(rt), x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, logits.data_ptr(),
+                emap_ptr, base, avail, out.data_ptr(), status.data_ptr(), stream)
         elif routing is None:
-            emap = None
-            if expert_map is not None:
-                emap = expert_map.to(device=dev, dtype=torch.int32).contiguous()
             rc = lib.b200moe_forward_topk(
-                C.byref(cfg), x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, tw.data_ptr(), ids.data_ptr(),
-                emap.data_ptr() if emap is not None else None, base, avail, out.data_ptr(),
-                status.data_ptr(), stream)
+                cfg_ref, x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, tw.data_ptr(), ids.data_ptr(),
+                emap_ptr, base, avail, out.data_ptr(), status.data_ptr(), stream)
         else:
             rc = lib.b200moe_forward_routed(
-                C.byref(cfg), x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, hist.data_ptr(),
+                cfg_ref, x.data_ptr(), w13.data_ptr(), w2.data_ptr(), qref, hist.data_ptr(),
                 topk_indx.data_ptr(), gate_scal.data_ptr(), base, avail, out.data_ptr(),
                 status.data_ptr(), stream)
-    _lib.check(rc, "fused_experts")
-    _deferred_status_check(dev, status)
-    if os.environ.get("B200MOE_CHECK_STATUS", "0") == "1":
+    if rc != _lib.OK:
+        _lib.check(rc, "fused_experts")
+    if not env or os.environ.get("B200MOE_DEFERRED_STATUS", "1") != "0":
+        _deferred_status_check(dev, status)
+    if env and os.environ.get("B200MOE_CHECK_STATUS", "0") == "1":
         check_status(dev)
     return out
 
@@ -538,6 +571,24 @@ def triton_kernel_fused_experts_with_bias(
     return out.view(hidden_states.shape[0], hidden_states.shape[1])
 
 
+_combine_class: dict = {}   # was sglang loaded at the look-up -> the result class of the hook
+
+
+def _combine_input():
+    """``StandardCombineInput`` of the running SGLang, or a namespace with the same field without
+    one.  Looked up once per state of ``sys.modules``: a failing import costs 100 us."""
+    loaded = "sglang" in sys.modules
+    cls = _combine_class.get(loaded)
+    if cls is None:
+        try:
+            from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput as cls
+        except Exception:
+            cls = SimpleNamespace
+        _combine_class["sglang" in sys.modules] = cls
+        _combine_class.setdefault(loaded, cls)
+    return cls
+
+
 def fused_moe_flagos(obj, layer: torch.nn.Module, dispatch_output):
     """SGLang plugin hook (src/flaggems_sglang/ops/fused_moe.py:312-406).
 
@@ -576,11 +627,7 @@ def fused_moe_flagos(obj, layer: torch.nn.Module, dispatch_output):
         routing_data, gather_indx, _ = topk_output
         routing = (routing_data.expt_hist, gather_indx.src_indx, routing_data.gate_scal, routing_data.n_expts_act)
         out = fused_experts(hidden_states, w13, layer.w2_weight, routing=routing, **common)
-    try:
-        from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput
-        return StandardCombineInput(hidden_states=out)
-    except Exception:
-        return SimpleNamespace(hidden_states=out)
+    return _combine_input()(hidden_states=out)
 
 
 _standard_topk_to_triton_kernels = topk_to_routing

@@ -118,6 +118,10 @@ typedef struct b200moe_quant {
 } b200moe_quant;
 
 int b200moe_version(void);
+
+/* 1 if the process environment holds any variable named B200MOE_*, else 0: one pass over the
+ * environment, so that a binding can skip looking the variables up one by one on every call. */
+int b200moe_env_set(void);
 const char *b200moe_status_string(int code);
 
 /* Token block the library would pick for this problem (16, 32, 64, 128 or 256). */
