@@ -36,6 +36,23 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// Index of the thread's warp as a value the compiler knows to be the same for the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+// True in exactly one lane of a converged warp.  The role threads that issue TMA loads and MMAs are
+// picked with it rather than with `lane == 0`: a branch on elect.sync is one the compiler knows to
+// hold a single thread, and it then issues the operands of a tcgen05.mma without a loop over the
+// active lanes.  Four dependent MMAs with a commit and a wait per stage: 137 cycles per MMA behind
+// `lane == 0`, 99 behind elect.sync (128 x 128 x 16; the tensor core itself needs 64).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -64,7 +64,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   int* s_blk_off = reinterpret_cast<int*>(s_col_ptr + 2 * 128);         // [E+1]
   constexpr int CPT = BT / NG;                                          // token columns per promotion thread
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -107,7 +107,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // row offset of the second weight block inside the expert
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
 
-  if (active && warp == 0 && lane == 0) {
+  if (active && warp == 0 && elect_one()) {
     // =============================== TMA producer ===============================
     int stage = 0;
     uint32_t phase = 0;
@@ -146,7 +146,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         mbar_wait_brief(smem_u32(&bar_full[s]), ph);
       }
     }
-  } else if (active && warp == 1 && lane == 0) {
+  } else if (active && warp == 1 && elect_one()) {
     // =============================== MMA issuer =================================
     const uint32_t idesc = make_idesc(0u /* e4m3 */, kTileRows, static_cast<uint32_t>(BT));
     int stage = 0;

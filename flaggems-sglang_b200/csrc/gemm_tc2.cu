@@ -170,14 +170,14 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   int* s_blk_off = reinterpret_cast<int*>(tmem_slot + 4);   // [E+1]
   int* s_pair_off = s_blk_off + (a.E + 1);                   // [E+1]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
-      mbar_init(smem_u32(&bar_full[s]), 2);     // one arrive.expect_tx per CTA of the pair
+      mbar_init(smem_u32(&bar_full[s]), 1);     // the leader announces the bytes of both CTAs
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -224,7 +224,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const int cl_eff = waves > 0 ? (total + waves - 1) / waves : 1;
   const bool active = cluster_id < cl_eff;
 
-  if (active && warp == 0 && lane == 0) {
+  if (active && warp == 0 && elect_one()) {
     // =============================== TMA producer (every CTA, its own operands) ===================
     int stage = 0;
     uint32_t phase = 0;
@@ -241,7 +241,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const uint32_t full = mapa_u32(smem_u32(&bar_full[stage]), 0);   // the leader's barrier
         const uint32_t sx = smem_u32(smem + static_cast<size_t>(stage) * kStageBytes2);
         const int k0 = kb * (kStageKBytes / static_cast<int>(sizeof(T)));
-        mbar_arrive_expect_tx_remote(full, static_cast<uint32_t>(kStageBytes2));
+        if (leader) mbar_arrive_expect_tx(smem_u32(&bar_full[stage]), static_cast<uint32_t>(2 * kStageBytes2));
         tma_load_2d_pair(sx, &tm_x, full, k0, t.blk * kTileRows);
         tma_load_3d_pair(sx + kTileBytes, &tm_w, full, k0, wrow, t.e);
         ++issued;
@@ -271,7 +271,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         }
       }
     }
-  } else if (active && warp == 1 && lane == 0 && leader) {
+  } else if (active && warp == 1 && leader && elect_one()) {
     // =============================== MMA issuer (leader CTA, for the pair) ========================
     const uint32_t fmt = (a.dtype == B200MOE_DTYPE_BF16) ? 1u : 0u;
     const uint32_t idesc = make_idesc(fmt, 256u, 256u);

@@ -106,7 +106,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   int* s_osum = reinterpret_cast<int*>(s_amax + 2 * 32);            // [2][32] tail: sums of the new integers
   int* s_blk_off = s_osum + 2 * 32;                                 // [E+1]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -154,7 +154,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
 
-  if (active && warp == 0 && lane == 0) {
+  if (active && warp == 0 && elect_one()) {
     // =============================== TMA producer ===============================
     int stage = 0;
     uint32_t phase = 0;
@@ -215,7 +215,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         mbar_wait_brief(smem_u32(&bar_full[s]), ph);
       }
     }
-  } else if (active && warp == 1 && lane == 0) {
+  } else if (active && warp == 1 && elect_one()) {
     // =============================== MMA issuer =================================
     const uint32_t idesc = make_idesc_i8(false, true, kTileRows, static_cast<uint32_t>(NB));
     int stage = 0, ost = 0;
