@@ -75,6 +75,22 @@ int make_tmap_3d(CUtensorMap* m, CUtensorMapDataType dt, int elem_bytes, const v
   return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
+// Stacked gate and up rows [experts][2][rows][inner] seen as [experts, rows, 2, inner], box = {box_inner, 2, box_rows,
+// 1}: one load brings the same rows of both halves, gate and up rows alternating.
+int make_tmap_gate_up(CUtensorMap* m, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
+                      uint64_t rows, uint64_t experts, uint32_t box_inner, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return B200MOE_ERR_CUDA;
+  cuuint64_t dims[4] = {inner, 2, rows, experts};
+  cuuint64_t strides[3] = {inner * rows * elem_bytes, inner * elem_bytes, 2 * inner * rows * elem_bytes};
+  cuuint32_t box[4] = {box_inner, 2, box_rows, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Optional per-kernel timing for the benchmark: CUDA events recorded around the two
@@ -129,6 +145,8 @@ struct Layout {
   bool align_multi; // alignment on 32 CTAs (many slots)
   bool quant_once; // FP8: quantise each token once, then gather the quantised rows (many pairs per token)
   bool pair_rows; // the down projection stores one 16-bit row per pair, the output conversion sums them
+  bool pairs2;    // 16-bit GEMMs on CTA pairs: rows padded to 32 per expert, tiles of up to `tile_tokens`
+  int tile_tokens;
   bool w4p;       // int4 decode path: integer MMAs on three-plane int8 activations
   int out_rows;   // rows of the fp32 output buffer: tokens, or pairs when nothing is combined
   int orient;     // GEMM tile orientation that goes with BT
@@ -152,7 +170,10 @@ int pick_bt(const b200moe_cfg* c) {
   }
   if (avg <= 10) return 16;
   if (avg <= 20) return 32;
-  if (avg <= 40) return 64;
+  // 16-bit weights: CTA pairs from here on (they pad to 32 rows and take whatever tiles an expert's rows give).
+  // At 25 tokens per expert they are 2 % (8 experts) to 7 % (128 experts) faster than 64-token blocks, at 10 to
+  // 13 tokens 4 % slower than 32-token ones.
+  if (avg <= 40 && c->wmode == B200MOE_W_INT4_AWQ) return 64;
   return 128;
 }
 
@@ -197,9 +218,15 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   // int4 always runs tokens-on-M (one MMA then covers 256 weight rows, which halves the number of
   // MMA instructions per streamed byte; blocks below 128 tokens simply load fewer token rows)
   if (c->wmode == B200MOE_W_INT4_AWQ) L->orient = (L->BT <= 128) ? 1 : 0;
-  else if (c->wmode == B200MOE_W_FP8_BLOCK)
-    L->orient = (L->BT == 128) ? 1 : 0;
-  else L->orient = (L->BT == 128) ? 1 : 0;
+  else L->orient = (c->wmode == B200MOE_W_FP8_BLOCK && L->BT == 128) ? 1 : 0;
+  const int sms_l = query_sms(c);
+  const int bt_asked = L->BT;
+  L->pairs2 = c->wmode == B200MOE_W_16BIT && L->BT >= 128 && !(c->flags & B200MOE_FLAG_SIMT) && gemm_tc2_ok(c->E, sms_l);
+  L->tile_tokens = c->block_tokens > 0 ? L->BT / 32 * 32 : 256;
+  if (L->pairs2) {
+    L->orient = 2;
+    L->BT = 32;
+  }
   L->P = c->M * c->topk;
   int cap = align_capacity(L->P, c->E, L->BT);
   if (cap < 0) return B200MOE_ERR_TOO_LARGE;
@@ -237,16 +264,15 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   // and let the output conversion sum a token's rows in a fixed order.  The combine buffer shrinks
   // to the pairs' validity bytes.  16-bit weights: only where the reference, too, rounds each
   // pair's row to the 16-bit type (or its rounding is not asked for).
-  const int sms_l = query_sms(c);
-  // (16-bit: from four waves of tiles on; below that the split reduction, which needs the atomics,
-  // is what keeps the last wave full)
-  const bool many_tiles = (static_cast<long long>(L->P) / L->BT) * ((c->H + 255) / 256) >=
+  // (16-bit without the reference's rounding: from four waves of 128 x 256 tiles on; below that the
+  // split reduction, which needs the atomics, is what keeps the last wave full)
+  const bool many_tiles = (static_cast<long long>(L->P) / bt_asked) * ((c->H + 255) / 256) >=
                           (fp8 ? 2LL : 4LL) * sms_l;
-  const bool pairs_ok16 = !fp8 && !L->w4p && L->orient == 1 &&
-                          (!(c->flags & B200MOE_FLAG_MIMIC_ROUNDING) ||
-                           reference_rounds_pairs(L->P, c->E, c->H, c->I, sms_l));
-  L->pair_rows = (fp8 || pairs_ok16) && L->BT == 128 && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
-                 !(c->flags & B200MOE_FLAG_SIMT) && many_tiles;
+  const bool pairs_ok16 = L->pairs2 && ((c->flags & B200MOE_FLAG_MIMIC_ROUNDING)
+                                            ? reference_rounds_pairs(L->P, c->E, c->H, c->I, sms_l)
+                                            : many_tiles);
+  L->pair_rows = ((fp8 && L->BT == 128 && many_tiles) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
+                 !(c->flags & B200MOE_FLAG_SIMT);
   L->out32 = take(L->pair_rows ? 16 : static_cast<size_t>(L->out_rows > 0 ? L->out_rows : 1) * c->H * 4);
   // Quantising inside the gather repeats the work topk times; beyond a few thousand pairs it pays to
   // quantise the M token rows once and gather bytes.
@@ -399,7 +425,7 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   g1.K = c->H;
   g1.N = c->I;
   g1.up_row_off = c->I;
-  g1.BT = L.BT;
+  g1.BT = L.pairs2 ? L.tile_tokens : L.BT;
   g1.orient = L.orient;
   g1.topk = c->topk;
   g1.P = L.P;
@@ -440,7 +466,10 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     g1.out_scale = reinterpret_cast<float*>(ws + L.a2_scale);
     g1.out_sum = reinterpret_cast<int*>(ws + L.a2_sum);
   }
-  if (fp8) gemm_plan_fp8(&g1); else if (w4p) gemm_plan_w4(&g1); else gemm_plan(&g1);
+  auto plan = [&](GemmArgs* g) {
+    if (fp8) gemm_plan_fp8(g); else if (w4p) gemm_plan_w4(g); else if (L.pairs2) gemm_plan_tc2(g); else gemm_plan(g);
+  };
+  plan(&g1);
 
   GemmArgs g2 = g1;
   g2.mode = 1;
@@ -498,15 +527,7 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     g2.out_scale = nullptr;
     g2.out_sum = nullptr;
   }
-  if (fp8) gemm_plan_fp8(&g2); else if (w4p) gemm_plan_w4(&g2); else gemm_plan(&g2);
-  // CTA pairs for the 16-bit prefill GEMMs (each GEMM by itself: the down projection only when its
-  // reduction is in one piece)
-  const bool pair_flag = (c->flags & B200MOE_FLAG_CTA_PAIR) != 0 && !(c->flags & B200MOE_FLAG_SIMT) && sms >= 2;
-  const bool pair1 = pair_flag && gemm_tc2_ok(g1);
-  const bool pair2 = pair_flag && gemm_tc2_ok(g2);
-  if (pair1) gemm_plan_tc2(&g1);
-  if (pair2) gemm_plan_tc2(&g2);
-
+  plan(&g2);
   if (c->flags & B200MOE_FLAG_SIMT) {
     rc = launch_gemm_simt(w1, xs, g1, st, L.cap);
     if (rc != B200MOE_OK) return rc;
@@ -530,25 +551,38 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
                              psw)) != B200MOE_OK)
         return rc;
     } else {
-      if ((rc = make_tmap_3d(&tm_w1, dt, eb, w1, c->H, 2ull * c->I, c->E, kbox, 128)) != B200MOE_OK) return rc;
-      if ((rc = make_tmap_3d(&tm_w2, dt, eb, w2, c->I, c->H, c->E, kbox, (L.orient == 1 && !fp8 && !pair2) ? 256 : 128)) != B200MOE_OK)
-        return rc;
+      rc = L.pairs2 ? make_tmap_gate_up(&tm_w1, dt, eb, w1, c->H, c->I, c->E, kbox, 64)
+                    : make_tmap_3d(&tm_w1, dt, eb, w1, c->H, 2ull * c->I, c->E, kbox, 128);
+      if (rc != B200MOE_OK) return rc;
+      if ((rc = make_tmap_3d(&tm_w2, dt, eb, w2, c->I, c->H, c->E, kbox, 128)) != B200MOE_OK) return rc;
     }
-    // int4 decode: a token block is 3 * BT consecutive rows (its three byte planes)
-    const uint64_t xrows = w4p ? 3ull * L.cap : static_cast<uint64_t>(L.cap);
-    const uint32_t xbox = w4p ? 3u * L.BT : static_cast<uint32_t>(L.BT);
-    if ((rc = make_tmap_2d(&tm_x, dt, eb, xs, c->H, xrows, kbox, xbox)) != B200MOE_OK) return rc;
-    if ((rc = make_tmap_2d(&tm_a2, dt, eb, a2, c->I, xrows, kbox, xbox)) != B200MOE_OK) return rc;
-    prof_mark(slot, 1, st);
-    rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, g1, sms, st)
-             : (w4p ? launch_gemm_w4(tm_w1, tm_x, g1, sms, st)
-                    : (pair1 ? launch_gemm_tc2(tm_w1, tm_x, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st)));
-    prof_mark(slot, 2, st);
-    if (rc != B200MOE_OK) return rc;
-    prof_mark(slot, 3, st);
-    rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, g2, sms, st)
-             : (w4p ? launch_gemm_w4(tm_w2, tm_a2, g2, sms, st)
-                    : (pair2 ? launch_gemm_tc2(tm_w2, tm_a2, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st)));
+    if (L.pairs2) {
+      PairTokenMaps tx1, tx2;
+      for (uint32_t b = 0; b < 8; ++b) {
+        if ((rc = make_tmap_2d(&tx1.m[b], dt, eb, xs, c->H, L.cap, kbox, 16 * (b + 1))) != B200MOE_OK) return rc;
+        if ((rc = make_tmap_2d(&tx2.m[b], dt, eb, a2, c->I, L.cap, kbox, 16 * (b + 1))) != B200MOE_OK) return rc;
+      }
+      prof_mark(slot, 1, st);
+      rc = launch_gemm_tc2(tm_w1, tx1, g1, sms, st);
+      prof_mark(slot, 2, st);
+      if (rc != B200MOE_OK) return rc;
+      prof_mark(slot, 3, st);
+      rc = launch_gemm_tc2(tm_w2, tx2, g2, sms, st);
+    } else {
+      // int4 decode: a token block is 3 * BT consecutive rows (its three byte planes)
+      const uint64_t xrows = w4p ? 3ull * L.cap : static_cast<uint64_t>(L.cap);
+      const uint32_t xbox = w4p ? 3u * L.BT : static_cast<uint32_t>(L.BT);
+      if ((rc = make_tmap_2d(&tm_x, dt, eb, xs, c->H, xrows, kbox, xbox)) != B200MOE_OK) return rc;
+      if ((rc = make_tmap_2d(&tm_a2, dt, eb, a2, c->I, xrows, kbox, xbox)) != B200MOE_OK) return rc;
+      prof_mark(slot, 1, st);
+      rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, g1, sms, st)
+               : (w4p ? launch_gemm_w4(tm_w1, tm_x, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st));
+      prof_mark(slot, 2, st);
+      if (rc != B200MOE_OK) return rc;
+      prof_mark(slot, 3, st);
+      rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, g2, sms, st)
+               : (w4p ? launch_gemm_w4(tm_w2, tm_a2, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st));
+    }
     prof_mark(slot, 4, st);
     if (rc != B200MOE_OK) return rc;
   }

@@ -17,8 +17,8 @@ struct GemmArgs {
   int K;           // reduction length (H for mode 0, I for mode 1)
   int N;           // output rows per expert covered by tiles of 128 (I for mode 0, H for mode 1)
   int up_row_off;  // mode 0: row of the first "up" weight inside an expert (= I)
-  int orient;      // 0: weight rows on the MMA's M side (decode); 1: tokens on the M side (BT = 128)
-  int BT;          // tokens per block (16..256, multiple of 16)
+  int orient;      // 0: weight rows on the MMA's M side (decode); 1: tokens on the M side (BT = 128); 2: CTA pairs
+  int BT;          // tokens per block (16..256, multiple of 16); CTA pairs: upper bound of the tokens per tile
   int stages;      // shared-memory ring depth
   int acc_stages;  // accumulator buffers in tensor memory (1 or 2)
   int tmem_cols;   // allocated tensor-memory columns (power of two >= 32)
@@ -99,11 +99,16 @@ int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Gemm
 void gemm_plan_w4(GemmArgs* a);
 int launch_gemm_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                    cudaStream_t stream);
-// 16-bit, 128-token blocks, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
-bool gemm_tc2_ok(const GemmArgs& a);
+// 16-bit, more than 64 tokens per expert, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
+bool gemm_tc2_ok(int E, int num_sms);
 int gemm_tc2_resident_pairs();   // CTA pairs the device kept resident for the last such launch (0: none yet)
 void gemm_plan_tc2(GemmArgs* a);
-int launch_gemm_tc2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
+// Token maps of a pair launch: m[i] has boxes of 16 (i + 1) rows, half of a tile of 32 (i + 1) tokens.
+struct PairTokenMaps {
+  CUtensorMap m[8];
+};
+// tm_w: mode 0 [E][2][I][K] in boxes of 64 rows of both halves, mode 1 [E][rows][K] in boxes of 128 rows
+int launch_gemm_tc2(const CUtensorMap& tm_w, const PairTokenMaps& tm_x, const GemmArgs& a, int num_sms,
                     cudaStream_t stream);
 int launch_gemm_simt(const void* w, const void* x, const GemmArgs& a, cudaStream_t stream, int cap);
 

@@ -11,8 +11,8 @@
 //   the block and the activation needs no data exchange.
 // mode 1 (down):    one 128-row tile; the reduction may be split over CTAs; the epilogue
 //   multiplies by the routing weight and adds into the fp32 combine buffer with
-//   red.global.add.f32 (which also merges the top-k experts of a token), or, with many pairs on
-//   128-token blocks, stores one 16-bit row per pair for the output conversion to sum.
+//   red.global.add.f32 (which also merges the top-k experts of a token).
+// 16-bit weights run here up to 20 tokens per expert; above that gemm_tc2.cu takes over.
 //
 // Every wait is bounded; on a time-out the CTA raises an abort flag, all roles leave their
 // loops, the status word is set, TMEM is freed and the kernel returns.
@@ -24,7 +24,7 @@ namespace {
 
 // Geometry of one pipeline stage and one accumulator for (MODE, ORIENT).
 //   ORIENT 0 ("weights on M"): decode-sized token blocks (BT = 16..256 tokens on the N side).
-//   ORIENT 1 ("tokens on M"):  BT = 128 tokens on the M side, 256 weight rows on the N side;
+//   ORIENT 1 ("tokens on M"):  int4 only: up to 128 tokens on the M side, 256 weight rows on the N side;
 //                              every epilogue thread owns one token row and stores contiguous
 //                              output columns with 16-byte accesses.
 template <int MODE, int ORIENT>
@@ -108,8 +108,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * kMaxBT);  // [2][kMaxBT]
   int* s_blk_off = reinterpret_cast<int*>(s_col_gam + 2 * kMaxBT);      // [E+1]
 
-  // see `issuer` below for the plain prefill kernels
-  const int warp = (ORIENT == 1 && !W4) ? static_cast<int>(threadIdx.x >> 5) : warp_index();
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -146,11 +145,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const Ctrl c = make_ctrl(a, MODE == 1);
   const int cols_per_acc = (ORIENT == 1) ? 256 : (MODE == 0 ? 2 : 1) * BT;
   const bool active = static_cast<int>(blockIdx.x) < c.grid_eff;
-  // 256-wide MMAs hide the issue cost either way, and under the power cap the steadier `lane == 0`
-  // issue ran 3 % faster there (4096 tokens of the Mixtral-shaped layer: 2733 vs 2821 us)
-  const bool issuer = (ORIENT == 1 && !W4) ? lane == 0 : elect_one();
 
-  if (active && warp == 0 && issuer) {
+  if (active && warp == 0 && elect_one()) {
     // =============================== TMA producer ===============================
     int stage = 0;
     uint32_t phase = 0;
@@ -209,7 +205,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         mbar_wait_brief(smem_u32(&bar_full[s]), ph);
       }
     }
-  } else if (active && warp == 1 && issuer) {
+  } else if (active && warp == 1 && elect_one()) {
     // =============================== MMA issuer =================================
     const uint32_t fmt = (a.dtype == B200MOE_DTYPE_BF16) ? 1u : 0u;
     const uint32_t idesc = make_idesc(fmt, kTileRows, ORIENT == 1 ? 256u : static_cast<uint32_t>(BT));
@@ -350,42 +346,15 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 u[j] += in ? __ldg(bg + a.N + j) : 0.f;
               }
             }
+            act_mul_array<T, EXT>(g, u, w_on_input, mimic, ap, [&](int) { return gam; });
             uint32_t pk[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float lo = act_mul<T, EXT>(g[2 * j], u[2 * j], w_on_input, gam, mimic, ap);
-              const float hi = act_mul<T, EXT>(g[2 * j + 1], u[2 * j + 1], w_on_input, gam, mimic, ap);
-              pk[j] = pack2<T>(lo, hi);
-            }
+            for (int j = 0; j < 8; ++j) pk[j] = pack2<T>(g[2 * j], g[2 * j + 1]);
             if (in_block && t.n0 + c0 + 8 <= a.N)
               *reinterpret_cast<uint4*>(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             if (in_block && t.n0 + c0 + 16 <= a.N)
               *reinterpret_cast<uint4*>(orow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
           }
-        } else if (a.out_pairs != nullptr) {
-          // one 16-bit row per (token, choice) pair, routing weight applied; the output conversion
-          // sums a token's rows in a fixed order (no atomics: a rerun gives the same bits)
-          T* prow = reinterpret_cast<T*>(a.out_pairs) + static_cast<size_t>(valid ? slot : 0) * a.N + t.n0;
-          const float scale = w_on_input ? 1.0f : gam;
-#pragma unroll 1
-          for (int c0 = 0; c0 < 256; c0 += 16) {
-            float v[16];
-            tmem_ld16_wait(taddr + c0, v);
-            if (valid) {
-              if (has_bias) {
-                const float* bo = a.bias + static_cast<size_t>(t.e) * a.N + t.n0 + c0;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] += (t.n0 + c0 + j < a.N) ? __ldg(bo + j) : 0.f;
-              }
-              uint32_t pk[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) pk[j] = pack2<T>(v[2 * j] * scale, v[2 * j + 1] * scale);
-              if (t.n0 + c0 + 8 <= a.N) *reinterpret_cast<uint4*>(prow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              if (t.n0 + c0 + 16 <= a.N)
-                *reinterpret_cast<uint4*>(prow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            }
-          }
-          if (valid && t.n0 == 0) a.pair_valid[slot] = 1;
         } else {
           const int orow_idx = valid ? slot / a.topk : 0;
           float* orow = reinterpret_cast<float*>(a.out) + static_cast<size_t>(orow_idx) * a.ld_out + t.n0;
@@ -439,11 +408,17 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           for (int c0 = 0; c0 < BT; c0 += 16) {
             float g[16], u[16];
             tmem_ld16x2_wait(taddr + c0, taddr + BT + c0, g, u);
+            if (has_bias) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float av = act_mul<T, EXT>(g[j] + bgate, u[j] + bup, w_on_input, col_gam[c0 + j], mimic, ap);
-              if (n_ok) out[static_cast<size_t>(c0 + j) * a.ld_out] = from_f32<T>(av);
+              for (int j = 0; j < 16; ++j) {
+                g[j] += bgate;
+                u[j] += bup;
+              }
             }
+            act_mul_array<T, EXT>(g, u, w_on_input, mimic, ap, [&](int j) { return col_gam[c0 + j]; });
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (n_ok) out[static_cast<size_t>(c0 + j) * a.ld_out] = from_f32<T>(g[j]);
           }
         } else {
           float* out = reinterpret_cast<float*>(a.out) + n;
@@ -542,9 +517,6 @@ static int launch_one(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Ge
 template <typename T, bool EXT>
 static int launch_typed(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                         cudaStream_t stream) {
-  if (a.orient == 1)
-    return a.mode == 0 ? launch_one<0, T, 1, false, EXT>(tm_w, tm_x, a, num_sms, stream)
-                       : launch_one<1, T, 1, false, EXT>(tm_w, tm_x, a, num_sms, stream);
   return a.mode == 0 ? launch_one<0, T, 0, false, EXT>(tm_w, tm_x, a, num_sms, stream)
                      : launch_one<1, T, 0, false, EXT>(tm_w, tm_x, a, num_sms, stream);
 }
@@ -552,7 +524,7 @@ static int launch_typed(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const 
 int launch_gemm_tc(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                    cudaStream_t stream) {
   if (a.BT < 16 || a.BT > kMaxBT || a.BT % 16 != 0) return B200MOE_ERR_BAD_ARG;
-  if (a.orient == 1 && a.BT > 128) return B200MOE_ERR_BAD_ARG;
+  if (a.orient == 1 && (a.BT > 128 || a.wmode != B200MOE_W_INT4_AWQ)) return B200MOE_ERR_BAD_ARG;
   if (a.wmode == B200MOE_W_INT4_AWQ) {
     if (a.dtype != B200MOE_DTYPE_FP16 || a.w_sz == nullptr) return B200MOE_ERR_UNSUPPORTED;
     const bool ext4 = a.bias != nullptr || a.activation == B200MOE_ACT_SWIGLU_OAI;

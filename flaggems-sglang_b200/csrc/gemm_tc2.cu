@@ -1,43 +1,77 @@
-// 16-bit grouped expert GEMMs on CTA pairs (tcgen05.mma.cta_group::2), prefill sizes.
+// 16-bit grouped expert GEMMs on CTA pairs (tcgen05.mma.cta_group::2) for blocks of more than 64 tokens.
 //
-// Two CTAs of a cluster share one tile of 256 tokens x 256 weight rows: each CTA stages ITS 128
-// token rows and HALF of the weight rows (128), the leader CTA issues one MMA for the pair and the
-// tensor cores of both SMs read the weight halves from both shared memories.  Per CTA and 64-k
-// stage that is 16 KiB of tokens + 16 KiB of weights instead of 16 + 32 with one CTA per tile:
-// a third less shared-memory fill, L2 traffic and operand reading for the same flops.
+// Two CTAs of a cluster share one tile of 256 weight rows x N tokens, N = 32..256 in steps of 32: weights sit
+// on the instruction's M side (each CTA stages its 128 rows), the tokens on its N side (each CTA
+// stages half of them), the leader CTA issues one MMA for the pair.  Both operands are then read from
+// shared memory once per pair, and N follows the tokens an expert really has: its rows are padded to 32 and
+// dealt out evenly over ceil(rows / max) tiles, where a kernel with tokens on the M side pays for whole
+// blocks of 128 (two experts of eight with 250 tokens on average hold more than 256: 25 % of that kernel's
+// MMAs were padding).  Every launch picks `max` from the tokens at hand (see pick_max_granules).
 //
-//   mode 0 (gate/up):  CTA 0 stages 128 gate rows, CTA 1 the 128 matching up rows; accumulator
-//                      columns 0..127 = gate, 128..255 = up, as in the single-CTA kernel.
-//   mode 1 (down):     CTA r stages weight rows n0 + 128 r ..; 256 output columns per tile.
-// The two token blocks of a tile are consecutive blocks of one expert; an expert with an odd number
-// of blocks leaves the second half of its last tile without a block (its rows are computed on
-// whatever the loads return and never stored).
+//   mode 0 (gate/up):  a CTA's 128 rows are 64 gate rows and the 64 matching up rows; the pair
+//                      covers 128 columns of the intermediate.
+//   mode 1 (down):     128 rows of the down projection per CTA.
+//
+// A stage is two TMA loads per CTA whatever the tile: the gate and up rows are one box of a 4-D view
+// [experts][gate | up][rows][K], and there is a token map for every half tile of 16..128 rows.  With
+// the same bytes in four smaller boxes the producer thread set the pace (4096 tokens of the
+// Mixtral-shaped layer, first GEMM: 1.77 ms, 1.34 ms with two loads issued behind elect.sync).
+//
+// An accumulator lane is a weight row, i.e. an output column, so the epilogue turns 16 tokens at a time in
+// shared memory and then stores 16 bytes of a token per thread, contiguous over the lanes of a warp.
+// In mode 0 gate and up rows alternate (the box puts row i of both halves next to each other), so the two
+// values of a column sit in neighbouring lanes: each lane trades half of its tokens with its
+// neighbour and turns finished 16-bit activations.  Turning fp32 gate and up values first cost four times
+// the shared-memory traffic and, at K = 1280, more time than the tile's MMAs.
 //
 // No load here has the cluster-multicast qualifier: every CTA loads its own operands with plain
 // tiled TMA loads.  Only tcgen05.commit is multicast (to the same barrier in both CTAs).
 // Synchronisation between the two CTAs:
 //   * operands staged: the loads of BOTH CTAs complete on the leader's `full` barrier (the
-//     cta_group::2 form of the tiled load lets the completion go to the peer CTA's barrier); each
-//     producer announces its bytes there with an arrive.expect_tx of its own (remote for the second
-//     CTA).  A first version that completed locally and forwarded each completion with a remote
-//     arrive ran at half speed: the extra hop made the refill loop longer than the seven stages
-//     of buffered work;
+//     cta_group::2 form of the tiled load lets the completion go to the peer CTA's barrier), and the
+//     leader alone announces the bytes of both.  Bytes of the second CTA may be counted before they
+//     are announced; the phase cannot end without the leader's arrival.  (An arrive.expect_tx by the
+//     second CTA on the leader's barrier, a release at cluster scope per stage, held its loads back
+//     so far that the pair ran at half speed.)
 //   * stage free / accumulator ready: tcgen05.commit of the leader, multicast to both CTAs;
 //   * accumulator drained: the epilogue warps of both CTAs arrive on the leader's `tempty`.
+// Asking for the weights in L2 ahead of the ring (cp.async.bulk.prefetch.tensor, 4 to 32 stages) was slower
+// at every size: 807 us without, 843 to 978 us with, at 1000 tokens of the Mixtral-shaped layer.
+//
+// What bounds it: the board's power cap at 4096 tokens (tensor pipe 90 % busy at 1.25 GHz, 2.45 ms against 2.74
+// for 128-token blocks on single CTAs), the weights' way from HBM at 1000 tokens (807 us, 975 before),
+// the activation epilogue at K = 1280 (1280 x 3072 x 64 experts, 2048 tokens: 605 us with routing, 729 before).
+//
 // Every wait is bounded (common.cuh); the cluster barriers at start and end are reached by every
 // thread whatever happened in between.
-//
-// Status: results are bit-identical to the one-CTA-per-tile kernel, but on the Mixtral-shaped
-// layer at M = 4096 this kernel takes 1.9x as long (tensor pipe 35 % active where the other shows
-// 87 %), whatever the stage count (4..7), the instruction's N, the epilogue or the commit pattern;
-// the cause has not been found.  It is therefore used only on request (B200MOE_FLAG_CTA_PAIR).
 #include "gemm_sched.cuh"
 
 namespace b200moe {
 
 namespace {
 
-constexpr int kStageBytes2 = 2 * kTileBytes;   // per CTA: 128 token rows + 128 weight rows, 64 k each
+constexpr int kPairThreads = 320;       // TMA producer, MMA issuer, two epilogue groups of four warps
+constexpr int kGran = 32;               // tokens: padding of an expert's rows and step of N
+constexpr int kMaxGran = 8;             // N <= 256
+constexpr int kMaxStages2 = 10;
+constexpr int kTurnTok = 16;            // tokens turned per epilogue step
+
+// Bytes per token in the turning buffer: 64 activations, 128 pair-row values (both 16-bit) or 128 fp32 sums, and
+// a pad that keeps the rows 16-byte aligned and spreads them over the banks.
+__host__ __device__ __forceinline__ int tc2_turn_pitch(int mode, bool pairs) {
+  return mode == 0 ? 160 : (pairs ? 272 : 528);
+}
+// Shared memory: token tables [2 groups][2 tiles][256] (slot, weight), barriers, granule and tile prefixes of the
+// experts, turning buffers [2 groups][2], then the operand ring (1024-byte aligned).
+constexpr size_t kTc2TableBytes = 2 * 2 * 256 * 8 + 512;
+__host__ __device__ __forceinline__ size_t tc2_turn_offset(int E) {
+  return (kTc2TableBytes + 2 * static_cast<size_t>(E + 1) * 4 + 127) & ~static_cast<size_t>(127);
+}
+__host__ __device__ __forceinline__ size_t tc2_fixed_bytes(int E, int mode, bool pairs) {
+  return (tc2_turn_offset(E) + 4 * kTurnTok * static_cast<size_t>(tc2_turn_pitch(mode, pairs)) + 1023) & ~static_cast<size_t>(1023);
+}
+// operand bytes of one 64-k stage in one CTA: 128 weight rows and half of up to n tokens
+__host__ __device__ __forceinline__ int tc2_stage_bytes(int n) { return kTileBytes + n / 2 * kStageKBytes; }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -59,10 +93,6 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx_remote(uint32_t cluster_addr, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(bytes)
-               : "memory");
-}
 // Tiled loads into this CTA's shared memory whose completion is counted on a barrier that may live
 // in the peer CTA (cluster address).  No multicast: one destination.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int c0, int c1) {
@@ -78,6 +108,14 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, "
       "%5}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int c0, int c1,
+                                                 int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, "
+      "%5, %6}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
@@ -107,88 +145,128 @@ __device__ __forceinline__ void tc_mma2_f16(uint32_t d_tmem, uint64_t adesc, uin
       : "memory");
 }
 
-__device__ __forceinline__ void red_add_v4_2(float* addr, float a, float b, float c, float d) {
+__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
   asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");
 }
 template <typename T>
-__device__ __forceinline__ uint32_t pack2_2(float lo, float hi);
+__device__ __forceinline__ uint32_t pack2(float lo, float hi);
 template <>
-__device__ __forceinline__ uint32_t pack2_2<__nv_bfloat16>(float lo, float hi) {
+__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 template <>
-__device__ __forceinline__ uint32_t pack2_2<__half>(float lo, float hi) {
+__device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   __half2 v = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Tile of one pair: N tokens of an expert from padded row row0, weight rows from n0, reduction [kb0, kb1).
 struct PairTile {
-  int e;        // expert
-  int n0;       // first weight row of the tile inside the expert (mode 0: of the gate rows)
-  int blk;      // this CTA's token block (index over all padded blocks)
-  bool has;     // the block belongs to the expert (false: second half of an odd expert's last tile)
+  int e, n0, row0, n, kb0, kb1;
 };
 
-// Tile `id` in expert-major, then n-tile, then block-pair order.  s_pair_off[e] = pairs before expert e.
-__device__ __forceinline__ PairTile decode_pair(int id, const int* s_pair_off, const int* s_blk_off, int E, int num_nt,
-                                                int tile_n, int rank) {
+// Tile `id` in expert-major, n-tile, reduction split, token tile order.  s_tile[e] = token tiles before
+// expert e, s_gran[e] = granules before it.
+__device__ __forceinline__ PairTile decode_pair(int id, const int* s_tile, const int* s_gran, int E, int num_nt,
+                                                int split, int kblocks, int tile_n) {
   int lo = 0, hi = E;
+  const int u = num_nt * split;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (s_pair_off[mid] * num_nt <= id) lo = mid; else hi = mid;
+    if (s_tile[mid] * u <= id) lo = mid; else hi = mid;
   }
   PairTile t;
   t.e = lo;
-  const int np = s_pair_off[lo + 1] - s_pair_off[lo];
-  const int local = id - s_pair_off[lo] * num_nt;
-  const int bp = local % np;
-  const int nt = local / np;
-  const int nb = s_blk_off[lo + 1] - s_blk_off[lo];
-  t.n0 = nt * tile_n;
-  t.blk = s_blk_off[lo] + 2 * bp + rank;
-  t.has = 2 * bp + rank < nb;
+  const int nt_e = s_tile[lo + 1] - s_tile[lo];
+  const int local = id - s_tile[lo] * u;
+  const int tt = local % nt_e;
+  const int rest = local / nt_e;
+  const int s = rest % split;
+  const int g = s_gran[lo + 1] - s_gran[lo];
+  const int g0 = tt * g / nt_e, g1 = (tt + 1) * g / nt_e;
+  t.n0 = (rest / split) * tile_n;
+  t.row0 = (s_gran[lo] + g0) * kGran;
+  t.n = (g1 - g0) * kGran;
+  t.kb0 = static_cast<int>((static_cast<long long>(s) * kblocks) / split);
+  t.kb1 = static_cast<int>((static_cast<long long>(s + 1) * kblocks) / split);
   return t;
 }
 
-template <int MODE, typename T>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+// Cycles of a 64-k stage of a tile with g granules: four MMAs of N / 2 cycles, or the time the stage's
+// operands take from L2 at about 80 bytes per clock and SM, whichever is longer.
+__device__ __forceinline__ float stage_cost(int g) {
+  return fmaxf(64.f * g, 200.f + 24.f * g) + 16.f;
+}
+
+// Largest number of granules per tile that this launch should use: the one with the shortest estimated
+// schedule, (sum of the tiles' costs) / pairs + half the longest tile (static round-robin over the pairs
+// ends that much later than a perfect split on average).  Wide tiles re-read the weights least; narrower ones fill the last wave
+// of a launch with few tiles.  Warp w < 6 rates 8 - w; result in every lane of the warp.
+__device__ __forceinline__ float rate_max_granules(int maxg, const int* s_gran, int E, int num_nt, int pairs, int lane) {
+  float sum = 0.f, longest = 0.f;
+  for (int e = lane; e < E; e += 32) {
+    const int g = s_gran[e + 1] - s_gran[e];
+    if (g > 0) {
+      const int t = (g + maxg - 1) / maxg;
+      const int lo = g / t, rem = g - lo * t;
+      sum += (t - rem) * stage_cost(lo) + rem * stage_cost(lo + 1);
+      longest = fmaxf(longest, stage_cost(rem > 0 ? lo + 1 : lo));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    longest = fmaxf(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  }
+  return sum * num_nt / pairs + 0.5f * longest;
+}
+
+template <int MODE, typename T, bool EXT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ PairTokenMaps tm_x,
                     const GemmArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  const int stages = a.stages;
-  uint8_t* ctrl_base = smem + static_cast<size_t>(stages) * kStageBytes2;
-  uint64_t* bar_full = reinterpret_cast<uint64_t*>(ctrl_base);   // leader: both CTAs' operands are staged
-  uint64_t* bar_empty = bar_full + stages;
-  uint64_t* bar_tfull = bar_empty + stages;
+  int* s_slot = reinterpret_cast<int*>(smem);                              // [2 groups][2][256]
+  float* s_gam = reinterpret_cast<float*>(s_slot + 4 * 256);               // [2 groups][2][256]
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(s_gam + 4 * 256);       // leader: both CTAs' operands are staged
+  uint64_t* bar_empty = bar_full + kMaxStages2;
+  uint64_t* bar_tfull = bar_empty + kMaxStages2;
   uint64_t* bar_tempty = bar_tfull + 2;          // leader: both CTAs' epilogues have drained the accumulator
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tempty + 2);
+  uint64_t* bar_meet = bar_tempty + 2;           // [2] the four warps of an epilogue group
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_meet + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_blk_off = reinterpret_cast<int*>(tmem_slot + 4);   // [E+1]
-  int* s_pair_off = s_blk_off + (a.E + 1);                   // [E+1]
+  int* s_nmax = reinterpret_cast<int*>(tmem_slot + 2);                     // tokens of the widest tile
+  float* s_rate = reinterpret_cast<float*>(tmem_slot + 4);                 // [6]
+  int* s_gran = reinterpret_cast<int*>(smem + kTc2TableBytes);             // [E+1]
+  int* s_tile = s_gran + (a.E + 1);                                        // [E+1]
+  const int pitch = tc2_turn_pitch(MODE, a.out_pairs != nullptr);
+  uint8_t* s_turn = smem + tc2_turn_offset(a.E);                           // [2 groups][2][16 tokens][pitch]
+  const size_t fixed = tc2_fixed_bytes(a.E, MODE, a.out_pairs != nullptr);
+  uint8_t* ring = smem + fixed;
 
-  const int warp = warp_index();
+  const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
+    for (int s = 0; s < kMaxStages2; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);     // the leader announces the bytes of both CTAs
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(&bar_tfull[s]), 1);
-      mbar_init(smem_u32(&bar_tempty[s]), 8);
+      mbar_init(smem_u32(&bar_tempty[s]), 16);
+      mbar_init(smem_u32(&bar_meet[s]), 4);
     }
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
     prefetch_tmap(&tm_w);
-    prefetch_tmap(&tm_x);
   }
   // barriers of both CTAs exist before either side signals the other
   cluster_arrive();
@@ -199,51 +277,83 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   }
   griddep_wait();
   griddep_launch_dependents();
-  for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
-  tc_fence_before();
+  for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_gran[e] = a.blk_off[e];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int e = 0; e < a.E; ++e) {
-      s_pair_off[e] = run;
-      run += (s_blk_off[e + 1] - s_blk_off[e] + 1) >> 1;
-    }
-    s_pair_off[a.E] = run;
+  const int num_nt = a.num_nt;
+  const int npairs = static_cast<int>(gridDim.x) >> 1;
+  if (warp < 6) {
+    const float r = rate_max_granules(kMaxGran - warp, s_gran, a.E, num_nt, npairs, lane);
+    if (lane == 0) s_rate[warp] = r;
   }
+  __syncthreads();
+  if (warp == 0) {
+    int best = 0;
+    for (int w = 1; w < 6; ++w)
+      if (s_rate[w] < s_rate[best]) best = w;
+    const int cap = a.BT / kGran;     // a caller that fixes the token block bounds the tile with it
+    const int maxg = min(kMaxGran - best, cap);
+    int run = 0, widest = 1;
+    for (int e0 = 0; e0 < a.E; e0 += 32) {
+      const int e = e0 + lane;
+      const int g = e < a.E ? s_gran[e + 1] - s_gran[e] : 0;
+      const int t = (g + maxg - 1) / maxg;
+      if (t > 0) widest = max(widest, (g + t - 1) / t);
+      int v = t;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (e < a.E) s_tile[e + 1] = run + v;
+      run += __shfl_sync(0xffffffffu, v, 31);
+    }
+    widest = __reduce_max_sync(0xffffffffu, widest);
+    if (lane == 0) {
+      s_tile[0] = 0;
+      *s_nmax = widest * kGran;
+    }
+  }
+  tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   constexpr int kTileN = (MODE == 1) ? 256 : 128;
-  const int num_nt = a.num_nt;
-  const int total = s_pair_off[a.E] * num_nt;
-  const int nclusters = static_cast<int>(gridDim.x) >> 1;
-  const int cluster_id = static_cast<int>(blockIdx.x) >> 1;
-  // spread the tiles evenly: with w waves, ceil(total / w) clusters do w tiles each
-  const int waves = (total + nclusters - 1) / nclusters;
-  const int cl_eff = waves > 0 ? (total + waves - 1) / waves : 1;
-  const bool active = cluster_id < cl_eff;
+  const int stage_bytes = tc2_stage_bytes(*s_nmax);
+  const int stages = min(kMaxStages2, static_cast<int>((kSmemLimit - 1024 - fixed) / stage_bytes));
+  const int tiles = s_tile[a.E] * num_nt;
+  const int split = (MODE == 1 && !(a.flags & B200MOE_FLAG_NO_SPLIT_K)) ? pick_split(tiles, a.kblocks, npairs, a.max_split) : 1;
+  const int total = tiles * split;
+  const int pair_id = static_cast<int>(blockIdx.x) >> 1;
+  auto tile_at = [&](int id) { return decode_pair(id, s_tile, s_gran, a.E, num_nt, split, a.kblocks, kTileN); };
 
-  if (active && warp == 0 && elect_one()) {
+  if (warp == 0 && elect_one()) {
     // =============================== TMA producer (every CTA, its own operands) ===================
     int stage = 0;
     uint32_t phase = 0;
     long long issued = 0;
     bool ok = true;
-    for (int tile = cluster_id; ok && tile < total; tile += cl_eff) {
-      const PairTile t = decode_pair(tile, s_pair_off, s_blk_off, a.E, num_nt, kTileN, static_cast<int>(rank));
-      const int wrow = (MODE == 0) ? (rank == 0 ? t.n0 : a.up_row_off + t.n0) : t.n0 + static_cast<int>(rank) * kTileRows;
-      for (int kb = 0; kb < a.kblocks; ++kb) {
+    constexpr int kKElems = kStageKBytes / static_cast<int>(sizeof(T));
+    constexpr int kRowsPerCta = MODE == 0 ? 64 : 128;
+    for (int tile = pair_id; ok && tile < total; tile += npairs) {
+      const PairTile t = tile_at(tile);
+      const int wrow = t.n0 + kRowsPerCta * static_cast<int>(rank);
+      const int half = t.n >> 1;
+      const int xrow = t.row0 + static_cast<int>(rank) * half;
+      const CUtensorMap* mx = &tm_x.m[half / 16 - 1];
+      for (int kb = t.kb0; kb < t.kb1; ++kb) {
         if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER)) {
           ok = false;
           break;
         }
         const uint32_t full = mapa_u32(smem_u32(&bar_full[stage]), 0);   // the leader's barrier
-        const uint32_t sx = smem_u32(smem + static_cast<size_t>(stage) * kStageBytes2);
-        const int k0 = kb * (kStageKBytes / static_cast<int>(sizeof(T)));
-        if (leader) mbar_arrive_expect_tx(smem_u32(&bar_full[stage]), static_cast<uint32_t>(2 * kStageBytes2));
-        tma_load_2d_pair(sx, &tm_x, full, k0, t.blk * kTileRows);
-        tma_load_3d_pair(sx + kTileBytes, &tm_w, full, k0, wrow, t.e);
+        const uint32_t sw = smem_u32(ring + static_cast<size_t>(stage) * stage_bytes);
+        const int k0 = kb * kKElems;
+        if (leader)
+          mbar_arrive_expect_tx(smem_u32(&bar_full[stage]), static_cast<uint32_t>(2 * kTileBytes + t.n * kStageKBytes));
+        if (MODE == 0) tma_load_4d_pair(sw, &tm_w, full, k0, 0, wrow, t.e);
+        else tma_load_3d_pair(sw, &tm_w, full, k0, wrow, t.e);
+        tma_load_2d_pair(sw + kTileBytes, mx, full, k0, xrow);
         ++issued;
         if (++stage == stages) {
           stage = 0;
@@ -271,29 +381,30 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         }
       }
     }
-  } else if (active && warp == 1 && leader && elect_one()) {
+  } else if (warp == 1 && leader && elect_one()) {
     // =============================== MMA issuer (leader CTA, for the pair) ========================
     const uint32_t fmt = (a.dtype == B200MOE_DTYPE_BF16) ? 1u : 0u;
-    const uint32_t idesc = make_idesc(fmt, 256u, 256u);
     constexpr int kSteps = kStageKBytes / 32;
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool ok = true;
-    for (int tile = cluster_id; ok && tile < total; tile += cl_eff) {
+    for (int tile = pair_id; ok && tile < total; tile += npairs) {
+      const PairTile t = tile_at(tile);
+      const uint32_t idesc = make_idesc(fmt, 256u, static_cast<uint32_t>(t.n));
       if (!mbar_wait(smem_u32(&bar_tempty[acc]), acc_phase ^ 1, abort_flag, DEV_TIMEOUT_MMA)) break;
       tc_fence_after();
       const uint32_t d0 = tmem_base + static_cast<uint32_t>(acc * 256);
-      for (int kb = 0; kb < a.kblocks; ++kb) {
+      for (int kb = t.kb0; kb < t.kb1; ++kb) {
         if (!mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag, DEV_TIMEOUT_MMA)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t sx = smem_u32(smem + static_cast<size_t>(stage) * kStageBytes2);
-        const uint64_t dx = smem_desc_k_sw128(sx);                 // token rows: the M side
-        const uint64_t dw = smem_desc_k_sw128(sx + kTileBytes);    // this CTA's half of the weight rows: the N side
+        const uint32_t sw = smem_u32(ring + static_cast<size_t>(stage) * stage_bytes);
+        const uint64_t dw = smem_desc_k_sw128(sw);                 // this CTA's weight rows: the M side
+        const uint64_t dx = smem_desc_k_sw128(sw + kTileBytes);    // this CTA's half of the tokens: the N side
 #pragma unroll
-        for (int k = 0; k < kSteps; ++k) tc_mma2_f16(d0, dx + 2 * k, dw + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < kSteps; ++k) tc_mma2_f16(d0, dw + 2 * k, dx + 2 * k, idesc, (kb > t.kb0 || k > 0) ? 1u : 0u);
         tc_commit2(smem_u32(&bar_empty[stage]));
         if (++stage == stages) {
           stage = 0;
@@ -307,87 +418,129 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         acc_phase ^= 1;
       }
     }
-  } else if (active && warp >= 2) {
-    // =============================== epilogue (every CTA, its own 128 token rows) =================
-    const int quad = warp & 3;
-    const int lrow = quad * 32 + lane;
+  } else if (warp >= 2) {
+    // =============================== epilogue (every CTA, its own 128 weight rows) ================
+    const int grp = (warp - 2) >> 2;              // steps of 16 tokens alternate between the two groups
+    const int quad = warp & 3;                    // TMEM lane quadrant this warp may read
+    const int gt = ((warp - 2) & 3) * 32 + lane;  // thread inside the group
     const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0;
     const bool mimic = (a.flags & B200MOE_FLAG_MIMIC_ROUNDING) != 0;
+    const bool round_pair = mimic && split == 1;
     const ActParams ap = act_params(a);
-    const uint32_t tempty_leader0 = mapa_u32(smem_u32(&bar_tempty[0]), 0);
-    const uint32_t tempty_leader1 = mapa_u32(smem_u32(&bar_tempty[1]), 0);
-    int acc = 0;
+    const bool has_bias = EXT && a.bias != nullptr;
+    const uint32_t meet = smem_u32(&bar_meet[grp]);
+    uint32_t meet_phase = 0;
+    int acc = 0, par = 0, step_no = 0;
     uint32_t acc_phase = 0;
-    for (int tile = cluster_id; tile < total; tile += cl_eff) {
-      const PairTile t = decode_pair(tile, s_pair_off, s_blk_off, a.E, num_nt, kTileN, static_cast<int>(rank));
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * 256);
-      const int r = t.blk * kTileRows + lrow;
-      int slot = -1;
-      float gam = 0.f;
-      if (t.has) {
-        slot = a.sorted_ids[r];
-        if (slot >= 0 && slot < a.P) gam = a.row_gamma[r]; else slot = -1;
+    bool ok = true;
+    for (int tile = pair_id; ok && tile < total; tile += npairs, par ^= 1) {
+      const PairTile t = tile_at(tile);
+      int* slots = s_slot + (grp * 2 + par) * 256;
+      float* gams = s_gam + (grp * 2 + par) * 256;
+      for (int i = gt; (MODE == 1 || w_on_input) && i < t.n; i += 128) {
+        const int slot = a.sorted_ids[t.row0 + i];
+        const bool valid = slot >= 0 && slot < a.P;
+        slots[i] = valid ? slot : -1;
+        gams[i] = valid ? a.row_gamma[t.row0 + i] : 0.f;
       }
-      const bool valid = slot >= 0;
+      // the tables are read before a step's meeting: they need one of their own
+      if (MODE == 1 || w_on_input) {
+        if (!warps_meet(meet, meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+      }
       if (!mbar_wait(smem_u32(&bar_tfull[acc]), acc_phase, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
-      if (MODE == 0) {
-        T* orow = reinterpret_cast<T*>(a.out) + static_cast<size_t>(t.has ? r : 0) * a.ld_out + t.n0;
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 16) {
-          float g[16], u[16];
-          tmem_ld16x2_wait(taddr + c0, taddr + 128 + c0, g, u);
-          uint32_t pk[8];
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * 256);
+      const int steps = t.n / kTurnTok;
+      // mode 0: output column of this lane pair; mode 1: of this lane
+      const int lcol = (MODE == 0) ? 64 * static_cast<int>(rank) + quad * 16 + (lane >> 1)
+                                   : 128 * static_cast<int>(rank) + quad * 32 + lane;
+      float bias0 = 0.f, bias1 = 0.f;
+      if (has_bias && t.n0 + lcol < a.N) {
+        if (MODE == 0) {
+          bias0 = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + t.n0 + lcol);
+          bias1 = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + a.N + t.n0 + lcol);
+        } else if (t.kb0 == 0) {      // the first reduction split carries the bias
+          bias0 = __ldg(a.bias + static_cast<size_t>(t.e) * a.N + t.n0 + lcol);
+        }
+      }
+      for (int st = grp; st < steps; st += 2, ++step_no) {
+        float v[16];
+        tmem_ld16_wait(taddr + st * kTurnTok, v);
+        if (st + 2 >= steps) {        // this warp has read its last part of the accumulator
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_tempty[acc]), 0));
+        }
+        uint8_t* buf = s_turn + static_cast<size_t>((grp * 2 + (step_no & 1)) * kTurnTok) * pitch;
+        if (MODE == 0) {
+          // even lanes hold gate values and finish the even tokens, odd lanes hold up values and finish the odd ones
+          const bool odd = (lane & 1) != 0;
+          float g[8], u[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float lo = act_mul<T>(g[2 * j], u[2 * j], w_on_input, gam, mimic, ap);
-            const float hi = act_mul<T>(g[2 * j + 1], u[2 * j + 1], w_on_input, gam, mimic, ap);
-            pk[j] = pack2_2<T>(lo, hi);
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
+            g[j] = (odd ? other : v[2 * j]) + bias0;
+            u[j] = (odd ? v[2 * j + 1] : other) + bias1;
           }
-          if (t.has && t.n0 + c0 + 8 <= a.N) *reinterpret_cast<uint4*>(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          if (t.has && t.n0 + c0 + 16 <= a.N)
-            *reinterpret_cast<uint4*>(orow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        }
-      } else if (a.out_pairs != nullptr) {
-        T* prow = reinterpret_cast<T*>(a.out_pairs) + static_cast<size_t>(valid ? slot : 0) * a.N + t.n0;
-        const float scale = w_on_input ? 1.0f : gam;
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 16) {
-          float v[16];
-          tmem_ld16_wait(taddr + c0, v);
-          if (valid) {
-            uint32_t pk[8];
+          act_mul_array<T, EXT>(g, u, w_on_input, mimic, ap,
+                                [&](int j) { return gams[st * kTurnTok + 2 * j + (odd ? 1 : 0)]; });
 #pragma unroll
-            for (int j = 0; j < 8; ++j) pk[j] = pack2_2<T>(v[2 * j] * scale, v[2 * j + 1] * scale);
-            if (t.n0 + c0 + 8 <= a.N) *reinterpret_cast<uint4*>(prow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (t.n0 + c0 + 16 <= a.N) *reinterpret_cast<uint4*>(prow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<T*>(buf + (2 * j + (odd ? 1 : 0)) * pitch + (quad * 16 + (lane >> 1)) * 2) = from_f32<T>(g[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float scale = w_on_input ? 1.0f : gams[st * kTurnTok + j];
+            v[j] = (v[j] + bias0) * scale;
+          }
+          if (a.out_pairs != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              *reinterpret_cast<T*>(buf + j * pitch + (quad * 32 + lane) * 2) = from_f32<T>(v[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              *reinterpret_cast<float*>(buf + j * pitch + (quad * 32 + lane) * 4) =
+                  round_pair ? to_f32<T>(from_f32<T>(v[j])) : v[j];
           }
         }
-        if (valid && t.n0 == 0) a.pair_valid[slot] = 1;
-      } else {
-        float* orow = reinterpret_cast<float*>(a.out) + static_cast<size_t>(valid ? slot / a.topk : 0) * a.ld_out + t.n0;
-        const float scale = w_on_input ? 1.0f : gam;
-        const bool round_pair = mimic;
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 16) {
-          float v[16];
-          tmem_ld16_wait(taddr + c0, v);
-          if (valid) {
+        // one meeting per step: a warp that writes this buffer again, two steps on, has met the others
+        // once more in between, after they had finished reading it
+        if (!warps_meet(meet, meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) {
+          ok = false;
+          break;
+        }
+        if (MODE == 0) {
+          const int tk = gt >> 3, ch = gt & 7;        // 16 tokens x 8 chunks of 16 bytes
+          const int col = t.n0 + 64 * static_cast<int>(rank) + ch * 8;
+          if (col < a.N)
+            *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out) +
+                                      static_cast<size_t>(t.row0 + st * kTurnTok + tk) * a.ld_out + col) =
+                *reinterpret_cast<const uint4*>(buf + tk * pitch + ch * 16);
+        } else if (a.out_pairs != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              v[j] *= scale;
-              if (round_pair) v[j] = to_f32<T>(from_f32<T>(v[j]));
+          for (int q = 0; q < 2; ++q) {
+            const int tk = q * 8 + (gt >> 4), ch = gt & 15;     // 16 tokens x 16 chunks
+            const int slot = slots[st * kTurnTok + tk];
+            const int col = t.n0 + 128 * static_cast<int>(rank) + ch * 8;
+            if (slot >= 0 && col < a.N) {
+              *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out_pairs) + static_cast<size_t>(slot) * a.N + col) =
+                  *reinterpret_cast<const uint4*>(buf + tk * pitch + ch * 16);
+              if (col == 0) a.pair_valid[slot] = 1;
             }
+          }
+        } else {
+          const int col = t.n0 + 128 * static_cast<int>(rank) + lane * 4;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (t.n0 + c0 + 4 * q + 4 <= a.N)
-                red_add_v4_2(orow + c0 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          for (int q = 0; q < 4; ++q) {
+            const int tk = q * 4 + (gt >> 5);
+            const int slot = slots[st * kTurnTok + tk];
+            if (slot < 0 || col >= a.N) continue;
+            const float4 y = *reinterpret_cast<const float4*>(buf + tk * pitch + lane * 16);
+            red_add_v4(reinterpret_cast<float*>(a.out) + static_cast<size_t>(slot / a.topk) * a.ld_out + col, y.x, y.y, y.z, y.w);
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_remote(acc == 0 ? tempty_leader0 : tempty_leader1);
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1;
@@ -409,87 +562,85 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(a.status, 0, *abort_flag);
 }
 
-size_t tc2_ctrl_bytes(const GemmArgs& a) { return 1024 + 2 * static_cast<size_t>(a.E + 1) * 4 + 64; }
-
 int g_tc2_pairs_seen = 0;   // resident CTA pairs found for the last launch (diagnostics)
 
 // How many CTA pairs of this kernel the device keeps resident at once.  The kernel is persistent with
 // a static tile assignment, so a grid with even one pair more than that would run its last pairs as a
 // second wave and take twice as long.
-template <int MODE, typename T>
-int max_resident_pairs(size_t smem, int num_sms) {
-  static int cached = 0;
-  static size_t cached_smem = 0;
-  if (cached > 0 && cached_smem == smem) return cached;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(num_sms & ~1);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, moe_gemm_tc2_kernel<MODE, T>, &cfg) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = (num_sms / 2) - 2;     // conservative guess
-  }
-  if (n > num_sms / 2) n = num_sms / 2;
-  cached = n;
-  cached_smem = smem;
-  return n;
+template <int MODE, typename T, bool EXT>
+int max_resident_pairs(int num_sms) {
+  static const int resident = [] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = kSmemLimit;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, moe_gemm_tc2_kernel<MODE, T, EXT>, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n;
+  }();
+  const int half = num_sms / 2;
+  const int n = resident > 0 ? resident : half - 2;     // conservative guess where the query fails
+  return n < half ? n : half;
 }
 
-template <int MODE, typename T>
-int launch_tc2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms, cudaStream_t stream) {
-  const size_t smem = 1024 + static_cast<size_t>(a.stages) * kStageBytes2 + tc2_ctrl_bytes(a);
-  if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
-  if (cudaFuncSetAttribute(moe_gemm_tc2_kernel<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
+template <int MODE, typename T, bool EXT>
+int launch_tc2(const CUtensorMap& tm_w, const PairTokenMaps& tm_x, const GemmArgs& a, int num_sms, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(moe_gemm_tc2_kernel<MODE, T, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kSmemLimit)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
-  const int pairs = max_resident_pairs<MODE, T>(smem, num_sms);
+  const int pairs = max_resident_pairs<MODE, T, EXT>(num_sms);
+  if (pairs <= 0) return B200MOE_ERR_UNSUPPORTED;
   g_tc2_pairs_seen = pairs;
   note_launch(MODE == 0 ? "moe_gemm_tc2_kernel<gate/up>" : "moe_gemm_tc2_kernel<down>");
-  cudaError_t err = launch_kernel(moe_gemm_tc2_kernel<MODE, T>, dim3(2 * pairs), dim3(kThreads), smem, stream,
+  cudaError_t err = launch_kernel(moe_gemm_tc2_kernel<MODE, T, EXT>, dim3(2 * pairs), dim3(kPairThreads), kSmemLimit, stream,
                                   a.pdl != 0, tm_w, tm_x, a);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
+template <typename T, bool EXT>
+int launch_typed(const CUtensorMap& tm_w, const PairTokenMaps& tm_x, const GemmArgs& a, int num_sms, cudaStream_t stream) {
+  return a.mode == 0 ? launch_tc2<0, T, EXT>(tm_w, tm_x, a, num_sms, stream)
+                     : launch_tc2<1, T, EXT>(tm_w, tm_x, a, num_sms, stream);
 }
 
 }  // namespace
 
 int gemm_tc2_resident_pairs() { return g_tc2_pairs_seen; }
 
-// Can this GEMM run on CTA pairs?  16-bit weights, 128-token blocks on the M side, plain epilogue,
-// whole reduction in one piece.
-bool gemm_tc2_ok(const GemmArgs& a) {
-  return a.wmode == B200MOE_W_16BIT && a.orient == 1 && a.BT == 128 && a.bias == nullptr &&
-         a.activation != B200MOE_ACT_SWIGLU_OAI && (a.mode == 0 || (a.flags & B200MOE_FLAG_NO_SPLIT_K) != 0) &&
-         a.n_peers <= 1;
+// The pair kernel keeps two prefixes over the experts in shared memory and needs a few stages beside them.
+bool gemm_tc2_ok(int E, int num_sms) {
+  return num_sms >= 6 && kSmemLimit - 1024 - tc2_fixed_bytes(E, 1, false) >= 3 * static_cast<size_t>(tc2_stage_bytes(256));
 }
 
+// a->BT: upper bound of the tokens per tile (a multiple of 32)
 void gemm_plan_tc2(GemmArgs* a) {
   const int tile_n = (a->mode == 1) ? 256 : kTileRows;
   a->num_nt = (a->N + tile_n - 1) / tile_n;
   a->kblocks = (a->K + 63) / 64;
   a->acc_stages = 2;
   a->tmem_cols = 512;
-  int st = static_cast<int>((kSmemLimit - 1024 - tc2_ctrl_bytes(*a)) / kStageBytes2);
-  if (st > 8) st = 8;
-  if (st < 2) st = 2;
-  a->stages = st;
+  if (a->max_split <= 0) a->max_split = 16;
 }
 
-int launch_gemm_tc2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
+int launch_gemm_tc2(const CUtensorMap& tm_w, const PairTokenMaps& tm_x, const GemmArgs& a, int num_sms,
                     cudaStream_t stream) {
-  if (!gemm_tc2_ok(a)) return B200MOE_ERR_UNSUPPORTED;
+  if (a.wmode != B200MOE_W_16BIT || a.BT < kGran || a.BT % kGran != 0) return B200MOE_ERR_UNSUPPORTED;
+  const bool ext = a.bias != nullptr || a.activation == B200MOE_ACT_SWIGLU_OAI;
   if (a.dtype == B200MOE_DTYPE_BF16)
-    return a.mode == 0 ? launch_tc2<0, __nv_bfloat16>(tm_w, tm_x, a, num_sms, stream)
-                       : launch_tc2<1, __nv_bfloat16>(tm_w, tm_x, a, num_sms, stream);
-  return a.mode == 0 ? launch_tc2<0, __half>(tm_w, tm_x, a, num_sms, stream)
-                     : launch_tc2<1, __half>(tm_w, tm_x, a, num_sms, stream);
+    return ext ? launch_typed<__nv_bfloat16, true>(tm_w, tm_x, a, num_sms, stream)
+               : launch_typed<__nv_bfloat16, false>(tm_w, tm_x, a, num_sms, stream);
+  return ext ? launch_typed<__half, true>(tm_w, tm_x, a, num_sms, stream)
+             : launch_typed<__half, false>(tm_w, tm_x, a, num_sms, stream);
 }
 
 }  // namespace b200moe

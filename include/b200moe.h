@@ -65,8 +65,8 @@ extern "C" {
                                            names the 16-bit type of the intermediate and the output   */
 #define B200MOE_FLAG_EP_DIAG_LOCAL_COMBINE 2048 /* tuning aid, expert parallelism: the down projection's rows stay on
                                            this GPU (WRONG results; isolates the cost of the peer stores)      */
-#define B200MOE_FLAG_CTA_PAIR 4096      /* 16-bit prefill (128-token blocks): run the grouped GEMMs on CTA pairs
-                                           (tcgen05.mma.cta_group::2) where the shape allows                   */
+#define B200MOE_FLAG_CTA_PAIR 4096      /* no effect: 16-bit problems of more than 64 tokens per block always run
+                                           on CTA pairs (tcgen05.mma.cta_group::2)                             */
 #define B200MOE_FLAG_ALIGN_ONE_CTA 512  /* tuning aid: single-CTA alignment however many slots           */
 #define B200MOE_FLAG_NO_COMBINE 256     /* out is [M*topk, H]: row t*topk+j holds pair j of token t,
                                            routing weight applied, nothing summed, routed_scaling ignored
