@@ -55,30 +55,68 @@ __device__ __forceinline__ int upper_expert(const int* offs, int n, int x) {
   return lo;
 }
 
-// Core: stable grouping of P slots by expert.  `ids` are expert ids (already
-// mapped to local experts when map != nullptr); slots with an id outside
-// [0, E) are dropped.  Each expert's group starts at a multiple of `block`.
-//   s_cnt   [nwarps][E] shared counters
-//   s_base  [E+1] shared: padded start row of each expert
-//   s_hist  [E]   shared: slots per expert
-// The caller provides place(slot, pos, pre[slot]) to record a placement.
-// `pre` (optional, [P]): a per-slot value fetched alongside the ids and handed to place().
+// The kernels below run as ONE cluster of 1..8 CTAs (the whole grid): CTA c owns the contiguous slots
+// [c * per, (c + 1) * per), the CTAs' counts meet through distributed shared memory, and stability follows from
+// ordering by (CTA, warp, lane).  One CTA pushed every store through one SM's memory pipe (77 us at 32768 slots), and
+// two launches of 32 CTAs with the counts in global memory took 47 us there.
+__device__ __forceinline__ int cluster_rank() {
+  int r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// the int at this CTA's shared-memory address `p`, read in CTA `rank` of the cluster
+__device__ __forceinline__ int ld_cluster(const int* p, int rank) {
+  uint32_t a;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+struct GroupSmem {
+  int* cnt;    // [nwarps][E] slots of each warp
+  int* tot;    // [E] slots of this CTA (read by the other CTAs)
+  int* hist;   // [E] slots of all CTAs
+  int* base;   // [E+1] padded start row of each expert
+  int* mine;   // [E] first row of this CTA's slots
+  int* scan;   // 33
+};
+__device__ __forceinline__ GroupSmem group_smem(int* smem, int nwarps, int E) {
+  GroupSmem g;
+  g.cnt = smem;
+  g.tot = g.cnt + nwarps * E;
+  g.hist = g.tot + E;
+  g.base = g.hist + E;
+  g.mine = g.base + (E + 1);
+  g.scan = g.mine + E;
+  return g;
+}
+size_t group_smem_bytes(int nwarps, int E) { return (static_cast<size_t>(nwarps) * E + 4 * static_cast<size_t>(E) + 1 + 40) * sizeof(int); }
+
+// Core: stable grouping of P slots by expert.  `ids` are expert ids (mapped to local experts when
+// map != nullptr); slots with an id outside [0, E) are dropped.  Each expert's group starts at a
+// multiple of `block`.  place(slot, pos, pre[slot]) records a placement; `pre` (optional, [P]) is a
+// per-slot value fetched alongside the ids.  Called by every thread of every CTA; the caller ends with
+// cluster_wait() (the CTAs' counts are read by their peers).
 template <typename Place>
 __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const int* map, int map_len, int P, int E,
-                                                int block, int* s_cnt, int* s_base, int* s_hist,
-                                                int* s_scan, int nwarps, const float* pre, Place place) {
+                                                int block, const GroupSmem& g, int nwarps, const float* pre, Place place) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) s_cnt[i] = 0;
+  const int rank = cluster_rank(), nctas = gridDim.x;
+  for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) g.cnt[i] = 0;
   __syncthreads();
 
-  // contiguous, 32-aligned segment of slots per counting warp
-  int seg = (P + nwarps - 1) / nwarps;
-  seg = (seg + 31) & ~31;
-  const int begin = warp * seg;
-  const int end = min(P, begin + seg);
+  // contiguous, 32-aligned shares of the slots per CTA and, inside it, per counting warp
+  const int per = ((P + nctas - 1) / nctas + 31) & ~31;
+  const int cta_begin = min(P, rank * per), cta_end = min(P, cta_begin + per);
+  const int seg = ((cta_end - cta_begin + nwarps - 1) / nwarps + 31) & ~31;
+  const int begin = cta_begin + warp * seg;
+  const int end = min(cta_end, begin + seg);
 
   // Both passes fetch the ids of kAhead iterations before they rank them: one dependent global
-  // load per 32 slots would otherwise set the pace of the whole kernel.
+  // load per 32 slots would otherwise set the pace.  A share that fits keeps them for the second pass.
   auto fetch = [&](int i) -> int {
     int e = -1;
     if (i < end) {
@@ -88,9 +126,9 @@ __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const
     }
     return e;
   };
+  int ev[kAhead];
   if (warp < nwarps) {
     for (int i0 = begin; i0 < end; i0 += 32 * kAhead) {
-      int ev[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) ev[u] = fetch(i0 + 32 * u + lane);
 #pragma unroll
@@ -98,47 +136,60 @@ __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const
         if (i0 + 32 * u >= end) break;
         const int e = ev[u];
         unsigned m = __match_any_sync(0xffffffffu, e);
-        if (e >= 0 && (m & ((1u << lane) - 1)) == 0) s_cnt[warp * E + e] += __popc(m);
+        if (e >= 0 && (m & ((1u << lane) - 1)) == 0) g.cnt[warp * E + e] += __popc(m);
         __syncwarp();
       }
     }
   }
   __syncthreads();
 
-  // per expert: totals and exclusive prefix over the counting warps
+  // per expert: this CTA's total and the exclusive prefix over its counting warps
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     int run = 0;
     for (int w = 0; w < nwarps; ++w) {
-      int t = s_cnt[w * E + e];
-      s_cnt[w * E + e] = run;
+      const int t = g.cnt[w * E + e];
+      g.cnt[w * E + e] = run;
       run += t;
     }
-    s_hist[e] = run;
+    g.tot[e] = run;
   }
-  __syncthreads();
+  cluster_arrive();
+  cluster_wait();
 
-  // padded starts: exclusive scan over experts (chunks of blockDim.x experts)
+  // totals and the slots of the CTAs before this one; padded starts by an exclusive scan over the
+  // experts (chunks of blockDim.x experts)
   int carry = 0;
   for (int e0 = 0; e0 < E; e0 += blockDim.x) {
-    int e = e0 + threadIdx.x;
-    int padded = 0;
-    if (e < E) padded = (s_hist[e] + block - 1) / block * block;
-    int total;
-    int ex = block_exclusive_scan(padded, s_scan, &total);
-    if (e < E) s_base[e] = carry + ex;
-    carry += total;
+    const int e = e0 + threadIdx.x;
+    int total = 0, before = 0;
+    if (e < E) {
+      for (int c = 0; c < nctas; ++c) {
+        const int t = ld_cluster(g.tot + e, c);
+        if (c < rank) before += t;
+        total += t;
+      }
+      g.hist[e] = total;
+    }
+    int sum;
+    const int ex = block_exclusive_scan((total + block - 1) / block * block, g.scan, &sum);
+    if (e < E) {
+      g.base[e] = carry + ex;
+      g.mine[e] = carry + ex + before;
+    }
+    carry += sum;
   }
-  if (threadIdx.x == 0) s_base[E] = carry;
+  if (threadIdx.x == 0) g.base[E] = carry;
+  cluster_arrive();       // the peers' counts have been read; the caller waits before it leaves
   __syncthreads();
 
   if (warp < nwarps) {
+    const bool kept = end - begin <= 32 * kAhead;
     for (int i0 = begin; i0 < end; i0 += 32 * kAhead) {
-      int ev[kAhead];
       float wv[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         const int i = i0 + 32 * u + lane;
-        ev[u] = fetch(i);
+        if (!kept) ev[u] = fetch(i);
         wv[u] = (pre != nullptr && i < end) ? pre[i] : 0.f;
       }
 #pragma unroll
@@ -147,19 +198,18 @@ __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const
         const int i = i0 + 32 * u + lane;
         const int e = ev[u];
         unsigned m = __match_any_sync(0xffffffffu, e);
-        int rank = __popc(m & ((1u << lane) - 1));
+        const int r = __popc(m & ((1u << lane) - 1));
         int cur = 0;
-        if (e >= 0) cur = s_cnt[warp * E + e];
+        if (e >= 0) cur = g.cnt[warp * E + e];
         __syncwarp();
         if (e >= 0) {
-          place(i, s_base[e] + cur + rank, wv[u]);
-          if (rank == 0) s_cnt[warp * E + e] = cur + __popc(m);
+          place(i, g.mine[e] + cur + r, wv[u]);
+          if (r == 0) g.cnt[warp * E + e] = cur + __popc(m);
         }
         __syncwarp();
       }
     }
   }
-  __syncthreads();
 }
 
 __global__ void __launch_bounds__(kAlignThreads)
@@ -170,199 +220,44 @@ align_block_kernel(const void* ids, int is64, const int* map, int map_len, const
   griddep_wait();             // the tables written below may still be read by the kernels of the previous call
   griddep_launch_dependents();
   wait_for_peers(fw);
-  int* s_cnt = smem;                    // nwarps * E
-  int* s_base = s_cnt + nwarps * E;     // E + 1
-  int* s_hist = s_base + (E + 1);       // E
-  int* s_scan = s_hist + E;             // 33
-
-  const int nblk_cap = (cap + block - 1) / block;
-  for (int i = threadIdx.x; i < cap; i += blockDim.x) {
-    sorted_ids[i] = P;
-    if (row_gamma != nullptr) row_gamma[i] = 0.f;
-  }
-  for (int i = threadIdx.x; i < nblk_cap; i += blockDim.x) expert_ids[i] = -1;
-  __syncthreads();
-
-  group_by_expert(ids, is64, map, map_len, P, E, block, s_cnt, s_base, s_hist, s_scan, nwarps,
-                  row_gamma != nullptr ? weights : nullptr, [&](int slot, int pos, float w) {
+  const GroupSmem g = group_smem(smem, nwarps, E);
+  group_by_expert(ids, is64, map, map_len, P, E, block, g, nwarps, row_gamma != nullptr ? weights : nullptr,
+                  [&](int slot, int pos, float w) {
                     sorted_ids[pos] = slot;
                     if (row_gamma != nullptr) row_gamma[pos] = w;
                   });
 
-  const int rows = s_base[E];
-  const int nblk = rows / block;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-    int e = upper_expert(s_base, E + 1, b * block);
-    expert_ids[b] = e;
+  // padding of every expert's group, then the unused tail of the tables
+  const int lane = threadIdx.x & 31;
+  const int tid = cluster_rank() * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  const int rows = g.base[E];
+  for (int e = tid >> 5; e < E; e += nthreads >> 5)
+    for (int r = g.base[e] + g.hist[e] + lane; r < g.base[e + 1]; r += 32) {
+      sorted_ids[r] = P;
+      if (row_gamma != nullptr) row_gamma[r] = 0.f;
+    }
+  for (int r = rows + tid; r < cap; r += nthreads) {
+    sorted_ids[r] = P;
+    if (row_gamma != nullptr) row_gamma[r] = 0.f;
   }
+  const int nblk_cap = (cap + block - 1) / block;
+  const int nblk = rows / block;
+  for (int b = tid; b < nblk_cap; b += nthreads) expert_ids[b] = b < nblk ? upper_expert(g.base, E + 1, b * block) : -1;
   if (blk_off != nullptr)
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) blk_off[e] = s_base[e] / block;
-  if (threadIdx.x == 0) {
+    for (int e = tid; e <= E; e += nthreads) blk_off[e] = g.base[e] / block;
+  if (tid == 0) {
     num_post_pad[0] = rows;
     if (meta != nullptr) {
       meta[0] = nblk;
       meta[1] = rows;
     }
   }
-}
-
-// ---------------------------------------------------------------------------------------------
-// The same grouping spread over kAlignCtas CTAs in two launches, for tens of thousands of slots
-// (one CTA pushes every store through one SM's memory pipe: 77 us at 32 k slots).  CTA c owns the
-// contiguous slots [c * per, (c + 1) * per); stability follows from ordering by (CTA, warp, lane).
-//   count  per-CTA slots per expert -> cnt[c][e]; all CTAs share the filling of the defaults
-//   place  each CTA derives the padded expert starts and its own first rows from cnt (CTA 0 also
-//          writes the block tables), recounts its chunk (cheaper than keeping the per-warp counts)
-//          and writes
-constexpr int kAlignCtas = 32;
-
-// warp-private counts of the chunk [begin, end): s_cnt[w][e]
-__device__ __forceinline__ void count_chunk(const void* ids, int is64, const int* map, int map_len, int begin, int end, int E,
-                                            int* s_cnt, int nwarps, int* seg_begin, int* seg_end) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) s_cnt[i] = 0;
-  __syncthreads();
-  int seg = (max(end - begin, 0) + nwarps - 1) / nwarps;
-  seg = (seg + 31) & ~31;
-  const int b = begin + warp * seg;
-  const int e_ = min(end, b + seg);
-  *seg_begin = b;
-  *seg_end = e_;
-  if (warp < nwarps) {
-    for (int i0 = b; i0 < e_; i0 += 32) {
-      const int i = i0 + lane;
-      int e = -1;
-      if (i < e_) {
-        e = load_id(ids, is64, i);
-        if (map != nullptr && e >= 0) e = (e < map_len) ? map[e] : -1;
-        if (e < 0 || e >= E) e = -1;
-      }
-      unsigned m = __match_any_sync(0xffffffffu, e);
-      if (e >= 0 && (m & ((1u << lane) - 1)) == 0) s_cnt[warp * E + e] += __popc(m);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(kAlignThreads)
-align_count_kernel(const void* ids, int is64, const int* map, int map_len, int P, int E, int block, int cap, int per, int nwarps,
-                   int* sorted_ids, int* expert_ids, float* row_gamma, int* cnt, const FlagWait fw) {
-  extern __shared__ int smem[];
-  int* s_cnt = smem;
-  griddep_wait();
-  griddep_launch_dependents();
-  wait_for_peers(fw);
-  const int nblk_cap = (cap + block - 1) / block;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += gridDim.x * blockDim.x) {
-    sorted_ids[i] = P;
-    if (row_gamma != nullptr) row_gamma[i] = 0.f;
-  }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nblk_cap; i += gridDim.x * blockDim.x) expert_ids[i] = -1;
-  const int begin = min(P, static_cast<int>(blockIdx.x) * per), end = min(P, begin + per);
-  int sb, se;
-  count_chunk(ids, is64, map, map_len, begin, end, E, s_cnt, nwarps, &sb, &se);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = 0;
-    for (int w = 0; w < nwarps; ++w) run += s_cnt[w * E + e];
-    cnt[blockIdx.x * E + e] = run;
-  }
-}
-
-__global__ void __launch_bounds__(kAlignThreads)
-align_place_kernel(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
-                   int block, int per, int nwarps, const int* cnt, int* sorted_ids, float* row_gamma, int* expert_ids,
-                   int* num_post_pad, int* blk_off, int* meta) {
-  extern __shared__ int smem[];
-  int* s_cnt = smem;                      // nwarps * E
-  int* s_base = s_cnt + nwarps * E;       // E + 1 padded expert starts
-  int* s_mine = s_base + (E + 1);         // E: first row of this CTA's slots of each expert
-  int* s_scan = s_mine + E;               // 33
-  griddep_wait();
-  griddep_launch_dependents();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nctas = gridDim.x;
-  // Every CTA derives the padded expert starts from the per-CTA counts by itself (a few thousand
-  // integers out of L2), which saves a single-CTA launch between counting and placing.
-  int carry = 0;
-  for (int e0 = 0; e0 < E; e0 += blockDim.x) {
-    const int e = e0 + threadIdx.x;
-    int total_e = 0, before = 0;
-    if (e < E) {
-      for (int c = 0; c < nctas; ++c) {
-        const int t = cnt[c * E + e];
-        if (c < static_cast<int>(blockIdx.x)) before += t;
-        total_e += t;
-      }
-    }
-    const int padded = (total_e + block - 1) / block * block;
-    int total;
-    const int ex = block_exclusive_scan(padded, s_scan, &total);
-    if (e < E) {
-      s_base[e] = carry + ex;
-      s_mine[e] = carry + ex + before;
-    }
-    carry += total;
-  }
-  if (threadIdx.x == 0) s_base[E] = carry;
-  __syncthreads();
-  if (blockIdx.x == 0) {
-    // the block tables, once
-    const int rows = s_base[E];
-    const int nblk = rows / block;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) expert_ids[b] = upper_expert(s_base, E + 1, b * block);
-    if (blk_off != nullptr)
-      for (int e = threadIdx.x; e <= E; e += blockDim.x) blk_off[e] = s_base[e] / block;
-    if (threadIdx.x == 0) {
-      num_post_pad[0] = rows;
-      if (meta != nullptr) {
-        meta[0] = nblk;
-        meta[1] = rows;
-      }
-    }
-  }
-  const int begin = min(P, static_cast<int>(blockIdx.x) * per), end = min(P, begin + per);
-  int sb, se;
-  count_chunk(ids, is64, map, map_len, begin, end, E, s_cnt, nwarps, &sb, &se);
-  // start of (warp, expert) = this CTA's first row of the expert + the counts of the warps before it
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = s_mine[e];
-    for (int w = 0; w < nwarps; ++w) {
-      const int t = s_cnt[w * E + e];
-      s_cnt[w * E + e] = run;
-      run += t;
-    }
-  }
-  __syncthreads();
-  if (warp < nwarps) {
-    for (int i0 = sb; i0 < se; i0 += 32) {
-      const int i = i0 + lane;
-      int e = -1;
-      float w = 0.f;
-      if (i < se) {
-        e = load_id(ids, is64, i);
-        if (map != nullptr && e >= 0) e = (e < map_len) ? map[e] : -1;
-        if (e < 0 || e >= E) e = -1;
-        if (row_gamma != nullptr) w = weights[i];
-      }
-      unsigned m = __match_any_sync(0xffffffffu, e);
-      const int rank = __popc(m & ((1u << lane) - 1));
-      int cur = 0;
-      if (e >= 0) cur = s_cnt[warp * E + e];
-      __syncwarp();
-      if (e >= 0) {
-        const int pos = cur + rank;
-        sorted_ids[pos] = i;
-        if (row_gamma != nullptr) row_gamma[pos] = w;
-        if (rank == 0) s_cnt[warp * E + e] = cur + __popc(m);
-      }
-      __syncwarp();
-    }
-  }
+  cluster_wait();
 }
 
 // Internal tables from the reference's routing triple: hist[E], topk_indx[P]
-// (sorted row -> slot), gate_scal[P] (sorted row order).
+// (sorted row -> slot), gate_scal[P] (sorted row order).  Every CTA scans hist by itself and fills its share of the
+// padded rows (one CTA took 19 us at 16384 slots).
 __global__ void __launch_bounds__(kAlignThreads)
 align_from_routing_kernel(const int* hist, const int* topk_indx, const float* gate_scal, int P, int E,
                           int block, int cap, int* sorted_ids, float* row_gamma, int* blk_off,
@@ -371,11 +266,8 @@ align_from_routing_kernel(const int* hist, const int* topk_indx, const float* ga
   int* s_base = smem;             // E + 1 padded starts
   int* s_raw = s_base + (E + 1);  // E + 1 raw starts
   int* s_scan = s_raw + (E + 1);  // 33
-
-  for (int i = threadIdx.x; i < cap; i += blockDim.x) {
-    sorted_ids[i] = P;
-    row_gamma[i] = 0.f;
-  }
+  griddep_wait();
+  griddep_launch_dependents();
   int carry_p = 0, carry_r = 0;
   for (int e0 = 0; e0 < E; e0 += blockDim.x) {
     int e = e0 + threadIdx.x;
@@ -393,89 +285,96 @@ align_from_routing_kernel(const int* hist, const int* topk_indx, const float* ga
     s_raw[E] = carry_r;
   }
   __syncthreads();
-  const int n_rows = min(P, s_raw[E]);
-  for (int q = threadIdx.x; q < n_rows; q += blockDim.x) {
-    int e = upper_expert(s_raw, E + 1, q);
-    int pos = s_base[e] + (q - s_raw[e]);
-    sorted_ids[pos] = topk_indx[q];
-    row_gamma[pos] = gate_scal[q];
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  for (int r = tid; r < cap; r += nthreads) {
+    int slot = P;
+    float w = 0.f;
+    if (r < carry_p) {
+      const int e = upper_expert(s_base, E + 1, r);
+      const int q = s_raw[e] + (r - s_base[e]);
+      if (q < s_raw[e + 1] && q < P) {
+        slot = topk_indx[q];
+        w = gate_scal[q];
+      }
+    }
+    sorted_ids[r] = slot;
+    row_gamma[r] = w;
   }
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) blk_off[e] = s_base[e] / block;
-  if (threadIdx.x == 0) {
-    meta[0] = s_base[E] / block;
-    meta[1] = s_base[E];
+  for (int e = tid; e <= E; e += nthreads) blk_off[e] = s_base[e] / block;
+  if (tid == 0) {
+    meta[0] = carry_p / block;
+    meta[1] = carry_p;
   }
 }
 
-// top-k -> the reference's routing tables.
+// top-k -> the reference's routing tables.  A token's experts are put in ascending order (stable): the place
+// of column j is the number of columns that precede it, so each slot finds its own with k reads
+// of its token's ids.  Grouping by expert needs no sorted ids: within an expert the order is by token, and by column
+// where a token names an expert twice, in either numbering.
 __global__ void __launch_bounds__(kAlignThreads)
 routing_from_topk_kernel(const float* weights, const void* ids, int is64, int M, int k, int E,
                          int max_tiles, int nwarps, int* expt_indx, int* topk_indx, int* gate_indx,
                          float* gate_scal, int* hist, int* token_offs_raw, int* token_offs_pad,
                          int* block_pid_map) {
   extern __shared__ int smem[];
-  int* s_cnt = smem;
-  int* s_base = s_cnt + nwarps * E;
-  int* s_hist = s_base + (E + 1);
-  int* s_scan = s_hist + E;
+  const GroupSmem g = group_smem(smem, nwarps, E);
   const int P = M * k;
-
-  // ascending (stable) insertion sort of each token's experts
-  for (int t = threadIdx.x; t < M; t += blockDim.x) {
-    for (int j = 0; j < k; ++j) {
-      int e = load_id(ids, is64, t * k + j);
-      int p = j;
-      while (p > 0 && expt_indx[t * k + p - 1] > e) {
-        expt_indx[t * k + p] = expt_indx[t * k + p - 1];
-        --p;
-      }
-      expt_indx[t * k + p] = e;
+  griddep_wait();
+  griddep_launch_dependents();
+  auto sorted_slot = [&](int i) {
+    const int t0 = i / k * k;
+    const int e = load_id(ids, is64, i);
+    int rank = 0;
+    for (int j = t0; j < t0 + k; ++j) {
+      const int ej = load_id(ids, is64, j);
+      rank += (ej < e) || (ej == e && j < i);
     }
-  }
-  for (int i = threadIdx.x; i < 4 * max_tiles; i += blockDim.x) block_pid_map[i] = -1;
+    return t0 + rank;
+  };
+  const int crank = cluster_rank(), nctas = gridDim.x;
+  const int tid = crank * blockDim.x + threadIdx.x, nthreads = nctas * blockDim.x;
+  for (int i = tid; i < P; i += nthreads) expt_indx[sorted_slot(i)] = load_id(ids, is64, i);
+
+  group_by_expert(ids, is64, nullptr, 0, P, E, 1, g, nwarps, weights, [&](int i, int pos, float w) {
+    const int slot = sorted_slot(i);
+    topk_indx[pos] = slot;
+    gate_indx[slot] = pos;
+    gate_scal[pos] = w;
+  });
+  for (int e = tid; e < E; e += nthreads) hist[e] = g.hist[e];
+  for (int e = tid; e <= E; e += nthreads) token_offs_raw[e] = g.base[e];
   __syncthreads();
 
-  group_by_expert(expt_indx, 0, nullptr, 0, P, E, 1, s_cnt, s_base, s_hist, s_scan, nwarps, nullptr,
-                  [&](int slot, int pos, float) {
-                    topk_indx[pos] = slot;
-                    gate_indx[slot] = pos;
-                    // the weight that the per-token sort moved to rank (slot % k):
-                    // the original column whose stable rank equals that position
-                    const int t = slot / k, want = slot - t * k;
-                    float w = 0.f;
-                    for (int j = 0; j < k; ++j) {
-                      int ej = load_id(ids, is64, t * k + j);
-                      int rank = 0;
-                      for (int i = 0; i < k; ++i) {
-                        int ei = load_id(ids, is64, t * k + i);
-                        rank += (ei < ej) || (ei == ej && i < j);
-                      }
-                      if (rank == want) w = weights[t * k + j];
-                    }
-                    gate_scal[pos] = w;
-                  });
-  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = s_hist[e];
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) token_offs_raw[e] = s_base[e];
-  __syncthreads();
-
-  // padded block tables for block sizes 16, 32, 64, 128
-  for (int v = 0; v < 4; ++v) {
+  // padded block tables for block sizes 16, 32, 64, 128, dealt out over the CTAs
+  int* s_off = g.cnt;     // E + 1 first blocks (the counters and totals behind them are no longer needed here)
+  cluster_wait();         // ... nor by the peers
+  for (int v = crank; v < 4; v += nctas) {
     const int bm = 16 << v;
     int carry = 0;
     for (int e0 = 0; e0 < E; e0 += blockDim.x) {
-      int e = e0 + threadIdx.x;
-      int tiles = (e < E) ? (s_hist[e] + bm - 1) / bm : 0;
+      const int e = e0 + threadIdx.x;
+      const int tiles = (e < E) ? (g.hist[e] + bm - 1) / bm : 0;
       int total;
-      int ex = block_exclusive_scan(tiles, s_scan, &total);
+      const int ex = block_exclusive_scan(tiles, g.scan, &total);
       if (e < E) {
-        int off = carry + ex;
-        token_offs_pad[v * (E + 1) + e] = off;
-        for (int b = 0; b < tiles; ++b)
-          if (off + b < max_tiles) block_pid_map[v * max_tiles + off + b] = (b << 16) + e;
+        s_off[e] = carry + ex;
+        token_offs_pad[v * (E + 1) + e] = carry + ex;
       }
       carry += total;
     }
-    if (threadIdx.x == 0) token_offs_pad[v * (E + 1) + E] = carry;
+    if (threadIdx.x == 0) {
+      s_off[E] = carry;
+      token_offs_pad[v * (E + 1) + E] = carry;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < max_tiles; b += blockDim.x) {
+      int w = -1;
+      if (b < carry) {
+        const int e = upper_expert(s_off, E + 1, b);
+        w = ((b - s_off[e]) << 16) + e;
+      }
+      block_pid_map[v * max_tiles + b] = w;
+    }
     __syncthreads();
   }
 }
@@ -485,6 +384,9 @@ int pick_warps(int E) {
   while (nw > 1 && static_cast<size_t>(nw) * E * 4 > 40 * 1024) nw >>= 1;
   return nw;
 }
+
+// CTAs of the cluster: one while a CTA's 32 warps hold a few rounds of slots at most
+int pick_ctas(int P) { return P < 1024 ? 1 : 8; }
 
 }  // namespace
 
@@ -508,59 +410,34 @@ int routing_max_tiles(int n_slots, int n_experts) {
 
 int launch_align_block(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
                        int block, int cap, int* sorted_ids, int* expert_ids, int* num_post_pad,
-                       float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl, const FlagWait* wait) {
+                       float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl, const FlagWait* wait, bool one_cta) {
   if (P < 0 || E <= 0 || block <= 0 || cap < 0) return B200MOE_ERR_BAD_ARG;
-  int nw = pick_warps(E);
-  size_t smem = (static_cast<size_t>(nw) * E + (E + 1) + E + 40) * sizeof(int);
+  const int nw = pick_warps(E);
+  const size_t smem = group_smem_bytes(nw, E);
   if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
   note_launch("align_block_kernel");
   FlagWait fw = {};
   if (wait != nullptr) fw = *wait;
-  cudaError_t err = launch_kernel(align_block_kernel, dim3(1), dim3(kAlignThreads), smem, stream, pdl, ids, is64, map,
-                                  map_len, weights, P, E, block, cap, nw, sorted_ids, expert_ids, num_post_pad,
-                                  row_gamma, blk_off, meta, fw);
-  return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
-}
-
-size_t align_multi_tmp_bytes(int E) { return static_cast<size_t>(kAlignCtas) * E * sizeof(int); }
-
-int launch_align_block_multi(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
-                             int block, int cap, int* sorted_ids, int* expert_ids, int* num_post_pad,
-                             float* row_gamma, int* blk_off, int* meta, int* tmp, cudaStream_t stream, bool pdl,
-                             const FlagWait* wait) {
-  if (P < 0 || E <= 0 || block <= 0 || cap < 0 || tmp == nullptr) return B200MOE_ERR_BAD_ARG;
-  const int nw = pick_warps(E);
-  const size_t smem = (static_cast<size_t>(nw) * E + 40) * sizeof(int);
-  const size_t smem_place = (static_cast<size_t>(nw) * E + 2 * static_cast<size_t>(E) + 1 + 40) * sizeof(int);
-  if (smem_place > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
-  int per = (P + kAlignCtas - 1) / kAlignCtas;
-  per = (per + 31) & ~31;
-  int* cnt = tmp;
-  FlagWait fw = {};
-  if (wait != nullptr) fw = *wait;
-  note_launch("align_count_kernel");
-  cudaError_t err = launch_kernel(align_count_kernel, dim3(kAlignCtas), dim3(kAlignThreads), smem, stream, pdl, ids,
-                                  is64, map, map_len, P, E, block, cap, per, nw, sorted_ids, expert_ids, row_gamma, cnt,
-                                  fw);
-  if (err != cudaSuccess) return B200MOE_ERR_CUDA;
-  note_launch("align_place_kernel");
-  err = launch_kernel(align_place_kernel, dim3(kAlignCtas), dim3(kAlignThreads), smem_place, stream, pdl, ids, is64, map,
-                      map_len, weights, P, E, block, per, nw, static_cast<const int*>(cnt), sorted_ids, row_gamma,
-                      expert_ids, num_post_pad, blk_off, meta);
+  const int ctas = one_cta ? 1 : pick_ctas(P);
+  cudaError_t err = launch_kernel_cluster(align_block_kernel, dim3(ctas), ctas, dim3(kAlignThreads), smem, stream, pdl, ids,
+                                          is64, map, map_len, weights, P, E, block, cap, nw, sorted_ids, expert_ids,
+                                          num_post_pad, row_gamma, blk_off, meta, fw);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
 int launch_align_from_routing(const int* hist, const int* topk_indx, const float* gate_scal, int P,
                               int E, int block, int cap, int* sorted_ids, float* row_gamma,
-                              int* blk_off, int* meta, cudaStream_t stream) {
+                              int* blk_off, int* meta, cudaStream_t stream, bool pdl) {
   if (P < 0 || E <= 0 || block <= 0) return B200MOE_ERR_BAD_ARG;
   size_t smem = (2 * static_cast<size_t>(E + 1) + 40) * sizeof(int);
   if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
   note_launch("align_from_routing_kernel");
-  align_from_routing_kernel<<<1, kAlignThreads, smem, stream>>>(hist, topk_indx, gate_scal, P, E, block,
-                                                                cap, sorted_ids, row_gamma, blk_off,
-                                                                meta);
-  return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
+  int ctas = (cap + kAlignThreads - 1) / kAlignThreads;
+  if (ctas > 32) ctas = 32;
+  if (ctas < 1) ctas = 1;
+  cudaError_t err = launch_kernel(align_from_routing_kernel, dim3(ctas), dim3(kAlignThreads), smem, stream, pdl, hist, topk_indx,
+                                  gate_scal, P, E, block, cap, sorted_ids, row_gamma, blk_off, meta);
+  return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
 int launch_routing_from_topk(const float* weights, const void* ids, int is64, int M, int k, int E,
@@ -568,15 +445,16 @@ int launch_routing_from_topk(const float* weights, const void* ids, int is64, in
                              int* hist, int* token_offs_raw, int* token_offs_pad, int* block_pid_map,
                              cudaStream_t stream) {
   if (M < 0 || k <= 0 || E <= 0) return B200MOE_ERR_BAD_ARG;
-  int nw = pick_warps(E);
-  size_t smem = (static_cast<size_t>(nw) * E + (E + 1) + E + 40) * sizeof(int);
+  const int nw = pick_warps(E);
+  const size_t smem = group_smem_bytes(nw, E);
   if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
-  int mt = routing_max_tiles(M * k, E);
+  const int mt = routing_max_tiles(M * k, E);
   note_launch("routing_from_topk_kernel");
-  routing_from_topk_kernel<<<1, kAlignThreads, smem, stream>>>(
-      weights, ids, is64, M, k, E, mt, nw, expt_indx, topk_indx, gate_indx, gate_scal, hist,
-      token_offs_raw, token_offs_pad, block_pid_map);
-  return cudaGetLastError() == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
+  const int ctas = pick_ctas(M * k);
+  cudaError_t err = launch_kernel_cluster(routing_from_topk_kernel, dim3(ctas), ctas, dim3(kAlignThreads), smem, stream, true,
+                                          weights, ids, is64, M, k, E, mt, nw, expt_indx, topk_indx, gate_indx, gate_scal,
+                                          hist, token_offs_raw, token_offs_pad, block_pid_map);
+  return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
 }  // namespace b200moe

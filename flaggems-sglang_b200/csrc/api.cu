@@ -142,7 +142,6 @@ void launch_log_new_call() {
 
 struct Layout {
   int BT, cap, P;
-  bool align_multi; // alignment on 32 CTAs (many slots)
   bool quant_once; // FP8: quantise each token once, then gather the quantised rows (many pairs per token)
   bool pair_rows; // the down projection stores one 16-bit row per pair, the output conversion sums them
   bool pairs2;    // 16-bit GEMMs on CTA pairs: rows padded to 32 per expert, tiles of up to `tile_tokens`
@@ -152,7 +151,7 @@ struct Layout {
   int orient;     // GEMM tile orientation that goes with BT
   int act_bytes;  // bytes per activation element fed to the GEMMs
   size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, xs_sum, a2, a2_scale,
-      a2_sum, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, align_tmp, total;
+      a2_sum, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
 };
 
 int pick_bt(const b200moe_cfg* c) {
@@ -210,7 +209,6 @@ int check_cfg(const b200moe_cfg* c) {
 
 int query_sms(const b200moe_cfg* c);
 bool reference_rounds_pairs(int P, int E, int n, int k, int sms);
-constexpr int kAlignMultiSlots = 8192;   // from here on the alignment runs on 32 CTAs
 
 int make_layout(const b200moe_cfg* c, Layout* L) {
   L->BT = pick_bt(c);
@@ -283,8 +281,6 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   L->pair_valid = take(L->pair_rows ? align_up(static_cast<size_t>(L->P), 16) : 0);
   L->route_w = take(static_cast<size_t>(L->P > 0 ? L->P : 1) * 4);    // router output when the call starts from logits
   L->route_ids = take(static_cast<size_t>(L->P > 0 ? L->P : 1) * 4);
-  L->align_multi = L->P >= kAlignMultiSlots && !(c->flags & B200MOE_FLAG_ALIGN_ONE_CTA);
-  L->align_tmp = take(L->align_multi ? align_multi_tmp_bytes(c->E) : 0);
   L->total = off;
   return B200MOE_OK;
 }
@@ -334,7 +330,7 @@ int query_sms(const b200moe_cfg* c) {
   return cached[dev];
 }
 
-// Block alignment into the workspace tables: one CTA, or 32 CTAs in three launches for many slots.
+// Block alignment into the workspace tables.
 int align_into_workspace(const b200moe_cfg* c, const Layout& L, uint8_t* ws, const void* ids, int is64,
                          const int32_t* expert_map, const float* weights, cudaStream_t st,
                          const FlagWait* wait = nullptr) {
@@ -345,12 +341,9 @@ int align_into_workspace(const b200moe_cfg* c, const Layout& L, uint8_t* ws, con
   float* row_gamma = reinterpret_cast<float*>(ws + L.row_gamma);
   int* blk_off = reinterpret_cast<int*>(ws + L.blk_off);
   int* meta = reinterpret_cast<int*>(ws + L.meta);
-  if (L.align_multi)
-    return launch_align_block_multi(ids, is64, expert_map, c->n_global_experts, weights, L.P, c->E, L.BT, L.cap, sorted_ids, expert_ids,
-                                    num_post, row_gamma, blk_off, meta, reinterpret_cast<int*>(ws + L.align_tmp), st, pdl,
-                                    wait);
   return launch_align_block(ids, is64, expert_map, c->n_global_experts, weights, L.P, c->E, L.BT, L.cap, sorted_ids,
-                            expert_ids, num_post, row_gamma, blk_off, meta, st, pdl, wait);
+                            expert_ids, num_post, row_gamma, blk_off, meta, st, pdl, wait,
+                            (c->flags & B200MOE_FLAG_ALIGN_ONE_CTA) != 0);
 }
 
 // Expert parallelism: where the down projection's output rows go (the buffers of the ranks that
@@ -871,7 +864,8 @@ int b200moe_forward_routed(const b200moe_cfg* cfg, const void* x, const void* w1
   rc = launch_align_from_routing(hist, topk_indx, gate_scal, L.P, cfg->E, L.BT, L.cap,
                                  reinterpret_cast<int*>(ws + L.sorted_ids),
                                  reinterpret_cast<float*>(ws + L.row_gamma),
-                                 reinterpret_cast<int*>(ws + L.blk_off), reinterpret_cast<int*>(ws + L.meta), st);
+                                 reinterpret_cast<int*>(ws + L.blk_off), reinterpret_cast<int*>(ws + L.meta), st,
+                                 (cfg->flags & B200MOE_FLAG_NO_PDL) == 0);
   if (rc != B200MOE_OK) return rc;
   return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot);
 }

@@ -6,7 +6,7 @@
 // shared memory once per pair, and N follows the tokens an expert really has: its rows are padded to 32 and
 // dealt out evenly over ceil(rows / max) tiles, where a kernel with tokens on the M side pays for whole
 // blocks of 128 (two experts of eight with 250 tokens on average hold more than 256: 25 % of that kernel's
-// MMAs were padding).  Every launch picks `max` from the tokens at hand (see pick_max_granules).
+// MMAs were padding).  Every launch picks `max` from the tokens at hand (see rate_max_granules).
 //
 //   mode 0 (gate/up):  a CTA's 128 rows are 64 gate rows and the 64 matching up rows; the pair
 //                      covers 128 columns of the intermediate.
