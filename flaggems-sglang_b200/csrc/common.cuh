@@ -338,17 +338,14 @@ __device__ __forceinline__ void tmem_ld16x2_wait(uint32_t taddr0, uint32_t taddr
   }
 }
 
-// Raw 32-bit words of two 16-column reads (for packed f32x2 arithmetic on register pairs).
-__device__ __forceinline__ void tmem_ld16x2_wait_u32(uint32_t taddr0, uint32_t taddr1, uint32_t (&r0)[16],
-                                                     uint32_t (&r1)[16]) {
+// Raw 32-bit words of a 16-column read (for packed f32x2 arithmetic on register pairs).
+__device__ __forceinline__ void tmem_ld16_wait_u32(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-      "%13, %14, %15}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, "
-      "%27, %28, %29, %30, %31}, [%33];\n\t"
+      "%13, %14, %15}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
-      : B200MOE_R16(r0, 0), B200MOE_R16(r1, 0)
-      : "r"(taddr0), "r"(taddr1)
+      : B200MOE_R16(r, 0)
+      : "r"(taddr)
       : "memory");
 }
 

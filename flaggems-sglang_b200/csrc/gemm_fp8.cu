@@ -294,14 +294,21 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           bg = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + n);
           bu = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + a.N + n);
         }
+        if (ext) {
+#pragma unroll
+          for (int i = 0; i < CPT; ++i) {
+            acc0[i] += bg;
+            acc1[i] += bu;
+          }
+          act_mul_array<__nv_bfloat16, true>(acc0, acc1, w_on_input, false, act_params(a), [&](int i) { return col_gam[i]; });
+        } else {
+          act_mul_array<__nv_bfloat16, false>(acc0, acc1, w_on_input, false, act_params(a), [&](int i) { return col_gam[i]; });
+        }
+        const bool bf = a.dtype == B200MOE_DTYPE_BF16;
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
-          float av = ext ? act_mul<__nv_bfloat16, true>(acc0[i] + bg, acc1[i] + bu, w_on_input, col_gam[i], false, act_params(a))
-                         : act_mul<__nv_bfloat16>(acc0[i], acc1[i], w_on_input, col_gam[i], false, act_params(a));
-          av = (a.dtype == B200MOE_DTYPE_BF16) ? __bfloat162float(__float2bfloat16_rn(av))
-                                               : __half2float(__float2half_rn(av));
-          acc0[i] = av;
-          const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(av)));
+          acc0[i] = bf ? __bfloat162float(__float2bfloat16_rn(acc0[i])) : __half2float(__float2half_rn(acc0[i]));
+          const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(acc0[i])));
           if (lane == 0) red[gw * 64 + i] = __uint_as_float(m);
         }
         if (!warps_meet(smem_u32(&bar_meet[grp]), meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
@@ -357,8 +364,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 // ------------------------------------------------------------------------------------------
 // Tokens-on-M variant for 128-token blocks (prefill-sized batches).
 //
-// One tcgen05.mma costs about the same issue time whatever its N, so with many tokens per
-// expert the token block goes on the M side (128 rows) and 256 weight rows on the N side:
+// With many tokens per expert the token block goes on the M side (128 rows) and 256 weight rows on the N side:
 // four MMAs per 128-wide reduction slice instead of sixteen.  An accumulator row is then a
 // token, so the activation scale is one scalar per thread and slice, the weight scale one
 // scalar per 128 columns; two promotion groups split the 256 columns (gate columns
@@ -366,8 +372,21 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 // and keep 128 accumulators per thread.  The 1x128 quantisation group of a token is the 64
 // activations of its thread in group 0 plus the 64 of its thread in group 1: the two partial
 // maxima meet in shared memory, no shuffles.
-constexpr int kThreadsFp8TokM = 7 * 32 + 128;
-constexpr int kPairStageBytes = 2 * 128 * 144;   // staging of 16-bit pair rows: two groups x 128 rows x (128 + 16) bytes
+//
+// What bounds it: the promotion's serial path per slice (wait, tensor-memory reads, FMAs, release), about 1000
+// cycles against 512 for the slice's MMAs, and the tail (5000 cycles per tile) that nothing overlaps: the
+// accumulators fill the registers and the two partial buffers all of tensor memory.  Kept off that
+// path: the tile's coordinates (decoded by the table warp), the activation scales (a ring filled per slice, which also
+// frees the room of a fourth stage), warp meetings around the staged stores (each warp transposes its own
+// rows).  256 experts, zipf-skewed routing: 4096 tokens 3367 -> 3140 us, 512 tokens 1093 -> 998 us.
+// Tried and slower: sixteen promotion warps, 32-column reads, scalar FMAs, partial buffers released by halves, hot and
+// cold experts' tiles interleaved.
+// warps 0-3: TMA, MMA, tables, idle; warps 4-11: promotion.  Launched with 168 registers a thread, the
+// first four warps keep 48 and the promotion warps take 224: 4 * 48 + 8 * 224 <= 12 * 168.
+constexpr int kThreadsFp8TokM = 12 * 32;
+constexpr int kPairStagePitch = 80;                               // 32 columns of a 16-bit pair row + 16 bytes
+constexpr int kPairStageBytes = 2 * 128 * kPairStagePitch;         // two groups x 128 rows
+constexpr int kXsSlots = 8;                                       // ring of activation scales, one slot per slice
 
 #ifdef B200MOE_STALL_STATS
 __device__ unsigned long long g_stall_fp8[16];
@@ -390,11 +409,11 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   constexpr int PCOLS = 256;
   const int stages = a.stages;
 
-  const int KBS = a.kblocks;   // reduction slices of a whole row: size of the per-tile scale tables
+  const int KBS = a.kblocks;   // reduction slices of a whole row: size of the per-tile weight-scale tables
   uint8_t* ctrl_base = smem + static_cast<size_t>(stages) * STAGE_BYTES;
-  float* s_xs = reinterpret_cast<float*>(ctrl_base);                    // [2][KBS][128] activation scales
-  float* s_ws = s_xs + 2 * KBS * BT;                                    // [2][2][KBS] weight scales
-  // mode 1 with rows stored per pair: staging for coalesced stores, [2 groups][128 rows][144 bytes]
+  float* s_xs = reinterpret_cast<float*>(ctrl_base);                    // [kXsSlots][128] activation scales
+  float* s_ws = s_xs + kXsSlots * BT;                                   // [2][2][KBS] weight scales
+  // mode 1 with rows stored per pair: staging for coalesced stores, [2 groups][128 rows][80 bytes]
   uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_ws + 2 * 2 * KBS);
   uint64_t* bar_full = reinterpret_cast<uint64_t*>(s_stage + ((MODE == 1 && a.out_pairs != nullptr) ? kPairStageBytes : 0));
   uint64_t* bar_empty = bar_full + stages;
@@ -402,15 +421,15 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   uint64_t* bar_pempty = bar_pfull + 2;
   uint64_t* bar_sfull = bar_pempty + 2;
   uint64_t* bar_sempty = bar_sfull + 2;
-  uint64_t* bar_meet = bar_sempty + 2;          // [2] one per promotion group: meetings around the staged stores
-  uint64_t* bar_meet8 = bar_meet + 2;           // both groups: the halves of a quantisation group's maximum
+  uint64_t* bar_meet8 = bar_sempty + 2;         // both groups: the halves of a quantisation group's maximum
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_meet8 + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_col_row = reinterpret_cast<int*>(tmem_slot + 4);               // [2][128] output row of each token
+  int* s_tile = reinterpret_cast<int*>(tmem_slot + 4);                  // [2][8] expert, row0, n0, kb0, kb1 of a tile
+  int* s_col_row = s_tile + 16;               // [2][128] output row of each token
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * 128);     // [2][128]
-  float* s_red = s_col_gam + 2 * 128;                                   // [2][2][128] partial group maxima
-  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + 2 * 2 * 128);   // [2][128] mode 1: base of each row's output row
-  int* s_blk_off = reinterpret_cast<int*>(s_col_ptr + 2 * 128);         // [E+1]
+  float* s_red = s_col_gam + 2 * 128;                                   // mode 0: [2][2][128] partial group maxima
+  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + (MODE == 0 ? 2 * 2 * 128 : 0));   // [2][128] mode 1: base of each row's output row
+  int* s_blk_off = reinterpret_cast<int*>(s_col_ptr + (MODE == 1 ? 2 * 128 : 0));   // [E+1]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -425,7 +444,6 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       mbar_init(smem_u32(&bar_pempty[s]), 8);
       mbar_init(smem_u32(&bar_sfull[s]), 1);
       mbar_init(smem_u32(&bar_sempty[s]), 8);
-      mbar_init(smem_u32(&bar_meet[s]), 4);
     }
     mbar_init(smem_u32(bar_meet8), 8);
     *abort_flag = 0;
@@ -451,11 +469,14 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
 
-  if (active && warp == 0 && lane == 0) {
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+  if (active && warp == 0 && elect_one()) {
     // =============================== TMA producer ===============================
     int stage = 0;
     uint32_t phase = 0;
     long long issued = 0;
+    uint32_t jx = 0;     // slices issued over the whole launch
     bool ok = true;
     unsigned long long w_empty = 0;
     const long long role_t0 = clock64();
@@ -466,8 +487,14 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
           ok = false;
           break;
         }
+        // The slice's activation scales go to a ring of their own, which the promotion warps read once the slice's
+        // MMAs are done (these wait for the whole stage, scales included).  The slot is free: this stage's last MMA has finished, and it was issued after the promotion of the slice two
+        // before it, which is at most stages + 2 <= kXsSlots slices back.
+        const uint32_t xs_slot = jx % kXsSlots;
+        ++jx;
         const uint32_t full = smem_u32(&bar_full[stage]);
-        mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES));
+        mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES + BT * 4));
+        bulk_copy_g2s(smem_u32(s_xs + xs_slot * BT), a.x_scale + static_cast<size_t>(kb) * a.ld_xscale + t.row0, BT * 4, full);
         const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
         const int k0 = kb * kStageKBytes;
         tma_load_3d(sw, &tm_w, full, k0, t.n0, t.e);
@@ -494,7 +521,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         mbar_wait_brief(smem_u32(&bar_full[s]), ph);
       }
     }
-  } else if (active && warp == 1 && lane == 0) {
+  } else if (active && warp == 1 && elect_one()) {
     // =============================== MMA issuer =================================
     const uint32_t idesc = make_idesc(0u /* e4m3 */, kTileRows, 256u);
     int stage = 0;
@@ -503,8 +530,13 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     unsigned long long w_full = 0, w_pempty = 0;
     const long long role_t0 = clock64();
     for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
-      for (int kb = t.kb0; kb < t.kb1; ++kb, ++j) {
+      int kb0 = 0, kb1 = a.kblocks;
+      if (c.split > 1) {       // only the slice count matters here
+        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+        kb0 = t.kb0;
+        kb1 = t.kb1;
+      }
+      for (int kb = kb0; kb < kb1; ++kb, ++j) {
         const uint32_t pb = j & 1u;
         if (!mbar_wait_t(smem_u32(&bar_full[stage]), phase, abort_flag, DEV_TIMEOUT_MMA, w_full) ||
             !mbar_wait_t(smem_u32(&bar_pempty[pb]), ((j >> 1) & 1u) ^ 1u, abort_flag, DEV_TIMEOUT_MMA, w_pempty)) {
@@ -529,7 +561,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     STALL_ADD8(1, w_pempty);
     STALL_ADD8(2, w_full);
     STALL_ADD8(9, static_cast<unsigned long long>(clock64() - role_t0));
-  } else if (active && warp == 6) {
+  } else if (active && warp == 2) {
     // =============================== per-tile table loader ======================
     const int kb_total = a.kblocks;
     int iter = 0;
@@ -559,17 +591,23 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         ws_t[i] = __ldg(ws0 + i);
         ws_t[KBS + i] = second_ok ? __ldg(ws1 + i) : 0.f;
       }
+      if (lane == 0) {
+        int* ti = s_tile + buf * 8;
+        ti[0] = t.e;
+        ti[1] = t.row0;
+        ti[2] = t.n0;
+        ti[3] = t.kb0;
+        ti[4] = t.kb1;
+      }
       __syncwarp();
-      const uint32_t sfull = smem_u32(&bar_sfull[buf]);
-      if (lane == 0) mbar_arrive_expect_tx(sfull, static_cast<uint32_t>(nkb * BT * 4));
-      __syncwarp();
-      for (int i = lane; i < nkb; i += 32)
-        bulk_copy_g2s(smem_u32(s_xs + (buf * KBS + i) * BT),
-                      a.x_scale + static_cast<size_t>(t.kb0 + i) * a.ld_xscale + t.row0, BT * 4, sfull);
+      if (lane == 0) mbar_arrive(smem_u32(&bar_sfull[buf]));
     }
-  } else if (active && warp >= 2 && warp != 6) {
+  }
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+  if (active) {
     // =============================== promotion + tail ===========================
-    const int grp = warp < 6 ? 0 : 1;
+    const int grp = warp < 8 ? 0 : 1;
     const int quad = warp & 3;
     const int lrow = quad * 32 + lane;  // token row inside the block = TMEM lane
     const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0;
@@ -577,17 +615,17 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     const uint32_t colA = (MODE == 0) ? 64u * grp : 128u * grp;
     const uint32_t colB = (MODE == 0) ? 128u + 64u * grp : 128u * grp + 64u;
     uint32_t j = 0;
-    uint32_t meet_phase = 0, meet8_phase = 0;
+    uint32_t meet8_phase = 0;
     int iter = 0;
     bool ok = true;
     unsigned long long w_pfull = 0, w_sfull = 0, t_tail = 0;
     const long long role_t0 = clock64();
     for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff, ++iter) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
       const int buf = iter & 1;
-      const float* xs_t = s_xs + buf * KBS * BT;
       const float* ws_t = s_ws + buf * 2 * KBS;
       if (!mbar_wait_t(smem_u32(&bar_sfull[buf]), (iter >> 1) & 1, abort_flag, DEV_TIMEOUT_EPILOGUE, w_sfull)) break;
+      const int* ti = s_tile + buf * 8;      // decoded by the table warp, off this critical path
+      const TileCoord t = {ti[0], ti[1], ti[2], ti[3], ti[4]};
       const int orow = s_col_row[buf * 128 + lrow];
       const float gam = s_col_gam[buf * 128 + lrow];
 
@@ -599,30 +637,32 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         pB[i] = 0ull;
       }
       for (int kb = t.kb0; kb < t.kb1; ++kb, ++j) {
-        const float sx = xs_t[(kb - t.kb0) * BT + lrow];
-        // mode 0: A columns belong to the first weight block, B columns to the second;
-        // mode 1: group g works entirely inside weight block g
-        const float fA = sx * ws_t[(MODE == 0 ? 0 : grp * KBS) + kb - t.kb0];
-        const float fB = sx * ws_t[(MODE == 0 ? KBS : grp * KBS) + kb - t.kb0];
         const uint32_t pb = j & 1u;
         if (!mbar_wait_t(smem_u32(&bar_pfull[pb]), (j >> 1) & 1u, abort_flag, DEV_TIMEOUT_EPILOGUE, w_pfull)) {
           ok = false;
           break;
         }
         tc_fence_after();
+        const uint32_t xs_slot = j % kXsSlots;
+        const float sx = s_xs[xs_slot * BT + lrow];
+        // mode 0: A columns belong to the first weight block, B columns to the second;
+        // mode 1: group g works entirely inside weight block g
+        const float fA = sx * ws_t[(MODE == 0 ? 0 : grp * KBS) + kb - t.kb0];
+        const float fB = sx * ws_t[(MODE == 0 ? KBS : grp * KBS) + kb - t.kb0];
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + pb * PCOLS;
-        // packed f32x2 FMAs on register pairs (one instruction per two accumulators), 16 columns of
-        // each half at a time to stay inside the register budget
+        // Packed f32x2 FMAs, 16 columns at a time.  They run at half the rate of scalar ones, so the FMA pipe is
+        // as busy, but they leave the MMA thread's scheduler twice the issue slots (with scalar FMAs the MMAs of a
+        // slice took 684 cycles instead of 516).  Wider reads spill: the accumulators alone take 128 registers.
         const unsigned long long fA2 = pack_f32x2(fA, fA), fB2 = pack_f32x2(fB, fB);
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 16) {
-          uint32_t g[16], u[16];
-          tmem_ld16x2_wait_u32(taddr + colA + c0, taddr + colB + c0, g, u);
+          uint32_t g[16];
+          tmem_ld16_wait_u32(taddr + colA + c0, g);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            ffma2_packed(pA[c0 / 2 + i], g[2 * i], g[2 * i + 1], fA2);
-            ffma2_packed(pB[c0 / 2 + i], u[2 * i], u[2 * i + 1], fB2);
-          }
+          for (int i = 0; i < 8; ++i) ffma2_packed(pA[c0 / 2 + i], g[2 * i], g[2 * i + 1], fA2);
+          tmem_ld16_wait_u32(taddr + colB + c0, g);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ffma2_packed(pB[c0 / 2 + i], g[2 * i], g[2 * i + 1], fB2);
         }
         tc_fence_before();
         __syncwarp();
@@ -661,14 +701,16 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             accB[i] += in ? __ldg(bgp + a.N + i) : 0.f;
           }
         }
+        if (ext) act_mul_array<__nv_bfloat16, true>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
+        else act_mul_array<__nv_bfloat16, false>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
+        const bool bf = a.dtype == B200MOE_DTYPE_BF16;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          float av = ext ? act_mul<__nv_bfloat16, true>(accA[i], accB[i], w_on_input, gam, false, act_params(a))
-                         : act_mul<__nv_bfloat16>(accA[i], accB[i], w_on_input, gam, false, act_params(a));
-          av = (a.dtype == B200MOE_DTYPE_BF16) ? __bfloat162float(__float2bfloat16_rn(av))
-                                               : __half2float(__float2half_rn(av));
-          accA[i] = av;
-          amax = fmaxf(amax, fabsf(av));
+        for (int i = 0; i < 64; i += 2) {
+          const float2 v = bf ? __bfloat1622float2(__floats2bfloat162_rn(accA[i], accA[i + 1]))
+                              : __half22float2(__floats2half2_rn(accA[i], accA[i + 1]));
+          accA[i] = v.x;
+          accA[i + 1] = v.y;
+          amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
         }
         float* red = s_red + buf * 2 * 128;
         red[grp * 128 + lrow] = amax;
@@ -694,19 +736,23 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       } else if (a.out_pairs != nullptr) {
         // The pair's row, weighted and rounded to the 16-bit type.  A thread owns 128 contiguous
         // columns of one row; storing them directly would touch 32 rows per warp instruction, so
-        // the group's four warps stage 64 columns at a time in shared memory (144-byte row pitch)
-        // and write them out with 16-byte stores that cover four rows per instruction.
+        // each warp stages 32 columns of its rows at a time in shared memory (80-byte row pitch)
+        // and writes them out with 16-byte stores that cover eight rows per instruction.
         const float scale = w_on_input ? 1.0f : gam;
         const bool bf = a.dtype == B200MOE_DTYPE_BF16;
-        uint8_t* stage_g = s_stage + grp * (128 * 144);
-        const int gtid = quad * 32 + lane;            // thread within the group
-        const uint32_t meet = smem_u32(&bar_meet[grp]);
-        auto group_meets = [&]() -> bool { return warps_meet(meet, meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE); };
+        uint8_t* stage_w = s_stage + (grp * 4 + quad) * (32 * kPairStagePitch);
+        uint16_t* dst[4];       // this lane stores chunk lane % 4 of rows lane / 4 + 8 it
 #pragma unroll
-        for (int round = 0; round < 2 && ok; ++round) {
-          const float* src = (round == 0) ? accA : accB;
+        for (int it = 0; it < 4; ++it) {
+          const int brow = buf * 128 + quad * 32 + it * 8 + (lane >> 2);
+          dst[it] = s_col_row[brow] >= 0 ? reinterpret_cast<uint16_t*>(s_col_ptr[brow]) + t.n0 + 128 * grp + (lane & 3) * 8 : nullptr;
+        }
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
+        for (int round = 0; round < 4; ++round) {
+          const float* src = (round < 2 ? accA : accB) + 32 * (round & 1);
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
             uint32_t w[4];
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
@@ -719,30 +765,17 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                 w[b] = *reinterpret_cast<uint32_t*>(&v);
               }
             }
-            *reinterpret_cast<uint4*>(stage_g + gtid * 144 + q * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(stage_w + lane * kPairStagePitch + q * 16) = make_uint4(w[0], w[1], w[2], w[3]);
           }
-          if (!group_meets()) {
-            ok = false;
-            break;
-          }
-          const int col0 = t.n0 + 128 * grp + 64 * round;
-          if (col0 < a.N) {
+          __syncwarp();
+          if (t.n0 + 128 * grp + 32 * round < a.N) {
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int idx = it * 128 + gtid;
-              const int row = idx >> 3, ch = idx & 7;
-              const int prow = s_col_row[buf * 128 + row];
-              if (prow >= 0)
-                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(s_col_ptr[buf * 128 + row]) + col0 + ch * 8) =
-                    *reinterpret_cast<const uint4*>(stage_g + row * 144 + ch * 16);
-            }
-          }
-          if (!group_meets()) {
-            ok = false;
-            break;
+            for (int it = 0; it < 4; ++it)
+              if (dst[it] != nullptr)
+                *reinterpret_cast<uint4*>(dst[it] + 32 * round) =
+                    *reinterpret_cast<const uint4*>(stage_w + (it * 8 + (lane >> 2)) * kPairStagePitch + (lane & 3) * 16);
           }
         }
-        if (!ok) break;
         if (orow >= 0 && t.n0 == 0 && grp == 0) mark_pair_valid(a, orow);
       } else if (orow >= 0) {
         const float scale = w_on_input ? 1.0f : gam;
@@ -764,12 +797,14 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
       t_tail += static_cast<unsigned long long>(clock64() - tail_t0);
     }
-    if (threadIdx.x == 2 * 32) {
+    if (threadIdx.x == 4 * 32) {
       STALL_ADD8(5, w_pfull);
       STALL_ADD8(6, w_sfull);
       STALL_ADD8(7, t_tail);
       STALL_ADD8(11, static_cast<unsigned long long>(clock64() - role_t0));
     }
+  }
+
   }
 
   // ---- teardown
@@ -784,9 +819,9 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 }
 
 size_t fp8_tokm_ctrl_bytes(const GemmArgs& a) {
-  const size_t kbs = static_cast<size_t>(a.kblocks);
-  return 2 * kbs * 128 * 4 + 2 * 2 * kbs * 4 + ((a.mode == 1 && a.out_pairs != nullptr) ? kPairStageBytes : 0) + 512 +
-         2 * 128 * 8 + 2 * 2 * 128 * 4 + 2 * 128 * 8 + static_cast<size_t>(a.E + 1) * 4 + 64;
+  return kXsSlots * 128 * 4 + 2 * 2 * static_cast<size_t>(a.kblocks) * 4 +
+         ((a.mode == 1 && a.out_pairs != nullptr) ? kPairStageBytes : 0) + 512 /*barriers, tile words*/ + 2 * 2 * 128 * 4 +
+         (a.mode == 0 ? 2 * 2 * 128 * 4 : 2 * 128 * 8) + static_cast<size_t>(a.E + 1) * 4 + 64;
 }
 
 template <int MODE>
@@ -853,6 +888,7 @@ void gemm_plan_fp8(GemmArgs* a) {
   if (a->orient == 1) {   // tokens on M, 128-token blocks
     a->tmem_cols = 512;
     st = static_cast<int>((kSmemLimit - 1024 - fp8_tokm_ctrl_bytes(*a)) / (3 * kTileBytes));
+    if (st > kXsSlots - 2) st = kXsSlots - 2;
   }
   if (st > 10) st = 10;
   if (st < 2) st = 2;
@@ -875,7 +911,6 @@ int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Gemm
     B200MOE_FP8_CASE(16, 1)
     B200MOE_FP8_CASE(32, 1)
     B200MOE_FP8_CASE(64, 2)
-    B200MOE_FP8_CASE(128, 2)
     default:
       return B200MOE_ERR_BAD_ARG;
   }
