@@ -78,7 +78,8 @@ int make_tmap_3d(CUtensorMap* m, CUtensorMapDataType dt, int elem_bytes, const v
 // Stacked gate and up rows [experts][2][rows][inner] seen as [experts, rows, 2, inner], box = {box_inner, 2, box_rows,
 // 1}: one load brings the same rows of both halves, gate and up rows alternating.
 int make_tmap_gate_up(CUtensorMap* m, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t inner,
-                      uint64_t rows, uint64_t experts, uint32_t box_inner, uint32_t box_rows) {
+                      uint64_t rows, uint64_t experts, uint32_t box_inner, uint32_t box_rows,
+                      CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return B200MOE_ERR_CUDA;
   cuuint64_t dims[4] = {inner, 2, rows, experts};
@@ -86,8 +87,38 @@ int make_tmap_gate_up(CUtensorMap* m, CUtensorMapDataType dt, int elem_bytes, co
   cuuint32_t box[4] = {box_inner, 2, box_rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(m, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
+// Scale / zero words [tables][halves][n], box = {box_n, halves, box_tables}, unswizzled.
+int make_tmap_words(CUtensorMap* m, const void* base, uint64_t n, uint32_t halves, uint64_t tables, uint32_t box_n,
+                    uint32_t box_tables) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return B200MOE_ERR_CUDA;
+  cuuint64_t dims[3] = {n, halves, tables};
+  cuuint64_t strides[2] = {n * 4, n * halves * 4};
+  cuuint32_t box[3] = {box_n, halves, box_tables};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
+// [rows, inner] 16-bit matrix seen as [inner / 64][rows][64], box = {64, box_rows, atoms}: one load brings 64 * atoms
+// k as swizzle atoms of box_rows rows.
+int make_tmap_group_rows(CUtensorMap* m, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t rows,
+                         uint32_t box_rows, uint32_t atoms) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return B200MOE_ERR_CUDA;
+  cuuint64_t dims[3] = {64, rows, inner / 64};
+  cuuint64_t strides[2] = {inner * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, atoms};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
@@ -145,13 +176,12 @@ struct Layout {
   bool quant_once; // FP8: quantise each token once, then gather the quantised rows (many pairs per token)
   bool pair_rows; // the down projection stores one 16-bit row per pair, the output conversion sums them
   bool pairs2;    // 16-bit GEMMs on CTA pairs: rows padded to 32 per expert, tiles of up to `tile_tokens`
+  bool w4_var;    // int4 above decode sizes: rows padded to 16 per expert, tiles of up to `tile_tokens`
   int tile_tokens;
-  bool w4p;       // int4 decode path: integer MMAs on three-plane int8 activations
   int out_rows;   // rows of the fp32 output buffer: tokens, or pairs when nothing is combined
   int orient;     // GEMM tile orientation that goes with BT
   int act_bytes;  // bytes per activation element fed to the GEMMs
-  size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, xs_sum, a2, a2_scale,
-      a2_sum, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
+  size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, a2, a2_scale, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
 };
 
 int pick_bt(const b200moe_cfg* c) {
@@ -200,7 +230,7 @@ int check_cfg(const b200moe_cfg* c) {
   } else if (c->wmode == B200MOE_W_INT4_AWQ) {
     if (c->H % 128 != 0 || c->I % 128 != 0) return B200MOE_ERR_UNSUPPORTED;   // whole groups of 128
     if (c->dtype != B200MOE_DTYPE_FP16) return B200MOE_ERR_UNSUPPORTED;
-    if (c->flags & B200MOE_FLAG_SIMT) return B200MOE_ERR_UNSUPPORTED;
+    if ((c->flags & B200MOE_FLAG_SIMT) || !gemm_w4_ok(c->E)) return B200MOE_ERR_UNSUPPORTED;
   } else {
     return B200MOE_ERR_UNSUPPORTED;
   }
@@ -212,18 +242,18 @@ bool reference_rounds_pairs(int P, int E, int n, int k, int sms);
 
 int make_layout(const b200moe_cfg* c, Layout* L) {
   L->BT = pick_bt(c);
-  // a block of 128 tokens sits on the M side of the MMA; smaller (and 256-token) blocks on the N side
-  // int4 always runs tokens-on-M (one MMA then covers 256 weight rows, which halves the number of
-  // MMA instructions per streamed byte; blocks below 128 tokens simply load fewer token rows)
-  if (c->wmode == B200MOE_W_INT4_AWQ) L->orient = (L->BT <= 128) ? 1 : 0;
-  else L->orient = (c->wmode == B200MOE_W_FP8_BLOCK && L->BT == 128) ? 1 : 0;
+  // FP8: a block of 128 tokens sits on the M side of the MMA; everything else keeps weight rows there
+  L->orient = (c->wmode == B200MOE_W_FP8_BLOCK && L->BT == 128) ? 1 : 0;
   const int sms_l = query_sms(c);
   const int bt_asked = L->BT;
   L->pairs2 = c->wmode == B200MOE_W_16BIT && L->BT >= 128 && !(c->flags & B200MOE_FLAG_SIMT) && gemm_tc2_ok(c->E, sms_l);
+  L->w4_var = c->wmode == B200MOE_W_INT4_AWQ && L->BT > 32;
   L->tile_tokens = c->block_tokens > 0 ? L->BT / 32 * 32 : 256;
   if (L->pairs2) {
     L->orient = 2;
     L->BT = 32;
+  } else if (L->w4_var) {
+    L->BT = 16;
   }
   L->P = c->M * c->topk;
   int cap = align_capacity(L->P, c->E, L->BT);
@@ -231,12 +261,7 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   cap = static_cast<int>(align_up(static_cast<size_t>(cap > 0 ? cap : 1), L->BT));
   L->cap = cap;
   const bool fp8 = c->wmode == B200MOE_W_FP8_BLOCK;
-  // decode-sized int4: nibbles converted straight into tensor memory, integer MMAs, group scales
-  // applied to the partial sums
-  L->w4p = c->wmode == B200MOE_W_INT4_AWQ && L->BT <= 32 && !(c->flags & B200MOE_FLAG_W4_SMEM_OPERANDS) &&
-           gemm_w4_planes_ok(c->H, L->BT) && gemm_w4_planes_ok(c->I, L->BT);
-  L->act_bytes = fp8 ? 1 : (L->w4p ? 3 : 2);
-  const bool tables = fp8 || L->w4p;   // per (128-k group, row) tables beside the activations
+  L->act_bytes = fp8 ? 1 : 2;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -250,11 +275,9 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   L->num_post = take(16);
   L->row_gamma = take(static_cast<size_t>(cap) * 4);
   L->xs = take(static_cast<size_t>(cap) * c->H * L->act_bytes);
-  L->xs_scale = take(tables ? static_cast<size_t>(cap) * (c->H / 128) * 4 : 0);
-  L->xs_sum = take(L->w4p ? static_cast<size_t>(cap) * (c->H / 128) * 4 : 0);
+  L->xs_scale = take(fp8 ? static_cast<size_t>(cap) * (c->H / 128) * 4 : 0);
   L->a2 = take(static_cast<size_t>(cap) * c->I * L->act_bytes);
-  L->a2_scale = take(tables ? static_cast<size_t>(cap) * (c->I / 128) * 4 : 0);
-  L->a2_sum = take(L->w4p ? static_cast<size_t>(cap) * (c->I / 128) * 4 : 0);
+  L->a2_scale = take(fp8 ? static_cast<size_t>(cap) * (c->I / 128) * 4 : 0);
   L->out_rows = (c->flags & B200MOE_FLAG_NO_COMBINE) ? L->P : c->M;   // one fp32 row per pair when nothing is summed
   // Many pairs on 128-token blocks: fp32 atomics into the combine buffer would bound the down
   // projection's tail (every add is a read-modify-write of a row another tile also touches), and
@@ -266,7 +289,7 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   // split reduction, which needs the atomics, is what keeps the last wave full)
   const bool many_tiles = (static_cast<long long>(L->P) / bt_asked) * ((c->H + 255) / 256) >=
                           (fp8 ? 2LL : 4LL) * sms_l;
-  const bool pairs_ok16 = L->pairs2 && ((c->flags & B200MOE_FLAG_MIMIC_ROUNDING)
+  const bool pairs_ok16 = (L->pairs2 || L->w4_var) && ((c->flags & B200MOE_FLAG_MIMIC_ROUNDING)
                                             ? reference_rounds_pairs(L->P, c->E, c->H, c->I, sms_l)
                                             : many_tiles);
   L->pair_rows = ((fp8 && L->BT == 128 && many_tiles) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
@@ -401,10 +424,6 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
       rc = launch_group_quant_fp8(x, c->dtype, xs, reinterpret_cast<float*>(ws + L.xs_scale), sorted_ids, meta,
                                   L.P, c->topk, L.cap, c->H, 1, L.cap, zero, zero_bytes, sms, st, pdl);
     }
-  } else if (L.w4p) {
-    rc = launch_group_split_i8(x, reinterpret_cast<uint8_t*>(xs), reinterpret_cast<float*>(ws + L.xs_scale),
-                               reinterpret_cast<int*>(ws + L.xs_sum), sorted_ids, meta, L.P, c->topk, L.cap, c->H,
-                               L.BT, L.cap, zero, zero_bytes, sms, st, pdl);
   } else {
     rc = launch_gather_rows(x, xs, sorted_ids, meta, L.P, c->topk, c->H * 2, L.cap, zero, zero_bytes, sms, st, pdl);
   }
@@ -418,7 +437,7 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   g1.K = c->H;
   g1.N = c->I;
   g1.up_row_off = c->I;
-  g1.BT = L.pairs2 ? L.tile_tokens : L.BT;
+  g1.BT = L.pairs2 || L.w4_var ? L.tile_tokens : L.BT;
   g1.orient = L.orient;
   g1.topk = c->topk;
   g1.P = L.P;
@@ -446,21 +465,8 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     g1.out_q = reinterpret_cast<uint8_t*>(a2);
     g1.out_scale = reinterpret_cast<float*>(ws + L.a2_scale);
   }
-  if (w4) {
-    g1.w_sz = quant->w1_sz;
-    g1.w_rows = 2 * c->I;
-  }
-  const bool w4p = L.w4p;
-  if (w4p) {
-    g1.x_scale = reinterpret_cast<float*>(ws + L.xs_scale);
-    g1.x_sum = reinterpret_cast<int*>(ws + L.xs_sum);
-    g1.ld_xscale = L.cap;
-    g1.out_q = reinterpret_cast<uint8_t*>(a2);
-    g1.out_scale = reinterpret_cast<float*>(ws + L.a2_scale);
-    g1.out_sum = reinterpret_cast<int*>(ws + L.a2_sum);
-  }
   auto plan = [&](GemmArgs* g) {
-    if (fp8) gemm_plan_fp8(g); else if (w4p) gemm_plan_w4(g); else if (L.pairs2) gemm_plan_tc2(g); else gemm_plan(g);
+    if (fp8) gemm_plan_fp8(g); else if (w4) gemm_plan_w4(g); else if (L.pairs2) gemm_plan_tc2(g); else gemm_plan(g);
   };
   plan(&g1);
 
@@ -474,10 +480,6 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   g2.max_split = 0;
   if (c->flags & B200MOE_FLAG_NO_COMBINE) g2.topk = 1;   // output row = pair slot instead of token
   g2.bias = quant != nullptr ? quant->b2 : nullptr;
-  if (w4) {
-    g2.w_sz = quant->w2_sz;
-    g2.w_rows = c->H;
-  }
   if (!fp8 && (c->flags & B200MOE_FLAG_MIMIC_ROUNDING)) {
     if (reference_rounds_pairs(L.P, c->E, c->H, c->I, sms)) g2.flags |= B200MOE_FLAG_NO_SPLIT_K;
     else g2.flags &= ~B200MOE_FLAG_MIMIC_ROUNDING;
@@ -513,13 +515,6 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     g2.out_scale = nullptr;
     g2.flags &= ~B200MOE_FLAG_MIMIC_ROUNDING;
   }
-  if (w4p) {
-    g2.x_scale = reinterpret_cast<float*>(ws + L.a2_scale);
-    g2.x_sum = reinterpret_cast<int*>(ws + L.a2_sum);
-    g2.out_q = nullptr;
-    g2.out_scale = nullptr;
-    g2.out_sum = nullptr;
-  }
   plan(&g2);
   if (c->flags & B200MOE_FLAG_SIMT) {
     rc = launch_gemm_simt(w1, xs, g1, st, L.cap);
@@ -527,29 +522,45 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     rc = launch_gemm_simt(w2, a2, g2, st, L.cap);
     if (rc != B200MOE_OK) return rc;
   } else {
-    const int eb = w4p ? 1 : L.act_bytes;
+    const int eb = L.act_bytes;
     const CUtensorMapDataType dt = tmap_dtype(c->dtype, eb);
     const uint32_t kbox = 128 / eb;
     CUtensorMap tm_w1, tm_x, tm_w2, tm_a2;
     if (w4) {
-      // packed int4 rows, K/2 bytes per row.  Shared-memory-operand kernels: 32 bytes (64 k) per
-      // stage, plain row-major staging; integer decode kernels: 64 bytes (one group) per stage with
-      // the 64-byte swizzle, so that threads reading whole rows do not collide on banks
-      const uint32_t pbox = w4p ? 64 : 32;
-      const CUtensorMapSwizzle psw = w4p ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE;
-      if ((rc = make_tmap_3d(&tm_w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w1, c->H / 2, 2ull * c->I, c->E, pbox, 128,
-                             psw)) != B200MOE_OK)
-        return rc;
-      if ((rc = make_tmap_3d(&tm_w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w2, c->I / 2, c->H, c->E, pbox, 128,
-                             psw)) != B200MOE_OK)
-        return rc;
+      // packed int4 rows, K/2 bytes per row: one group (64 bytes) or, at decode sizes, two per stage, with the swizzle of
+      // that width, so that threads reading whole rows do not collide on banks
+      constexpr CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
+      const uint32_t pbox = L.w4_var ? 64 : 128;
+      const CUtensorMapSwizzle psw = L.w4_var ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
+      if ((rc = make_tmap_gate_up(&tm_w1, u8, 1, w1, c->H / 2, c->I, c->E, pbox, 64, psw)) != B200MOE_OK) return rc;
+      if ((rc = make_tmap_3d(&tm_w2, u8, 1, w2, c->I / 2, c->H, c->E, pbox, 128, psw)) != B200MOE_OK) return rc;
     } else {
       rc = L.pairs2 ? make_tmap_gate_up(&tm_w1, dt, eb, w1, c->H, c->I, c->E, kbox, 64)
                     : make_tmap_3d(&tm_w1, dt, eb, w1, c->H, 2ull * c->I, c->E, kbox, 128);
       if (rc != B200MOE_OK) return rc;
       if ((rc = make_tmap_3d(&tm_w2, dt, eb, w2, c->I, c->H, c->E, kbox, 128)) != B200MOE_OK) return rc;
     }
-    if (L.pairs2) {
+    if (w4) {
+      CUtensorMap tm_sz1, tm_sz2;
+      W4TokenMaps tx1, tx2;
+      if ((rc = make_tmap_words(&tm_sz1, quant->w1_sz, c->I, 2, static_cast<uint64_t>(c->E) * (c->H / 128), 64,
+                                L.w4_var ? 1 : 2)) != B200MOE_OK)
+        return rc;
+      if ((rc = make_tmap_words(&tm_sz2, quant->w2_sz, c->H, 1, static_cast<uint64_t>(c->E) * (c->I / 128), 128,
+                                L.w4_var ? 1 : 2)) != B200MOE_OK)
+        return rc;
+      const uint32_t n0 = L.w4_var ? 16 : L.BT;
+      for (uint32_t b = 0; b < (L.w4_var ? 12u : 1u); ++b) {
+        if ((rc = make_tmap_group_rows(&tx1.m[b], dt, xs, c->H, L.cap, n0 + 16 * b, L.w4_var ? 2 : 4)) != B200MOE_OK) return rc;
+        if ((rc = make_tmap_group_rows(&tx2.m[b], dt, a2, c->I, L.cap, n0 + 16 * b, L.w4_var ? 2 : 4)) != B200MOE_OK) return rc;
+      }
+      prof_mark(slot, 1, st);
+      rc = launch_gemm_w4(tm_w1, tm_sz1, tx1, g1, sms, st);
+      prof_mark(slot, 2, st);
+      if (rc != B200MOE_OK) return rc;
+      prof_mark(slot, 3, st);
+      rc = launch_gemm_w4(tm_w2, tm_sz2, tx2, g2, sms, st);
+    } else if (L.pairs2) {
       PairTokenMaps tx1, tx2;
       for (uint32_t b = 0; b < 8; ++b) {
         if ((rc = make_tmap_2d(&tx1.m[b], dt, eb, xs, c->H, L.cap, kbox, 16 * (b + 1))) != B200MOE_OK) return rc;
@@ -562,19 +573,14 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
       prof_mark(slot, 3, st);
       rc = launch_gemm_tc2(tm_w2, tx2, g2, sms, st);
     } else {
-      // int4 decode: a token block is 3 * BT consecutive rows (its three byte planes)
-      const uint64_t xrows = w4p ? 3ull * L.cap : static_cast<uint64_t>(L.cap);
-      const uint32_t xbox = w4p ? 3u * L.BT : static_cast<uint32_t>(L.BT);
-      if ((rc = make_tmap_2d(&tm_x, dt, eb, xs, c->H, xrows, kbox, xbox)) != B200MOE_OK) return rc;
-      if ((rc = make_tmap_2d(&tm_a2, dt, eb, a2, c->I, xrows, kbox, xbox)) != B200MOE_OK) return rc;
+      if ((rc = make_tmap_2d(&tm_x, dt, eb, xs, c->H, L.cap, kbox, L.BT)) != B200MOE_OK) return rc;
+      if ((rc = make_tmap_2d(&tm_a2, dt, eb, a2, c->I, L.cap, kbox, L.BT)) != B200MOE_OK) return rc;
       prof_mark(slot, 1, st);
-      rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, g1, sms, st)
-               : (w4p ? launch_gemm_w4(tm_w1, tm_x, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st));
+      rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st);
       prof_mark(slot, 2, st);
       if (rc != B200MOE_OK) return rc;
       prof_mark(slot, 3, st);
-      rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, g2, sms, st)
-               : (w4p ? launch_gemm_w4(tm_w2, tm_a2, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st));
+      rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st);
     }
     prof_mark(slot, 4, st);
     if (rc != B200MOE_OK) return rc;

@@ -166,6 +166,15 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2,
+                                            int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+      "[%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
 // Untiled bulk copy global -> shared (both addresses 16-byte aligned, size a multiple of 16),
 // completing on an mbarrier like the tiled loads.
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -220,31 +229,7 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, 
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Integer form: A (tensor memory, four consecutive k per 32-bit column, lowest byte first) and
-// B (shared memory) hold 8-bit integers, the accumulator is int32.
-__device__ __forceinline__ void tc_mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Each thread of the warp writes 32 consecutive 32-bit columns of its own TMEM lane and waits
-// until the store has landed.
-__device__ __forceinline__ void tmem_st32_wait(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n\t"
-      "tcgen05.wait::st.sync.aligned;" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-// Same for 8-bit float inputs (e4m3 / e5m2).
+// D[tmem] (+)= A[smem] * B[smem] for 8-bit float inputs (e4m3 / e5m2).
 __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -275,50 +260,10 @@ __device__ __forceinline__ void tmem_ld16_wait(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Two loads (e.g. gate and up accumulators) in flight before the single wait.
-// Six 8-column reads of raw 32-bit accumulators, one wait.
 #define B200MOE_R8(r, o)                                                                             \
   "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]),   \
       "=r"(r[o + 6]), "=r"(r[o + 7])
-__device__ __forceinline__ void tmem_ld8x6_wait_b32(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t a4,
-                                                    uint32_t a5, int (&v)[48]) {
-  uint32_t r[48];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%48];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%49];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%50];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%51];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%32, %33, %34, %35, %36, %37, %38, %39}, [%52];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%40, %41, %42, %43, %44, %45, %46, %47}, [%53];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : B200MOE_R8(r, 0), B200MOE_R8(r, 8), B200MOE_R8(r, 16), B200MOE_R8(r, 24), B200MOE_R8(r, 32), B200MOE_R8(r, 40)
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 48; ++i) v[i] = static_cast<int>(r[i]);
-}
-// Three 16-column reads of raw 32-bit accumulators (integer MMAs), one wait.
-__device__ __forceinline__ void tmem_ld16x3_wait_b32(uint32_t taddr0, uint32_t taddr1, uint32_t taddr2,
-                                                     int (&v0)[16], int (&v1)[16], int (&v2)[16]) {
-  uint32_t r[48];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-      "%13, %14, %15}, [%48];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, "
-      "%27, %28, %29, %30, %31}, [%49];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, "
-      "%43, %44, %45, %46, %47}, [%50];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : B200MOE_R16(r, 0), B200MOE_R16(r, 16), B200MOE_R16(r, 32)
-      : "r"(taddr0), "r"(taddr1), "r"(taddr2)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    v0[i] = static_cast<int>(r[i]);
-    v1[i] = static_cast<int>(r[16 + i]);
-    v2[i] = static_cast<int>(r[32 + i]);
-  }
-}
+// Two loads (e.g. gate and up accumulators) in flight before the single wait.
 __device__ __forceinline__ void tmem_ld16x2_wait(uint32_t taddr0, uint32_t taddr1, float (&v0)[16],
                                                  float (&v1)[16]) {
   uint32_t r[32];
@@ -404,18 +349,6 @@ __host__ __device__ __forceinline__ uint32_t make_idesc(uint32_t fmt, uint32_t m
   d |= 1u << 4;           // accumulator format fp32
   d |= (fmt & 7u) << 7;   // A format
   d |= (fmt & 7u) << 10;  // B format
-  d |= (n >> 3) << 17;
-  d |= (m >> 4) << 24;
-  return d;
-}
-
-// Integer instruction descriptor (kind::i8): int32 accumulate, A unsigned or signed 8-bit, B
-// unsigned or signed 8-bit, both with the reduction dim contiguous.
-__host__ __device__ __forceinline__ uint32_t make_idesc_i8(bool a_signed, bool b_signed, uint32_t m, uint32_t n) {
-  uint32_t d = 0;
-  d |= 2u << 4;                       // accumulator format s32
-  d |= (a_signed ? 1u : 0u) << 7;     // A format: 0 = u8, 1 = s8
-  d |= (b_signed ? 1u : 0u) << 10;    // B format
   d |= (n >> 3) << 17;
   d |= (m >> 4) << 24;
   return d;

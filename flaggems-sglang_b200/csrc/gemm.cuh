@@ -45,21 +45,14 @@ struct GemmArgs {
   const float* bias;      // optional per-expert bias of this GEMM's output rows: [E, rows] fp32 (mode 0: gate rows then up rows)
   float act_alpha;        // B200MOE_ACT_SWIGLU_OAI: s = g * sigmoid(alpha * g)
   float act_limit;        // B200MOE_ACT_SWIGLU_OAI: clamp gate to <= limit and linear to [-limit, limit]; <= 0: none
-  const void* w_sz;       // int4: per (expert, group of 128 k, weight row) fp16 scale | fp16 (1024 + zero)
-  int w_rows;             // int4: weight rows per expert (2I for mode 0, H for mode 1)
   uint8_t* out_q;         // mode 0 FP8: quantised activations [cap, N]
   float* out_scale;       // mode 0 FP8: [N/128][ld_xscale]
-  // int4 decode path (integer MMAs): activations are three int8 planes per token block
-  // ([block][plane][BT rows][K], rows of one block consecutive) + per (128-k group, row) a
-  // power-of-two scale (x_scale / out_scale, [K/128][ld_xscale]) and the sum of the integers
   // mode 1, optional: instead of adding into the fp32 combine buffer, store each (token, choice)
   // pair's weighted row in the 16-bit type at out_pairs[slot][N] and mark pair_valid[slot]; the
   // output conversion then sums a token's rows.  Plain 16-byte stores instead of fp32 atomics,
   // which bound the tail once M * topk * N is large.  Requires an unsplit reduction.
   void* out_pairs;
   uint8_t* pair_valid;
-  const int* x_sum;       // [K/128][ld_xscale]
-  int* out_sum;           // mode 0: [N/128][ld_xscale]; planes go to out_q with row stride ld_out
   // mode 1 under expert parallelism (FP8 kernels): the output row of a token (fp32 combine buffer)
   // or of a pair (16-bit pair rows) lives on the rank that owns the token.  Output row index r
   // (token, or pair slot, numbered rank-major over all ranks) -> rank r / rows_per_peer, row
@@ -87,7 +80,6 @@ __device__ __forceinline__ void mark_pair_valid(const GemmArgs& a, int slot) {
 }
 
 size_t gemm_smem_bytes(const GemmArgs& a);
-bool gemm_w4_planes_ok(int K, int BT);   // can the integer int4 path take this reduction length / token block?
 void gemm_plan(GemmArgs* a);  // fills stages / acc_stages / tmem_cols / num_nt / kblocks from the rest
 
 int launch_gemm_tc(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
@@ -95,11 +87,18 @@ int launch_gemm_tc(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmA
 void gemm_plan_fp8(GemmArgs* a);
 int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                     cudaStream_t stream);
-// int4 AWQ, token blocks of 16 / 32: exact (q - zero) operands, group scales applied to partial sums
+// int4 AWQ: see gemm_w4.cu.  Token maps: boxes of 16 (i + 1) rows x the 64-k halves of a group;
+// decode blocks use m[0] (their rows, two groups).
+struct W4TokenMaps {
+  CUtensorMap m[12];
+};
+bool gemm_w4_ok(int E);
 void gemm_plan_w4(GemmArgs* a);
-int launch_gemm_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
-                   cudaStream_t stream);
-// 16-bit, more than 64 tokens per expert, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
+// tm_w: packed rows, mode 0 [E][I][2][K/2] in boxes of 64 rows of both halves, mode 1 [E][rows][K/2] in boxes of 128
+// rows; tm_sz: their scale / zero words [E * K/128][2][I] in boxes of 64 of both halves, or [E * K/128][1][rows] in boxes of 128
+int launch_gemm_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4TokenMaps& tm_x, const GemmArgs& a,
+                   int num_sms, cudaStream_t stream);
+// 16-bit, more than 20 tokens per expert, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
 bool gemm_tc2_ok(int E, int num_sms);
 int gemm_tc2_resident_pairs();   // CTA pairs the device kept resident for the last such launch (0: none yet)
 void gemm_plan_tc2(GemmArgs* a);

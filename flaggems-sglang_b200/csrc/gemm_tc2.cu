@@ -44,7 +44,7 @@
 //
 // Every wait is bounded (common.cuh); the cluster barriers at start and end are reached by every
 // thread whatever happened in between.
-#include "gemm_sched.cuh"
+#include "gemm_turn.cuh"
 
 namespace b200moe {
 
@@ -54,21 +54,15 @@ constexpr int kPairThreads = 320;       // TMA producer, MMA issuer, two epilogu
 constexpr int kGran = 32;               // tokens: padding of an expert's rows and step of N
 constexpr int kMaxGran = 8;             // N <= 256
 constexpr int kMaxStages2 = 10;
-constexpr int kTurnTok = 16;            // tokens turned per epilogue step
 
-// Bytes per token in the turning buffer: 64 activations, 128 pair-row values (both 16-bit) or 128 fp32 sums, and
-// a pad that keeps the rows 16-byte aligned and spreads them over the banks.
-__host__ __device__ __forceinline__ int tc2_turn_pitch(int mode, bool pairs) {
-  return mode == 0 ? 160 : (pairs ? 272 : 528);
-}
-// Shared memory: token tables [2 groups][2 tiles][256] (slot, weight), barriers, granule and tile prefixes of the
-// experts, turning buffers [2 groups][2], then the operand ring (1024-byte aligned).
-constexpr size_t kTc2TableBytes = 2 * 2 * 256 * 8 + 512;
+// Shared memory: token tables, barriers, granule and tile prefixes of the experts, turning buffers, then the operand
+// ring (1024-byte aligned).
+constexpr size_t kTc2TableBytes = kTurnTableBytes + 512;
 __host__ __device__ __forceinline__ size_t tc2_turn_offset(int E) {
   return (kTc2TableBytes + 2 * static_cast<size_t>(E + 1) * 4 + 127) & ~static_cast<size_t>(127);
 }
 __host__ __device__ __forceinline__ size_t tc2_fixed_bytes(int E, int mode, bool pairs) {
-  return (tc2_turn_offset(E) + 4 * kTurnTok * static_cast<size_t>(tc2_turn_pitch(mode, pairs)) + 1023) & ~static_cast<size_t>(1023);
+  return (tc2_turn_offset(E) + turn_bytes(mode, pairs) + 1023) & ~static_cast<size_t>(1023);
 }
 // operand bytes of one 64-k stage in one CTA: 128 weight rows and half of up to n tokens
 __host__ __device__ __forceinline__ int tc2_stage_bytes(int n) { return kTileBytes + n / 2 * kStageKBytes; }
@@ -145,82 +139,10 @@ __device__ __forceinline__ void tc_mma2_f16(uint32_t d_tmem, uint64_t adesc, uin
       : "memory");
 }
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-template <typename T>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi);
-template <>
-__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <>
-__device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
-  __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-// Tile of one pair: N tokens of an expert from padded row row0, weight rows from n0, reduction [kb0, kb1).
-struct PairTile {
-  int e, n0, row0, n, kb0, kb1;
-};
-
-// Tile `id` in expert-major, n-tile, reduction split, token tile order.  s_tile[e] = token tiles before
-// expert e, s_gran[e] = granules before it.
-__device__ __forceinline__ PairTile decode_pair(int id, const int* s_tile, const int* s_gran, int E, int num_nt,
-                                                int split, int kblocks, int tile_n) {
-  int lo = 0, hi = E;
-  const int u = num_nt * split;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (s_tile[mid] * u <= id) lo = mid; else hi = mid;
-  }
-  PairTile t;
-  t.e = lo;
-  const int nt_e = s_tile[lo + 1] - s_tile[lo];
-  const int local = id - s_tile[lo] * u;
-  const int tt = local % nt_e;
-  const int rest = local / nt_e;
-  const int s = rest % split;
-  const int g = s_gran[lo + 1] - s_gran[lo];
-  const int g0 = tt * g / nt_e, g1 = (tt + 1) * g / nt_e;
-  t.n0 = (rest / split) * tile_n;
-  t.row0 = (s_gran[lo] + g0) * kGran;
-  t.n = (g1 - g0) * kGran;
-  t.kb0 = static_cast<int>((static_cast<long long>(s) * kblocks) / split);
-  t.kb1 = static_cast<int>((static_cast<long long>(s + 1) * kblocks) / split);
-  return t;
-}
-
 // Cycles of a 64-k stage of a tile with g granules: four MMAs of N / 2 cycles, or the time the stage's
 // operands take from L2 at about 80 bytes per clock and SM, whichever is longer.
 __device__ __forceinline__ float stage_cost(int g) {
   return fmaxf(64.f * g, 200.f + 24.f * g) + 16.f;
-}
-
-// Largest number of granules per tile that this launch should use: the one with the shortest estimated
-// schedule, (sum of the tiles' costs) / pairs + half the longest tile (static round-robin over the pairs
-// ends that much later than a perfect split on average).  Wide tiles re-read the weights least; narrower ones fill the last wave
-// of a launch with few tiles.  Warp w < 6 rates 8 - w; result in every lane of the warp.
-__device__ __forceinline__ float rate_max_granules(int maxg, const int* s_gran, int E, int num_nt, int pairs, int lane) {
-  float sum = 0.f, longest = 0.f;
-  for (int e = lane; e < E; e += 32) {
-    const int g = s_gran[e + 1] - s_gran[e];
-    if (g > 0) {
-      const int t = (g + maxg - 1) / maxg;
-      const int lo = g / t, rem = g - lo * t;
-      sum += (t - rem) * stage_cost(lo) + rem * stage_cost(lo + 1);
-      longest = fmaxf(longest, stage_cost(rem > 0 ? lo + 1 : lo));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    longest = fmaxf(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-  }
-  return sum * num_nt / pairs + 0.5f * longest;
 }
 
 template <int MODE, typename T, bool EXT>
@@ -243,7 +165,6 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   float* s_rate = reinterpret_cast<float*>(tmem_slot + 4);                 // [6]
   int* s_gran = reinterpret_cast<int*>(smem + kTc2TableBytes);             // [E+1]
   int* s_tile = s_gran + (a.E + 1);                                        // [E+1]
-  const int pitch = tc2_turn_pitch(MODE, a.out_pairs != nullptr);
   uint8_t* s_turn = smem + tc2_turn_offset(a.E);                           // [2 groups][2][16 tokens][pitch]
   const size_t fixed = tc2_fixed_bytes(a.E, MODE, a.out_pairs != nullptr);
   uint8_t* ring = smem + fixed;
@@ -282,7 +203,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const int num_nt = a.num_nt;
   const int npairs = static_cast<int>(gridDim.x) >> 1;
   if (warp < 6) {
-    const float r = rate_max_granules(kMaxGran - warp, s_gran, a.E, num_nt, npairs, lane);
+    const float r = rate_max_granules(kMaxGran - warp, s_gran, a.E, num_nt, npairs, lane, stage_cost);
     if (lane == 0) s_rate[warp] = r;
   }
   __syncthreads();
@@ -292,26 +213,8 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       if (s_rate[w] < s_rate[best]) best = w;
     const int cap = a.BT / kGran;     // a caller that fixes the token block bounds the tile with it
     const int maxg = min(kMaxGran - best, cap);
-    int run = 0, widest = 1;
-    for (int e0 = 0; e0 < a.E; e0 += 32) {
-      const int e = e0 + lane;
-      const int g = e < a.E ? s_gran[e + 1] - s_gran[e] : 0;
-      const int t = (g + maxg - 1) / maxg;
-      if (t > 0) widest = max(widest, (g + t - 1) / t);
-      int v = t;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-      }
-      if (e < a.E) s_tile[e + 1] = run + v;
-      run += __shfl_sync(0xffffffffu, v, 31);
-    }
-    widest = __reduce_max_sync(0xffffffffu, widest);
-    if (lane == 0) {
-      s_tile[0] = 0;
-      *s_nmax = widest * kGran;
-    }
+    const int widest = plan_row_tiles(maxg, s_gran, a.E, s_tile, lane);
+    if (lane == 0) *s_nmax = widest * kGran;
   }
   tc_fence_before();
   __syncthreads();
@@ -325,7 +228,8 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const int split = (MODE == 1 && !(a.flags & B200MOE_FLAG_NO_SPLIT_K)) ? pick_split(tiles, a.kblocks, npairs, a.max_split) : 1;
   const int total = tiles * split;
   const int pair_id = static_cast<int>(blockIdx.x) >> 1;
-  auto tile_at = [&](int id) { return decode_pair(id, s_tile, s_gran, a.E, num_nt, split, a.kblocks, kTileN); };
+  const RowTiles grid = {s_tile, s_gran, a.E, num_nt, split, a.kblocks, kTileN, kGran};
+  auto tile_at = [&](int id) { return row_tile_at(id, grid); };
 
   if (warp == 0 && elect_one()) {
     // =============================== TMA producer (every CTA, its own operands) ===================
@@ -336,7 +240,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     constexpr int kKElems = kStageKBytes / static_cast<int>(sizeof(T));
     constexpr int kRowsPerCta = MODE == 0 ? 64 : 128;
     for (int tile = pair_id; ok && tile < total; tile += npairs) {
-      const PairTile t = tile_at(tile);
+      const RowTile t = tile_at(tile);
       const int wrow = t.n0 + kRowsPerCta * static_cast<int>(rank);
       const int half = t.n >> 1;
       const int xrow = t.row0 + static_cast<int>(rank) * half;
@@ -389,7 +293,7 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     uint32_t phase = 0, acc_phase = 0;
     bool ok = true;
     for (int tile = pair_id; ok && tile < total; tile += npairs) {
-      const PairTile t = tile_at(tile);
+      const RowTile t = tile_at(tile);
       const uint32_t idesc = make_idesc(fmt, 256u, static_cast<uint32_t>(t.n));
       if (!mbar_wait(smem_u32(&bar_tempty[acc]), acc_phase ^ 1, abort_flag, DEV_TIMEOUT_MMA)) break;
       tc_fence_after();
@@ -420,127 +324,22 @@ moe_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
   } else if (warp >= 2) {
     // =============================== epilogue (every CTA, its own 128 weight rows) ================
-    const int grp = (warp - 2) >> 2;              // steps of 16 tokens alternate between the two groups
-    const int quad = warp & 3;                    // TMEM lane quadrant this warp may read
-    const int gt = ((warp - 2) & 3) * 32 + lane;  // thread inside the group
-    const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0;
-    const bool mimic = (a.flags & B200MOE_FLAG_MIMIC_ROUNDING) != 0;
-    const bool round_pair = mimic && split == 1;
-    const ActParams ap = act_params(a);
-    const bool has_bias = EXT && a.bias != nullptr;
-    const uint32_t meet = smem_u32(&bar_meet[grp]);
-    uint32_t meet_phase = 0;
-    int acc = 0, par = 0, step_no = 0;
+    TurnEpilogue<MODE, T, EXT> ep(a, s_turn, s_slot, s_gam, bar_meet, abort_flag, warp - 2, warp, lane,
+                                  (MODE == 0 ? 64 : 128) * static_cast<int>(rank), split);
+    int acc = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
-    for (int tile = pair_id; ok && tile < total; tile += npairs, par ^= 1) {
-      const PairTile t = tile_at(tile);
-      int* slots = s_slot + (grp * 2 + par) * 256;
-      float* gams = s_gam + (grp * 2 + par) * 256;
-      for (int i = gt; (MODE == 1 || w_on_input) && i < t.n; i += 128) {
-        const int slot = a.sorted_ids[t.row0 + i];
-        const bool valid = slot >= 0 && slot < a.P;
-        slots[i] = valid ? slot : -1;
-        gams[i] = valid ? a.row_gamma[t.row0 + i] : 0.f;
-      }
-      // the tables are read before a step's meeting: they need one of their own
-      if (MODE == 1 || w_on_input) {
-        if (!warps_meet(meet, meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
-      }
+    for (int tile = pair_id; tile < total; tile += npairs) {
+      const RowTile t = tile_at(tile);
+      if (!ep.load_tables(t)) break;
       if (!mbar_wait(smem_u32(&bar_tfull[acc]), acc_phase, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(acc * 256);
-      const int steps = t.n / kTurnTok;
-      // mode 0: output column of this lane pair; mode 1: of this lane
-      const int lcol = (MODE == 0) ? 64 * static_cast<int>(rank) + quad * 16 + (lane >> 1)
-                                   : 128 * static_cast<int>(rank) + quad * 32 + lane;
-      float bias0 = 0.f, bias1 = 0.f;
-      if (has_bias && t.n0 + lcol < a.N) {
-        if (MODE == 0) {
-          bias0 = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + t.n0 + lcol);
-          bias1 = __ldg(a.bias + static_cast<size_t>(t.e) * 2 * a.N + a.N + t.n0 + lcol);
-        } else if (t.kb0 == 0) {      // the first reduction split carries the bias
-          bias0 = __ldg(a.bias + static_cast<size_t>(t.e) * a.N + t.n0 + lcol);
-        }
-      }
-      for (int st = grp; st < steps; st += 2, ++step_no) {
-        float v[16];
-        tmem_ld16_wait(taddr + st * kTurnTok, v);
-        if (st + 2 >= steps) {        // this warp has read its last part of the accumulator
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_tempty[acc]), 0));
-        }
-        uint8_t* buf = s_turn + static_cast<size_t>((grp * 2 + (step_no & 1)) * kTurnTok) * pitch;
-        if (MODE == 0) {
-          // even lanes hold gate values and finish the even tokens, odd lanes hold up values and finish the odd ones
-          const bool odd = (lane & 1) != 0;
-          float g[8], u[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
-            g[j] = (odd ? other : v[2 * j]) + bias0;
-            u[j] = (odd ? v[2 * j + 1] : other) + bias1;
-          }
-          act_mul_array<T, EXT>(g, u, w_on_input, mimic, ap,
-                                [&](int j) { return gams[st * kTurnTok + 2 * j + (odd ? 1 : 0)]; });
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<T*>(buf + (2 * j + (odd ? 1 : 0)) * pitch + (quad * 16 + (lane >> 1)) * 2) = from_f32<T>(g[j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float scale = w_on_input ? 1.0f : gams[st * kTurnTok + j];
-            v[j] = (v[j] + bias0) * scale;
-          }
-          if (a.out_pairs != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              *reinterpret_cast<T*>(buf + j * pitch + (quad * 32 + lane) * 2) = from_f32<T>(v[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              *reinterpret_cast<float*>(buf + j * pitch + (quad * 32 + lane) * 4) =
-                  round_pair ? to_f32<T>(from_f32<T>(v[j])) : v[j];
-          }
-        }
-        // one meeting per step: a warp that writes this buffer again, two steps on, has met the others
-        // once more in between, after they had finished reading it
-        if (!warps_meet(meet, meet_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) {
-          ok = false;
-          break;
-        }
-        if (MODE == 0) {
-          const int tk = gt >> 3, ch = gt & 7;        // 16 tokens x 8 chunks of 16 bytes
-          const int col = t.n0 + 64 * static_cast<int>(rank) + ch * 8;
-          if (col < a.N)
-            *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out) +
-                                      static_cast<size_t>(t.row0 + st * kTurnTok + tk) * a.ld_out + col) =
-                *reinterpret_cast<const uint4*>(buf + tk * pitch + ch * 16);
-        } else if (a.out_pairs != nullptr) {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int tk = q * 8 + (gt >> 4), ch = gt & 15;     // 16 tokens x 16 chunks
-            const int slot = slots[st * kTurnTok + tk];
-            const int col = t.n0 + 128 * static_cast<int>(rank) + ch * 8;
-            if (slot >= 0 && col < a.N) {
-              *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out_pairs) + static_cast<size_t>(slot) * a.N + col) =
-                  *reinterpret_cast<const uint4*>(buf + tk * pitch + ch * 16);
-              if (col == 0) a.pair_valid[slot] = 1;
-            }
-          }
-        } else {
-          const int col = t.n0 + 128 * static_cast<int>(rank) + lane * 4;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int tk = q * 4 + (gt >> 5);
-            const int slot = slots[st * kTurnTok + tk];
-            if (slot < 0 || col >= a.N) continue;
-            const float4 y = *reinterpret_cast<const float4*>(buf + tk * pitch + lane * 16);
-            red_add_v4(reinterpret_cast<float*>(a.out) + static_cast<size_t>(slot / a.topk) * a.ld_out + col, y.x, y.y, y.z, y.w);
-          }
-        }
-      }
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ep.quad * 32) << 16) + static_cast<uint32_t>(acc * 256);
+      if (!ep.run(t, taddr, [&] {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_tempty[acc]), 0));
+          }))
+        break;
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1;

@@ -432,8 +432,7 @@ struct StagedW4 {
   int* vsum;         // [rows][K / 32] sum of the integers of every 32-k segment
 };
 
-// fp16 rows -> planes, scales and segment sums; one warp per (row, group), the arithmetic of
-// group_split_i8_kernel (prep.cu).  fold[row] multiplies the stored scale (nullptr: 1).
+// fp16 rows -> planes, scales and segment sums; one warp per (row, group).  fold[row] multiplies the stored scale (nullptr: 1).
 __device__ __forceinline__ void stage_w4(const __half* src, int rows, int K, const StagedW4& st, const float* fold,
                                          int nthreads) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

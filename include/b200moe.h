@@ -58,7 +58,7 @@ extern "C" {
 #define B200MOE_FLAG_NO_SPLIT_K 16      /* keep GEMM-2's reduction in one piece                */
 #define B200MOE_FLAG_NO_GRID_BALANCE 32 /* tuning aid: every CTA takes tiles round-robin       */
 #define B200MOE_FLAG_NO_PDL 64          /* launch every kernel fully serialised                */
-#define B200MOE_FLAG_W4_SMEM_OPERANDS 128 /* int4: always stage fp16 operands in shared memory (tuning aid) */
+#define B200MOE_FLAG_W4_SMEM_OPERANDS 128 /* int4: grouped GEMMs at every size, none of the small-batch kernels (tuning aid) */
 #define B200MOE_FLAG_X_FP8 1024         /* FP8 weights only: x is already e4m3 [M, H], quantised per
                                            1 x 128 group with scales quant->x_scale [M, H/128] (what
                                            b200moe_per_token_group_quant_fp8 writes); cfg->dtype still
