@@ -4,7 +4,7 @@
 
 namespace b200moe {
 
-// xs[r] = x[sorted_ids[r] / topk] for r < meta[1]; padding rows zero-filled.  Also clears
+// xs[r] = x[sorted_ids[r] / topk] for r < meta[1]; padding rows are left alone.  Also clears
 // `zero_bytes` bytes at `zero` (the fp32 combine buffer) in the same launch.  With sc_src
 // ([tokens][G] group scales of already quantised rows) the scales follow their rows into the
 // group-major table sc_dst [G][ld].  `wait` (expert parallelism): every CTA first waits for the
