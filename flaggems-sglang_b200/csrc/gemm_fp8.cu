@@ -377,15 +377,15 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 // cycles against 512 for the slice's MMAs, and the tail (5000 cycles per tile) that nothing overlaps: the
 // accumulators fill the registers and the two partial buffers all of tensor memory.  Kept off that
 // path: the tile's coordinates (decoded by the table warp), the activation scales (a ring filled per slice, which also
-// frees the room of a fourth stage), warp meetings around the staged stores (each warp transposes its own
-// rows).  256 experts, zipf-skewed routing: 4096 tokens 3367 -> 3140 us, 512 tokens 1093 -> 998 us.
+// frees the room of a fourth stage).  A warp whose 32 rows are all padding (three of four in the block of a cold expert)
+// keeps in step with the others and promotes nothing, which leaves the board's power to the rest.  256 experts,
+// zipf-skewed routing, 4096 tokens: 3367 -> 3140 us with the first two, 3205 -> 3058 (another board) with direct stores and
+// idle warps; 512 tokens 1093 -> 998, 1045 -> 984.
 // Tried and slower: sixteen promotion warps, 32-column reads, scalar FMAs, partial buffers released by halves, hot and
 // cold experts' tiles interleaved.
 // warps 0-3: TMA, MMA, tables, idle; warps 4-11: promotion.  Launched with 168 registers a thread, the
 // first four warps keep 48 and the promotion warps take 224: 4 * 48 + 8 * 224 <= 12 * 168.
 constexpr int kThreadsFp8TokM = 12 * 32;
-constexpr int kPairStagePitch = 80;                               // 32 columns of a 16-bit pair row + 16 bytes
-constexpr int kPairStageBytes = 2 * 128 * kPairStagePitch;         // two groups x 128 rows
 constexpr int kXsSlots = 8;                                       // ring of activation scales, one slot per slice
 
 #ifdef B200MOE_STALL_STATS
@@ -394,6 +394,13 @@ __device__ unsigned long long g_stall_fp8[16];
 #else
 #define STALL_ADD8(slot, v) ((void)0)
 #endif
+
+// 32 bytes of one thread, a whole sector.
+__device__ __forceinline__ void st_global_v8(uint8_t* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreadsFp8TokM, 1)
@@ -413,9 +420,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   uint8_t* ctrl_base = smem + static_cast<size_t>(stages) * STAGE_BYTES;
   float* s_xs = reinterpret_cast<float*>(ctrl_base);                    // [kXsSlots][128] activation scales
   float* s_ws = s_xs + kXsSlots * BT;                                   // [2][2][KBS] weight scales
-  // mode 1 with rows stored per pair: staging for coalesced stores, [2 groups][128 rows][80 bytes]
-  uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_ws + 2 * 2 * KBS);
-  uint64_t* bar_full = reinterpret_cast<uint64_t*>(s_stage + ((MODE == 1 && a.out_pairs != nullptr) ? kPairStageBytes : 0));
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(s_ws + 2 * 2 * KBS);
   uint64_t* bar_empty = bar_full + stages;
   uint64_t* bar_pfull = bar_empty + stages;
   uint64_t* bar_pempty = bar_pfull + 2;
@@ -628,6 +633,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       const TileCoord t = {ti[0], ti[1], ti[2], ti[3], ti[4]};
       const int orow = s_col_row[buf * 128 + lrow];
       const float gam = s_col_gam[buf * 128 + lrow];
+      const bool idle = !__any_sync(0xffffffffu, orow >= 0);   // 32 padding rows: keep in step, promote and store nothing
 
       // running sums stay packed two to a 64-bit register for the whole reduction
       unsigned long long pA[32], pB[32];
@@ -641,6 +647,10 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         if (!mbar_wait_t(smem_u32(&bar_pfull[pb]), (j >> 1) & 1u, abort_flag, DEV_TIMEOUT_EPILOGUE, w_pfull)) {
           ok = false;
           break;
+        }
+        if (idle) {
+          if (lane == 0) mbar_arrive(smem_u32(&bar_pempty[pb]));
+          continue;
         }
         tc_fence_after();
         const uint32_t xs_slot = j % kXsSlots;
@@ -670,6 +680,12 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       }
       if (!ok) break;
       const long long tail_t0 = clock64();
+      if (idle) {
+        if (MODE == 0 && !warps_meet(smem_u32(bar_meet8), meet8_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
+        continue;
+      }
       float accA[64], accB[64];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
@@ -730,33 +746,24 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                                                        __NV_SATFINITE, __NV_E4M3);
           pk[q] = lo | (hi << 16);
         }
-        uint4* dst = reinterpret_cast<uint4*>(a.out_q + static_cast<size_t>(r) * a.ld_out + t.n0 + 64 * grp);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dst[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+        uint8_t* dst = a.out_q + static_cast<size_t>(r) * a.ld_out + t.n0 + 64 * grp;
+        st_global_v8(dst, pk);
+        st_global_v8(dst + 32, pk + 8);
       } else if (a.out_pairs != nullptr) {
-        // The pair's row, weighted and rounded to the 16-bit type.  A thread owns 128 contiguous
-        // columns of one row; storing them directly would touch 32 rows per warp instruction, so
-        // each warp stages 32 columns of its rows at a time in shared memory (80-byte row pitch)
-        // and writes them out with 16-byte stores that cover eight rows per instruction.
+        // The pair's row, weighted and rounded to the 16-bit type.  A thread owns 128 contiguous columns of one row and
+        // stores them as whole sectors straight from its registers.  (Turning them in shared memory so that a store
+        // covers eight rows made the tail 4700 cycles of a 20000-cycle tile: 4096 tokens 3205 -> 3065 us.)
         const float scale = w_on_input ? 1.0f : gam;
         const bool bf = a.dtype == B200MOE_DTYPE_BF16;
-        uint8_t* stage_w = s_stage + (grp * 4 + quad) * (32 * kPairStagePitch);
-        uint16_t* dst[4];       // this lane stores chunk lane % 4 of rows lane / 4 + 8 it
+        if (orow >= 0) {
+          uint8_t* dst = reinterpret_cast<uint8_t*>(s_col_ptr[buf * 128 + lrow]) + (t.n0 + 128 * grp) * 2;
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          const int brow = buf * 128 + quad * 32 + it * 8 + (lane >> 2);
-          dst[it] = s_col_row[brow] >= 0 ? reinterpret_cast<uint16_t*>(s_col_ptr[brow]) + t.n0 + 128 * grp + (lane & 3) * 8 : nullptr;
-        }
+          for (int q = 0; q < 8; ++q) {
+            const float* src = (q < 4 ? accA : accB) + 16 * (q & 3);
+            uint32_t w[8];
 #pragma unroll
-        for (int round = 0; round < 4; ++round) {
-          const float* src = (round < 2 ? accA : accB) + 32 * (round & 1);
-          __syncwarp();
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t w[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              const float lo = src[8 * q + 2 * b] * scale, hi = src[8 * q + 2 * b + 1] * scale;
+            for (int b = 0; b < 8; ++b) {
+              const float lo = src[2 * b] * scale, hi = src[2 * b + 1] * scale;
               if (bf) {
                 __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
                 w[b] = *reinterpret_cast<uint32_t*>(&v);
@@ -765,15 +772,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                 w[b] = *reinterpret_cast<uint32_t*>(&v);
               }
             }
-            *reinterpret_cast<uint4*>(stage_w + lane * kPairStagePitch + q * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          __syncwarp();
-          if (t.n0 + 128 * grp + 32 * round < a.N) {
-#pragma unroll
-            for (int it = 0; it < 4; ++it)
-              if (dst[it] != nullptr)
-                *reinterpret_cast<uint4*>(dst[it] + 32 * round) =
-                    *reinterpret_cast<const uint4*>(stage_w + (it * 8 + (lane >> 2)) * kPairStagePitch + (lane & 3) * 16);
+            if (t.n0 + 128 * grp < a.N) st_global_v8(dst + 32 * q, w);
           }
         }
         if (orow >= 0 && t.n0 == 0 && grp == 0) mark_pair_valid(a, orow);
@@ -820,7 +819,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 
 size_t fp8_tokm_ctrl_bytes(const GemmArgs& a) {
   return kXsSlots * 128 * 4 + 2 * 2 * static_cast<size_t>(a.kblocks) * 4 +
-         ((a.mode == 1 && a.out_pairs != nullptr) ? kPairStageBytes : 0) + 512 /*barriers, tile words*/ + 2 * 2 * 128 * 4 +
+         512 /*barriers, tile words*/ + 2 * 2 * 128 * 4 +
          (a.mode == 0 ? 2 * 2 * 128 * 4 : 2 * 128 * 8) + static_cast<size_t>(a.E + 1) * 4 + 64;
 }
 
