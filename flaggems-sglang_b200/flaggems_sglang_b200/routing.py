@@ -9,6 +9,7 @@ are accepted as well.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from dataclasses import dataclass, field
 from typing import Optional
@@ -18,6 +19,11 @@ import torch
 from . import _lib
 
 BLOCK_MS = (16, 32, 64, 128)
+
+# The conversion is a dozen microseconds on the device; device guard, stream handle and views are the cheap forms (one
+# token through the operator: 100 -> 80 us of host time).
+_SAME_DEVICE = contextlib.nullcontext()
+_current_device = torch._C._cuda_getDevice
 
 
 @dataclass
@@ -51,7 +57,11 @@ class RoutingData:
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def _on_device(device):
+    return _SAME_DEVICE if _current_device() == device.index else torch.cuda.device(device)
 
 
 def _require_cuda(t: torch.Tensor, name: str) -> None:
@@ -88,7 +98,7 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: i
     emap = None
     if expert_map is not None:
         emap = expert_map.to(device=dev, dtype=torch.int32).contiguous()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = lib.b200moe_align_block_size(
             ids.data_ptr(), int(ids.dtype == torch.int64), n_slots, num_experts, block_size,
             emap.data_ptr() if emap is not None else None, emap.numel() if emap is not None else 0,
@@ -114,28 +124,27 @@ def topk_to_routing(topk_weights: torch.Tensor, topk_ids: torch.Tensor, n_expts_
     w32 = topk_weights.to(torch.float32).contiguous()
     lib = _lib.lib()
     mt = lib.b200moe_routing_max_tiles(p, n_expts_tot)
-    i32 = dict(dtype=torch.int32, device=dev)
-    expt_indx = torch.empty(p, **i32)
-    topk_indx = torch.empty(p, **i32)
-    gate_indx = torch.empty(p, **i32)
+    i32 = torch.int32
+    expt_indx = torch.empty(p, dtype=i32, device=dev)
+    topk_indx = torch.empty(p, dtype=i32, device=dev)
+    gate_indx = torch.empty(p, dtype=i32, device=dev)
     gate_scal = torch.empty(p, dtype=torch.float32, device=dev)
-    hist = torch.empty(n_expts_tot, **i32)
-    offs_raw = torch.empty(n_expts_tot + 1, **i32)
-    offs_pad = torch.empty(4, n_expts_tot + 1, **i32)
-    pid_map = torch.empty(4 * max(mt, 1), **i32)   # four block maps back to back, stride max_tiles
-    with torch.cuda.device(dev):
+    hist = torch.empty(n_expts_tot, dtype=i32, device=dev)
+    offs_raw = torch.empty(n_expts_tot + 1, dtype=i32, device=dev)
+    offs_pad = torch.empty(4, n_expts_tot + 1, dtype=i32, device=dev)
+    pid_map = torch.empty(4, max(mt, 1), dtype=i32, device=dev)   # four block maps back to back, stride max_tiles
+    with _on_device(dev):
         rc = lib.b200moe_routing_from_topk(
             w32.data_ptr(), ids.data_ptr(), int(ids.dtype == torch.int64), m, k, n_expts_tot,
             expt_indx.data_ptr(), topk_indx.data_ptr(), gate_indx.data_ptr(), gate_scal.data_ptr(),
             hist.data_ptr(), offs_raw.data_ptr(), offs_pad.data_ptr(),
             pid_map.data_ptr(), _stream_ptr(dev))
     _lib.check(rc, "topk_to_routing")
-    maps = pid_map[: 4 * mt].view(4, mt)
     expt_data = ExptData(
         hist=hist,
         token_offs_raw=offs_raw,
-        token_offs_pad={bm: offs_pad[i] for i, bm in enumerate(BLOCK_MS)},
-        block_pid_map={bm: maps[i] for i, bm in enumerate(BLOCK_MS)},
+        token_offs_pad=dict(zip(BLOCK_MS, offs_pad.unbind(0))),
+        block_pid_map=dict(zip(BLOCK_MS, (pid_map if mt > 0 else pid_map[:, :0]).unbind(0))),
     )
     gs = gate_scal if topk_weights.dtype == torch.float32 else gate_scal.to(topk_weights.dtype)
     routing = RoutingData(gs, hist, n_expts_tot, k, expt_data)
