@@ -14,6 +14,11 @@
 //                promotion warps.  Weights and activations are then exact up to the fp32 sums.  (The version before
 //                this one multiplied 20-bit integers split into three byte planes: three times the accumulator columns and
 //                activation bytes, and a kernel in front to split them.)
+//                NT = 16 expands nothing: a masked nibble already is the fp16 subnormal q * 2^-24, and eight more MMAs per
+//                group add -zero (times the same 2^-24) against every k.  The schedulers, which all roles
+//                share, then see 7 instructions per eight weights instead of 9, none of them half-precision arithmetic.  2
+//                tokens of the Mixtral-shaped layer 111.8 -> 102.8 us, 4: 164.7 -> 156.7, 16: 222 -> 219, 32: 234 -> 232.
+//                At NT = 32 the extra MMAs are the longer path (64 tokens 269 -> 285).
 //
 // Packed rows and tokens have rings of their own: the packed rows of a group are needed a conversion (about 900 cycles)
 // earlier than its tokens, and at 192 tokens only three stages of tokens fit.  The MMA thread works on units of one (NT =
@@ -24,7 +29,7 @@
 // either of them; two operand stages keep them apart), at decode sizes the hand-over between them (about 650 cycles a
 // group, of which HBM needs 380).  Mixtral-shaped layer (8 experts, top-2), us per call, against 128-token blocks on
 // the M side with the nibbles expanded into shared memory: 64 tokens 269 (368), 256: 374 (511), 600: 560 (921), 2048:
-// 1455 (2037); against the integer kernel: 4 tokens 164 (160), 16: 220 (227), 32: 231 (242).
+// 1455 (2037); against the integer kernel: 2 tokens 103 (123), 4: 157 (160), 16: 219 (227), 32: 230 (242).
 //
 // Warps: 0 packed rows, 1 MMA, 2 tokens, from 4 on the conversion (two or three sets of four warps), then the epilogue or
 // promotion (one or two groups of four).
@@ -50,6 +55,10 @@ struct W4Geo {
   static constexpr int kPacked = NT > 0 ? 8 : 4;
   static constexpr int kWords = NT > 0 ? 64 : 16;
   static constexpr int kPartials = NT == 16 ? 4 : 2;      // units (NT = 0: tiles) whose accumulators are in flight
+  // NT = 16: the nibbles go in as they are and the zero points as an operand of their own (8 columns a group)
+  static constexpr bool kZeroMma = NT == 16;
+  static constexpr int kSlots = NT == 16 ? 2 : 3;         // NT > 0: units whose operands are in flight
+  static constexpr int kSlotCols = kGroups * (kZeroMma ? 72 : 64);   // tensor-memory columns of a unit's operands
   // Conversion sets: at decode a group's conversion takes one set about 1000 cycles, most of them latency, and HBM
   // delivers a group every 380.  One promotion group holds all 16 tokens of a block.
   static constexpr int kSets = NT > 0 ? 3 : 2;
@@ -75,6 +84,9 @@ __host__ __device__ __forceinline__ int w4_token_bytes(int n, int groups) { retu
 // Cycles per group of a tile with g granules: eight MMAs of N / 2 cycles, or the conversion.
 __device__ __forceinline__ float w4_cost(int g) { return fmaxf(64.f * g, 320.f) + 30.f; }
 
+__device__ __forceinline__ void tmem_st8_same(uint32_t taddr, uint32_t v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -209,7 +221,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   // tensor memory: accumulators first, then the operand stages
   const int acc_cols = NT > 0 ? GP * NT : nmax;
   const uint32_t a_col0 = static_cast<uint32_t>(G::kPartials * acc_cols);
-  const int slots_a = NT > 0 ? 3 : min(4, (512 - 2 * nmax) / 64);
+  const int slots_a = NT > 0 ? G::kSlots : min(4, (512 - 2 * nmax) / 64);
   const int first = blockIdx.x, stride = gridDim.x;
   // units of this CTA over the whole launch
   int units = 0;
@@ -289,7 +301,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           return false;
         tc_fence_after();
         const uint32_t idesc = make_idesc(0u, kTileRows, static_cast<uint32_t>(n));
-        const uint32_t a0 = tmem_base + a_col0 + static_cast<uint32_t>(slot) * (64u * GP);
+        const uint32_t a0 = tmem_base + a_col0 + static_cast<uint32_t>(slot) * G::kSlotCols;
         const uint64_t dx = smem_desc_k_sw128(smem_u32(tokens + static_cast<size_t>(stage) * token_bytes));
         const uint64_t atom = static_cast<uint64_t>(n * 128) >> 4;
 #pragma unroll
@@ -299,6 +311,11 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           for (int k = 0; k < 8; ++k)
             tc_mma_f16_ts(dg, a0 + 64u * g + 8 * k, dx + (2 * g + (k >> 2)) * atom + 2 * (k & 3), idesc,
                           (!fresh || k > 0) ? 1u : 0u);
+          if (G::kZeroMma) {       // the zero points: the same 16 columns of -zero against every 16 k of the tokens
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              tc_mma_f16_ts(dg, a0 + 64u * GP + 8u * g, dx + (2 * g + (k >> 2)) * atom + 2 * (k & 3), idesc, 1u);
+          }
         }
         tc_commit(smem_u32(&bar_done[u % kDone]));
         ++u;
@@ -357,7 +374,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const __half2 zp = __half2half2(__ushort_as_half(static_cast<unsigned short>(szv >> 16)));
       const __half2 mz = __hsub2(__float2half2_rn(960.f), zp);       // -(64 + zero)
       const uint32_t dst = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + a_col0 +
-                           static_cast<uint32_t>(u % slots_a) * (64u * GP) + static_cast<uint32_t>(g % GP) * 64u;
+                           static_cast<uint32_t>(u % slots_a) * G::kSlotCols + static_cast<uint32_t>(g % GP) * 64u;
       // As much as the registers hold is converted before the wait for a free operand stage: with two stages (192
       // tokens) the time from there to the MMA would otherwise add to every second unit.
       constexpr int kBefore = NT == 0 ? 2 : 1;
@@ -367,7 +384,14 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         for (int c = 0; c < 2; ++c) {
           const uint32_t w[4] = {v[2 * b + c].x, v[2 * b + c].y, v[2 * b + c].z, v[2 * b + c].w};
 #pragma unroll
-          for (int q = 0; q < 4; ++q) expand8<NT == 0>(w[q], zp, mz, sc, o[b] + 16 * c + 4 * q);
+          for (int q = 0; q < 4; ++q) {
+            if (!G::kZeroMma) {
+              expand8<NT == 0>(w[q], zp, mz, sc, o[b] + 16 * c + 4 * q);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) o[b][16 * c + 4 * q + i] = (w[q] >> (4 * i)) & 0x000F000Fu;
+            }
+          }
         }
       };
 #pragma unroll
@@ -379,6 +403,12 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       tmem_st32(dst, o[0]);
       if (kBefore == 1) convert(1);
       tmem_st32(dst + 32, o[1]);
+      if (G::kZeroMma) {
+        const uint32_t z = 0x8000u | ((szv >> 16) & 0x3FFu);       // -zero as a subnormal, like the nibbles
+        tmem_st8_same(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + a_col0 +
+                          static_cast<uint32_t>(u % slots_a) * G::kSlotCols + 64u * GP + static_cast<uint32_t>(g % GP) * 8u,
+                      z | (z << 16));
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -453,8 +483,9 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar_tempty[acc]));
-        const float s0 = __half2float(__ushort_as_half(static_cast<unsigned short>(sz0 & 0xFFFFu)));
-        const float s1 = __half2float(__ushort_as_half(static_cast<unsigned short>(sz1 & 0xFFFFu)));
+        constexpr float kUnit = G::kZeroMma ? 16777216.f : 1.f;     // the operands are integers times 2^-24
+        const float s0 = kUnit * __half2float(__ushort_as_half(static_cast<unsigned short>(sz0 & 0xFFFFu)));
+        const float s1 = kUnit * __half2float(__ushort_as_half(static_cast<unsigned short>(sz1 & 0xFFFFu)));
 #pragma unroll
         for (int i = 0; i < HT; ++i) sum[i] = fmaf(s1, w[i], fmaf(s0, v[i], sum[i]));
         if (++acc == G::kPartials) acc = 0;
