@@ -7,13 +7,17 @@ namespace b200moe {
 
 namespace {
 
-// One thread per 16-byte chunk of a padded row (grid-stride), so that a handful of rows at
-// decode sizes still spreads over many threads.  Padding rows are left alone, whatever they hold: every GEMM keeps a
+// A warp copies 2 KiB of a row at a time: one row id, then four 16-byte loads per lane, then the stores.  What bounds it is
+// the write to HBM at prefill sizes and two memory latencies at decode; with a row id and a 64-bit division per
+// 16-byte chunk it was bound by its instructions (32768 rows of 7168 bytes: 118 -> 80 us; decode graph of the 128-expert layer 182.0 -> 179.4).
+// Padding rows are left alone, whatever they hold: every GEMM keeps a
 // row's results to itself and none of a padding row's is ever stored where it is read.  (Zeroing them was three
 // quarters of the writes of a 64-token call on 256 experts; quantising them, likewise: 439 -> 431 us for that call.)
 // The same launch clears the fp32 combine buffer (`zero`, `zero_chunks`).
 // With sc_src: the rows are already quantised (one byte per element) and each has G group scales
 // [tokens][G]; they are re-laid group-major for the GEMMs, sc_dst [G][ld].
+constexpr int kGatherSeg = 128;      // 16-byte chunks per warp and step
+
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const int* __restrict__ sorted_ids,
                    const int* __restrict__ meta, int P, int topk, int chunks_per_row, int cap,
@@ -23,48 +27,39 @@ gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const in
   griddep_launch_dependents();
   wait_for_peers(fw);     // expert parallelism: the rows come from the peers
   const int rows = min(meta[1], cap);
-  const long long n_copy = static_cast<long long>(rows) * chunks_per_row;
-  const long long total = n_copy + zero_chunks;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  const int threads = gridDim.x * blockDim.x;
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x;
   if (sc_src != nullptr) {
-    const long long n_sc = static_cast<long long>(rows) * G;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_sc; i += stride) {
-      const int g = static_cast<int>(i / rows);
-      const int r = static_cast<int>(i - static_cast<long long>(g) * rows);
+    // lanes along the rows: a group's scales of 32 rows are one store
+    const int blocks = (rows + 31) >> 5;
+    for (int u = thread >> 5; u < blocks * G; u += threads >> 5) {
+      const int g = u / blocks;
+      const int r = ((u - g * blocks) << 5) + (thread & 31);
+      if (r >= rows) continue;
       const int slot = sorted_ids[r];
       if (slot >= 0 && slot < P)
         sc_dst[static_cast<size_t>(g) * ld + r] = __ldg(sc_src + static_cast<size_t>(slot / topk) * G + g);
     }
   }
-  // four chunks per thread and trip: first the four row ids, then the four loads, then the stores
-  for (long long i0 = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
-    int slot[4];
-    int col[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + u * stride;
-      slot[u] = -1;
-      col[u] = 0;
-      if (i < n_copy) {
-        const int r = static_cast<int>(i / chunks_per_row);
-        col[u] = static_cast<int>(i - static_cast<long long>(r) * chunks_per_row);
-        slot[u] = sorted_ids[r];
-      }
-    }
+  const int lane = thread & 31;
+  const int segs = (chunks_per_row + kGatherSeg - 1) / kGatherSeg;
+  const int units = rows * segs;       // (2 KiB each, or a shorter row of at most 2^25: far below 2^31)
+  for (int u = thread >> 5; u < units; u += threads >> 5) {
+    const int r = u / segs;
+    const int slot = sorted_ids[r];
+    if (slot < 0 || slot >= P) continue;
+    const int c0 = (u - r * segs) * kGatherSeg + lane;
+    const uint4* src = x + static_cast<size_t>(slot / topk) * chunks_per_row;
+    uint4* dst = xs + static_cast<size_t>(r) * chunks_per_row;
     uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      v[u] = make_uint4(0, 0, 0, 0);
-      if (slot[u] >= 0 && slot[u] < P) v[u] = __ldg(x + static_cast<size_t>(slot[u] / topk) * chunks_per_row + col[u]);
-    }
+    for (int q = 0; q < 4; ++q)
+      if (c0 + 32 * q < chunks_per_row) v[q] = __ldg(src + c0 + 32 * q);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + u * stride;
-      if (i < n_copy) {
-        if (slot[u] >= 0 && slot[u] < P) xs[i] = v[u];
-      } else if (i < total) zero[i - n_copy] = make_uint4(0, 0, 0, 0);
-    }
+    for (int q = 0; q < 4; ++q)
+      if (c0 + 32 * q < chunks_per_row) dst[c0 + 32 * q] = v[q];
   }
+  for (long long i = thread; i < zero_chunks; i += threads) zero[i] = make_uint4(0, 0, 0, 0);
 }
 
 template <typename T>
@@ -237,8 +232,9 @@ int launch_gather_rows(const void* x, void* xs, const int* sorted_ids, const int
   FlagWait fw = {};
   if (wait != nullptr) fw = *wait;
   if (row_bytes % 16 != 0 || zero_bytes % 16 != 0) return B200MOE_ERR_UNSUPPORTED;
-  const long long work = static_cast<long long>(cap) * (row_bytes / 16) + static_cast<long long>(zero_bytes / 16);
-  long long ctas = (work + 255) / 256;
+  const int segs = (row_bytes / 16 + kGatherSeg - 1) / kGatherSeg;
+  const long long copy_warps = static_cast<long long>(cap) * segs, zero_threads = static_cast<long long>(zero_bytes / 16);
+  long long ctas = (copy_warps * 32 > zero_threads ? copy_warps * 32 + 255 : zero_threads + 255) / 256;
   if (ctas > static_cast<long long>(num_sms) * 8) ctas = static_cast<long long>(num_sms) * 8;
   if (ctas < 1) ctas = 1;
   note_launch("gather_rows_kernel");
