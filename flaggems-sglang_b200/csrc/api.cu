@@ -197,12 +197,14 @@ int pick_bt(const b200moe_cfg* c) {
     if (avg < 8) return 32;
     return 128;  // tokens-on-M kernels
   }
-  if (avg <= 10) return 16;
-  if (avg <= 20) return 32;
-  // 16-bit weights: CTA pairs from here on (they pad to 32 rows and take whatever tiles an expert's rows give).
-  // At 25 tokens per expert they are 2 % (8 experts) to 7 % (128 experts) faster than 64-token blocks, at 10 to
-  // 13 tokens 4 % slower than 32-token ones.
-  if (avg <= 40 && c->wmode == B200MOE_W_INT4_AWQ) return 64;
+  // 16-bit and int4: the smaller block until too many experts need a second one.  16 against 32 tokens per block cross at
+  // an average of 13 for layers of 8, 64 and 128 experts (us, 16 / 32: 128 experts, average 12.6: 212 / 217, 15: 220 / 218;
+  // int4, 12: 240 / 265, 14: 272 / 267).
+  if (avg <= 13) return 16;
+  // 32-token blocks against what follows.  16-bit weights, CTA pairs (they pad to 32 rows and take whatever tiles an expert's
+  // rows give): average 20, 128 experts: 215 / 225, 24: 226 / 233, 64 experts, 24: 264 / 272, 8 experts, 24: 454 / 456,
+  // 32: 475 / 449.  int4, variable tiles: average 25: 284 / 317, 27.5: 322 / 321, 30: 360 / 327.
+  if (avg <= (c->wmode == B200MOE_W_INT4_AWQ ? 27 : 25)) return 32;
   return 128;
 }
 
