@@ -98,7 +98,7 @@ void gemm_plan_w4(GemmArgs* a);
 // rows; tm_sz: their scale / zero words [E * K/128][2][I] in boxes of 64 of both halves, or [E * K/128][1][rows] in boxes of 128
 int launch_gemm_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4TokenMaps& tm_x, const GemmArgs& a,
                    int num_sms, cudaStream_t stream);
-// 16-bit, more than 20 tokens per expert, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
+// 16-bit, more than 25 tokens per expert, on CTA pairs (tcgen05.mma.cta_group::2): see gemm_tc2.cu
 bool gemm_tc2_ok(int E, int num_sms);
 int gemm_tc2_resident_pairs();   // CTA pairs the device kept resident for the last such launch (0: none yet)
 void gemm_plan_tc2(GemmArgs* a);

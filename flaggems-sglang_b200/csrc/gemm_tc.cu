@@ -12,7 +12,7 @@
 // mode 1 (down):    one 128-row tile; the reduction may be split over CTAs; the epilogue
 //   multiplies by the routing weight and adds into the fp32 combine buffer with
 //   red.global.add.f32 (which also merges the top-k experts of a token).
-// 16-bit weights run here up to 20 tokens per expert; above that gemm_tc2.cu takes over.
+// 16-bit weights run here up to 25 tokens per expert; above that gemm_tc2.cu takes over.
 //
 // Every wait is bounded; on a time-out the CTA raises an abort flag, all roles leave their
 // loops, the status word is set, TMEM is freed and the kernel returns.
