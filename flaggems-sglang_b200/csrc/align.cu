@@ -388,6 +388,22 @@ int pick_warps(int E) {
 // CTAs of the cluster: one while a CTA's 32 warps hold a few rounds of slots at most
 int pick_ctas(int P) { return P < 1024 ? 1 : 8; }
 
+// Experts a grouping launch takes; pick_warps keeps its tables below kMaxGroupSmem up to there.
+constexpr int kMaxGroupExperts = 3061;
+constexpr size_t kMaxGroupSmem = 96 * 1024;
+
+// Shared memory of a grouping launch; above 48 KiB (from 613 experts on, depending on the warps that count) the
+// kernel has to be told.  Always the same limit: two threads may launch with different sizes.
+template <typename Kernel>
+int group_smem_for(Kernel* kernel, int nwarps, int E, size_t* bytes) {
+  *bytes = group_smem_bytes(nwarps, E);
+  if (E > kMaxGroupExperts || *bytes > kMaxGroupSmem) return B200MOE_ERR_TOO_LARGE;
+  if (*bytes > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(kMaxGroupSmem)) != cudaSuccess)
+    return B200MOE_ERR_CUDA;
+  return B200MOE_OK;
+}
+
 }  // namespace
 
 int align_capacity(int n_slots, int n_experts, int block) {
@@ -413,8 +429,8 @@ int launch_align_block(const void* ids, int is64, const int* map, int map_len, c
                        float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl, const FlagWait* wait, bool one_cta) {
   if (P < 0 || E <= 0 || block <= 0 || cap < 0) return B200MOE_ERR_BAD_ARG;
   const int nw = pick_warps(E);
-  const size_t smem = group_smem_bytes(nw, E);
-  if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
+  size_t smem;
+  if (const int rc = group_smem_for(align_block_kernel, nw, E, &smem)) return rc;
   note_launch("align_block_kernel");
   FlagWait fw = {};
   if (wait != nullptr) fw = *wait;
@@ -446,8 +462,8 @@ int launch_routing_from_topk(const float* weights, const void* ids, int is64, in
                              cudaStream_t stream) {
   if (M < 0 || k <= 0 || E <= 0) return B200MOE_ERR_BAD_ARG;
   const int nw = pick_warps(E);
-  const size_t smem = group_smem_bytes(nw, E);
-  if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
+  size_t smem;
+  if (const int rc = group_smem_for(routing_from_topk_kernel, nw, E, &smem)) return rc;
   const int mt = routing_max_tiles(M * k, E);
   note_launch("routing_from_topk_kernel");
   const int ctas = pick_ctas(M * k);

@@ -147,7 +147,8 @@ size_t b200moe_workspace_bytes(const b200moe_cfg *cfg);
  *   num_tokens_post_padded[1]
  * cap = b200moe_align_capacity(n_slots, n_experts, block).  expert_map (may be
  * NULL; expert_map_len entries) maps global ids to local experts, negative = not
- * local (slot dropped); ids outside [0, expert_map_len) are dropped too.
+ * local (slot dropped); ids outside [0, expert_map_len) are dropped too.  At most
+ * 3061 experts here and in b200moe_routing_from_topk (B200MOE_ERR_TOO_LARGE beyond).
  */
 int b200moe_align_capacity(int n_slots, int n_experts, int block);
 int b200moe_align_block_size(const void *topk_ids, int ids_are_i64, int n_slots,

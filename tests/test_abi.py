@@ -53,6 +53,21 @@ def test_argument_errors(built_lib):
     assert built_lib.b200moe_status_string(_lib.ERR_WORKSPACE).decode().startswith("workspace")
 
 
+def test_alignment_takes_every_expert_count(built_lib):
+    """No number of experts up to the documented limit is refused for want of shared memory.  Without a GPU an accepted
+    call ends at its launch, with the CUDA error, before anything is read or written."""
+    import torch
+    from flaggems_sglang_b200 import _lib
+    if torch.cuda.is_available():
+        pytest.skip("would launch on host memory")
+    buf = (C.c_int32 * 8)()
+    p = C.addressof(buf)
+    for e in (*range(1, 3062), 3062, 5000):
+        want = _lib.ERR_CUDA if e <= 3061 else _lib.ERR_TOO_LARGE
+        assert built_lib.b200moe_align_block_size(p, 0, 2, e, 16, None, 0, p, p, p, None) == want, e
+        assert built_lib.b200moe_routing_from_topk(p, p, 0, 1, 2, e, p, p, p, p, p, p, p, p, None) == want, e
+
+
 def test_matrix_vector_path_selection(built_lib):
     """Which problems the forward calls run on the two matrix-vector kernels (host arithmetic only)."""
     from flaggems_sglang_b200 import _lib

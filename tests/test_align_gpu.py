@@ -23,6 +23,7 @@ def _rand_ids(m, k, e, seed, dtype=torch.int32):
     (1, 2, 8, 16), (7, 2, 8, 4), (33, 4, 16, 16), (64, 2, 8, 64), (17, 8, 64, 16), (1024, 8, 64, 128),
     (4096, 2, 8, 256), (256, 8, 128, 16), (4096, 8, 256, 128), (5, 1, 3, 128), (3, 2, 1000, 16),
     (2, 8, 128, 64), (0, 2, 8, 16),
+    (40, 8, 640, 16), (1500, 8, 1024, 32), (33, 4, 1200, 16), (2000, 2, 2300, 16), (600, 2, 3061, 16),
 ])
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 def test_align_block_size_bit_exact(cuda_device, m, k, e, bs, dtype):
@@ -82,7 +83,8 @@ def test_routing_from_topk_matches_reference_golden(cuda_device, name):
         np.testing.assert_array_equal(rd.expt_data.block_pid_map[bm].cpu().numpy(), g[f"block_pid_map_{bm}"])
 
 
-@pytest.mark.parametrize("m,k,e", [(4096, 8, 256), (2048, 8, 64), (4096, 2, 8), (3, 8, 128)])
+@pytest.mark.parametrize("m,k,e", [(4096, 8, 256), (2048, 8, 64), (4096, 2, 8), (3, 8, 128), (40, 8, 640),
+                                   (1500, 8, 1024), (33, 4, 1200), (600, 2, 3061)])
 def test_routing_from_topk_full_size(cuda_device, m, k, e):
     import flaggems_sglang_b200 as F
     from flaggems_sglang_b200.testing import route

@@ -66,7 +66,7 @@ def test_grouped_topk_deepseek_shapes(cuda_device, m):
     _check(logits, 8, cuda_device, scoring="sigmoid")
 
 
-@pytest.mark.parametrize("shape", [(7, 128, 256, 8, 2), (300, 256, 384, 64, 8)], ids=str)
+@pytest.mark.parametrize("shape", [(7, 128, 256, 8, 2), (300, 256, 384, 64, 8), (300, 128, 128, 1024, 8)], ids=str)
 def test_layer_from_logits(cuda_device, shape):
     """fused_moe(x, w13, w2, logits, k) == the experts applied to the oracle's routing."""
     import flaggems_sglang_b200 as F
