@@ -250,11 +250,14 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   const int bt_asked = L->BT;
   L->pairs2 = c->wmode == B200MOE_W_16BIT && L->BT >= 128 && !(c->flags & B200MOE_FLAG_SIMT) && gemm_tc2_ok(c->E, sms_l);
   L->w4_var = c->wmode == B200MOE_W_INT4_AWQ && L->BT > 32;
-  L->tile_tokens = c->block_tokens > 0 ? L->BT / 32 * 32 : 256;
+  // a caller that fixes the token block bounds the tiles with it, in whole granules of the rows' padding
+  L->tile_tokens = 256;
   if (L->pairs2) {
+    if (c->block_tokens > 0) L->tile_tokens = L->BT / 32 * 32;
     L->orient = 2;
     L->BT = 32;
   } else if (L->w4_var) {
+    if (c->block_tokens > 0) L->tile_tokens = L->BT;
     L->BT = 16;
   }
   L->P = c->M * c->topk;
@@ -440,6 +443,7 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   g1.N = c->I;
   g1.up_row_off = c->I;
   g1.BT = L.pairs2 || L.w4_var ? L.tile_tokens : L.BT;
+  g1.w4_var = L.w4_var ? 1 : 0;
   g1.orient = L.orient;
   g1.topk = c->topk;
   g1.P = L.P;

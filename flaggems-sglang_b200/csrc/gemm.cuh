@@ -18,7 +18,8 @@ struct GemmArgs {
   int N;           // output rows per expert covered by tiles of 128 (I for mode 0, H for mode 1)
   int up_row_off;  // mode 0: row of the first "up" weight inside an expert (= I)
   int orient;      // 0: weight rows on the MMA's M side (decode); 1: tokens on the M side (BT = 128); 2: CTA pairs
-  int BT;          // tokens per block (16..256, multiple of 16); CTA pairs: upper bound of the tokens per tile
+  int BT;          // tokens per block (16..256, multiple of 16); CTA pairs, w4_var: upper bound of the tokens per tile
+  int w4_var;      // int4: 1 = tiles of a variable number of tokens (16..192), 0 = decode blocks of BT (16 or 32) tokens
   int stages;      // shared-memory ring depth
   int acc_stages;  // accumulator buffers in tensor memory (1 or 2)
   int tmem_cols;   // allocated tensor-memory columns (power of two >= 32)

@@ -551,9 +551,12 @@ int launch_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4TokenMa
 template <int MODE, bool EXT>
 int launch_mode(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4TokenMaps& tm_x, const GemmArgs& a, int num_sms,
                 cudaStream_t stream) {
+  // a field of its own decides: the tables and tensor maps are laid out for one of the variants, and a tile bound of 16 or
+  // 32 tokens is not a decode block of that size
+  if (a.w4_var) return launch_w4<MODE, EXT, 0>(tm_w, tm_sz, tm_x, a, num_sms, stream);
   if (a.BT == 16) return launch_w4<MODE, EXT, 16>(tm_w, tm_sz, tm_x, a, num_sms, stream);
   if (a.BT == 32) return launch_w4<MODE, EXT, 32>(tm_w, tm_sz, tm_x, a, num_sms, stream);
-  return launch_w4<MODE, EXT, 0>(tm_w, tm_sz, tm_x, a, num_sms, stream);
+  return B200MOE_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -564,12 +567,12 @@ bool gemm_w4_ok(int E) {
          kSmemLimit - 1024 >= w4_fixed_bytes<32>(E, 1, false) + 2 * static_cast<size_t>(w4_token_bytes(32, 2));
 }
 
-// a->BT: 16 or 32 (decode blocks), otherwise the upper bound of the tokens per tile
+// a->BT: 16 or 32 (decode blocks); with a->w4_var the upper bound of the tokens per tile
 void gemm_plan_w4(GemmArgs* a) {
   const int tile_n = a->mode == 0 ? 64 : 128;
   a->num_nt = (a->N + tile_n - 1) / tile_n;
   // reduction unit: one quantisation group, two for decode blocks
-  a->kblocks = a->BT <= 32 ? (a->K + 255) / 256 : a->K / 128;
+  a->kblocks = a->w4_var ? a->K / 128 : (a->K + 255) / 256;
   if (a->max_split <= 0) a->max_split = 16;
 }
 
