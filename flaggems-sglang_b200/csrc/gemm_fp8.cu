@@ -649,6 +649,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
           break;
         }
         if (idle) {
+          __syncwarp();      // every lane has seen this phase: two slices on, the barrier has the same parity again
           if (lane == 0) mbar_arrive(smem_u32(&bar_pempty[pb]));
           continue;
         }

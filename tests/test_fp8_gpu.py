@@ -62,6 +62,22 @@ def test_fp8_every_token_block(cuda_device, bt):
     assert_parity(out, ref, what=f"fp8 BT={bt}")
 
 
+@pytest.mark.parametrize("m,k", [(40, 8), (1, 1)])
+def test_fp8_blocks_of_mostly_padding(cuda_device, m, k):
+    """128-token blocks with a handful of rows each: three of four promotion warps keep step over a long reduction
+    without promoting anything."""
+    import flaggems_sglang_b200 as F
+    x, tw, ids, w13q, s13, w2q, s2 = _fp8_case(7168, 256, 64, k, m, seed=m, skew=True)
+    d = cuda_device
+    args = (x.to(d), w13q.to(d), w2q.to(d), tw.to(d), ids.to(d))
+    kw = dict(use_fp8_w8a8=True, w13_scale=s13.to(d), w2_scale=s2.to(d), block_tokens=128)
+    ref = OM.fused_experts_fp8(x, w13q, w2q, s13, s2, tw, ids)
+    for _ in range(10):
+        out = F.fused_experts(*args, **kw)
+        F.check_status()
+        assert_parity(out, ref, what=f"fp8 mostly padding m={m}")
+
+
 def test_fp8_through_reference_signature(cuda_device):
     """The reference's signature already carries use_fp8_w8a8 / w1_scale / w2_scale /
     block_shape (fused_moe.py:143-151) and asserts them away; here they work."""
