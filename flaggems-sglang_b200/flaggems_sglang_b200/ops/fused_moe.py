@@ -571,22 +571,22 @@ def triton_kernel_fused_experts_with_bias(
     return out.view(hidden_states.shape[0], hidden_states.shape[1])
 
 
-_combine_class: dict = {}   # was sglang loaded at the look-up -> the result class of the hook
+_sglang_missing = False      # the import failed and `sglang` was not in sys.modules
 
 
 def _combine_input():
     """``StandardCombineInput`` of the running SGLang, or a namespace with the same field without
-    one.  Looked up once per state of ``sys.modules``: a failing import costs 100 us."""
-    loaded = "sglang" in sys.modules
-    cls = _combine_class.get(loaded)
-    if cls is None:
-        try:
-            from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput as cls
+    one.  A failing import costs 100 us, so that SGLang is missing is remembered until something
+    loads it; an import that fails while it is in ``sys.modules`` (it may be half imported) is
+    tried again by the next call."""
+    global _sglang_missing
+    if not _sglang_missing or "sglang" in sys.modules:
+        try:      # once loaded this is a look-up in sys.modules
+            from sglang.srt.layers.moe.token_dispatcher.standard import StandardCombineInput
+            return StandardCombineInput
         except Exception:
-            cls = SimpleNamespace
-        _combine_class["sglang" in sys.modules] = cls
-        _combine_class.setdefault(loaded, cls)
-    return cls
+            _sglang_missing = "sglang" not in sys.modules
+    return SimpleNamespace
 
 
 def fused_moe_flagos(obj, layer: torch.nn.Module, dispatch_output):

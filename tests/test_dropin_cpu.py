@@ -2,6 +2,8 @@
 signatures, and the per-weight layout caches survive a second look-up with the same tensor."""
 import importlib
 import inspect
+import sys
+from types import ModuleType, SimpleNamespace
 
 import torch
 
@@ -87,3 +89,21 @@ def test_workspace_cache_is_bounded():
     assert fm.MAX_CACHED_WORKSPACES >= 2
     fm.release_workspaces()
     assert len(fm._workspaces) == 0
+
+
+def test_hook_result_class_survives_a_failed_import(monkeypatch):
+    """Without SGLang the hook returns a namespace; an import that fails while SGLang is being loaded must not
+    decide the class for the rest of the process."""
+    fm = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")   # (the package also exports a function of that name)
+    name = "sglang.srt.layers.moe.token_dispatcher.standard"
+    for part in [m for m in sys.modules if m == "sglang" or m.startswith("sglang.")]:
+        monkeypatch.delitem(sys.modules, part)
+    monkeypatch.setitem(sys.modules, "sglang", ModuleType("sglang"))     # half imported: not even a package yet
+    assert fm._combine_input() is SimpleNamespace
+    parts = name.split(".")
+    for n in range(2, len(parts) + 1):
+        monkeypatch.setitem(sys.modules, ".".join(parts[:n]), ModuleType(".".join(parts[:n])))
+    combine = type("StandardCombineInput", (), {})
+    sys.modules[name].StandardCombineInput = combine
+    assert fm._combine_input() is combine
+    assert fm._combine_input() is combine
