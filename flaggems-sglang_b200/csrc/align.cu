@@ -459,7 +459,7 @@ int launch_align_from_routing(const int* hist, const int* topk_indx, const float
 int launch_routing_from_topk(const float* weights, const void* ids, int is64, int M, int k, int E,
                              int* expt_indx, int* topk_indx, int* gate_indx, float* gate_scal,
                              int* hist, int* token_offs_raw, int* token_offs_pad, int* block_pid_map,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, bool pdl) {
   if (M < 0 || k <= 0 || E <= 0) return B200MOE_ERR_BAD_ARG;
   const int nw = pick_warps(E);
   size_t smem;
@@ -467,7 +467,7 @@ int launch_routing_from_topk(const float* weights, const void* ids, int is64, in
   const int mt = routing_max_tiles(M * k, E);
   note_launch("routing_from_topk_kernel");
   const int ctas = pick_ctas(M * k);
-  cudaError_t err = launch_kernel_cluster(routing_from_topk_kernel, dim3(ctas), ctas, dim3(kAlignThreads), smem, stream, true,
+  cudaError_t err = launch_kernel_cluster(routing_from_topk_kernel, dim3(ctas), ctas, dim3(kAlignThreads), smem, stream, pdl,
                                           weights, ids, is64, M, k, E, mt, nw, expt_indx, topk_indx, gate_indx, gate_scal,
                                           hist, token_offs_raw, token_offs_pad, block_pid_map);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;

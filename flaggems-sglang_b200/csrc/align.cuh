@@ -26,6 +26,6 @@ int launch_align_from_routing(const int* hist, const int* topk_indx, const float
 int launch_routing_from_topk(const float* weights, const void* ids, int is64, int M, int k, int E,
                              int* expt_indx, int* topk_indx, int* gate_indx, float* gate_scal,
                              int* hist, int* token_offs_raw, int* token_offs_pad, int* block_pid_map,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool pdl);
 
 }  // namespace b200moe

@@ -779,9 +779,10 @@ int b200moe_routing_from_topk(const float* topk_weights, const void* topk_ids, i
       !block_pid_map)
     return B200MOE_ERR_BAD_ARG;
   if (n_tokens > 0 && (!topk_weights || !topk_ids)) return B200MOE_ERR_BAD_ARG;
-  return launch_routing_from_topk(topk_weights, topk_ids, ids_are_i64, n_tokens, topk, n_experts, expt_indx,
-                                  topk_indx, gate_indx, gate_scal, hist, token_offs_raw, token_offs_pad,
-                                  block_pid_map, static_cast<cudaStream_t>(stream));
+  return launch_routing_from_topk(topk_weights, topk_ids, (ids_are_i64 & ~B200MOE_FLAG_NO_PDL) != 0, n_tokens, topk,
+                                  n_experts, expt_indx, topk_indx, gate_indx, gate_scal, hist, token_offs_raw,
+                                  token_offs_pad, block_pid_map, static_cast<cudaStream_t>(stream),
+                                  (ids_are_i64 & B200MOE_FLAG_NO_PDL) == 0);
 }
 
 static int forward_common(const b200moe_cfg* cfg, const void* x, const void* w1, const void* w2, void* workspace,

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import os
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -124,6 +125,9 @@ def topk_to_routing(topk_weights: torch.Tensor, topk_ids: torch.Tensor, n_expts_
     w32 = topk_weights.to(torch.float32).contiguous()
     lib = _lib.lib()
     mt = lib.b200moe_routing_max_tiles(p, n_expts_tot)
+    flags = int(ids.dtype == torch.int64)
+    if _lib.env_set() and os.environ.get("B200MOE_NO_PDL", "0") == "1":
+        flags |= _lib.FLAG_NO_PDL
     i32 = torch.int32
     expt_indx = torch.empty(p, dtype=i32, device=dev)
     topk_indx = torch.empty(p, dtype=i32, device=dev)
@@ -135,7 +139,7 @@ def topk_to_routing(topk_weights: torch.Tensor, topk_ids: torch.Tensor, n_expts_
     pid_map = torch.empty(4, max(mt, 1), dtype=i32, device=dev)   # four block maps back to back, stride max_tiles
     with _on_device(dev):
         rc = lib.b200moe_routing_from_topk(
-            w32.data_ptr(), ids.data_ptr(), int(ids.dtype == torch.int64), m, k, n_expts_tot,
+            w32.data_ptr(), ids.data_ptr(), flags, m, k, n_expts_tot,
             expt_indx.data_ptr(), topk_indx.data_ptr(), gate_indx.data_ptr(), gate_scal.data_ptr(),
             hist.data_ptr(), offs_raw.data_ptr(), offs_pad.data_ptr(),
             pid_map.data_ptr(), _stream_ptr(dev))

@@ -164,6 +164,7 @@ int b200moe_align_block_size(const void *topk_ids, int ids_are_i64, int n_slots,
  *   expt_indx[P], topk_indx[P], gate_indx[P], gate_scal[P] (fp32), hist[E],
  *   token_offs_raw[E+1], token_offs_pad[4][E+1], block_pid_map[4][max_tiles]
  * for block sizes 16, 32, 64, 128; max_tiles = b200moe_routing_max_tiles(P, E).
+ * ids_are_i64: 0 or 1, plus B200MOE_FLAG_NO_PDL for a fully serialised launch.
  */
 int b200moe_routing_max_tiles(int n_slots, int n_experts);
 int b200moe_routing_from_topk(const float *topk_weights, const void *topk_ids,

@@ -102,3 +102,22 @@ def test_routing_from_topk_full_size(cuda_device, m, k, e):
     # size-independent property: gate_indx is the inverse permutation of topk_indx
     ti, gi_ = gi.src_indx.long(), gi.dst_indx.long()
     assert torch.equal(gi_[ti], torch.arange(m * k, device=cuda_device))
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("no_pdl", ["0", "1"])
+def test_routing_from_topk_serialised(cuda_device, monkeypatch, dtype, no_pdl):
+    """B200MOE_NO_PDL reaches the routing conversion too, for both id types."""
+    import flaggems_sglang_b200 as F
+    from flaggems_sglang_b200 import _lib
+    monkeypatch.setenv("B200MOE_NO_PDL", no_pdl)
+    seen = []
+    call = _lib.lib().b200moe_routing_from_topk
+    monkeypatch.setattr(_lib.lib(), "b200moe_routing_from_topk", lambda *a: seen.append(a[2]) or call(*a))
+    ids = _rand_ids(50, 4, 16, 2, dtype)
+    w = torch.rand(50, 4)
+    rd, gi, _ = F.topk_to_routing(w.to(cuda_device), ids.to(cuda_device), 16)
+    assert bool(seen[0] & _lib.FLAG_NO_PDL) == (no_pdl == "1")
+    r = R.topk_to_routing(w.numpy(), ids.numpy(), 16)
+    np.testing.assert_array_equal(gi.src_indx.cpu().numpy(), r["topk_indx"])
+    np.testing.assert_array_equal(rd.gate_scal.cpu().numpy(), r["gate_scal"])
