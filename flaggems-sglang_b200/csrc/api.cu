@@ -613,7 +613,7 @@ bool gemv_eligible(const b200moe_cfg* c, const Layout& L) {
   // layer at M = 1 took 152 us this way, 97 us on the grouped tensor-core path)
   const bool w4 = c->wmode == B200MOE_W_INT4_AWQ;
   if (L.P <= 0 || L.P > kGemvMaxPairs || c->block_tokens != 0) return false;
-  if ((c->wmode != B200MOE_W_16BIT && !w4) || (c->flags & (B200MOE_FLAG_SIMT | B200MOE_FLAG_W4_SMEM_OPERANDS)))
+  if ((c->wmode != B200MOE_W_16BIT && !w4) || (c->flags & (B200MOE_FLAG_SIMT | B200MOE_FLAG_NO_MATRIX_VECTOR)))
     return false;
   // the pairs' 16-bit activations go where the grouped path keeps GEMM-1's output
   if (static_cast<size_t>(L.cap) * c->I * L.act_bytes < static_cast<size_t>(L.P) * c->I * 2) return false;

@@ -260,9 +260,6 @@ __device__ __forceinline__ void tmem_ld16_wait(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-#define B200MOE_R8(r, o)                                                                             \
-  "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]),   \
-      "=r"(r[o + 6]), "=r"(r[o + 7])
 // Two loads (e.g. gate and up accumulators) in flight before the single wait.
 __device__ __forceinline__ void tmem_ld16x2_wait(uint32_t taddr0, uint32_t taddr1, float (&v0)[16],
                                                  float (&v1)[16]) {
@@ -295,20 +292,6 @@ __device__ __forceinline__ void tmem_ld16_wait_u32(uint32_t taddr, uint32_t (&r)
 }
 
 #define B200MOE_R32(r, o) B200MOE_R16(r, o), B200MOE_R16(r, o + 16)
-// 32 consecutive fp32 columns of the thread's TMEM lane (load + wait in one statement).
-__device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : B200MOE_R32(r, 0)
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Two 32-column loads in flight before the single wait.
 __device__ __forceinline__ void tmem_ld32x2_wait(uint32_t taddr0, uint32_t taddr1, float (&v0)[32],
                                                  float (&v1)[32]) {
@@ -487,7 +470,6 @@ __device__ __forceinline__ __half from_f32<__half>(float v) {
   return __float2half_rn(v);
 }
 
-__device__ __forceinline__ float silu_f32(float g) { return g / (1.0f + __expf(-g)); }
 __device__ __forceinline__ float gelu_f32(float g) {
   return 0.5f * g * (1.0f + erff(g * 0.70710678118654752f));
 }

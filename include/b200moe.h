@@ -58,15 +58,13 @@ extern "C" {
 #define B200MOE_FLAG_NO_SPLIT_K 16      /* keep GEMM-2's reduction in one piece                */
 #define B200MOE_FLAG_NO_GRID_BALANCE 32 /* tuning aid: every CTA takes tiles round-robin       */
 #define B200MOE_FLAG_NO_PDL 64          /* launch every kernel fully serialised                */
-#define B200MOE_FLAG_W4_SMEM_OPERANDS 128 /* int4: grouped GEMMs at every size, none of the small-batch kernels (tuning aid) */
+#define B200MOE_FLAG_NO_MATRIX_VECTOR 128 /* tuning aid: grouped GEMMs at every size, 16-bit and int4 */
 #define B200MOE_FLAG_X_FP8 1024         /* FP8 weights only: x is already e4m3 [M, H], quantised per
                                            1 x 128 group with scales quant->x_scale [M, H/128] (what
                                            b200moe_per_token_group_quant_fp8 writes); cfg->dtype still
                                            names the 16-bit type of the intermediate and the output   */
 #define B200MOE_FLAG_EP_DIAG_LOCAL_COMBINE 2048 /* tuning aid, expert parallelism: the down projection's rows stay on
                                            this GPU (WRONG results; isolates the cost of the peer stores)      */
-#define B200MOE_FLAG_CTA_PAIR 4096      /* no effect: 16-bit problems of more than 64 tokens per block always run
-                                           on CTA pairs (tcgen05.mma.cta_group::2)                             */
 #define B200MOE_FLAG_ALIGN_ONE_CTA 512  /* tuning aid: single-CTA alignment however many slots           */
 #define B200MOE_FLAG_NO_COMBINE 256     /* out is [M*topk, H]: row t*topk+j holds pair j of token t,
                                            routing weight applied, nothing summed, routed_scaling ignored
@@ -373,8 +371,8 @@ int b200moe_profile_end(double *gemm1_ms, double *gemm2_ms, double *total_ms, do
  * characters).  Returns the number of kernels in that list.
  */
 int b200moe_launch_stats(long long *total_launches, char *last_call_names, size_t names_bytes);
-/* CTA pairs the device kept resident for the last grouped GEMM launched on CTA pairs
- * (B200MOE_FLAG_CTA_PAIR); 0 before the first such launch.  Diagnostics. */
+/* CTA pairs the device kept resident for the last grouped GEMM launched on CTA pairs (16-bit
+ * problems on token blocks of 128 and more); 0 before the first such launch.  Diagnostics. */
 int b200moe_debug_resident_cta_pairs(void);
 
 /*

@@ -85,6 +85,7 @@ def test_matrix_vector_path_selection(built_lib):
     assert uses(1, 7168, 2048, 256, 8, wmode=_lib.W_FP8_BLOCK) == 0
     assert uses(1, 4096, 14336, 8, 2, wmode=_lib.W_INT4_AWQ, dtype=1) == 1
     assert uses(1, 4096, 14336, 8, 2, flags=_lib.FLAG_SIMT) == 0
+    assert uses(1, 2048, 768, 128, 8, flags=_lib.FLAG_NO_MATRIX_VECTOR) == 0
     assert uses(1, 4096, 32768, 8, 4) == 0                     # 4 x 32768 fp32 activations do not fit in shared memory
     bad = _lib.Cfg(4, 1, 128, 128, 8, 2, 0, 0, 0, 0, 0, 0, 1.0, 0)
     assert built_lib.b200moe_uses_matrix_vector_path(C.byref(bad)) == _lib.ERR_BAD_ARG
