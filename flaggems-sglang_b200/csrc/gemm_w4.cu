@@ -396,8 +396,13 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       };
 #pragma unroll
       for (int b = 0; b < kBefore; ++b) convert(b);
+      // The loads of the rows are issued here, but nothing needs their data before the operands are stored, and the next
+      // rows are written by another proxy (TMA), which the arrival alone does not hold back: at 176-192 tokens a tile, where
+      // the MMAs and the token loads take all of shared memory's bandwidth, one refill in about 10^5 overtook the loads of
+      // some lanes of a warp.  The fence orders them (2048 tokens 1415 -> 1432 us, 32 tokens 222 -> 224).
+      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_wempty[ws]));         // every lane has read its row
+      if (lane == 0) mbar_arrive(smem_u32(&bar_wempty[ws]));
       if (!wait_done(u - slots_a, DEV_TIMEOUT_MMA)) break;
       tc_fence_after();
       tmem_st32(dst, o[0]);

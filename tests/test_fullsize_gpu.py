@@ -172,3 +172,37 @@ def test_mixtral_int4_awq_full_layer(cuda_device, mixtral_awq, M):
     ref = OM.fused_experts(x, w13f, w2f, tw, ids)
     assert out.dtype == torch.float16
     assert_parity(out, ref, rtol=2e-2, atol=2e-2, what=f"mixtral int4 awq I=14336 M={M}")
+
+
+@pytest.mark.parametrize("M", [600, 2048])
+def test_mixtral_int4_awq_prefill_repeats_and_stays_close(cuda_device, mixtral_awq, M):
+    """The variable-tile int4 kernel accumulates in a fixed order and stores a row per pair, so a rerun gives the same
+    bits; and no row is further from an fp64 evaluation of the same operands than its roundings to fp16 explain
+    (projections, activation, pair row, output: at most 2^-11 of a value each, adding up in quadrature).  A quantisation group that
+    is wrong in a single column of a tile is beyond that in the tile's rows."""
+    import flaggems_sglang_b200 as F
+    from flaggems_sglang_b200.testing import make_tokens
+    h, i, e, k, p1, z1, p2, z2, w13f, w2f = mixtral_awq
+    d = cuda_device
+    x, tw, ids = (t.to(d) for t in make_tokens(M, h, e, k, dtype=torch.float16, seed=0))
+    kw = dict(use_int4_w4a16=True, w13_sz=z1, w2_sz=z2)
+    out = F.fused_experts(x, p1, p2, tw, ids, **kw)
+    for call in range(60):
+        again = F.fused_experts(x, p1, p2, tw, ids, **kw)
+        if call % 4 == 0:          # back to back and after a pause
+            torch.cuda.synchronize()
+        assert torch.equal(out, again), f"rerun {call} differs"
+    F.check_status()
+
+    ref = torch.zeros(M, h, dtype=torch.float64, device=d)
+    for ex in range(e):
+        a13, a2 = (w[ex].to(d).half().double().t() for w in (w13f, w2f))      # (q - z) * s rounded once to fp16
+        for c in range(k):
+            t = (ids[:, c] == ex).nonzero()[:, 0]
+            y = x[t].double() @ a13
+            g, u = y[:, :i], y[:, i:]
+            ref[t] += tw[t, c].double()[:, None] * ((g / (1 + torch.exp(-g)) * u) @ a2)
+    err = (out.double() - ref).norm(dim=1) / ref.norm(dim=1)
+    bound = 5 ** 0.5 * 2.0 ** -11
+    print(f"[rows] M={M}: largest error of a row {float(err.max()):.3e}, median {float(err.median()):.3e}, bound {bound:.3e}")
+    assert float(err.max()) <= bound, f"row {int(err.argmax())} is {float(err.max()):.3e} off (bound {bound:.3e})"
