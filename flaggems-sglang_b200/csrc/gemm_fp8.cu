@@ -475,336 +475,336 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
 
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-  if (active && warp == 0 && elect_one()) {
-    // =============================== TMA producer ===============================
-    int stage = 0;
-    uint32_t phase = 0;
-    long long issued = 0;
-    uint32_t jx = 0;     // slices issued over the whole launch
-    bool ok = true;
-    unsigned long long w_empty = 0;
-    const long long role_t0 = clock64();
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
-      for (int kb = t.kb0; kb < t.kb1; ++kb) {
-        if (!mbar_wait_t(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER, w_empty)) {
-          ok = false;
-          break;
-        }
-        // The slice's activation scales go to a ring of their own, which the promotion warps read once the slice's
-        // MMAs are done (these wait for the whole stage, scales included).  The slot is free: this stage's last MMA has finished, and it was issued after the promotion of the slice two
-        // before it, which is at most stages + 2 <= kXsSlots slices back.
-        const uint32_t xs_slot = jx % kXsSlots;
-        ++jx;
-        const uint32_t full = smem_u32(&bar_full[stage]);
-        mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES + BT * 4));
-        bulk_copy_g2s(smem_u32(s_xs + xs_slot * BT), a.x_scale + static_cast<size_t>(kb) * a.ld_xscale + t.row0, BT * 4, full);
-        const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
-        const int k0 = kb * kStageKBytes;
-        tma_load_3d(sw, &tm_w, full, k0, t.n0, t.e);
-        tma_load_3d(sw + kTileBytes, &tm_w, full, k0, second_off + t.n0, t.e);
-        tma_load_2d(sw + W_BYTES, &tm_x, full, k0, t.row0);
-        ++issued;
-        if (++stage == stages) {
-          stage = 0;
-          phase ^= 1;
-        }
-      }
-    }
-    STALL_ADD8(0, w_empty);
-    STALL_ADD8(8, static_cast<unsigned long long>(clock64() - role_t0));
-    if (!ok) {
-      const int n = static_cast<int>(issued < stages ? issued : stages);
-      for (int i = 1; i <= n; ++i) {
-        int s = stage - i;
-        uint32_t ph = phase;
-        if (s < 0) {
-          s += stages;
-          ph ^= 1;
-        }
-        mbar_wait_brief(smem_u32(&bar_full[s]), ph);
-      }
-    }
-  } else if (active && warp == 1 && elect_one()) {
-    // =============================== MMA issuer =================================
-    const uint32_t idesc = make_idesc(0u /* e4m3 */, kTileRows, 256u);
-    int stage = 0;
-    uint32_t phase = 0, j = 0;
-    bool ok = true;
-    unsigned long long w_full = 0, w_pempty = 0;
-    const long long role_t0 = clock64();
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-      int kb0 = 0, kb1 = a.kblocks;
-      if (c.split > 1) {       // only the slice count matters here
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    if (active && warp == 0 && elect_one()) {
+      // =============================== TMA producer ===============================
+      int stage = 0;
+      uint32_t phase = 0;
+      long long issued = 0;
+      uint32_t jx = 0;     // slices issued over the whole launch
+      bool ok = true;
+      unsigned long long w_empty = 0;
+      const long long role_t0 = clock64();
+      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
         const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
-        kb0 = t.kb0;
-        kb1 = t.kb1;
-      }
-      for (int kb = kb0; kb < kb1; ++kb, ++j) {
-        const uint32_t pb = j & 1u;
-        if (!mbar_wait_t(smem_u32(&bar_full[stage]), phase, abort_flag, DEV_TIMEOUT_MMA, w_full) ||
-            !mbar_wait_t(smem_u32(&bar_pempty[pb]), ((j >> 1) & 1u) ^ 1u, abort_flag, DEV_TIMEOUT_MMA, w_pempty)) {
-          ok = false;
-          break;
+        for (int kb = t.kb0; kb < t.kb1; ++kb) {
+          if (!mbar_wait_t(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER, w_empty)) {
+            ok = false;
+            break;
+          }
+          // The slice's activation scales go to a ring of their own, which the promotion warps read once the slice's
+          // MMAs are done (these wait for the whole stage, scales included).  The slot is free: this stage's last MMA has
+          // finished, and it was issued after the promotion of the slice two before it, which is at most
+          // stages + 2 <= kXsSlots slices back.
+          const uint32_t xs_slot = jx % kXsSlots;
+          ++jx;
+          const uint32_t full = smem_u32(&bar_full[stage]);
+          mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES + BT * 4));
+          bulk_copy_g2s(smem_u32(s_xs + xs_slot * BT), a.x_scale + static_cast<size_t>(kb) * a.ld_xscale + t.row0, BT * 4, full);
+          const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
+          const int k0 = kb * kStageKBytes;
+          tma_load_3d(sw, &tm_w, full, k0, t.n0, t.e);
+          tma_load_3d(sw + kTileBytes, &tm_w, full, k0, second_off + t.n0, t.e);
+          tma_load_2d(sw + W_BYTES, &tm_x, full, k0, t.row0);
+          ++issued;
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        tc_fence_after();
-        const uint32_t d0 = tmem_base + pb * PCOLS;
-        const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
-        const uint64_t dw = smem_desc_k_sw128(sw);             // 256 weight rows: N side
-        const uint64_t dx = smem_desc_k_sw128(sw + W_BYTES);   // 128 token rows: M side
+      }
+      STALL_ADD8(0, w_empty);
+      STALL_ADD8(8, static_cast<unsigned long long>(clock64() - role_t0));
+      if (!ok) {
+        const int n = static_cast<int>(issued < stages ? issued : stages);
+        for (int i = 1; i <= n; ++i) {
+          int s = stage - i;
+          uint32_t ph = phase;
+          if (s < 0) {
+            s += stages;
+            ph ^= 1;
+          }
+          mbar_wait_brief(smem_u32(&bar_full[s]), ph);
+        }
+      }
+    } else if (active && warp == 1 && elect_one()) {
+      // =============================== MMA issuer =================================
+      const uint32_t idesc = make_idesc(0u /* e4m3 */, kTileRows, 256u);
+      int stage = 0;
+      uint32_t phase = 0, j = 0;
+      bool ok = true;
+      unsigned long long w_full = 0, w_pempty = 0;
+      const long long role_t0 = clock64();
+      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
+        int kb0 = 0, kb1 = a.kblocks;
+        if (c.split > 1) {       // only the slice count matters here
+          const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+          kb0 = t.kb0;
+          kb1 = t.kb1;
+        }
+        for (int kb = kb0; kb < kb1; ++kb, ++j) {
+          const uint32_t pb = j & 1u;
+          if (!mbar_wait_t(smem_u32(&bar_full[stage]), phase, abort_flag, DEV_TIMEOUT_MMA, w_full) ||
+              !mbar_wait_t(smem_u32(&bar_pempty[pb]), ((j >> 1) & 1u) ^ 1u, abort_flag, DEV_TIMEOUT_MMA, w_pempty)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d0 = tmem_base + pb * PCOLS;
+          const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
+          const uint64_t dw = smem_desc_k_sw128(sw);             // 256 weight rows: N side
+          const uint64_t dx = smem_desc_k_sw128(sw + W_BYTES);   // 128 token rows: M side
 #pragma unroll
-        for (int k = 0; k < 4; ++k) tc_mma_f8(d0, dx + 2 * k, dw + 2 * k, idesc, k > 0 ? 1u : 0u);
-        tc_commit(smem_u32(&bar_empty[stage]));
-        tc_commit(smem_u32(&bar_pfull[pb]));
-        if (++stage == stages) {
-          stage = 0;
-          phase ^= 1;
+          for (int k = 0; k < 4; ++k) tc_mma_f8(d0, dx + 2 * k, dw + 2 * k, idesc, k > 0 ? 1u : 0u);
+          tc_commit(smem_u32(&bar_empty[stage]));
+          tc_commit(smem_u32(&bar_pfull[pb]));
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
+      STALL_ADD8(1, w_pempty);
+      STALL_ADD8(2, w_full);
+      STALL_ADD8(9, static_cast<unsigned long long>(clock64() - role_t0));
+    } else if (active && warp == 2) {
+      // =============================== per-tile table loader ======================
+      const int kb_total = a.kblocks;
+      int iter = 0;
+      for (int tile = blockIdx.x; tile < c.total; tile += c.grid_eff, ++iter) {
+        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+        const int buf = iter & 1;
+        if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+        const int nkb = t.kb1 - t.kb0;
+        for (int cidx = lane; cidx < BT; cidx += 32) {
+          const int slot = a.sorted_ids[t.row0 + cidx];
+          const bool valid = slot >= 0 && slot < a.P;
+          // mode 1: output row = token, or the pair's own slot when rows are stored per pair
+          const int orow = valid ? ((MODE == 1 && a.out_pairs == nullptr) ? slot / a.topk : slot) : -1;
+          s_col_row[buf * 128 + cidx] = orow;
+          s_col_gam[buf * 128 + cidx] = valid ? a.row_gamma[t.row0 + cidx] : 0.f;
+          if (MODE == 1 && valid)
+            s_col_ptr[buf * 128 + cidx] = reinterpret_cast<unsigned long long>(
+                a.out_pairs != nullptr ? out_row_base(a, a.out_pairs, orow, static_cast<size_t>(a.N) * 2)
+                                       : out_row_base(a, a.out, orow, static_cast<size_t>(a.ld_out) * sizeof(float)));
+        }
+        const int nb0 = t.n0 / 128, nb1 = (second_off + t.n0) / 128;
+        const float* ws0 = a.w_scale + (static_cast<size_t>(t.e) * a.w_scale_rows + nb0) * kb_total + t.kb0;
+        const float* ws1 = a.w_scale + (static_cast<size_t>(t.e) * a.w_scale_rows + nb1) * kb_total + t.kb0;
+        const bool second_ok = nb1 < a.w_scale_rows;
+        float* ws_t = s_ws + buf * 2 * KBS;
+        for (int i = lane; i < nkb; i += 32) {
+          ws_t[i] = __ldg(ws0 + i);
+          ws_t[KBS + i] = second_ok ? __ldg(ws1 + i) : 0.f;
+        }
+        if (lane == 0) {
+          int* ti = s_tile + buf * 8;
+          ti[0] = t.e;
+          ti[1] = t.row0;
+          ti[2] = t.n0;
+          ti[3] = t.kb0;
+          ti[4] = t.kb1;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_sfull[buf]));
+      }
     }
-    STALL_ADD8(1, w_pempty);
-    STALL_ADD8(2, w_full);
-    STALL_ADD8(9, static_cast<unsigned long long>(clock64() - role_t0));
-  } else if (active && warp == 2) {
-    // =============================== per-tile table loader ======================
-    const int kb_total = a.kblocks;
-    int iter = 0;
-    for (int tile = blockIdx.x; tile < c.total; tile += c.grid_eff, ++iter) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
-      const int buf = iter & 1;
-      if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
-      const int nkb = t.kb1 - t.kb0;
-      for (int cidx = lane; cidx < BT; cidx += 32) {
-        const int slot = a.sorted_ids[t.row0 + cidx];
-        const bool valid = slot >= 0 && slot < a.P;
-        // mode 1: output row = token, or the pair's own slot when rows are stored per pair
-        const int orow = valid ? ((MODE == 1 && a.out_pairs == nullptr) ? slot / a.topk : slot) : -1;
-        s_col_row[buf * 128 + cidx] = orow;
-        s_col_gam[buf * 128 + cidx] = valid ? a.row_gamma[t.row0 + cidx] : 0.f;
-        if (MODE == 1 && valid)
-          s_col_ptr[buf * 128 + cidx] = reinterpret_cast<unsigned long long>(
-              a.out_pairs != nullptr ? out_row_base(a, a.out_pairs, orow, static_cast<size_t>(a.N) * 2)
-                                     : out_row_base(a, a.out, orow, static_cast<size_t>(a.ld_out) * sizeof(float)));
-      }
-      const int nb0 = t.n0 / 128, nb1 = (second_off + t.n0) / 128;
-      const float* ws0 = a.w_scale + (static_cast<size_t>(t.e) * a.w_scale_rows + nb0) * kb_total + t.kb0;
-      const float* ws1 = a.w_scale + (static_cast<size_t>(t.e) * a.w_scale_rows + nb1) * kb_total + t.kb0;
-      const bool second_ok = nb1 < a.w_scale_rows;
-      float* ws_t = s_ws + buf * 2 * KBS;
-      for (int i = lane; i < nkb; i += 32) {
-        ws_t[i] = __ldg(ws0 + i);
-        ws_t[KBS + i] = second_ok ? __ldg(ws1 + i) : 0.f;
-      }
-      if (lane == 0) {
-        int* ti = s_tile + buf * 8;
-        ti[0] = t.e;
-        ti[1] = t.row0;
-        ti[2] = t.n0;
-        ti[3] = t.kb0;
-        ti[4] = t.kb1;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_sfull[buf]));
-    }
-  }
   } else {
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-  if (active) {
-    // =============================== promotion + tail ===========================
-    const int grp = warp < 8 ? 0 : 1;
-    const int quad = warp & 3;
-    const int lrow = quad * 32 + lane;  // token row inside the block = TMEM lane
-    const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0;
-    // columns of this thread: mode 0 -> gate [64g, 64g+64) and up [128+64g, ..+64); mode 1 -> [128g, 128g+128)
-    const uint32_t colA = (MODE == 0) ? 64u * grp : 128u * grp;
-    const uint32_t colB = (MODE == 0) ? 128u + 64u * grp : 128u * grp + 64u;
-    uint32_t j = 0;
-    uint32_t meet8_phase = 0;
-    int iter = 0;
-    bool ok = true;
-    unsigned long long w_pfull = 0, w_sfull = 0, t_tail = 0;
-    const long long role_t0 = clock64();
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff, ++iter) {
-      const int buf = iter & 1;
-      const float* ws_t = s_ws + buf * 2 * KBS;
-      if (!mbar_wait_t(smem_u32(&bar_sfull[buf]), (iter >> 1) & 1, abort_flag, DEV_TIMEOUT_EPILOGUE, w_sfull)) break;
-      const int* ti = s_tile + buf * 8;      // decoded by the table warp, off this critical path
-      const TileCoord t = {ti[0], ti[1], ti[2], ti[3], ti[4]};
-      const int orow = s_col_row[buf * 128 + lrow];
-      const float gam = s_col_gam[buf * 128 + lrow];
-      const bool idle = !__any_sync(0xffffffffu, orow >= 0);   // 32 padding rows: keep in step, promote and store nothing
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    if (active) {
+      // =============================== promotion + tail ===========================
+      const int grp = warp < 8 ? 0 : 1;
+      const int quad = warp & 3;
+      const int lrow = quad * 32 + lane;  // token row inside the block = TMEM lane
+      const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0;
+      // columns of this thread: mode 0 -> gate [64g, 64g+64) and up [128+64g, ..+64); mode 1 -> [128g, 128g+128)
+      const uint32_t colA = (MODE == 0) ? 64u * grp : 128u * grp;
+      const uint32_t colB = (MODE == 0) ? 128u + 64u * grp : 128u * grp + 64u;
+      uint32_t j = 0;
+      uint32_t meet8_phase = 0;
+      int iter = 0;
+      bool ok = true;
+      unsigned long long w_pfull = 0, w_sfull = 0, t_tail = 0;
+      const long long role_t0 = clock64();
+      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff, ++iter) {
+        const int buf = iter & 1;
+        const float* ws_t = s_ws + buf * 2 * KBS;
+        if (!mbar_wait_t(smem_u32(&bar_sfull[buf]), (iter >> 1) & 1, abort_flag, DEV_TIMEOUT_EPILOGUE, w_sfull)) break;
+        const int* ti = s_tile + buf * 8;      // decoded by the table warp, off this critical path
+        const TileCoord t = {ti[0], ti[1], ti[2], ti[3], ti[4]};
+        const int orow = s_col_row[buf * 128 + lrow];
+        const float gam = s_col_gam[buf * 128 + lrow];
+        const bool idle = !__any_sync(0xffffffffu, orow >= 0);   // 32 padding rows: keep in step, promote and store nothing
 
-      // running sums stay packed two to a 64-bit register for the whole reduction
-      unsigned long long pA[32], pB[32];
+        // running sums stay packed two to a 64-bit register for the whole reduction
+        unsigned long long pA[32], pB[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        pA[i] = 0ull;
-        pB[i] = 0ull;
-      }
-      for (int kb = t.kb0; kb < t.kb1; ++kb, ++j) {
-        const uint32_t pb = j & 1u;
-        if (!mbar_wait_t(smem_u32(&bar_pfull[pb]), (j >> 1) & 1u, abort_flag, DEV_TIMEOUT_EPILOGUE, w_pfull)) {
-          ok = false;
-          break;
+        for (int i = 0; i < 32; ++i) {
+          pA[i] = 0ull;
+          pB[i] = 0ull;
         }
-        if (idle) {
-          __syncwarp();      // every lane has seen this phase: two slices on, the barrier has the same parity again
+        for (int kb = t.kb0; kb < t.kb1; ++kb, ++j) {
+          const uint32_t pb = j & 1u;
+          if (!mbar_wait_t(smem_u32(&bar_pfull[pb]), (j >> 1) & 1u, abort_flag, DEV_TIMEOUT_EPILOGUE, w_pfull)) {
+            ok = false;
+            break;
+          }
+          if (idle) {
+            __syncwarp();      // every lane has seen this phase: two slices on, the barrier has the same parity again
+            if (lane == 0) mbar_arrive(smem_u32(&bar_pempty[pb]));
+            continue;
+          }
+          tc_fence_after();
+          const uint32_t xs_slot = j % kXsSlots;
+          const float sx = s_xs[xs_slot * BT + lrow];
+          // mode 0: A columns belong to the first weight block, B columns to the second;
+          // mode 1: group g works entirely inside weight block g
+          const float fA = sx * ws_t[(MODE == 0 ? 0 : grp * KBS) + kb - t.kb0];
+          const float fB = sx * ws_t[(MODE == 0 ? KBS : grp * KBS) + kb - t.kb0];
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + pb * PCOLS;
+          // Packed f32x2 FMAs, 16 columns at a time.  They run at half the rate of scalar ones, so the FMA pipe is
+          // as busy, but they leave the MMA thread's scheduler twice the issue slots (with scalar FMAs the MMAs of a
+          // slice took 684 cycles instead of 516).  Wider reads spill: the accumulators alone take 128 registers.
+          const unsigned long long fA2 = pack_f32x2(fA, fA), fB2 = pack_f32x2(fB, fB);
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            uint32_t g[16];
+            tmem_ld16_wait_u32(taddr + colA + c0, g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ffma2_packed(pA[c0 / 2 + i], g[2 * i], g[2 * i + 1], fA2);
+            tmem_ld16_wait_u32(taddr + colB + c0, g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ffma2_packed(pB[c0 / 2 + i], g[2 * i], g[2 * i + 1], fB2);
+          }
+          tc_fence_before();
+          __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bar_pempty[pb]));
+        }
+        if (!ok) break;
+        const long long tail_t0 = clock64();
+        if (idle) {
+          if (MODE == 0 && !warps_meet(smem_u32(bar_meet8), meet8_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
           continue;
         }
-        tc_fence_after();
-        const uint32_t xs_slot = j % kXsSlots;
-        const float sx = s_xs[xs_slot * BT + lrow];
-        // mode 0: A columns belong to the first weight block, B columns to the second;
-        // mode 1: group g works entirely inside weight block g
-        const float fA = sx * ws_t[(MODE == 0 ? 0 : grp * KBS) + kb - t.kb0];
-        const float fB = sx * ws_t[(MODE == 0 ? KBS : grp * KBS) + kb - t.kb0];
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + pb * PCOLS;
-        // Packed f32x2 FMAs, 16 columns at a time.  They run at half the rate of scalar ones, so the FMA pipe is
-        // as busy, but they leave the MMA thread's scheduler twice the issue slots (with scalar FMAs the MMAs of a
-        // slice took 684 cycles instead of 516).  Wider reads spill: the accumulators alone take 128 registers.
-        const unsigned long long fA2 = pack_f32x2(fA, fA), fB2 = pack_f32x2(fB, fB);
+        float accA[64], accB[64];
 #pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-          uint32_t g[16];
-          tmem_ld16_wait_u32(taddr + colA + c0, g);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) ffma2_packed(pA[c0 / 2 + i], g[2 * i], g[2 * i + 1], fA2);
-          tmem_ld16_wait_u32(taddr + colB + c0, g);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) ffma2_packed(pB[c0 / 2 + i], g[2 * i], g[2 * i + 1], fB2);
+        for (int i = 0; i < 32; ++i) {
+          unpack_f32x2(pA[i], accA[2 * i], accA[2 * i + 1]);
+          unpack_f32x2(pB[i], accB[2 * i], accB[2 * i + 1]);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_pempty[pb]));
-      }
-      if (!ok) break;
-      const long long tail_t0 = clock64();
-      if (idle) {
-        if (MODE == 0 && !warps_meet(smem_u32(bar_meet8), meet8_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
-        continue;
-      }
-      float accA[64], accB[64];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        unpack_f32x2(pA[i], accA[2 * i], accA[2 * i + 1]);
-        unpack_f32x2(pB[i], accB[2 * i], accB[2 * i + 1]);
-      }
 
-      if (MODE == 1 && a.bias != nullptr && t.kb0 == 0) {
-        // bias of columns n0 + 128 grp + [0, 128): accA holds the first 64, accB the next 64
-        const float* bo = a.bias + static_cast<size_t>(t.e) * a.N + t.n0 + 128 * grp;
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          accA[i] += (t.n0 + 128 * grp + i < a.N) ? __ldg(bo + i) : 0.f;
-          accB[i] += (t.n0 + 128 * grp + 64 + i < a.N) ? __ldg(bo + 64 + i) : 0.f;
-        }
-      }
-      if (MODE == 0) {
-        // 64 activations of this token; the other 64 of its quantisation group live in the
-        // same lane of the other promotion group
-        float amax = 0.f;
-        const bool ext = a.bias != nullptr || a.activation == B200MOE_ACT_SWIGLU_OAI;
-        if (a.bias != nullptr) {
-          // gate columns n0 + 64 grp + i and the matching up / linear columns of the same expert
-          const float* bgp = a.bias + static_cast<size_t>(t.e) * 2 * a.N + t.n0 + 64 * grp;
+        if (MODE == 1 && a.bias != nullptr && t.kb0 == 0) {
+          // bias of columns n0 + 128 grp + [0, 128): accA holds the first 64, accB the next 64
+          const float* bo = a.bias + static_cast<size_t>(t.e) * a.N + t.n0 + 128 * grp;
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
-            const bool in = t.n0 + 64 * grp + i < a.N;
-            accA[i] += in ? __ldg(bgp + i) : 0.f;
-            accB[i] += in ? __ldg(bgp + a.N + i) : 0.f;
+            accA[i] += (t.n0 + 128 * grp + i < a.N) ? __ldg(bo + i) : 0.f;
+            accB[i] += (t.n0 + 128 * grp + 64 + i < a.N) ? __ldg(bo + 64 + i) : 0.f;
           }
         }
-        if (ext) act_mul_array<__nv_bfloat16, true>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
-        else act_mul_array<__nv_bfloat16, false>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
-        const bool bf = a.dtype == B200MOE_DTYPE_BF16;
+        if (MODE == 0) {
+          // 64 activations of this token; the other 64 of its quantisation group live in the
+          // same lane of the other promotion group
+          float amax = 0.f;
+          const bool ext = a.bias != nullptr || a.activation == B200MOE_ACT_SWIGLU_OAI;
+          if (a.bias != nullptr) {
+            // gate columns n0 + 64 grp + i and the matching up / linear columns of the same expert
+            const float* bgp = a.bias + static_cast<size_t>(t.e) * 2 * a.N + t.n0 + 64 * grp;
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float2 v = bf ? __bfloat1622float2(__floats2bfloat162_rn(accA[i], accA[i + 1]))
-                              : __half22float2(__floats2half2_rn(accA[i], accA[i + 1]));
-          accA[i] = v.x;
-          accA[i + 1] = v.y;
-          amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
-        }
-        float* red = s_red + buf * 2 * 128;
-        red[grp * 128 + lrow] = amax;
-        if (!warps_meet(smem_u32(bar_meet8), meet8_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
-        amax = fmaxf(red[lrow], red[128 + lrow]);
-        const float sc = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
-        const float inv = __fdiv_rn(1.0f, sc);
-        const int r = t.row0 + lrow;
-        if (grp == 0) a.out_scale[static_cast<size_t>(t.n0 / 128) * a.ld_xscale + r] = sc;
-        uint32_t pk[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          // two values per conversion instruction
-          const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(accA[4 * q] * inv, accA[4 * q + 1] * inv),
-                                                       __NV_SATFINITE, __NV_E4M3);
-          const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(accA[4 * q + 2] * inv, accA[4 * q + 3] * inv),
-                                                       __NV_SATFINITE, __NV_E4M3);
-          pk[q] = lo | (hi << 16);
-        }
-        uint8_t* dst = a.out_q + static_cast<size_t>(r) * a.ld_out + t.n0 + 64 * grp;
-        st_global_v8(dst, pk);
-        st_global_v8(dst + 32, pk + 8);
-      } else if (a.out_pairs != nullptr) {
-        // The pair's row, weighted and rounded to the 16-bit type.  A thread owns 128 contiguous columns of one row and
-        // stores them as whole sectors straight from its registers.  (Turning them in shared memory so that a store
-        // covers eight rows made the tail 4700 cycles of a 20000-cycle tile: 4096 tokens 3205 -> 3065 us.)
-        const float scale = w_on_input ? 1.0f : gam;
-        const bool bf = a.dtype == B200MOE_DTYPE_BF16;
-        if (orow >= 0) {
-          uint8_t* dst = reinterpret_cast<uint8_t*>(s_col_ptr[buf * 128 + lrow]) + (t.n0 + 128 * grp) * 2;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float* src = (q < 4 ? accA : accB) + 16 * (q & 3);
-            uint32_t w[8];
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-              const float lo = src[2 * b] * scale, hi = src[2 * b + 1] * scale;
-              if (bf) {
-                __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-                w[b] = *reinterpret_cast<uint32_t*>(&v);
-              } else {
-                __half2 v = __floats2half2_rn(lo, hi);
-                w[b] = *reinterpret_cast<uint32_t*>(&v);
-              }
+            for (int i = 0; i < 64; ++i) {
+              const bool in = t.n0 + 64 * grp + i < a.N;
+              accA[i] += in ? __ldg(bgp + i) : 0.f;
+              accB[i] += in ? __ldg(bgp + a.N + i) : 0.f;
             }
-            if (t.n0 + 128 * grp < a.N) st_global_v8(dst + 32 * q, w);
           }
-        }
-        if (orow >= 0 && t.n0 == 0 && grp == 0) mark_pair_valid(a, orow);
-      } else if (orow >= 0) {
-        const float scale = w_on_input ? 1.0f : gam;
-        float* out = reinterpret_cast<float*>(s_col_ptr[buf * 128 + lrow]) + t.n0 + 128 * grp;
-        if (t.n0 + 128 * grp < a.N) {
+          if (ext) act_mul_array<__nv_bfloat16, true>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
+          else act_mul_array<__nv_bfloat16, false>(accA, accB, w_on_input, false, act_params(a), [&](int) { return gam; });
+          const bool bf = a.dtype == B200MOE_DTYPE_BF16;
+#pragma unroll
+          for (int i = 0; i < 64; i += 2) {
+            const float2 v = bf ? __bfloat1622float2(__floats2bfloat162_rn(accA[i], accA[i + 1]))
+                                : __half22float2(__floats2half2_rn(accA[i], accA[i + 1]));
+            accA[i] = v.x;
+            accA[i + 1] = v.y;
+            amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
+          }
+          float* red = s_red + buf * 2 * 128;
+          red[grp * 128 + lrow] = amax;
+          if (!warps_meet(smem_u32(bar_meet8), meet8_phase, lane, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+          amax = fmaxf(red[lrow], red[128 + lrow]);
+          const float sc = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
+          const float inv = __fdiv_rn(1.0f, sc);
+          const int r = t.row0 + lrow;
+          if (grp == 0) a.out_scale[static_cast<size_t>(t.n0 / 128) * a.ld_xscale + r] = sc;
+          uint32_t pk[16];
 #pragma unroll
           for (int q = 0; q < 16; ++q) {
-            asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(out + 4 * q), "f"(accA[4 * q] * scale),
-                         "f"(accA[4 * q + 1] * scale), "f"(accA[4 * q + 2] * scale), "f"(accA[4 * q + 3] * scale)
-                         : "memory");
-            asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(out + 64 + 4 * q),
-                         "f"(accB[4 * q] * scale), "f"(accB[4 * q + 1] * scale), "f"(accB[4 * q + 2] * scale),
-                         "f"(accB[4 * q + 3] * scale)
-                         : "memory");
+            // two values per conversion instruction
+            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(accA[4 * q] * inv, accA[4 * q + 1] * inv),
+                                                         __NV_SATFINITE, __NV_E4M3);
+            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(accA[4 * q + 2] * inv, accA[4 * q + 3] * inv),
+                                                         __NV_SATFINITE, __NV_E4M3);
+            pk[q] = lo | (hi << 16);
+          }
+          uint8_t* dst = a.out_q + static_cast<size_t>(r) * a.ld_out + t.n0 + 64 * grp;
+          st_global_v8(dst, pk);
+          st_global_v8(dst + 32, pk + 8);
+        } else if (a.out_pairs != nullptr) {
+          // The pair's row, weighted and rounded to the 16-bit type.  A thread owns 128 contiguous columns of one row and
+          // stores them as whole sectors straight from its registers.  (Turning them in shared memory so that a store
+          // covers eight rows made the tail 4700 cycles of a 20000-cycle tile: 4096 tokens 3205 -> 3065 us.)
+          const float scale = w_on_input ? 1.0f : gam;
+          const bool bf = a.dtype == B200MOE_DTYPE_BF16;
+          if (orow >= 0) {
+            uint8_t* dst = reinterpret_cast<uint8_t*>(s_col_ptr[buf * 128 + lrow]) + (t.n0 + 128 * grp) * 2;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float* src = (q < 4 ? accA : accB) + 16 * (q & 3);
+              uint32_t w[8];
+#pragma unroll
+              for (int b = 0; b < 8; ++b) {
+                const float lo = src[2 * b] * scale, hi = src[2 * b + 1] * scale;
+                if (bf) {
+                  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+                  w[b] = *reinterpret_cast<uint32_t*>(&v);
+                } else {
+                  __half2 v = __floats2half2_rn(lo, hi);
+                  w[b] = *reinterpret_cast<uint32_t*>(&v);
+                }
+              }
+              if (t.n0 + 128 * grp < a.N) st_global_v8(dst + 32 * q, w);
+            }
+          }
+          if (orow >= 0 && t.n0 == 0 && grp == 0) mark_pair_valid(a, orow);
+        } else if (orow >= 0) {
+          const float scale = w_on_input ? 1.0f : gam;
+          float* out = reinterpret_cast<float*>(s_col_ptr[buf * 128 + lrow]) + t.n0 + 128 * grp;
+          if (t.n0 + 128 * grp < a.N) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(out + 4 * q), "f"(accA[4 * q] * scale),
+                           "f"(accA[4 * q + 1] * scale), "f"(accA[4 * q + 2] * scale), "f"(accA[4 * q + 3] * scale)
+                           : "memory");
+              asm volatile("red.global.v4.f32.add [%0], {%1, %2, %3, %4};" ::"l"(out + 64 + 4 * q),
+                           "f"(accB[4 * q] * scale), "f"(accB[4 * q + 1] * scale), "f"(accB[4 * q + 2] * scale),
+                           "f"(accB[4 * q + 3] * scale)
+                           : "memory");
+            }
           }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
+        t_tail += static_cast<unsigned long long>(clock64() - tail_t0);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[buf]));
-      t_tail += static_cast<unsigned long long>(clock64() - tail_t0);
+      if (threadIdx.x == 4 * 32) {
+        STALL_ADD8(5, w_pfull);
+        STALL_ADD8(6, w_sfull);
+        STALL_ADD8(7, t_tail);
+        STALL_ADD8(11, static_cast<unsigned long long>(clock64() - role_t0));
+      }
     }
-    if (threadIdx.x == 4 * 32) {
-      STALL_ADD8(5, w_pfull);
-      STALL_ADD8(6, w_sfull);
-      STALL_ADD8(7, t_tail);
-      STALL_ADD8(11, static_cast<unsigned long long>(clock64() - role_t0));
-    }
-  }
-
   }
 
   // ---- teardown
