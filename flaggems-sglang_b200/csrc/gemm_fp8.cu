@@ -379,8 +379,8 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 // path: the tile's coordinates (decoded by the table warp), the activation scales (a ring filled per slice, which also
 // frees the room of a fourth stage).  A warp whose 32 rows are all padding (three of four in the block of a cold expert)
 // keeps in step with the others and promotes nothing, which leaves the board's power to the rest.  256 experts,
-// zipf-skewed routing, 4096 tokens: 3367 -> 3140 us with the first two, 3205 -> 3058 (another board) with direct stores and
-// idle warps; 512 tokens 1093 -> 998, 1045 -> 984.
+// zipf-skewed routing, one board: 4096 tokens 3045 us, 512: 1056; with the tables on the promotion's path, results turned in
+// shared memory before the store and padding rows promoted 3402 and 1155.
 // Tried and slower: sixteen promotion warps, 32-column reads, scalar FMAs, partial buffers released by halves, hot and
 // cold experts' tiles interleaved.
 // warps 0-3: TMA, MMA, tables, idle; warps 4-11: promotion.  Launched with 168 registers a thread, the

@@ -1,4 +1,4 @@
-// 16-bit grouped expert GEMMs on CTA pairs (tcgen05.mma.cta_group::2) for blocks of more than 64 tokens.
+// 16-bit grouped expert GEMMs on CTA pairs (tcgen05.mma.cta_group::2) for token blocks of 128 and more.
 //
 // Two CTAs of a cluster share one tile of 256 weight rows x N tokens, N = 32..256 in steps of 32: weights sit
 // on the instruction's M side (each CTA stages its 128 rows), the tokens on its N side (each CTA
@@ -38,9 +38,14 @@
 // Asking for the weights in L2 ahead of the ring (cp.async.bulk.prefetch.tensor, 4 to 32 stages) was slower
 // at every size: 807 us without, 843 to 978 us with, at 1000 tokens of the Mixtral-shaped layer.
 //
-// What bounds it: the board's power cap at 4096 tokens (tensor pipe 90 % busy at 1.25 GHz, 2.45 ms against 2.74
-// for 128-token blocks on single CTAs), the weights' way from HBM at 1000 tokens (807 us, 975 before),
-// the activation epilogue at K = 1280 (1280 x 3072 x 64 experts, 2048 tokens: 605 us with routing, 729 before).
+// What bounds it, from cycle counters around the waits:
+//   4096 tokens of the Mixtral-shaped layer: the tensor pipe, 476 cycles per stage for 464 of MMA, at the clock that the
+//     board's power cap leaves (1.15 - 1.25 GHz; 2.41 - 2.46 ms against 2.65 - 2.70 for 128-token blocks on single CTAs);
+//   1000 tokens: 403 - 459 cycles per stage for about 350 of MMA, in a train of calls and after a pause; the weights' way from
+//     HBM is the nearest other limit (739 - 765 us, 833 - 873 before);
+//   K = 1280 (1280 x 3072 x 64 experts, 2048 tokens): the activation epilogue in the first GEMM, whose warps wait only 5 % of the
+//     time for a tile and hold the accumulators for 13 % of the MMA thread's; HBM in the second (496 - 500 us with
+//     routing, 707 before).
 //
 // Every wait is bounded (common.cuh); the cluster barriers at start and end are reached by every
 // thread whatever happened in between.

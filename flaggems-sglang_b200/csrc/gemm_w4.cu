@@ -6,30 +6,34 @@
 // takes its A operand: the expanded weights never touch shared memory, which carries only the packed
 // rows and the tokens.  (Expanding into shared memory moved 104 KiB per 64 k through it for 512 cycles of MMA.)
 //
-// Two variants of the same kernel:
+// Two variants of the same kernel (GemmArgs::w4_var):
 //   NT = 0       any number of tokens per tile (16..192, dealt out evenly over an expert's tiles); the operand is
 //                (q - zero) * scale, rounded once to fp16, and the reduction accumulates in tensor memory.
 //   NT = 16, 32  decode: a tile is one block of NT tokens; the operand is the exact integer q - zero, each group's
 //                sum goes into a partial accumulator of its own and is added as acc += scale * sum in fp32 by the
-//                promotion warps.  Weights and activations are then exact up to the fp32 sums.  (The version before
-//                this one multiplied 20-bit integers split into three byte planes: three times the accumulator columns and
-//                activation bytes, and a kernel in front to split them.)
+//                promotion warps.  Weights and activations are then exact up to the fp32 sums.
 //                NT = 16 expands nothing: a masked nibble already is the fp16 subnormal q * 2^-24, and eight more MMAs per
 //                group add -zero (times the same 2^-24) against every k.  The schedulers, which all roles
-//                share, then see 7 instructions per eight weights instead of 9, none of them half-precision arithmetic.  2
-//                tokens of the Mixtral-shaped layer 111.8 -> 102.8 us, 4: 164.7 -> 156.7, 16: 222 -> 219, 32: 234 -> 232.
-//                At NT = 32 the extra MMAs are the longer path (64 tokens 269 -> 285).
+//                share, then see 7 instructions per eight weights instead of 9, none of them half-precision arithmetic
+//                (Mixtral-shaped layer, us, expanded / unexpanded: 2 tokens 111.8 / 102.8, 4: 164.7 / 156.7, 16: 222 / 219).
+//                At NT = 32 the extra MMAs are the longer path (64 tokens 269 / 285).
 //
 // Packed rows and tokens have rings of their own: the packed rows of a group are needed a conversion (about 900 cycles)
 // earlier than its tokens, and at 192 tokens only three stages of tokens fit.  The MMA thread works on units of one (NT =
 // 0) or two groups and commits once per unit to one barrier, on which the token producer, the conversion warps and
 // the promotion warps all wait; with three commits and three waits per group that thread set the pace at decode.
 //
-// What bounds it: with many tokens the MMA thread and the conversion together (about 700 cycles a group at 192 tokens,
-// either of them; two operand stages keep them apart), at decode sizes the hand-over between them (about 650 cycles a
-// group, of which HBM needs 380).  Mixtral-shaped layer (8 experts, top-2), us per call, against 128-token blocks on
-// the M side with the nibbles expanded into shared memory: 64 tokens 269 (368), 256: 374 (511), 600: 560 (921), 2048:
-// 1455 (2037); against the integer kernel: 2 tokens 103 (123), 4: 157 (160), 16: 219 (227), 32: 230 (242).
+// What bounds it, from cycle counters around every wait on the Mixtral-shaped layer (8 experts, top-2):
+//   2048 tokens  the MMAs: a unit of the first GEMM takes 894 cycles, 704 of them MMAs of 176 tokens; its thread waits 9 %
+//                of the time for operands and 10 % for tokens, never for an accumulator.  The conversion keeps the same pace
+//                (1786 cycles per group and set, two sets) and waits 23 % of the time for a free operand slot.
+//   32 tokens    no single role.  A unit takes 1047 cycles in the first GEMM and 1273 in the second, where HBM needs 770; the
+//                MMA thread spends about 650 issuing its 32 MMAs of 16 tokens, and waits 19 % of the time for operands, 10 %
+//                for tokens and 9 % for partial accumulators (second GEMM: 25 %, whose tails add 16 tokens to the combine
+//                buffer with atomics).  A conversion set is busy about 1000 cycles per group of its own.
+// us per call on one board: 2 tokens 124, 4: 158, 16: 215, 32: 222, 64: 258, 256: 368, 600: 552, 2048: 1423 (integer MMAs on
+// three byte planes up to 32 tokens, above them 128-token blocks on the M side with the nibbles expanded into shared memory:
+// 144, 178, 237, 244, 365, 494, 939, 2027).
 //
 // Warps: 0 packed rows, 1 MMA, 2 tokens, from 4 on the conversion (two or three sets of four warps), then the epilogue or
 // promotion (one or two groups of four).

@@ -405,7 +405,7 @@ moe_gemv_down_kernel(const GemvArgs a) {
 // ==========================================================================================
 // int4 (AWQ) weights: the same two launches on integer dot products.
 //
-// The activations take the form the integer tensor-core kernels use (gemm_w4.cu): per 128-k group
+// The activations become integers: per 128-k group
 // a power-of-two scale f = 2^(e-18) for a group maximum in [2^e, 2^(e+1)) and the exact integers
 // v = rint(x / f), |v| < 2^19, as three signed byte planes v = p0 + 256 p1 + 65536 p2.  A packed
 // word holds eight weights; `w & 0x0F0F0F0F` and `(w >> 4) & 0x0F0F0F0F` are their raw nibbles as

@@ -8,10 +8,11 @@ namespace b200moe {
 namespace {
 
 // A warp copies 2 KiB of a row at a time: one row id, then four 16-byte loads per lane, then the stores.  What bounds it is
-// the write to HBM at prefill sizes and two memory latencies at decode; with a row id and a 64-bit division per
-// 16-byte chunk it was bound by its instructions (32768 rows of 7168 bytes: 118 -> 80 us; a decode graph of the 128-expert
-// layer 182.0 -> 179.4).  Padding rows are left alone, whatever they hold: every GEMM keeps a row's results to itself
-// and none of a padding row's is ever stored where it is read.  (Zeroing them was three quarters of the writes of a 64-token call on 256 experts; quantising them, likewise: 439 -> 431 us for that call.)
+// the write to HBM at prefill sizes and two memory latencies at decode (a row id and a 64-bit division per 16-byte chunk
+// bound it by its instructions: 32768 rows of 7168 bytes 118 us, 80 like this; a decode graph of the 128-expert layer
+// 182.0 and 179.4).  Padding rows are left alone, whatever they hold: every GEMM keeps a row's results to itself and none
+// of a padding row's is ever stored where it is read.  (Quantising and zeroing them, three quarters of the rows of a
+// 64-token call on 256 experts, cost 8 us of 439.)
 // The same launch clears the fp32 combine buffer (`zero`, `zero_chunks`).
 // With sc_src: the rows are already quantised (one byte per element) and each has G group scales
 // [tokens][G]; they are re-laid group-major for the GEMMs, sc_dst [G][ld].

@@ -119,8 +119,8 @@ def test_fp8_many_pairs_stored_per_pair(cuda_device, masked):
 
 
 def test_alignment_on_many_ctas_matches_single_cta(cuda_device, monkeypatch):
-    """From 8192 slots on, the alignment runs on 32 CTAs in three launches; it must order the rows
-    exactly like the single-CTA kernel.  The FP8 path with pair rows has no atomics, so the two
+    """From 1024 slots on, the alignment runs on a cluster of eight CTAs; it must order the rows
+    exactly like a single one.  The FP8 path with pair rows has no atomics, so the two
     outputs must be bit-equal."""
     import flaggems_sglang_b200 as F
     h, i, e, k, m = 2048, 256, 64, 8, 1100          # 8800 slots, skewed routing, some experts empty

@@ -153,8 +153,9 @@ def _awq_case(h, i, e, k, m, seed, device):
 @pytest.mark.parametrize("h,i,e,k,m", [(1024, 512, 8, 2, 1), (4096, 1024, 8, 2, 1), (512, 384, 64, 8, 2),
                                         (256, 128, 16, 4, 1), (2048, 1152, 64, 4, 3)])
 def test_gemv_int4_integer_dot_products(cuda_device, h, i, e, k, m):
-    """int4 (AWQ) weights: dp4a on raw nibbles and three int8 activation planes, the arithmetic of the
-    integer tensor-core kernels, so the two paths agree far inside the tolerance."""
+    """int4 (AWQ) weights: dp4a on raw nibbles and three int8 activation planes.  The grouped decode
+    kernels, too, multiply exact integers q - zero and scale a group's sum in fp32, so the two paths agree far
+    inside the tolerance."""
     import flaggems_sglang_b200 as F
     d = cuda_device
     x, tw, ids, q1, q2, kw, p1, p2 = _awq_case(h, i, e, k, m, seed=h + m, device=d)

@@ -70,8 +70,8 @@ def test_int4_through_reference_signature(cuda_device):
 
 @pytest.mark.parametrize("m,bt", [(20, 16), (60, 32), (300, 64), (300, 128)])
 def test_int4_bias_and_clamped_swiglu(cuda_device, m, bt):
-    """Per-expert biases and the bias variant's activation on both int4 kernels (integer MMAs for
-    blocks of 16 / 32 tokens, fp16 operands above)."""
+    """Per-expert biases and the bias variant's activation on every int4 variant (exact integers and
+    group sums for blocks of 16 / 32 tokens, operands rounded to fp16 above)."""
     import flaggems_sglang_b200 as F
     from flaggems_sglang_b200.quant import repack_awq_for_kernel
     h, i, e, k = 512, 256, 4, 2
