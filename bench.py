@@ -58,8 +58,8 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the
 # ncu capture summarised under profiles/ (None until such a capture exists for the workload).
-NCU_TRAFFIC = {("mixtral", 4096): {"kernel": "moe_gemm_tc_kernel<gate/up>", "bytes": 2189100000,
-                                   "source": "profiles/moe_gemm_tc_mixtral_m4096_launch_list.md"}}
+NCU_TRAFFIC = {("mixtral", 4096): {"kernel": "moe_gemm_tc2_kernel<gate/up>", "bytes": 3404000000,
+                                   "source": "profiles/moe_gemm_tc2_mixtral_m4096_launch_list.md"}}
 
 
 def load_peaks():
