@@ -232,7 +232,7 @@ int check_cfg(const b200moe_cfg* c) {
   } else if (c->wmode == B200MOE_W_INT4_AWQ) {
     if (c->H % 128 != 0 || c->I % 128 != 0) return B200MOE_ERR_UNSUPPORTED;   // whole groups of 128
     if (c->dtype != B200MOE_DTYPE_FP16) return B200MOE_ERR_UNSUPPORTED;
-    if ((c->flags & B200MOE_FLAG_SIMT) || !gemm_w4_ok(c->E)) return B200MOE_ERR_UNSUPPORTED;
+    if (c->flags & B200MOE_FLAG_SIMT) return B200MOE_ERR_UNSUPPORTED;
   } else {
     return B200MOE_ERR_UNSUPPORTED;
   }
@@ -403,6 +403,7 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   const bool pdl = (c->flags & B200MOE_FLAG_NO_PDL) == 0;
   int rc;
   if (w4 && (quant == nullptr || quant->w1_sz == nullptr || quant->w2_sz == nullptr)) return B200MOE_ERR_BAD_ARG;
+  if (w4 && !gemm_w4_ok(c->E)) return B200MOE_ERR_UNSUPPORTED;
 
   // cleared alongside the first row mover: the fp32 combine buffer, or the pairs' validity bytes
   // when rows are stored per pair

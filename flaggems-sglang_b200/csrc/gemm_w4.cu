@@ -75,7 +75,8 @@ static_assert(W4Geo<16>::kWords >= 2 * W4Geo<16>::kPacked + W4Geo<16>::kSets + 2
 
 template <int NT>
 __host__ __device__ __forceinline__ size_t w4_turn_offset(int E) {
-  return (W4Geo<NT>::kTableBytes + 2 * static_cast<size_t>(E + 1) * 4 + 127) & ~static_cast<size_t>(127);
+  // prefixes over the experts: granules and tiles, which at decode are the same
+  return (W4Geo<NT>::kTableBytes + (NT > 0 ? 1 : 2) * static_cast<size_t>(E + 1) * 4 + 127) & ~static_cast<size_t>(127);
 }
 template <int NT>
 __host__ __device__ __forceinline__ size_t w4_fixed_bytes(int E, int mode, bool pairs) {
@@ -150,7 +151,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   int* s_nmax = reinterpret_cast<int*>(tmem_slot + 2);
   float* s_rate = reinterpret_cast<float*>(tmem_slot + 4);                   // [6]
   int* s_gran = reinterpret_cast<int*>(smem + G::kTableBytes);               // [E+1] granules (NT > 0: blocks) before e
-  int* s_tile = s_gran + (a.E + 1);                                          // [E+1]
+  int* s_tile = NT > 0 ? s_gran : s_gran + (a.E + 1);                        // [E+1] tiles before e
   uint8_t* s_turn = smem + w4_turn_offset<NT>(a.E);
   const size_t fixed = w4_fixed_bytes<NT>(a.E, MODE, a.out_pairs != nullptr);
   uint8_t* packed = smem + fixed - G::kPacked * G::kPackedStage;
@@ -205,9 +206,6 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       const int widest = plan_row_tiles(min(maxg, a.BT / kGranW4), s_gran, a.E, s_tile, lane);
       if (lane == 0) *s_nmax = widest * kGranW4;
     }
-  } else if (warp == 0) {
-    plan_row_tiles(1, s_gran, a.E, s_tile, lane);   // a tile per block
-    if (lane == 0) *s_nmax = NT;
   }
   tc_fence_before();
   __syncthreads();
@@ -570,7 +568,7 @@ int launch_mode(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4Token
 
 }  // namespace
 
-// Two prefixes over the experts beside at least two stages of tokens.
+// The prefixes over the experts beside at least two stages of tokens.
 bool gemm_w4_ok(int E) {
   return kSmemLimit - 1024 >= w4_fixed_bytes<0>(E, 1, false) + 2 * static_cast<size_t>(w4_token_bytes(kMaxGranW4 * kGranW4, 1)) &&
          kSmemLimit - 1024 >= w4_fixed_bytes<32>(E, 1, false) + 2 * static_cast<size_t>(w4_token_bytes(32, 2));

@@ -84,6 +84,7 @@ def test_matrix_vector_path_selection(built_lib):
     assert uses(1, 2048, 768, 128, 8, block_tokens=16) == 0    # the caller asked for the grouped GEMMs
     assert uses(1, 7168, 2048, 256, 8, wmode=_lib.W_FP8_BLOCK) == 0
     assert uses(1, 4096, 14336, 8, 2, wmode=_lib.W_INT4_AWQ, dtype=1) == 1
+    assert uses(1, 128, 128, 8000, 2, wmode=_lib.W_INT4_AWQ, dtype=1) == 1     # no table of the experts on this path
     assert uses(1, 4096, 14336, 8, 2, flags=_lib.FLAG_SIMT) == 0
     assert uses(1, 2048, 768, 128, 8, flags=_lib.FLAG_NO_MATRIX_VECTOR) == 0
     assert uses(1, 4096, 32768, 8, 4) == 0                     # 4 x 32768 fp32 activations do not fit in shared memory
@@ -176,4 +177,5 @@ def test_workspace_grows_with_the_optional_paths(built_lib):
     assert ws(4096, 7168, 2048, 256, 8, _lib.W_FP8_BLOCK, flags=_lib.FLAG_X_FP8) < big_fp8     # no quantise-once buffers
     assert ws(32, 4096, 14336, 8, 2, _lib.W_INT4_AWQ, dtype=_lib.DTYPE_FP16) > 0
     assert ws(32, 4096, 14336, 8, 2, _lib.W_INT4_AWQ) == 0      # int4 needs fp16 activations
+    assert ws(40, 128, 128, 5000, 2, _lib.W_INT4_AWQ, dtype=_lib.DTYPE_FP16) > 0               # any number of experts
     assert ws(64, 1024, 512, 8, 2, _lib.W_16BIT, flags=_lib.FLAG_X_FP8) == 0                   # FP8 rows need FP8 weights

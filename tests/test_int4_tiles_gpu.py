@@ -49,6 +49,32 @@ def test_int4_ragged_tiles(cuda_device, h, i, e, k, m, bt):
                   atol=2e-2, what=f"int4 weight on input {(h, i, e, k, m, bt)}")
 
 
+@pytest.mark.parametrize("m,bt", [(40, 16), (40, 32), (40, 64), (1, 0)])
+def test_int4_many_experts(cuda_device, m, bt):
+    """More experts than any router here serves: the prefixes over them still fit beside the rings."""
+    import flaggems_sglang_b200 as F
+    from flaggems_sglang_b200.quant import quantize_awq, repack_awq_for_kernel
+    from oracle import routing as R
+    h, i, e, k = 256, 128, 5000, 2
+    d = cuda_device
+    g = torch.Generator(device=d).manual_seed(m + bt)
+    q1 = quantize_awq(torch.randn(e, h, 2 * i, generator=g, device=d) * 0.05)
+    q2 = quantize_awq(torch.randn(e, i, h, generator=g, device=d) * 0.05)
+    p1, z1 = repack_awq_for_kernel(*q1)
+    p2, z2 = repack_awq_for_kernel(*q2)
+    x = torch.randn(m, h, generator=g, device=d).to(torch.float16)
+    ids = torch.stack([torch.randperm(e, generator=g, device=d)[:k] for _ in range(m)]).sort(dim=1).values.cpu()
+    ids[:, 0] = ids[:, 0] % 3                  # a few experts with many rows, the first ones
+    ids[0, 1] = e - 1
+    tw = torch.rand(m, k, generator=g, device=d).cpu()
+    r = R.topk_to_routing(tw.numpy(), ids.numpy(), e)
+    routing = tuple(torch.from_numpy(r[n]).to(d) for n in ("hist", "topk_indx", "gate_scal"))
+    out = F.fused_experts(x, p1, p2, routing=(*routing, k), use_int4_w4a16=True, w13_sz=z1, w2_sz=z2, block_tokens=bt)
+    F.check_status()
+    ref = OM.fused_experts_awq(x.cpu(), *[t.cpu() for t in q1], *[t.cpu() for t in q2], tw, ids)
+    assert_parity(out, ref, rtol=2e-2, atol=2e-2, what=f"int4 E=5000 M={m} BT={bt}")
+
+
 @pytest.mark.parametrize("h,i,e,k,m,bt", [(264, 136, 5, 2, 33, 128), (512, 200, 3, 1, 257, 256), (128, 320, 6, 2, 900, 160)])
 def test_pair_kernel_ragged_tiles(cuda_device, h, i, e, k, m, bt):
     import flaggems_sglang_b200 as F
