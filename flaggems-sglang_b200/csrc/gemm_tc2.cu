@@ -39,7 +39,7 @@
 // at every size: 807 us without, 843 to 978 us with, at 1000 tokens of the Mixtral-shaped layer.
 //
 // What bounds it, from cycle counters around the waits:
-//   4096 tokens of the Mixtral-shaped layer: the tensor pipe, 476 cycles per stage for 464 of MMA, at the clock that the
+//   4096 tokens of the Mixtral-shaped layer: the tensor pipe, 476 cycles per stage for about 470 of MMA, at the clock that the
 //     board's power cap leaves (1.15 - 1.25 GHz; 2.41 - 2.46 ms against 2.65 - 2.70 for 128-token blocks on single CTAs);
 //   1000 tokens: 403 - 459 cycles per stage for about 350 of MMA, in a train of calls and after a pause; the weights' way from
 //     HBM is the nearest other limit (739 - 765 us, 833 - 873 before);
