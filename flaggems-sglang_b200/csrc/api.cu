@@ -178,6 +178,7 @@ struct Layout {
   bool pairs2;    // 16-bit GEMMs on CTA pairs: rows padded to 32 per expert, tiles of up to `tile_tokens`
   bool w4_var;    // int4 above decode sizes: rows padded to 16 per expert, tiles of up to `tile_tokens`
   int tile_tokens;
+  bool own;       // decode sizes: the GEMMs sort the slots themselves and fetch the token rows where they lie (gemm_route.cuh)
   int out_rows;   // rows of the fp32 output buffer: tokens, or pairs when nothing is combined
   int orient;     // GEMM tile orientation that goes with BT
   int act_bytes;  // bytes per activation element fed to the GEMMs
@@ -239,6 +240,20 @@ int check_cfg(const b200moe_cfg* c) {
   return B200MOE_OK;
 }
 
+// Calls whose GEMMs sort the slots themselves.  Every CTA counts the slots by itself, 2 to 3 us in front of its first weights
+// against 15 to 20 for the launches of an alignment and a gather.  128 experts, top-8, us with / without them: 8 tokens 90.6 /
+// 80.2, 64: 203 / 188, 200: 209 / 199, 300: 216 / 214.5; int4, 8 experts: 8 tokens 198 / 185, 64: 248 / 230.  Beyond 4096 slots
+// the scan for a tile's slots, which grows with them, would be longer than a tile of a short reduction.
+constexpr int kOwnMaxSlots = 4096, kOwnMaxExperts = 1024;
+bool route_by_gemm(const b200moe_cfg* c, const Layout& L) {
+  if (c->flags & B200MOE_FLAG_SIMT) return false;
+  if (L.pairs2 || L.w4_var || L.BT > 32 || (c->flags & B200MOE_FLAG_X_FP8)) return false;
+  // FP8 beyond 1024 slots: the blocks of hot experts make tiles short beside a scan of the slots (256 experts, zipf-skewed, us
+  // aligned / sorted by the GEMMs: 8 tokens 200 / 191, 200 tokens 656 / 661)
+  if (L.P > (c->wmode == B200MOE_W_FP8_BLOCK ? 1024 : kOwnMaxSlots) || c->E > kOwnMaxExperts) return false;
+  return c->wmode != B200MOE_W_INT4_AWQ || gemm_w4_own_ok(c->E, L.P, L.BT);
+}
+
 int query_sms(const b200moe_cfg* c);
 bool reference_rounds_pairs(int P, int E, int n, int k, int sms);
 
@@ -261,6 +276,7 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
     L->BT = 16;
   }
   L->P = c->M * c->topk;
+  L->own = route_by_gemm(c, *L);
   int cap = align_capacity(L->P, c->E, L->BT);
   if (cap < 0) return B200MOE_ERR_TOO_LARGE;
   cap = static_cast<int>(align_up(static_cast<size_t>(cap > 0 ? cap : 1), L->BT));
@@ -374,6 +390,16 @@ int align_into_workspace(const b200moe_cfg* c, const Layout& L, uint8_t* ws, con
                             (c->flags & B200MOE_FLAG_ALIGN_ONE_CTA) != 0);
 }
 
+RouteSource topk_source(const b200moe_cfg* c, const void* ids, int is64, const int32_t* expert_map, const float* weights) {
+  RouteSource r = {};
+  r.ids = ids;
+  r.is64 = is64;
+  r.map = expert_map;
+  r.map_len = c->n_global_experts;
+  r.weights = weights;
+  return r;
+}
+
 // Expert parallelism: where the down projection's output rows go (the buffers of the ranks that
 // own the tokens) instead of this call's workspace.
 struct PeerOut {
@@ -385,11 +411,12 @@ struct PeerOut {
   const FlagWait* rows_wait = nullptr;   // the gather waits for the peers' "rows" flags in its prologue
 };
 
-// Everything after the internal routing tables exist in the workspace.  With `peers` the results
+// Everything after the internal routing tables exist in the workspace; `route`: there are none, the GEMMs sort for
+// themselves (Layout::own).  With `peers` the results
 // land on their owners and nothing is cleared or converted here.
 int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void* w1, const void* w2,
                 const b200moe_quant* quant, uint8_t* ws, void* out, int32_t* status, cudaStream_t st,
-                int slot, const PeerOut* peers = nullptr) {
+                int slot, const RouteSource* route, const PeerOut* peers = nullptr) {
   const int sms = query_sms(c);
   int* meta = reinterpret_cast<int*>(ws + L.meta);
   int* blk_off = reinterpret_cast<int*>(ws + L.blk_off);
@@ -411,8 +438,20 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   size_t zero_bytes = L.pair_rows ? align_up(static_cast<size_t>(L.P), 16)
                                   : static_cast<size_t>(L.out_rows) * c->H * 4;
   if (peers != nullptr) zero_bytes = 0;   // the owners cleared their buffers before they signalled "ready"
-  if (fp8) {
-    if (quant == nullptr || quant->w1_scale == nullptr || quant->w2_scale == nullptr) return B200MOE_ERR_BAD_ARG;
+  const bool own = route != nullptr;
+  bool cleared = false;      // own: a kernel in front of GEMM-1 puts the rows in order and clears the combine buffer
+  rc = B200MOE_OK;
+  if (fp8 && (quant == nullptr || quant->w1_scale == nullptr || quant->w2_scale == nullptr)) return B200MOE_ERR_BAD_ARG;
+  if (own) {
+    if (fp8) {
+      rc = launch_group_quant_routed(x, c->dtype, xs, reinterpret_cast<float*>(ws + L.xs_scale), *route, L.P, c->E, L.BT, c->topk,
+                                     c->M, c->H, L.cap, zero, zero_bytes, sms, st, pdl);
+      cleared = true;
+    } else if (w4) {
+      rc = launch_gather_routed(x, xs, *route, L.P, c->E, L.BT, c->topk, c->H * 2, zero, zero_bytes, sms, st, pdl);
+      cleared = true;
+    }
+  } else if (fp8) {
     if (c->flags & B200MOE_FLAG_X_FP8) {
       // rows arrive quantised (e.g. from an expert-parallel dispatch that sends bytes): gather only
       if (quant->x_scale == nullptr) return B200MOE_ERR_BAD_ARG;
@@ -464,6 +503,15 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     g1.act_alpha = quant->swiglu_alpha;
     g1.act_limit = quant->swiglu_limit;
   }
+  if (own) {
+    g1.route = *route;
+    g1.route.own = 1;
+    // the quantisation of the rows, or their gathering, stands between the routing input and GEMM-1
+    g1.route.early = cleared ? 1 : 0;
+    g1.rows = x;
+    g1.zero = zero;
+    g1.zero_chunks = cleared ? 0 : static_cast<long long>(zero_bytes / 16);
+  }
   if (fp8) {
     g1.w_scale = quant->w1_scale;
     g1.w_scale_rows = (2 * c->I + 127) / 128;
@@ -485,6 +533,8 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   g2.out = out32;
   g2.ld_out = c->H;
   g2.max_split = 0;
+  g2.route.early = g1.route.own;
+  g2.zero_chunks = 0;
   if (c->flags & B200MOE_FLAG_NO_COMBINE) g2.topk = 1;   // output row = pair slot instead of token
   g2.bias = quant != nullptr ? quant->b2 : nullptr;
   if (!fp8 && (c->flags & B200MOE_FLAG_MIMIC_ROUNDING)) {
@@ -817,10 +867,14 @@ int b200moe_forward_topk(const b200moe_cfg* cfg, const void* x, const void* w1, 
   rc = run_gemv(cfg, L, x, w1, w2, quant, topk_weights, topk_ids, expert_map, nullptr, nullptr, nullptr, ws, out, st,
                 slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
-  rc = align_into_workspace(cfg, L, ws, topk_ids, (cfg->flags & B200MOE_FLAG_IDS_I64) ? 1 : 0, expert_map,
-                            topk_weights, st);
+  const int is64 = (cfg->flags & B200MOE_FLAG_IDS_I64) ? 1 : 0;
+  if (L.own) {
+    const RouteSource src = topk_source(cfg, topk_ids, is64, expert_map, topk_weights);
+    return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, &src);
+  }
+  rc = align_into_workspace(cfg, L, ws, topk_ids, is64, expert_map, topk_weights, st);
   if (rc != B200MOE_OK) return rc;
-  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot);
+  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr);
 }
 
 int b200moe_route_topk(const b200moe_router* router, const void* logits, int n_tokens, int n_experts, int topk,
@@ -850,13 +904,18 @@ int b200moe_forward_logits(const b200moe_cfg* cfg, const b200moe_router* router,
   int* ids = reinterpret_cast<int*>(ws + L.route_ids);
   const int slot = prof_slot();
   prof_mark(slot, 0, st);
-  rc = launch_route_topk(router, logits, cfg->M, cfg->E, cfg->topk, tw, ids, query_sms(cfg), st);
+  rc = launch_route_topk(router, logits, cfg->M, cfg->E, cfg->topk, tw, ids, query_sms(cfg), st,
+                         (cfg->flags & B200MOE_FLAG_NO_PDL) == 0);
   if (rc != B200MOE_OK) return rc;
   rc = run_gemv(cfg, L, x, w1, w2, quant, tw, ids, expert_map, nullptr, nullptr, nullptr, ws, out, st, slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
+  if (L.own) {
+    const RouteSource src = topk_source(cfg, ids, 0, expert_map, tw);
+    return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, &src);
+  }
   rc = align_into_workspace(cfg, L, ws, ids, 0, expert_map, tw, st);
   if (rc != B200MOE_OK) return rc;
-  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot);
+  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr);
 }
 
 int b200moe_forward_routed(const b200moe_cfg* cfg, const void* x, const void* w1, const void* w2,
@@ -875,13 +934,20 @@ int b200moe_forward_routed(const b200moe_cfg* cfg, const void* x, const void* w1
   prof_mark(slot, 0, st);
   rc = run_gemv(cfg, L, x, w1, w2, quant, nullptr, nullptr, nullptr, hist, topk_indx, gate_scal, ws, out, st, slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
+  if (L.own && cfg->wmode != B200MOE_W_FP8_BLOCK) {   // (the quantisation looks its rows up by slot)
+    RouteSource src = {};
+    src.hist = hist;
+    src.topk_indx = topk_indx;
+    src.gate_scal = gate_scal;
+    return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, &src);
+  }
   rc = launch_align_from_routing(hist, topk_indx, gate_scal, L.P, cfg->E, L.BT, L.cap,
                                  reinterpret_cast<int*>(ws + L.sorted_ids),
                                  reinterpret_cast<float*>(ws + L.row_gamma),
                                  reinterpret_cast<int*>(ws + L.blk_off), reinterpret_cast<int*>(ws + L.meta), st,
                                  (cfg->flags & B200MOE_FLAG_NO_PDL) == 0);
   if (rc != B200MOE_OK) return rc;
-  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot);
+  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1097,7 +1163,7 @@ int b200moe_ep_forward(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, void* c
       po.pairs[r] = h + H.pairs;
       po.pair_valid[r] = h + H.pair_valid;
     }
-    if ((rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, &po)) != B200MOE_OK) return rc;
+    if ((rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, nullptr, &po)) != B200MOE_OK) return rc;
     uint8_t* hp[kMaxPeers];
     for (int r = 0; r < ep->world; ++r) hp[r] = reinterpret_cast<uint8_t*>(heaps[r]);
     if ((rc = launch_ep_signal(hp, H, kEpFlagDone, ep->world, ep->rank, st, pdl)) != B200MOE_OK) return rc;

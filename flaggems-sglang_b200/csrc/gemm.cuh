@@ -9,6 +9,20 @@ namespace b200moe {
 // block of 16 wastes nothing and a prefill block of 256 fills the widest shape.
 constexpr int kMaxPeers = 8;   // ranks of one NVSwitch domain that an expert-parallel call may span
 
+// Routing input of a call whose GEMMs sort the slots by expert themselves (gemm_route.cuh).
+struct RouteSource {
+  int own;                   // 1: they do; 0: the tables come from an alignment launch, the rows lie in expert order
+  int early;                 // own: a kernel of this call lies between the routing input and this one (see griddep_wait below)
+  const void* ids;           // [P] expert of each slot, with an optional global -> local map
+  int is64;
+  const int* map;
+  int map_len;
+  const float* weights;      // [P]
+  const int* hist;           // or the routing triple: slots per expert, slots by expert, their weights
+  const int* topk_indx;
+  const float* gate_scal;
+};
+
 struct GemmArgs {
   int mode;        // 0: gate/up projection + activation; 1: down projection + weighted scatter-add
   int dtype;       // B200MOE_DTYPE_* of activations / 16-bit weights
@@ -63,6 +77,10 @@ struct GemmArgs {
   int rows_per_peer;
   void* peer_out[kMaxPeers];          // out (fp32) or out_pairs (16-bit) of every rank
   uint8_t* peer_valid[kMaxPeers];     // pair_valid of every rank (pair rows only)
+  RouteSource route;
+  const void* rows;       // mode 0, route.own: the token rows
+  void* zero;             // mode 0, route.own: the combine buffer, cleared here
+  long long zero_chunks;  // of 16 bytes
 };
 
 // Base address of output row `orow` (row_bytes bytes per row): local, or on the owning rank.
@@ -94,6 +112,7 @@ struct W4TokenMaps {
   CUtensorMap m[12];
 };
 bool gemm_w4_ok(int E);
+bool gemm_w4_own_ok(int E, int P, int BT);
 void gemm_plan_w4(GemmArgs* a);
 // tm_w: packed rows, mode 0 [E][I][2][K/2] in boxes of 64 rows of both halves, mode 1 [E][rows][K/2] in boxes of 128
 // rows; tm_sz: their scale / zero words [E * K/128][2][I] in boxes of 64 of both halves, or [E * K/128][1][rows] in boxes of 128

@@ -21,6 +21,7 @@
 // loader warp that prepares the next tile's per-token tables (output row, routing weight,
 // activation scales by bulk copy, weight scales) in double-buffered shared memory, so that no
 // global-memory latency sits between two tiles of the promotion warps.
+#include "gemm_route.cuh"
 #include "gemm_sched.cuh"
 
 namespace b200moe {
@@ -61,11 +62,13 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * 128);     // [2][128]
   float* s_red = s_col_gam + 2 * 128;                                   // [2][NG][4][64]
   unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + 2 * 2 * 4 * 64);   // [2][128] mode 1: base of each token's output row
-  int* s_blk_off = reinterpret_cast<int*>(s_col_ptr + 2 * 128);         // [E+1]
+  const RowTables rt = row_tables(s_col_ptr + 2 * 128, a.E);            // own tables, or only the blocks' starts
+  int* s_blk_off = rt.blk;                                              // [E+1]
   constexpr int CPT = BT / NG;                                          // token columns per promotion thread
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
+  const bool own = BT <= 32 && a.route.own != 0, early = own && a.route.early != 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -91,17 +94,18 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(a.tmem_cols));
     tmem_relinquish();
   }
-  // everything above touched only shared / tensor memory and kernel parameters; the routing
-  // tables and activations below come from the preceding kernels
-  griddep_wait();
+  // everything above touched only shared / tensor memory and kernel parameters
+  if (!early) griddep_wait();
   griddep_launch_dependents();
-  for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
+  if (own) count_slots(a.route, a.P, a.E, BT, rt);
+  else
+    for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const Ctrl c = make_ctrl(a, MODE == 1);
+  const Ctrl c = make_ctrl(a, own ? s_blk_off[a.E] : a.meta[0], MODE == 1);
   const bool active = static_cast<int>(blockIdx.x) < c.grid_eff;
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;  // output rows advanced per n-tile
   // row offset of the second weight block inside the expert
@@ -113,20 +117,35 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     uint32_t phase = 0;
     long long issued = 0;
     bool ok = true;
+    auto load_weights = [&](const TileCoord& t, int kb, int s) {
+      const uint32_t full = smem_u32(&bar_full[s]);
+      const uint32_t sw = smem_u32(smem + static_cast<size_t>(s) * STAGE_BYTES);
+      const int k0 = kb * kStageKBytes;  // one byte per element
+      mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES));
+      tma_load_3d(sw, &tm_w, full, k0, t.n0, t.e);
+      tma_load_3d(sw + kTileBytes, &tm_w, full, k0, second_off + t.n0, t.e);  // rows past the expert zero-fill
+    };
+    // the ring's first round of weights, before the activations may be read
+    int ahead = 0;
+    if (early) {
+      for (int tile = blockIdx.x; ahead < stages && tile < c.total; tile += c.grid_eff) {
+        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+        for (int kb = t.kb0; ahead < stages && kb < t.kb1; ++kb, ++ahead) load_weights(t, kb, ahead);
+      }
+      griddep_wait();
+    }
     for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
       const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
       for (int kb = t.kb0; kb < t.kb1; ++kb) {
-        if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER)) {
-          ok = false;
-          break;
+        if (issued >= ahead) {
+          if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER)) {
+            ok = false;
+            break;
+          }
+          load_weights(t, kb, stage);
         }
-        const uint32_t full = smem_u32(&bar_full[stage]);
-        mbar_arrive_expect_tx(full, static_cast<uint32_t>(STAGE_BYTES));
-        const uint32_t sw = smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES);
-        const int k0 = kb * kStageKBytes;  // one byte per element
-        tma_load_3d(sw, &tm_w, full, k0, t.n0, t.e);
-        tma_load_3d(sw + kTileBytes, &tm_w, full, k0, second_off + t.n0, t.e);  // rows past the expert zero-fill
-        tma_load_2d(sw + W_BYTES, &tm_x, full, k0, t.row0);
+        tma_load_2d(smem_u32(smem + static_cast<size_t>(stage) * STAGE_BYTES) + W_BYTES, &tm_x, smem_u32(&bar_full[stage]),
+                    kb * kStageKBytes, t.row0);
         ++issued;
         if (++stage == stages) {
           stage = 0;
@@ -182,6 +201,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
   } else if (active && warp == 6) {
     // =============================== per-tile table loader ======================
+    griddep_wait();
     const int kb_total = a.kblocks;
     int iter = 0;
     for (int tile = blockIdx.x; tile < c.total; tile += c.grid_eff, ++iter) {
@@ -189,12 +209,13 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const int buf = iter & 1;
       if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
       const int nkb = t.kb1 - t.kb0;
-      for (int cidx = lane; cidx < BT; cidx += 32) {
-        const int slot = a.sorted_ids[t.row0 + cidx];
-        const bool valid = slot >= 0 && slot < a.P;
+      for (int r = 0; r < BT; r += 32) {
+        const int slot = rows_slot(a, rt, BT, t.e, t.row0 + r, BT < 32 ? BT : 32), cidx = r + lane;
+        if (cidx >= BT) continue;
+        const bool valid = slot >= 0;
         const int orow = valid ? (MODE == 1 ? slot / a.topk : slot) : -1;
         s_col_row[buf * 128 + cidx] = orow;
-        s_col_gam[buf * 128 + cidx] = valid ? a.row_gamma[t.row0 + cidx] : 0.f;
+        s_col_gam[buf * 128 + cidx] = rows_weight(a, rt, BT, t.e, t.row0 + r, slot);
         if (MODE == 1 && valid)
           s_col_ptr[buf * 128 + cidx] = reinterpret_cast<unsigned long long>(
               out_row_base(a, a.out, orow, static_cast<size_t>(a.ld_out) * sizeof(float)));
@@ -219,6 +240,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
   } else if (active && warp >= 2 && warp != 6) {
     // =============================== promotion + tail ===========================
+    griddep_wait();
     const int grp = warp < 6 ? 0 : 1;               // promotion group
     const int gw = warp < 6 ? warp - 2 : warp - 7;  // warp inside the group
     const int quad = warp & 3;                      // TMEM lane quadrant (each group covers all four)
@@ -469,7 +491,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const Ctrl c = make_ctrl(a, MODE == 1);
+  const Ctrl c = make_ctrl(a, a.meta[0], MODE == 1);
   const bool active = static_cast<int>(blockIdx.x) < c.grid_eff;
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
@@ -843,7 +865,8 @@ size_t fp8_stage_bytes(const GemmArgs& a) {
 }
 size_t fp8_ctrl_bytes(const GemmArgs& a) {
   return 2 * static_cast<size_t>(kMaxKB) * a.BT * 4 + 2 * 2 * kMaxKB * 4 + 512 /*barriers*/ + 2 * 128 * 8 +
-         2 * 2 * 4 * 64 * 4 + 2 * 128 * 8 + static_cast<size_t>(a.E + 1) * 4 + 64;
+         2 * 2 * 4 * 64 * 4 + 2 * 128 * 8 +
+         (a.route.own ? route_table_bytes(a.E, a.P) : static_cast<size_t>(a.E + 1) * 4) + 64;
 }
 
 template <int MODE, int BT, int NG>

@@ -5,7 +5,6 @@
 
 namespace b200moe {
 
-constexpr int kThreads = 192;
 constexpr int kTileRows = 128;           // weight rows per MMA (the instruction's M)
 constexpr int kStageKBytes = 128;        // bytes of the reduction dim per stage row (one swizzle atom)
 constexpr int kTileBytes = kTileRows * kStageKBytes;  // 16 KiB
@@ -157,9 +156,9 @@ __device__ __forceinline__ ActParams act_params(const GemmArgs& a) {
 }
 
 // Work decomposition for one launch; identical in every thread of every CTA.
-__device__ __forceinline__ Ctrl make_ctrl(const GemmArgs& a, bool may_split) {
+__device__ __forceinline__ Ctrl make_ctrl(const GemmArgs& a, int nblocks, bool may_split) {
   Ctrl c;
-  c.nblocks = a.meta[0];
+  c.nblocks = nblocks;
   c.split = 1;
   if (may_split && !(a.flags & B200MOE_FLAG_NO_SPLIT_K))
     c.split = pick_split(c.nblocks * a.num_nt, a.kblocks, gridDim.x, a.max_split);

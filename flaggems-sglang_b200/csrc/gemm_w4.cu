@@ -35,8 +35,15 @@
 // three byte planes up to 32 tokens, above them 128-token blocks on the M side with the nibbles expanded into shared memory:
 // 144, 178, 237, 244, 365, 494, 939, 2027).
 //
+// Decode calls sort their slots in here (gemm_route.cuh) behind a launch that gathers the rows; the packed rows and their
+// conversion start before those are there.  (Fetching the rows from here was slower: gather4 loads take about 80 cycles each,
+// four rows of 128 bytes, and set the pace of a unit, 32 tokens 205 -> 233 us; a copying warp waits for a proxy fence per unit, 217.)
+// A lane looks one row's slot and weight up and tells the others: one after the other they cost a tile two memory latencies
+// per row (32 tokens 205 -> 200).
+//
 // Warps: 0 packed rows, 1 MMA, 2 tokens, from 4 on the conversion (two or three sets of four warps), then the epilogue or
 // promotion (one or two groups of four).
+#include "gemm_route.cuh"
 #include "gemm_turn.cuh"
 
 namespace b200moe {
@@ -57,7 +64,7 @@ template <int NT>
 struct W4Geo {
   static constexpr int kGroups = NT > 0 ? 2 : 1;
   static constexpr int kPacked = NT > 0 ? 8 : 4;
-  static constexpr int kWords = NT > 0 ? 64 : 16;
+  static constexpr int kWords = NT > 0 ? 48 : 16;
   static constexpr int kPartials = NT == 16 ? 4 : 2;      // units (NT = 0: tiles) whose accumulators are in flight
   // NT = 16: the nibbles go in as they are and the zero points as an operand of their own (8 columns a group)
   static constexpr bool kZeroMma = NT == 16;
@@ -78,9 +85,11 @@ __host__ __device__ __forceinline__ size_t w4_turn_offset(int E) {
   // prefixes over the experts: granules and tiles, which at decode are the same
   return (W4Geo<NT>::kTableBytes + (NT > 0 ? 1 : 2) * static_cast<size_t>(E + 1) * 4 + 127) & ~static_cast<size_t>(127);
 }
+// own_slots: slots of a decode call that sorts them itself (its tables stand in the place of the prefixes), or 0
 template <int NT>
-__host__ __device__ __forceinline__ size_t w4_fixed_bytes(int E, int mode, bool pairs) {
-  return ((w4_turn_offset<NT>(E) + (NT == 0 ? turn_bytes(mode, pairs) : 0) + 1023) & ~static_cast<size_t>(1023)) +
+__host__ __device__ __forceinline__ size_t w4_fixed_bytes(int E, int mode, bool pairs, int own_slots = 0) {
+  return (((NT > 0 && own_slots > 0 ? W4Geo<NT>::kTableBytes + route_table_bytes(E, own_slots)
+                                    : w4_turn_offset<NT>(E) + (NT == 0 ? turn_bytes(mode, pairs) : 0)) + 1023) & ~static_cast<size_t>(1023)) +
          W4Geo<NT>::kPacked * W4Geo<NT>::kPackedStage;
 }
 // tokens of one unit: swizzle atoms of 64 k
@@ -153,7 +162,9 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   int* s_gran = reinterpret_cast<int*>(smem + G::kTableBytes);               // [E+1] granules (NT > 0: blocks) before e
   int* s_tile = NT > 0 ? s_gran : s_gran + (a.E + 1);                        // [E+1] tiles before e
   uint8_t* s_turn = smem + w4_turn_offset<NT>(a.E);
-  const size_t fixed = w4_fixed_bytes<NT>(a.E, MODE, a.out_pairs != nullptr);
+  const bool own = NT > 0 && a.route.own != 0, early = own && a.route.early != 0;
+  const RowTables rt = row_tables(s_gran, a.E);
+  const size_t fixed = w4_fixed_bytes<NT>(a.E, MODE, a.out_pairs != nullptr, own ? a.P : 0);
   uint8_t* packed = smem + fixed - G::kPacked * G::kPackedStage;
   uint8_t* tokens = smem + fixed;
 
@@ -183,9 +194,11 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tmem_alloc(smem_u32(tmem_slot), 512u);
     tmem_relinquish();
   }
-  griddep_wait();
+  if (!early) griddep_wait();
   griddep_launch_dependents();
-  for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_gran[e] = a.blk_off[e];
+  if (NT > 0 && own) count_slots(a.route, a.P, a.E, NT, rt);
+  else
+    for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_gran[e] = a.blk_off[e];
   __syncthreads();
   const int num_nt = a.num_nt;
   if (NT == 0) {
@@ -271,6 +284,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   } else if (warp == 2) {
     if (elect_one()) {
       // =============================== tokens =====================================
+      griddep_wait();       // (the packed rows and their conversion need not wait for the activations)
       int u = 0;
       bool ok = true;
       for (int tile = first; ok && tile < total; tile += stride) {
@@ -447,6 +461,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
   } else {
     // =============================== promotion + tail ============================
+    griddep_wait();
     constexpr int HT = NT > 0 ? NT / G::kTailGroups : 16;         // tokens per thread
     const int grp = (warp - 4 - 4 * G::kSets) >> 2, quad = warp & 3;
     const int row = quad * 32 + lane;
@@ -465,12 +480,15 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       // output row and routing weight of this group's tokens, fetched ahead of the reduction (uniform over the warp)
       int orow[HT];
       float gam[HT];
+      if (MODE == 1 || w_on_input) {      // a lane looks one row up and tells the others
+        const int slot = rows_slot(a, rt, NT, t.e, r0, HT);
+        const float weight = rows_weight(a, rt, NT, t.e, r0, slot);
+        const int token = slot >= 0 ? slot / a.topk : -1;
 #pragma unroll
-      for (int i = 0; i < HT; ++i) {
-        const int slot = (MODE == 1 || w_on_input) ? a.sorted_ids[r0 + i] : 0;
-        const bool valid = slot >= 0 && slot < a.P;
-        orow[i] = valid ? slot / a.topk : -1;
-        gam[i] = ((MODE == 1 || w_on_input) && valid) ? a.row_gamma[r0 + i] : 0.f;
+        for (int i = 0; i < HT; ++i) {
+          orow[i] = __shfl_sync(0xffffffffu, token, i);
+          gam[i] = __shfl_sync(0xffffffffu, weight, i);
+        }
       }
       float sum[HT];
 #pragma unroll
@@ -572,6 +590,12 @@ int launch_mode(const CUtensorMap& tm_w, const CUtensorMap& tm_sz, const W4Token
 bool gemm_w4_ok(int E) {
   return kSmemLimit - 1024 >= w4_fixed_bytes<0>(E, 1, false) + 2 * static_cast<size_t>(w4_token_bytes(kMaxGranW4 * kGranW4, 1)) &&
          kSmemLimit - 1024 >= w4_fixed_bytes<32>(E, 1, false) + 2 * static_cast<size_t>(w4_token_bytes(32, 2));
+}
+
+// Tables of a call whose GEMMs sort its P slots themselves, beside as many stages of tokens as they leave at least.
+bool gemm_w4_own_ok(int E, int P, int BT) {
+  const size_t fixed = BT == 16 ? w4_fixed_bytes<16>(E, 1, false, P) : w4_fixed_bytes<32>(E, 1, false, P);
+  return kSmemLimit - 1024 >= fixed + 3 * static_cast<size_t>(w4_token_bytes(BT, 2));
 }
 
 // a->BT: 16 or 32 (decode blocks); with a->w4_var the upper bound of the tokens per tile

@@ -1,6 +1,7 @@
 // Row movers around the grouped GEMMs: gather token rows into expert-sorted,
 // block-padded order (optionally quantising them to FP8 per 1x128 group),
 // and turn the fp32 combine buffer into the 16-bit output.
+#include "gemm_route.cuh"
 #include "prep.cuh"
 
 namespace b200moe {
@@ -62,6 +63,65 @@ gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const in
   for (long long i = thread; i < zero_chunks; i += threads) zero[i] = make_uint4(0, 0, 0, 0);
 }
 
+// The same for a call whose GEMMs sort the slots themselves (gemm_route.cuh): a warp takes 2 KiB of a slot's row and puts it where
+// the GEMMs look for it.
+// Padded row of slot i (triple: of the i-th sorted row); -1: no expert here.  Whole warp.
+__device__ __forceinline__ int routed_row(const RouteSource& route, const RowTables& t, int P, int E, int BT, int i) {
+  if (route.hist == nullptr) {
+    const unsigned e = t.ids[ids_at(i)];
+    return e == kNoSlot ? -1 : t.blk[e] * BT + slot_rank(t, i, e);
+  }
+  const int slot = __ldcg(route.topk_indx + i);
+  if (i >= t.raw[E] || slot < 0 || slot >= P) return -1;
+  int lo = 0, hi = E;         // last expert that starts at or before row i
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (t.raw[mid] <= i) lo = mid; else hi = mid;
+  }
+  return t.blk[lo] * BT + i - t.raw[lo];
+}
+
+__global__ void __launch_bounds__(256)
+gather_routed_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const RouteSource route, int P, int E, int BT, int topk,
+                     int chunks_per_row, uint4* __restrict__ zero, long long zero_chunks) {
+  extern __shared__ __align__(16) uint8_t route_smem[];
+  const RowTables t = row_tables(route_smem, E);
+  griddep_wait();
+  griddep_launch_dependents();
+  const int threads = gridDim.x * blockDim.x;
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = thread & 31;
+  const int segs = (chunks_per_row + kGatherSeg - 1) / kGatherSeg;
+  // The first unit's row is on its way while the slots are counted: the next kernel's weights fill the memory's queues by then,
+  // and a second trip through them costs 4 us.
+  uint4 v[4];
+  auto fetch = [&](int u) {
+    const int i = u / segs, c0 = (u - i * segs) * kGatherSeg + lane;
+    int slot = route.hist == nullptr ? i : __ldcg(route.topk_indx + i);
+    if (slot < 0 || slot >= P) slot = 0;
+    const uint4* src = x + static_cast<size_t>(slot / topk) * chunks_per_row;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c0 + 32 * q < chunks_per_row) v[q] = __ldg(src + c0 + 32 * q);
+  };
+  const int units = P * segs;
+  int u = thread >> 5;
+  if (u < units) fetch(u);
+  for (long long i = thread; i < zero_chunks; i += threads) zero[i] = make_uint4(0, 0, 0, 0);
+  count_slots(route, P, E, BT, t);
+  for (bool first = true; u < units; u += threads >> 5, first = false) {
+    if (!first) fetch(u);
+    const int i = u / segs;
+    const int r = routed_row(route, t, P, E, BT, i);
+    if (r < 0) continue;
+    const int c0 = (u - i * segs) * kGatherSeg + lane;
+    uint4* dst = xs + static_cast<size_t>(r) * chunks_per_row;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c0 + 32 * q < chunks_per_row) dst[c0 + 32 * q] = v[q];
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ void load4(const T* p, float (&v)[4]);
 template <>
@@ -79,10 +139,24 @@ __device__ __forceinline__ void load4<__half>(const __half* p, float (&v)[4]) {
   v[0] = __low2float(a); v[1] = __high2float(a); v[2] = __low2float(b); v[3] = __high2float(b);
 }
 
+// One 128-wide group over a warp: four e4m3 values of this lane; lane u receives the group's scale in `mine`.
+// scale = max(amax, eps)/448, q = rne_satfinite(x / scale) with an IEEE divide so that the bits match a CPU restatement.
+__device__ __forceinline__ uint32_t quantise_group(const float (&v)[4], int lane, int u, float& mine) {
+  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+  // non-negative floats order like their bit patterns: one redux instead of five shuffles
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  const float s = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
+  if (lane == u) mine = s;
+  uint32_t packed = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    packed |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(__fdiv_rn(v[i], s), __NV_SATFINITE, __NV_E4M3)) << (8 * i);
+  return packed;
+}
+
 // One warp per (row, run of up to eight 128-wide groups): the loads of the run are issued
 // together (one 8-byte load per lane and group in flight is too little to cover the memory
-// latency), then per group amax by shuffles, scale = max(amax, eps)/448,
-// q = rne_satfinite(x / scale) with an IEEE divide so that the bits match a CPU restatement.
+// latency), then quantise_group per group.
 // sorted_ids == nullptr: rows map to themselves.
 // scale_t != 0: scales stored [K/128][ld_scale] (group-major) instead of [rows][K/128].
 template <typename T>
@@ -124,20 +198,73 @@ group_quant_fp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* 
     for (int u = 0; u < RUN; ++u) {
       const int g = g0 + u;
       if (g >= groups) break;
-      float amax = fmaxf(fmaxf(fabsf(v[u][0]), fabsf(v[u][1])), fmaxf(fabsf(v[u][2]), fabsf(v[u][3])));
-      // non-negative floats order like their bit patterns: one redux instead of five shuffles
-      amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
-      const float s = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
-      uint32_t packed = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        __nv_fp8_storage_t b = __nv_cvt_float_to_fp8(__fdiv_rn(v[u][i], s), __NV_SATFINITE, __NV_E4M3);
-        packed |= static_cast<uint32_t>(b) << (8 * i);
-      }
-      *reinterpret_cast<uint32_t*>(q + static_cast<size_t>(r) * K + g * 128 + lane * 4) = packed;
+      float s = 0.f;
+      *reinterpret_cast<uint32_t*>(q + static_cast<size_t>(r) * K + g * 128 + lane * 4) = quantise_group(v[u], lane, 0, s);
       if (lane == 0) {
         if (scale_t) scales[static_cast<size_t>(g) * ld_scale + r] = s;
         else scales[static_cast<size_t>(r) * groups + g] = s;
+      }
+    }
+  }
+}
+
+// The quantisation for a call whose GEMMs sort the slots themselves (gemm_route.cuh): a warp quantises a run of groups of a
+// token once and stores it for each of the token's slots, where the GEMMs look for the row.  The kernel is a few
+// microseconds long, so its loops stay rolled: straight-line code for eight groups and eight slots spent more time being
+// fetched than executed (64 tokens of 56 groups, top-8: 18.5 us; an alignment and one warp per slot: 20).
+constexpr int kQuantRun = 8;      // groups of a run at most; few tokens are dealt out in shorter ones
+template <typename T>
+__global__ void __launch_bounds__(256)
+group_quant_routed_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, const RouteSource route,
+                          int P, int E, int BT, int topk, int M, int K, int run, int ld_scale, uint4* __restrict__ zero,
+                          long long zero_chunks) {
+  extern __shared__ __align__(16) uint8_t route_smem[];
+  __shared__ __align__(16) uint2 s_x[8][kQuantRun][32];
+  const RowTables t = row_tables(route_smem, E);
+  griddep_wait();
+  griddep_launch_dependents();
+  const int threads = gridDim.x * blockDim.x;
+  const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+  const int groups = K >> 7, runs = (groups + run - 1) / run, lane = thread & 31;
+  uint2(*mine)[32] = s_x[threadIdx.x >> 5];
+  auto fetch = [&](int w) {
+    const int tok = w / runs, g0 = (w - tok * runs) * run, n = min(run, groups - g0);
+    const T* src = x + static_cast<size_t>(tok) * K + g0 * 128 + lane * 4;
+#pragma unroll 1
+    for (int u = 0; u < n; ++u)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(&mine[u][lane])), "l"(src + u * 128) : "memory");
+  };
+  // the first run is on its way while the slots are counted: by then the next kernel's weights fill the memory's queues
+  int w = thread >> 5;
+  if (w < M * runs) fetch(w);
+  for (long long i = thread; i < zero_chunks; i += threads) zero[i] = make_uint4(0, 0, 0, 0);
+  count_slots(route, P, E, BT, t);
+  for (bool first_run = true; w < M * runs; w += threads >> 5, first_run = false) {
+    if (!first_run) fetch(w);
+    const int tok = w / runs, g0 = (w - tok * runs) * run, n = min(run, groups - g0);
+    asm volatile("cp.async.wait_all;" ::: "memory");        // (a lane reads only what it copied)
+    for (int j0 = 0; j0 < topk; j0 += 32) {
+      const int nj = min(32, topk - j0);
+      int row = -1;             // lane j: padded row of the token's slot j0 + j
+#pragma unroll 1
+      for (int j = 0; j < nj; ++j) {
+        const int slot = tok * topk + j0 + j;
+        const unsigned e = t.ids[ids_at(slot)];
+        const int rank = e == kNoSlot ? -1 : slot_rank(t, slot, e);
+        if (lane == j && rank >= 0) row = t.blk[e] * BT + rank;
+      }
+#pragma unroll 1
+      for (int u = 0; u < n; ++u) {
+        float v[4];
+        load4<T>(reinterpret_cast<const T*>(&mine[u][lane]), v);
+        float scale = 0.f;
+        const uint32_t packed = quantise_group(v, 0, 0, scale);      // (every lane has the scale)
+#pragma unroll 1
+        for (int j = 0; j < nj; ++j) {
+          const int r = __shfl_sync(0xffffffffu, row, j);
+          if (r >= 0) *reinterpret_cast<uint32_t*>(q + static_cast<size_t>(r) * K + (g0 + u) * 128 + lane * 4) = packed;
+        }
+        if (row >= 0) scales[static_cast<size_t>(g0 + u) * ld_scale + row] = scale;
       }
     }
   }
@@ -245,6 +372,22 @@ int launch_gather_rows(const void* x, void* xs, const int* sorted_ids, const int
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
+int launch_gather_routed(const void* x, void* xs, const RouteSource& route, int P, int E, int BT, int topk, int row_bytes, void* zero,
+                         size_t zero_bytes, int num_sms, cudaStream_t stream, bool pdl) {
+  if (row_bytes % 16 != 0 || zero_bytes % 16 != 0) return B200MOE_ERR_UNSUPPORTED;
+  const size_t smem = route_table_bytes(E, P);
+  if (smem > 48 * 1024) return B200MOE_ERR_TOO_LARGE;
+  const int segs = (row_bytes / 16 + kGatherSeg - 1) / kGatherSeg;
+  int ctas = (P * segs + 7) / 8;
+  if (ctas > 2 * num_sms) ctas = 2 * num_sms;
+  if (ctas < 1) ctas = 1;
+  note_launch("gather_routed_kernel");
+  cudaError_t err = launch_kernel(gather_routed_kernel, dim3(ctas), dim3(256), smem, stream, pdl, reinterpret_cast<const uint4*>(x),
+                                  reinterpret_cast<uint4*>(xs), route, P, E, BT, topk, row_bytes / 16,
+                                  reinterpret_cast<uint4*>(zero), static_cast<long long>(zero_bytes / 16));
+  return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
 int launch_group_quant_fp8(const void* x, int dtype, void* q, float* scales, const int* sorted_ids,
                            const int* meta, int P, int topk, int rows, int K, int scale_t, int ld_scale,
                            void* zero, size_t zero_bytes, int num_sms, cudaStream_t stream, bool pdl) {
@@ -264,6 +407,32 @@ int launch_group_quant_fp8(const void* x, int dtype, void* q, float* scales, con
     err = launch_kernel(group_quant_fp8_kernel<__half>, dim3(static_cast<unsigned>(ctas)), dim3(256), 0, stream, pdl,
                         reinterpret_cast<const __half*>(x), reinterpret_cast<uint8_t*>(q), scales, sorted_ids, meta, P,
                         topk, rows, K, scale_t, ld_scale, reinterpret_cast<uint4*>(zero), zc);
+  return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
+}
+
+int launch_group_quant_routed(const void* x, int dtype, void* q, float* scales, const RouteSource& route, int P, int E, int BT,
+                              int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms, cudaStream_t stream,
+                              bool pdl) {
+  const size_t smem = route_table_bytes(E, P);
+  if (K % 128 != 0 || zero_bytes % 16 != 0 || route.hist != nullptr) return B200MOE_ERR_UNSUPPORTED;
+  if (smem > 30 * 1024) return B200MOE_ERR_TOO_LARGE;
+  const int groups = K / 128;
+  int run = (M * groups + 16 * num_sms - 1) / (16 * num_sms);
+  if (run > kQuantRun) run = kQuantRun;
+  int ctas = (M * ((groups + run - 1) / run) + 7) / 8;
+  if (ctas > 2 * num_sms) ctas = 2 * num_sms;
+  if (ctas < 1) ctas = 1;
+  const long long zc = static_cast<long long>(zero_bytes / 16);
+  note_launch("group_quant_routed_kernel");
+  cudaError_t err;
+  if (dtype == B200MOE_DTYPE_BF16)
+    err = launch_kernel(group_quant_routed_kernel<__nv_bfloat16>, dim3(ctas), dim3(256), smem, stream, pdl,
+                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, route, P, E, BT, topk, M, K,
+                        run, ld_scale, reinterpret_cast<uint4*>(zero), zc);
+  else
+    err = launch_kernel(group_quant_routed_kernel<__half>, dim3(ctas), dim3(256), smem, stream, pdl, reinterpret_cast<const __half*>(x),
+                        reinterpret_cast<uint8_t*>(q), scales, route, P, E, BT, topk, M, K, run, ld_scale,
+                        reinterpret_cast<uint4*>(zero), zc);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 

@@ -1,6 +1,6 @@
 // Host-callable launchers of the row movers around the grouped GEMMs.
 #pragma once
-#include "common.cuh"
+#include "gemm.cuh"
 
 namespace b200moe {
 
@@ -13,6 +13,14 @@ int launch_gather_rows(const void* x, void* xs, const int* sorted_ids, const int
                        int row_bytes, int cap, void* zero, size_t zero_bytes, int num_sms,
                        cudaStream_t stream, bool pdl, const float* sc_src = nullptr, float* sc_dst = nullptr,
                        int G = 0, int ld = 0, const FlagWait* wait = nullptr);
+
+// The same from the routing input, for calls whose GEMMs sort the slots themselves (gemm_route.cuh).
+int launch_gather_routed(const void* x, void* xs, const RouteSource& route, int P, int E, int BT, int topk, int row_bytes, void* zero,
+                         size_t zero_bytes, int num_sms, cudaStream_t stream, bool pdl);
+
+int launch_group_quant_routed(const void* x, int dtype, void* q, float* scales, const RouteSource& route, int P, int E, int BT,
+                              int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms, cudaStream_t stream,
+                              bool pdl);
 
 // Per-token-group (1x128) FP8 quantisation, optionally gathering rows through
 // sorted_ids like launch_gather_rows.  scale_t: store scales group-major.

@@ -55,6 +55,8 @@ route_topk_kernel(const TL* __restrict__ logits, const float* __restrict__ bias,
   float* s_key = s_score + E;                                  // selection keys
   const int gsize = n_group > 1 ? E / n_group : E;
 
+  griddep_wait();
+  griddep_launch_dependents();
   for (int t = blockIdx.x * kRouterWarps + warp; t < M; t += gridDim.x * kRouterWarps) {
     const size_t base = static_cast<size_t>(t) * E;
     float denom = 1.0f;
@@ -174,7 +176,7 @@ int check_router(const b200moe_router* r, int E, int topk) {
 }
 
 int launch_route_topk(const b200moe_router* r, const void* logits, int M, int E, int topk, float* out_w,
-                      int* out_ids, int num_sms, cudaStream_t stream) {
+                      int* out_ids, int num_sms, cudaStream_t stream, bool pdl) {
   int rc = check_router(r, E, topk);
   if (rc != B200MOE_OK) return rc;
   if (M == 0) return B200MOE_OK;
@@ -186,7 +188,7 @@ int launch_route_topk(const b200moe_router* r, const void* logits, int M, int E,
   cudaError_t err;
   note_launch("route_topk_kernel");
 #define B200MOE_ROUTE(TL)                                                                                     \
-  err = launch_kernel(route_topk_kernel<TL>, dim3(ctas), dim3(kRouterWarps * 32), smem, stream, false,          \
+  err = launch_kernel(route_topk_kernel<TL>, dim3(ctas), dim3(kRouterWarps * 32), smem, stream, pdl,            \
                       reinterpret_cast<const TL*>(logits), r->bias, M, E, topk, r->scoring, r->renormalize,     \
                       r->n_group, r->topk_group, scale, out_w, out_ids)
   if (r->logits_dtype == B200MOE_DTYPE_FP32) B200MOE_ROUTE(float);
