@@ -19,17 +19,22 @@ struct Ctrl {
   int grid_eff;
 };
 
+// Called by whole warps.  A lane rates one split; with the rates one after the other the two divisions of each stood in the
+// way of a launch's first loads for 2 us (reductions of 224 steps, up to 16 splits).
 __device__ __forceinline__ int pick_split(int tiles, int kblocks, int grid, int max_split) {
+  const int smax = min(max_split, max(1, kblocks / 4));
   int best = 1;
   float best_eff = -1.f;
-  int smax = min(max_split, max(1, kblocks / 4));
-  for (int s = 1; s <= smax; ++s) {
-    int total = tiles * s;
-    int waves = (total + grid - 1) / grid;
-    float eff = static_cast<float>(total) / static_cast<float>(waves * grid);
-    if (eff > best_eff + 0.04f) {
-      best_eff = eff;
-      best = s;
+  for (int s0 = 1; s0 <= smax; s0 += 32) {
+    const int total = tiles * (s0 + static_cast<int>(threadIdx.x & 31));
+    const int waves = (total + grid - 1) / grid;
+    const float eff = static_cast<float>(total) / static_cast<float>(waves * grid);
+    for (int i = 0; i < 32 && s0 + i <= smax; ++i) {
+      const float e = __shfl_sync(0xffffffffu, eff, i);
+      if (e > best_eff + 0.04f) {
+        best_eff = e;
+        best = s0 + i;
+      }
     }
   }
   return best;
@@ -62,11 +67,14 @@ __device__ __forceinline__ TileCoord decode_tile(int id, const Ctrl& c, const in
   const int nt = rest / c.split;
   t.row0 = (first + b) * BT;
   t.n0 = nt * tile_n;
-  t.kb0 = static_cast<int>((static_cast<long long>(s) * kblocks) / c.split);
-  t.kb1 = static_cast<int>((static_cast<long long>(s + 1) * kblocks) / c.split);
+  t.kb0 = 0;
+  t.kb1 = kblocks;
+  if (c.split > 1) {      // (32 bits: the reduction has at most 2^20 steps, the split is at most 1024)
+    t.kb0 = static_cast<int>(static_cast<unsigned>(s) * static_cast<unsigned>(kblocks) / static_cast<unsigned>(c.split));
+    t.kb1 = static_cast<int>(static_cast<unsigned>(s + 1) * static_cast<unsigned>(kblocks) / static_cast<unsigned>(c.split));
+  }
   return t;
 }
-
 
 // Fused tail of the gate/up projection.
 //   SiLU / GELU (the reference's plain op, fused_moe.py:198-206): optional routing weight on the

@@ -45,8 +45,12 @@ __device__ __forceinline__ RowTile row_tile_at(int id, const RowTiles& r) {
   t.n0 = (rest / r.split) * r.tile_n;
   t.row0 = (r.gran[lo] + g0) * r.gran_rows;
   t.n = (g1 - g0) * r.gran_rows;
-  t.kb0 = static_cast<int>((static_cast<long long>(s) * r.kblocks) / r.split);
-  t.kb1 = static_cast<int>((static_cast<long long>(s + 1) * r.kblocks) / r.split);
+  t.kb0 = 0;
+  t.kb1 = r.kblocks;
+  if (r.split > 1) {      // (32 bits: see decode_tile)
+    t.kb0 = static_cast<int>(static_cast<unsigned>(s) * static_cast<unsigned>(r.kblocks) / static_cast<unsigned>(r.split));
+    t.kb1 = static_cast<int>(static_cast<unsigned>(s + 1) * static_cast<unsigned>(r.kblocks) / static_cast<unsigned>(r.split));
+  }
   return t;
 }
 

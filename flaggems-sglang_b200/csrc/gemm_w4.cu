@@ -238,15 +238,17 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const uint32_t a_col0 = static_cast<uint32_t>(G::kPartials * acc_cols);
   const int slots_a = NT > 0 ? G::kSlots : min(4, (512 - 2 * nmax) / 64);
   const int first = blockIdx.x, stride = gridDim.x;
-  // units of this CTA over the whole launch
+  // units of this CTA over the whole launch; a lane takes a tile (every thread taking all of them one after the other
+  // cost the second GEMM of a decode call 8 us before its first load)
   int units = 0;
   if (split == 1) {
     units = first < total ? ((total - first + stride - 1) / stride) * a.kblocks : 0;
   } else {
-    for (int tile = first; tile < total; tile += stride) {
+    for (int tile = first + lane * stride; tile < total; tile += 32 * stride) {
       const RowTile t = row_tile_at(tile, grid);
       units += t.kb1 - t.kb0;
     }
+    units = __reduce_add_sync(0xffffffffu, units);
   }
   // The MMAs of unit u have finished.  Nobody falls a whole ring behind: the MMA thread needs every waiter's
   // product (tokens, operands, free partial sums) within fewer units than the ring has barriers.
