@@ -98,11 +98,12 @@ size_t group_smem_bytes(int nwarps, int E) { return (static_cast<size_t>(nwarps)
 // Core: stable grouping of P slots by expert.  `ids` are expert ids (mapped to local experts when
 // map != nullptr); slots with an id outside [0, E) are dropped.  Each expert's group starts at a
 // multiple of `block`.  place(slot, pos, pre[slot]) records a placement; `pre` (optional, [P]) is a
-// per-slot value fetched alongside the ids.  Called by every thread of every CTA; the caller ends with
+// per-slot value fetched alongside the ids; dropped[slot] (optional) becomes -1 for a dropped slot.  Called by every thread of every CTA; the caller ends with
 // cluster_wait() (the CTAs' counts are read by their peers).
 template <typename Place>
 __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const int* map, int map_len, int P, int E,
-                                                int block, const GroupSmem& g, int nwarps, const float* pre, Place place) {
+                                                int block, const GroupSmem& g, int nwarps, const float* pre, Place place,
+                                                int* dropped = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rank = cluster_rank(), nctas = gridDim.x;
   for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) g.cnt[i] = 0;
@@ -205,6 +206,8 @@ __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const
         if (e >= 0) {
           place(i, g.mine[e] + cur + r, wv[u]);
           if (r == 0) g.cnt[warp * E + e] = cur + __popc(m);
+        } else if (dropped != nullptr && i < end) {
+          dropped[i] = -1;
         }
         __syncwarp();
       }
@@ -215,7 +218,7 @@ __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const
 __global__ void __launch_bounds__(kAlignThreads)
 align_block_kernel(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
                    int block, int cap, int nwarps, int* sorted_ids, int* expert_ids, int* num_post_pad,
-                   float* row_gamma, int* blk_off, int* meta, const FlagWait fw) {
+                   float* row_gamma, int* blk_off, int* meta, int* slot_row, const FlagWait fw) {
   extern __shared__ int smem[];
   griddep_wait();             // the tables written below may still be read by the kernels of the previous call
   griddep_launch_dependents();
@@ -225,7 +228,9 @@ align_block_kernel(const void* ids, int is64, const int* map, int map_len, const
                   [&](int slot, int pos, float w) {
                     sorted_ids[pos] = slot;
                     if (row_gamma != nullptr) row_gamma[pos] = w;
-                  });
+                    if (slot_row != nullptr) slot_row[slot] = pos;
+                  },
+                  slot_row);
 
   // padding of every expert's group, then the unused tail of the tables
   const int lane = threadIdx.x & 31;
@@ -426,7 +431,8 @@ int routing_max_tiles(int n_slots, int n_experts) {
 
 int launch_align_block(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
                        int block, int cap, int* sorted_ids, int* expert_ids, int* num_post_pad,
-                       float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl, const FlagWait* wait, bool one_cta) {
+                       float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl, const FlagWait* wait, bool one_cta,
+                       int* slot_row) {
   if (P < 0 || E <= 0 || block <= 0 || cap < 0) return B200MOE_ERR_BAD_ARG;
   const int nw = pick_warps(E);
   size_t smem;
@@ -437,7 +443,7 @@ int launch_align_block(const void* ids, int is64, const int* map, int map_len, c
   const int ctas = one_cta ? 1 : pick_ctas(P);
   cudaError_t err = launch_kernel_cluster(align_block_kernel, dim3(ctas), ctas, dim3(kAlignThreads), smem, stream, pdl, ids,
                                           is64, map, map_len, weights, P, E, block, cap, nw, sorted_ids, expert_ids,
-                                          num_post_pad, row_gamma, blk_off, meta, fw);
+                                          num_post_pad, row_gamma, blk_off, meta, slot_row, fw);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 

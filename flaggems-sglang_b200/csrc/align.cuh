@@ -14,9 +14,10 @@ int routing_max_tiles(int n_slots, int n_experts);
 int launch_align_block(const void* ids, int is64, const int* map, int map_len, const float* weights, int P, int E,
                        int block, int cap, int* sorted_ids, int* expert_ids, int* num_post_pad,
                        float* row_gamma, int* blk_off, int* meta, cudaStream_t stream, bool pdl = false,
-                       const FlagWait* wait = nullptr, bool one_cta = false);
+                       const FlagWait* wait = nullptr, bool one_cta = false, int* slot_row = nullptr);
 // `pdl`: launch with programmatic stream serialisation; `wait` (expert parallelism): the kernel
-// waits for the peers' flags before it reads the ids; `one_cta`: however many slots.
+// waits for the peers' flags before it reads the ids; `one_cta`: however many slots; `slot_row` (optional, [P]): padded row
+// of each slot, -1 for a dropped one (may be the array of 32-bit ids itself: a slot's id is read by the lane that writes its row).
 
 // Same internal tables from hist / topk_indx / gate_scal of the routing triple.
 int launch_align_from_routing(const int* hist, const int* topk_indx, const float* gate_scal, int P,

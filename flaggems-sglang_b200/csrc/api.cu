@@ -191,12 +191,10 @@ int pick_bt(const b200moe_cfg* c) {
   if (c->wmode == B200MOE_W_FP8_BLOCK) {
     // many-expert FP8 layers route unevenly: hot experts hold several times the average, and every
     // extra block of an expert streams its weights once more from L2, so lean towards larger blocks
-    // (measured on the 256-expert zipf-skewed layer: average 2 (M = 64) -> 16 is best; average 4: 16 / 32 /
-    // 64 within 4 %; average 8 (M = 256): tokens-on-M blocks of 128 and 64-token blocks beat 32-token blocks
-    // by 10 %; average 12 / 16: blocks of 128 win by 20 % / 11 %)
+    // and blocks of 128 take the experts of at most 16 tokens as blocks of 16 anyway (256 experts, zipf-skewed, us,
+    // blocks of 16 or 32 / 128: average 2: 400 / 403, 3.1: 445 / 463, 4.1: 583 / 475, 5.6: 605 / 561, 7.8: 705 / 617)
     if (avg <= 4) return 16;
-    if (avg < 8) return 32;
-    return 128;  // tokens-on-M kernels
+    return 128;
   }
   // 16-bit and int4: the smaller block until too many experts need a second one.  16 against 32 tokens per block cross at
   // an average of 13 for layers of 8, 64 and 128 experts (us, 16 / 32: 128 experts, average 12.6: 212 / 217, 15: 220 / 218;
@@ -377,7 +375,7 @@ int query_sms(const b200moe_cfg* c) {
 // Block alignment into the workspace tables.
 int align_into_workspace(const b200moe_cfg* c, const Layout& L, uint8_t* ws, const void* ids, int is64,
                          const int32_t* expert_map, const float* weights, cudaStream_t st,
-                         const FlagWait* wait = nullptr) {
+                         const FlagWait* wait = nullptr, int* slot_row = nullptr) {
   const bool pdl = (c->flags & B200MOE_FLAG_NO_PDL) == 0;
   int* sorted_ids = reinterpret_cast<int*>(ws + L.sorted_ids);
   int* expert_ids = reinterpret_cast<int*>(ws + L.expert_ids);
@@ -387,7 +385,7 @@ int align_into_workspace(const b200moe_cfg* c, const Layout& L, uint8_t* ws, con
   int* meta = reinterpret_cast<int*>(ws + L.meta);
   return launch_align_block(ids, is64, expert_map, c->n_global_experts, weights, L.P, c->E, L.BT, L.cap, sorted_ids,
                             expert_ids, num_post, row_gamma, blk_off, meta, st, pdl, wait,
-                            (c->flags & B200MOE_FLAG_ALIGN_ONE_CTA) != 0);
+                            (c->flags & B200MOE_FLAG_ALIGN_ONE_CTA) != 0, slot_row);
 }
 
 RouteSource topk_source(const b200moe_cfg* c, const void* ids, int is64, const int32_t* expert_map, const float* weights) {
@@ -398,6 +396,13 @@ RouteSource topk_source(const b200moe_cfg* c, const void* ids, int is64, const i
   r.map_len = c->n_global_experts;
   r.weights = weights;
   return r;
+}
+
+// FP8 rows are quantised by token and stored per slot: the alignment then also says where each slot's row is, in the place
+// of the router's ids (its own input at most; nothing reads them after it).
+int* slot_rows(const b200moe_cfg* c, const Layout& L, uint8_t* ws) {
+  const bool wanted = c->wmode == B200MOE_W_FP8_BLOCK && !(c->flags & B200MOE_FLAG_X_FP8);
+  return wanted ? reinterpret_cast<int*>(ws + L.route_ids) : nullptr;
 }
 
 // Expert parallelism: where the down projection's output rows go (the buffers of the ranks that
@@ -416,7 +421,7 @@ struct PeerOut {
 // land on their owners and nothing is cleared or converted here.
 int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void* w1, const void* w2,
                 const b200moe_quant* quant, uint8_t* ws, void* out, int32_t* status, cudaStream_t st,
-                int slot, const RouteSource* route, const PeerOut* peers = nullptr) {
+                int slot, const RouteSource* route, const int* slot_row = nullptr, const PeerOut* peers = nullptr) {
   const int sms = query_sms(c);
   int* meta = reinterpret_cast<int*>(ws + L.meta);
   int* blk_off = reinterpret_cast<int*>(ws + L.blk_off);
@@ -444,8 +449,8 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
   if (fp8 && (quant == nullptr || quant->w1_scale == nullptr || quant->w2_scale == nullptr)) return B200MOE_ERR_BAD_ARG;
   if (own) {
     if (fp8) {
-      rc = launch_group_quant_routed(x, c->dtype, xs, reinterpret_cast<float*>(ws + L.xs_scale), *route, L.P, c->E, L.BT, c->topk,
-                                     c->M, c->H, L.cap, zero, zero_bytes, sms, st, pdl);
+      rc = launch_group_quant_slots(x, c->dtype, xs, reinterpret_cast<float*>(ws + L.xs_scale), *route, nullptr, L.P, c->E, L.BT,
+                                    c->topk, c->M, c->H, L.cap, zero, zero_bytes, sms, st, pdl);
       cleared = true;
     } else if (w4) {
       rc = launch_gather_routed(x, xs, *route, L.P, c->E, L.BT, c->topk, c->H * 2, zero, zero_bytes, sms, st, pdl);
@@ -458,6 +463,9 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
       rc = launch_gather_rows(x, xs, sorted_ids, meta, L.P, c->topk, c->H, L.cap, zero, zero_bytes, sms, st, pdl,
                               quant->x_scale, reinterpret_cast<float*>(ws + L.xs_scale), c->H / 128, L.cap,
                               peers != nullptr ? peers->rows_wait : nullptr);
+    } else if (slot_row != nullptr) {
+      rc = launch_group_quant_slots(x, c->dtype, xs, reinterpret_cast<float*>(ws + L.xs_scale), RouteSource{}, slot_row, L.P, c->E,
+                                    L.BT, c->topk, c->M, c->H, L.cap, zero, zero_bytes, sms, st, pdl);
     } else if (L.quant_once) {
       float* tok_scale = reinterpret_cast<float*>(ws + L.xq_scale);
       rc = launch_group_quant_fp8(x, c->dtype, ws + L.xq_tok, tok_scale, nullptr, nullptr, L.P, c->topk, c->M, c->H, 0,
@@ -632,12 +640,17 @@ int run_experts(const b200moe_cfg* c, const Layout& L, const void* x, const void
     } else {
       if ((rc = make_tmap_2d(&tm_x, dt, eb, xs, c->H, L.cap, kbox, L.BT)) != B200MOE_OK) return rc;
       if ((rc = make_tmap_2d(&tm_a2, dt, eb, a2, c->I, L.cap, kbox, L.BT)) != B200MOE_OK) return rc;
+      CUtensorMap tm_xc = {}, tm_a2c = {};
+      if (fp8 && L.BT == 128) {
+        if ((rc = make_tmap_2d(&tm_xc, dt, eb, xs, c->H, L.cap, kbox, 16)) != B200MOE_OK) return rc;
+        if ((rc = make_tmap_2d(&tm_a2c, dt, eb, a2, c->I, L.cap, kbox, 16)) != B200MOE_OK) return rc;
+      }
       prof_mark(slot, 1, st);
-      rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st);
+      rc = fp8 ? launch_gemm_fp8(tm_w1, tm_x, tm_xc, g1, sms, st) : launch_gemm_tc(tm_w1, tm_x, g1, sms, st);
       prof_mark(slot, 2, st);
       if (rc != B200MOE_OK) return rc;
       prof_mark(slot, 3, st);
-      rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st);
+      rc = fp8 ? launch_gemm_fp8(tm_w2, tm_a2, tm_a2c, g2, sms, st) : launch_gemm_tc(tm_w2, tm_a2, g2, sms, st);
     }
     prof_mark(slot, 4, st);
     if (rc != B200MOE_OK) return rc;
@@ -872,9 +885,10 @@ int b200moe_forward_topk(const b200moe_cfg* cfg, const void* x, const void* w1, 
     const RouteSource src = topk_source(cfg, topk_ids, is64, expert_map, topk_weights);
     return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, &src);
   }
-  rc = align_into_workspace(cfg, L, ws, topk_ids, is64, expert_map, topk_weights, st);
+  int* slot_row = slot_rows(cfg, L, ws);
+  rc = align_into_workspace(cfg, L, ws, topk_ids, is64, expert_map, topk_weights, st, nullptr, slot_row);
   if (rc != B200MOE_OK) return rc;
-  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr);
+  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr, slot_row);
 }
 
 int b200moe_route_topk(const b200moe_router* router, const void* logits, int n_tokens, int n_experts, int topk,
@@ -913,9 +927,10 @@ int b200moe_forward_logits(const b200moe_cfg* cfg, const b200moe_router* router,
     const RouteSource src = topk_source(cfg, ids, 0, expert_map, tw);
     return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, &src);
   }
-  rc = align_into_workspace(cfg, L, ws, ids, 0, expert_map, tw, st);
+  int* slot_row = slot_rows(cfg, L, ws);
+  rc = align_into_workspace(cfg, L, ws, ids, 0, expert_map, tw, st, nullptr, slot_row);
   if (rc != B200MOE_OK) return rc;
-  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr);
+  return run_experts(cfg, L, x, w1, w2, quant, ws, out, status, st, slot, nullptr, slot_row);
 }
 
 int b200moe_forward_routed(const b200moe_cfg* cfg, const void* x, const void* w1, const void* w2,
@@ -991,6 +1006,14 @@ int b200moe_forward_topk_noalloc(const b200moe_cfg* cfg, const void* x, const vo
   if (rc != B200MOE_OK) return rc;
   Layout L;
   if ((rc = make_layout(cfg, &L)) != B200MOE_OK) return rc;
+  // Blocks of 128 need the most room: an FP8 call of fewer than eight slots per expert also runs on blocks of 32.
+  b200moe_cfg small = *cfg;
+  if (L.total > static_cast<size_t>(B200MOE_NOALLOC_SCRATCH_BYTES) && cfg->wmode == B200MOE_W_FP8_BLOCK && cfg->block_tokens == 0 &&
+      static_cast<long long>(cfg->M) * cfg->topk < 8LL * cfg->E) {
+    small.block_tokens = 32;
+    cfg = &small;
+    if ((rc = make_layout(cfg, &L)) != B200MOE_OK) return rc;
+  }
   if (L.total > static_cast<size_t>(B200MOE_NOALLOC_SCRATCH_BYTES)) return B200MOE_ERR_TOO_LARGE;
   void* scratch = noalloc_scratch_for_current_device();
   if (scratch == nullptr) return B200MOE_ERR_CUDA;
@@ -1163,7 +1186,7 @@ int b200moe_ep_forward(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, void* c
       po.pairs[r] = h + H.pairs;
       po.pair_valid[r] = h + H.pair_valid;
     }
-    if ((rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, nullptr, &po)) != B200MOE_OK) return rc;
+    if ((rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, nullptr, nullptr, &po)) != B200MOE_OK) return rc;
     uint8_t* hp[kMaxPeers];
     for (int r = 0; r < ep->world; ++r) hp[r] = reinterpret_cast<uint8_t*>(heaps[r]);
     if ((rc = launch_ep_signal(hp, H, kEpFlagDone, ep->world, ep->rank, st, pdl)) != B200MOE_OK) return rc;

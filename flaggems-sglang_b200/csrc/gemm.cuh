@@ -35,6 +35,8 @@ struct GemmArgs {
   int BT;          // tokens per block (16..256, multiple of 16); CTA pairs, w4_var: upper bound of the tokens per tile
   int w4_var;      // int4: 1 = tiles of a variable number of tokens (16..192), 0 = decode blocks of BT (16 or 32) tokens
   int stages;      // shared-memory ring depth
+  int table_off;   // FP8 blocks of 128: where the block tables stand in shared memory
+  int stages_cold; // FP8 blocks of 128: the same of the CTAs that take the blocks of at most 16 tokens
   int acc_stages;  // accumulator buffers in tensor memory (1 or 2)
   int tmem_cols;   // allocated tensor-memory columns (power of two >= 32)
   int num_nt;      // ceil(N / 128)
@@ -104,7 +106,8 @@ void gemm_plan(GemmArgs* a);  // fills stages / acc_stages / tmem_cols / num_nt 
 int launch_gemm_tc(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                    cudaStream_t stream);
 void gemm_plan_fp8(GemmArgs* a);
-int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
+// tm_xc (blocks of 128): boxes of 16 rows for blocks that hold no more
+int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_xc, const GemmArgs& a, int num_sms,
                     cudaStream_t stream);
 // int4 AWQ: see gemm_w4.cu.  Token maps: boxes of 16 (i + 1) rows x the 64-k halves of a group;
 // decode blocks use m[0] (their rows, two groups).

@@ -15,6 +15,7 @@
 //           dynamic 1x128 quantisation (the 128 lanes are exactly one group) -> e4m3 + scale.
 //   mode 1: rows n0.. and n0+128.. of the down projection; tail = routing weight and
 //           red.global.add.f32 into the combine buffer (K may be split across CTAs).
+// Blocks of 128 tokens run in a launch of their own kind (moe_gemm_fp8_mixed_kernel, below).
 //
 // Warps: TMA producer, MMA issuer (owns tensor memory), four promotion warps per group of up
 // to 64 tokens (one group for blocks of 16/32/64, two for blocks of 128), and a
@@ -29,23 +30,32 @@ namespace b200moe {
 namespace {
 
 constexpr int kMaxKB = 64;  // 128-wide reduction slices per tile whose scales are staged in shared memory
-constexpr int fp8_threads(int ng) { return 7 * 32 + (ng - 1) * 128; }
+__host__ __device__ constexpr int fp8_threads(int ng) { return 7 * 32 + (ng - 1) * 128; }
+
+// A CTA's share of a launch: tiles cta, cta + c.grid_eff, ... of c.total.
+struct Fp8Part {
+  Ctrl c;
+  int cta;
+  const int* off;   // [E+1] blocks of this share before expert e
+  const int* blk;   // [E+1] blocks before expert e
+  int rows;         // padded rows of a block
+};
+__device__ __forceinline__ TileCoord part_tile(int id, const Fp8Part& p, const GemmArgs& a, int tile_n) {
+  TileCoord t = decode_tile(id, p.c, p.off, a.E, 1, a.num_nt, a.kblocks, tile_n);
+  t.row0 = (p.blk[t.e] + t.row0 - p.off[t.e]) * p.rows;
+  return t;
+}
 
 // NG = promotion groups; group g owns token columns [g * BT / NG, (g + 1) * BT / NG)
-template <int MODE, int BT, int NG>
-__global__ void __launch_bounds__(fp8_threads(NG), 1)
-moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
-                    const GemmArgs a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+// MIXED: part of a launch with two kinds of tiles (moe_gemm_fp8_mixed_kernel), which hands over its share and the tensor memory
+template <int MODE, int BT, int NG, bool MIXED>
+__device__ __forceinline__ void weights_on_m(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, uint8_t* smem,
+                                             const int stages, Fp8Part& part, uint32_t tmem_base) {
   constexpr int W_BYTES = 2 * kTileBytes;
   constexpr int X_BYTES = BT * kStageKBytes;
   constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
   constexpr int PCOLS = 2 * BT;  // columns of one partial accumulator (both row blocks)
   constexpr int NPB = (512 / PCOLS) >= 4 ? 4 : 2;  // partial accumulators in flight
-  const int stages = a.stages;
-
   uint8_t* ctrl_base = smem + static_cast<size_t>(stages) * STAGE_BYTES;
   float* s_xs = reinterpret_cast<float*>(ctrl_base);                    // [2][kMaxKB][BT] activation scales
   float* s_ws = s_xs + 2 * kMaxKB * BT;                                 // [2][2][kMaxKB] weight scales
@@ -68,7 +78,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 
   const int warp = warp_index();
   const int lane = threadIdx.x & 31;
-  const bool own = BT <= 32 && a.route.own != 0, early = own && a.route.early != 0;
+  const bool own = !MIXED && BT <= 32 && a.route.own != 0, early = own && a.route.early != 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -90,23 +100,30 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     prefetch_tmap(&tm_w);
     prefetch_tmap(&tm_x);
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(a.tmem_cols));
-    tmem_relinquish();
+  if constexpr (!MIXED) {
+    if (warp == 1) {
+      tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(a.tmem_cols));
+      tmem_relinquish();
+    }
+    // everything above touched only shared / tensor memory and kernel parameters
+    if (!early) griddep_wait();
+    griddep_launch_dependents();
+    if (own) count_slots(a.route, a.P, a.E, BT, rt);
+    else
+      for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
+    tc_fence_before();
   }
-  // everything above touched only shared / tensor memory and kernel parameters
-  if (!early) griddep_wait();
-  griddep_launch_dependents();
-  if (own) count_slots(a.route, a.P, a.E, BT, rt);
-  else
-    for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  const Ctrl c = make_ctrl(a, own ? s_blk_off[a.E] : a.meta[0], MODE == 1);
-  const bool active = static_cast<int>(blockIdx.x) < c.grid_eff;
+  if constexpr (!MIXED) {
+    tc_fence_after();
+    tmem_base = *tmem_slot;
+    part.c = make_ctrl(a, own ? s_blk_off[a.E] : a.meta[0], MODE == 1);
+    part.cta = blockIdx.x;
+    part.off = part.blk = s_blk_off;
+    part.rows = BT;
+  }
+  const Ctrl& c = part.c;
+  const bool active = part.cta < c.grid_eff;
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;  // output rows advanced per n-tile
   // row offset of the second weight block inside the expert
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
@@ -128,14 +145,14 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     // the ring's first round of weights, before the activations may be read
     int ahead = 0;
     if (early) {
-      for (int tile = blockIdx.x; ahead < stages && tile < c.total; tile += c.grid_eff) {
-        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+      for (int tile = part.cta; ahead < stages && tile < c.total; tile += c.grid_eff) {
+        const TileCoord t = part_tile(tile, part, a, kTileN);
         for (int kb = t.kb0; ahead < stages && kb < t.kb1; ++kb, ++ahead) load_weights(t, kb, ahead);
       }
       griddep_wait();
     }
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+    for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff) {
+      const TileCoord t = part_tile(tile, part, a, kTileN);
       for (int kb = t.kb0; kb < t.kb1; ++kb) {
         if (issued >= ahead) {
           if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER)) {
@@ -171,8 +188,8 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     int stage = 0;
     uint32_t phase = 0, j = 0;  // j counts reduction slices over the whole launch
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+    for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff) {
+      const TileCoord t = part_tile(tile, part, a, kTileN);
       for (int kb = t.kb0; kb < t.kb1; ++kb, ++j) {
         const uint32_t pb = j % NPB;
         if (!mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag, DEV_TIMEOUT_MMA) ||
@@ -204,8 +221,8 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     griddep_wait();
     const int kb_total = a.kblocks;
     int iter = 0;
-    for (int tile = blockIdx.x; tile < c.total; tile += c.grid_eff, ++iter) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+    for (int tile = part.cta; tile < c.total; tile += c.grid_eff, ++iter) {
+      const TileCoord t = part_tile(tile, part, a, kTileN);
       const int buf = iter & 1;
       if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
       const int nkb = t.kb1 - t.kb0;
@@ -213,12 +230,14 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const int slot = rows_slot(a, rt, BT, t.e, t.row0 + r, BT < 32 ? BT : 32), cidx = r + lane;
         if (cidx >= BT) continue;
         const bool valid = slot >= 0;
-        const int orow = valid ? (MODE == 1 ? slot / a.topk : slot) : -1;
+        const bool pairs = MIXED && MODE == 1 && a.out_pairs != nullptr;      // the output row is the pair's own slot
+        const int orow = valid ? (MODE == 1 && !pairs ? slot / a.topk : slot) : -1;
         s_col_row[buf * 128 + cidx] = orow;
         s_col_gam[buf * 128 + cidx] = rows_weight(a, rt, BT, t.e, t.row0 + r, slot);
         if (MODE == 1 && valid)
           s_col_ptr[buf * 128 + cidx] = reinterpret_cast<unsigned long long>(
-              out_row_base(a, a.out, orow, static_cast<size_t>(a.ld_out) * sizeof(float)));
+              pairs ? out_row_base(a, a.out_pairs, orow, static_cast<size_t>(a.N) * 2)
+                    : out_row_base(a, a.out, orow, static_cast<size_t>(a.ld_out) * sizeof(float)));
       }
       const int nb0 = t.n0 / 128, nb1 = (second_off + t.n0) / 128;
       const float* ws0 = a.w_scale + (static_cast<size_t>(t.e) * a.w_scale_rows + nb0) * kb_total + t.kb0;
@@ -238,7 +257,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         bulk_copy_g2s(smem_u32(s_xs + (buf * kMaxKB + i) * BT),
                       a.x_scale + static_cast<size_t>(t.kb0 + i) * a.ld_xscale + t.row0, BT * 4, sfull);
     }
-  } else if (active && warp >= 2 && warp != 6) {
+  } else if (active && warp >= 2 && warp != 6 && warp < fp8_threads(NG) / 32) {
     // =============================== promotion + tail ===========================
     griddep_wait();
     const int grp = warp < 6 ? 0 : 1;               // promotion group
@@ -252,8 +271,8 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     uint32_t meet_phase = 0;
     int iter = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff, ++iter) {
-      const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+    for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff, ++iter) {
+      const TileCoord t = part_tile(tile, part, a, kTileN);
       const int buf = iter & 1;
       const int* col_row = s_col_row + buf * 128 + cb;
       const float* col_gam = s_col_gam + buf * 128 + cb;
@@ -355,6 +374,23 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           if (n < a.N) b0 = __ldg(a.bias + static_cast<size_t>(t.e) * a.N + n);
           if (second) b1 = __ldg(a.bias + static_cast<size_t>(t.e) * a.N + n + kTileRows);
         }
+        if (MIXED && a.out_pairs != nullptr) {
+          // the pair's row, weighted and rounded to the 16-bit type; a warp stores 64 contiguous bytes of it
+          const bool bf = a.dtype == B200MOE_DTYPE_BF16;
+          auto half_bits = [&](float v) -> uint16_t {
+            return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+          };
+#pragma unroll
+          for (int i = 0; i < CPT; ++i) {
+            const int orow = col_row[i];
+            if (orow < 0) continue;
+            const float gam = w_on_input ? 1.0f : col_gam[i];
+            uint16_t* out = reinterpret_cast<uint16_t*>(col_ptr[i]) + n;
+            out[0] = half_bits((acc0[i] + b0) * gam);
+            if (second) out[kTileRows] = half_bits((acc1[i] + b1) * gam);
+            if (n == 0) mark_pair_valid(a, orow);
+          }
+        } else {
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
           const int orow = col_row[i];
@@ -364,6 +400,7 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             atomicAdd(out, (acc0[i] + b0) * gam);
             if (second) atomicAdd(out + kTileRows, (acc1[i] + b1) * gam);
           }
+        }
         }
       }
       // the tables of this tile may now be overwritten
@@ -375,12 +412,23 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   // ---- teardown
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (!MIXED && warp == 1) {
     __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, static_cast<uint32_t>(a.tmem_cols));
   }
   if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(a.status, 0, *abort_flag);
+}
+
+template <int MODE, int BT, int NG>
+__global__ void __launch_bounds__(fp8_threads(NG), 1)
+moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                    const GemmArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  Fp8Part part;
+  weights_on_m<MODE, BT, NG, false>(tm_w, tm_x, a, smem, a.stages, part, 0);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -395,18 +443,20 @@ moe_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 // activations of its thread in group 0 plus the 64 of its thread in group 1: the two partial
 // maxima meet in shared memory, no shuffles.
 //
-// What bounds it: the promotion's serial path per slice (wait, tensor-memory reads, FMAs, release), about 1000
-// cycles against 512 for the slice's MMAs, and the tail (5000 cycles per tile) that nothing overlaps: the
-// accumulators fill the registers and the two partial buffers all of tensor memory.  Kept off that
-// path: the tile's coordinates (decoded by the table warp), the activation scales (a ring filled per slice, which also
-// frees the room of a fourth stage).  A warp whose 32 rows are all padding (three of four in the block of a cold expert)
-// keeps in step with the others and promotes nothing, which leaves the board's power to the rest.  256 experts,
-// zipf-skewed routing, one board: 4096 tokens 3045 us, 512: 1056; with the tables on the promotion's path, results turned in
-// shared memory before the store and padding rows promoted 3402 and 1155.
+// What bounds it, from the CTAs' cycles at 4096 tokens (256 experts, zipf-skewed) with and without parts of the work: the
+// promotion, about 970 cycles per slice in the gate/up projection and 800 in the down projection against 512 for the
+// slice's MMAs, and the tail that nothing overlaps (11400 and 5300 cycles per tile: the accumulators fill the registers
+// and the two partial buffers all of tensor memory).  With a third of the operand loads left out the cycles stay and the
+// clock rises by 9 %: in a train of calls the board is at its power cap.  Alone, with operands that stay in shared
+// memory, the same promotion takes 696 cycles per slice, its tensor-memory reads 513.
+// Kept off that path: the tile's coordinates (decoded by the table warp), the activation scales (a ring filled per slice, which
+// also frees the room of a fourth stage).  A warp whose 32 rows are all padding keeps in step with the others and promotes
+// nothing, which leaves the board's power to the rest.
 // Tried and slower: sixteen promotion warps, 32-column reads, scalar FMAs, partial buffers released by halves, hot and
-// cold experts' tiles interleaved.
-// warps 0-3: TMA, MMA, tables, idle; warps 4-11: promotion.  Launched with 168 registers a thread, the
-// first four warps keep 48 and the promotion warps take 224: 4 * 48 + 8 * 224 <= 12 * 168.
+// cold experts' tiles interleaved on every CTA.
+// warps 0-3: TMA, MMA, tables, idle; warps 4-11: promotion.  Launched with 168 registers a thread; the first four warps
+// give some up for the promotion, within 12 * 168: 72 and 216 in mode 0, where the other roles spill with less (their
+// spills cost the whole tile 10 %), 56 and 224 in mode 1, whose promotion does with less.
 constexpr int kThreadsFp8TokM = 12 * 32;
 constexpr int kXsSlots = 8;                                       // ring of activation scales, one slot per slice
 
@@ -425,12 +475,8 @@ __device__ __forceinline__ void st_global_v8(uint8_t* p, const uint32_t* w) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kThreadsFp8TokM, 1)
-moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
-                         const GemmArgs a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+__device__ __forceinline__ void tokens_on_m(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, uint8_t* smem,
+                                            const Fp8Part& part, const uint32_t tmem_base) {
   constexpr int BT = 128;
   constexpr int W_BYTES = 2 * kTileBytes;
   constexpr int X_BYTES = BT * kStageKBytes;
@@ -449,14 +495,12 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   uint64_t* bar_sfull = bar_pempty + 2;
   uint64_t* bar_sempty = bar_sfull + 2;
   uint64_t* bar_meet8 = bar_sempty + 2;         // both groups: the halves of a quantisation group's maximum
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_meet8 + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_tile = reinterpret_cast<int*>(tmem_slot + 4);                  // [2][8] expert, row0, n0, kb0, kb1 of a tile
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_meet8 + 1);
+  int* s_tile = reinterpret_cast<int*>(bar_meet8 + 3);                  // [2][8] expert, row0, n0, kb0, kb1 of a tile
   int* s_col_row = s_tile + 16;               // [2][128] output row of each token
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * 128);     // [2][128]
   float* s_red = s_col_gam + 2 * 128;                                   // mode 0: [2][2][128] partial group maxima
   unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + (MODE == 0 ? 2 * 2 * 128 : 0));   // [2][128] mode 1: base of each row's output row
-  int* s_blk_off = reinterpret_cast<int*>(s_col_ptr + (MODE == 1 ? 2 * 128 : 0));   // [E+1]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -479,25 +523,16 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     prefetch_tmap(&tm_w);
     prefetch_tmap(&tm_x);
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 512u);
-    tmem_relinquish();
-  }
-  griddep_wait();
-  griddep_launch_dependents();
-  for (int e = threadIdx.x; e <= a.E; e += blockDim.x) s_blk_off[e] = a.blk_off[e];
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
 
-  const Ctrl c = make_ctrl(a, a.meta[0], MODE == 1);
-  const bool active = static_cast<int>(blockIdx.x) < c.grid_eff;
+  const Ctrl& c = part.c;
+  const bool active = part.cta < c.grid_eff;
   constexpr int kTileN = (MODE == 0) ? kTileRows : 2 * kTileRows;
   const int second_off = (MODE == 0) ? a.up_row_off : kTileRows;
 
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    if (MODE == 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (active && warp == 0 && elect_one()) {
       // =============================== TMA producer ===============================
       int stage = 0;
@@ -507,8 +542,8 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       bool ok = true;
       unsigned long long w_empty = 0;
       const long long role_t0 = clock64();
-      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
-        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+      for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff) {
+        const TileCoord t = part_tile(tile, part, a, kTileN);
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
           if (!mbar_wait_t(smem_u32(&bar_empty[stage]), phase ^ 1, abort_flag, DEV_TIMEOUT_PRODUCER, w_empty)) {
             ok = false;
@@ -557,10 +592,10 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       bool ok = true;
       unsigned long long w_full = 0, w_pempty = 0;
       const long long role_t0 = clock64();
-      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff) {
+      for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff) {
         int kb0 = 0, kb1 = a.kblocks;
         if (c.split > 1) {       // only the slice count matters here
-          const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+          const TileCoord t = part_tile(tile, part, a, kTileN);
           kb0 = t.kb0;
           kb1 = t.kb1;
         }
@@ -593,8 +628,8 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       // =============================== per-tile table loader ======================
       const int kb_total = a.kblocks;
       int iter = 0;
-      for (int tile = blockIdx.x; tile < c.total; tile += c.grid_eff, ++iter) {
-        const TileCoord t = decode_tile(tile, c, s_blk_off, a.E, BT, a.num_nt, a.kblocks, kTileN);
+      for (int tile = part.cta; tile < c.total; tile += c.grid_eff, ++iter) {
+        const TileCoord t = part_tile(tile, part, a, kTileN);
         const int buf = iter & 1;
         if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
         const int nkb = t.kb1 - t.kb0;
@@ -632,7 +667,8 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    if (MODE == 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     if (active) {
       // =============================== promotion + tail ===========================
       const int grp = warp < 8 ? 0 : 1;
@@ -648,7 +684,7 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       bool ok = true;
       unsigned long long w_pfull = 0, w_sfull = 0, t_tail = 0;
       const long long role_t0 = clock64();
-      for (int tile = blockIdx.x; ok && tile < c.total; tile += c.grid_eff, ++iter) {
+      for (int tile = part.cta; ok && tile < c.total; tile += c.grid_eff, ++iter) {
         const int buf = iter & 1;
         const float* ws_t = s_ws + buf * 2 * KBS;
         if (!mbar_wait_t(smem_u32(&bar_sfull[buf]), (iter >> 1) & 1, abort_flag, DEV_TIMEOUT_EPILOGUE, w_sfull)) break;
@@ -829,50 +865,152 @@ moe_gemm_fp8_tokm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     }
   }
 
-  // ---- teardown
+  // ---- teardown (the launch frees tensor memory)
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(a.status, 0, *abort_flag);
+}
+
+// ------------------------------------------------------------------------------------------
+// Prefill-sized batches: one launch for both kinds of blocks.  Routing of many-expert layers is skewed: of 4096 tokens' 397
+// blocks of 128 on 256 experts, 107 hold at most 16 tokens.  Such a cold block's time is its expert's weights' way from
+// HBM, a hot one's is the promotion; one kind after the other, as the experts come, leaves either idle.  So some CTAs
+// take the hot blocks (tokens on M) and the rest the cold ones (weights on M, 16 tokens on N, which also spares the
+// MMAs of 112 padding rows), in proportion to what they cost.  The rows lie in the same blocks of 128 for both.
+// us per call, all blocks with tokens on M / mixed, one board: 130 tokens 583 (blocks of 32) / 475, 300: 745 / 647, 1024: 1265 /
+// 1070, 2048: - / 1650, 4096: 3010 / 2750.
+constexpr int kColdRows = 16;
+// Cycles of a 128-wide reduction slice and of a tile's tail, from the CTAs' times at 4096 tokens: hot tiles 65800 (gate/up, 56
+// slices) and 18000 cycles (down, 16), 40000 and 13500 with a quarter of the promotion, cold ones 31800 and 11800.  The
+// cold slices of mode 0 count for more than the 525 measured: 4096 tokens 2800 us with that, 2750 with 600, 2766 with 680.
+template <int MODE>
+struct MixedCost {
+  static constexpr float kHotSlice = MODE == 0 ? 970.f : 800.f, kHotTail = MODE == 0 ? 11400.f : 5300.f;
+  static constexpr float kColdSlice = MODE == 0 ? 600.f : 580.f, kColdTail = 2500.f;
+};
+
+__host__ __device__ __forceinline__ size_t mixed_table_bytes(int E) {
+  return (3 * static_cast<size_t>(E + 1) * 4 + 16 + sizeof(Fp8Part) + 1023) & ~static_cast<size_t>(1023);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreadsFp8TokM, 1)
+moe_gemm_fp8_mixed_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                          const __grid_constant__ CUtensorMap tm_xc, const GemmArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  // tables behind the larger of the two kinds' shared memory (whose addresses then need no offset: the promotion has no
+  // register left for one)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + a.table_off);
+  Fp8Part* s_part = reinterpret_cast<Fp8Part*>(tmem_slot + 4);
+  int* s_blk = reinterpret_cast<int*>(s_part + 1);      // [E+1] blocks before expert e
+  int* s_hot = s_blk + (a.E + 1);                       // [E+1] hot blocks before expert e
+  int* s_cold = s_hot + (a.E + 1);                      // [E+1] cold ones
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 512u);
+    tmem_relinquish();
+  }
+  griddep_wait();
+  griddep_launch_dependents();
+  if (warp == 0) {
+    unsigned long long run = 0;      // running sums: hot blocks below, cold ones above
+    for (int e0 = 0; e0 < a.E; e0 += 32) {
+      const int e = e0 + lane;
+      int first = 0, n = 0;
+      bool cold = false;
+      if (e < a.E) {
+        first = a.blk_off[e];
+        n = a.blk_off[e + 1] - first;
+        cold = n == 1 && a.sorted_ids[first * 128 + kColdRows] == a.P;      // an expert's rows stand in front of its padding
+        s_blk[e] = first;
+        if (e == a.E - 1) s_blk[a.E] = first + n;
+      }
+      unsigned long long v = cold ? 1ull << 32 : static_cast<unsigned long long>(n);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (e < a.E) {
+        s_hot[e + 1] = static_cast<int>(run + v);
+        s_cold[e + 1] = static_cast<int>((run + v) >> 32);
+      }
+      run += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) s_hot[0] = s_cold[0] = 0;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int hot = s_hot[a.E], cold = s_cold[a.E], grid = gridDim.x;
+  int split = 1;
+  if (MODE == 1 && !(a.flags & B200MOE_FLAG_NO_SPLIT_K)) split = pick_split((hot + cold) * a.num_nt, a.kblocks, grid, a.max_split);
+  const int units = a.num_nt * split;
+  const float slices = static_cast<float>(a.kblocks) / split;
+  using Cost = MixedCost<MODE>;
+  const float hot_cost = hot * (slices * Cost::kHotSlice + Cost::kHotTail), cold_cost = cold * (slices * Cost::kColdSlice + Cost::kColdTail);
+  int cold_ctas = 0;
+  if (cold > 0) {
+    cold_ctas = static_cast<int>(grid * cold_cost / (hot_cost + cold_cost) + 0.5f);
+    cold_ctas = hot > 0 ? max(1, min(grid - 1, cold_ctas)) : grid;
+  }
+  const bool cold_cta = static_cast<int>(blockIdx.x) < cold_ctas;
+  if (threadIdx.x == 0) {
+    Fp8Part part;
+    part.cta = cold_cta ? blockIdx.x : blockIdx.x - cold_ctas;
+    part.off = cold_cta ? s_cold : s_hot;
+    part.blk = s_blk;
+    part.rows = 128;
+    part.c = spread_tiles(cold_cta ? cold : hot, units, split, cold_cta ? cold_ctas : grid - cold_ctas, a.flags);
+    *s_part = part;
+  }
+  if (cold_cta) weights_on_m<MODE, kColdRows, 1, true>(tm_w, tm_xc, a, smem, a.stages_cold, *s_part, tmem_base);
+  else tokens_on_m<MODE>(tm_w, tm_x, a, smem, *s_part, tmem_base);
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, 512u);
   }
-  if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(a.status, 0, *abort_flag);
 }
 
+size_t fp8_stage_bytes(int bt) { return 2 * static_cast<size_t>(kTileBytes) + static_cast<size_t>(bt) * kStageKBytes; }
+size_t fp8_ctrl_bytes(const GemmArgs& a, int bt) {
+  return 2 * static_cast<size_t>(kMaxKB) * bt * 4 + 2 * 2 * kMaxKB * 4 + 512 /*barriers*/ + 2 * 128 * 8 +
+         2 * 2 * 4 * 64 * 4 + 2 * 128 * 8 +
+         (a.route.own ? route_table_bytes(a.E, a.P) : static_cast<size_t>(a.E + 1) * 4) + 64;
+}
 size_t fp8_tokm_ctrl_bytes(const GemmArgs& a) {
   return kXsSlots * 128 * 4 + 2 * 2 * static_cast<size_t>(a.kblocks) * 4 +
          512 /*barriers, tile words*/ + 2 * 2 * 128 * 4 +
-         (a.mode == 0 ? 2 * 2 * 128 * 4 : 2 * 128 * 8) + static_cast<size_t>(a.E + 1) * 4 + 64;
+         (a.mode == 0 ? 2 * 2 * 128 * 4 : 2 * 128 * 8) + 64;
 }
 
 template <int MODE>
-int launch_fp8_tokm(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
-                    cudaStream_t stream) {
-  const size_t smem = 1024 + static_cast<size_t>(a.stages) * (3 * kTileBytes) + fp8_tokm_ctrl_bytes(a);
+int launch_fp8_mixed(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_xc, const GemmArgs& a, int num_sms,
+                     cudaStream_t stream) {
+  const size_t hot = static_cast<size_t>(a.stages) * (3 * kTileBytes) + fp8_tokm_ctrl_bytes(a);
+  const size_t cold = a.stages_cold * fp8_stage_bytes(kColdRows) + fp8_ctrl_bytes(a, kColdRows);
+  GemmArgs g = a;
+  g.table_off = static_cast<int>(((hot > cold ? hot : cold) + 1023) & ~static_cast<size_t>(1023));
+  const size_t smem = 1024 + g.table_off + mixed_table_bytes(a.E);
   if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
-  if (cudaFuncSetAttribute(moe_gemm_fp8_tokm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(moe_gemm_fp8_mixed_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
-  note_launch(MODE == 0 ? "moe_gemm_fp8_tokm_kernel<gate/up>" : "moe_gemm_fp8_tokm_kernel<down>");
-  cudaError_t err = launch_kernel(moe_gemm_fp8_tokm_kernel<MODE>, dim3(num_sms), dim3(kThreadsFp8TokM), smem, stream,
-                                  a.pdl != 0, tm_w, tm_x, a);
+  note_launch(MODE == 0 ? "moe_gemm_fp8_mixed_kernel<gate/up>" : "moe_gemm_fp8_mixed_kernel<down>");
+  cudaError_t err = launch_kernel(moe_gemm_fp8_mixed_kernel<MODE>, dim3(num_sms), dim3(kThreadsFp8TokM), smem, stream,
+                                  a.pdl != 0, tm_w, tm_x, tm_xc, g);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
-}
-
-size_t fp8_stage_bytes(const GemmArgs& a) {
-  return 2 * static_cast<size_t>(kTileBytes) + static_cast<size_t>(a.BT) * kStageKBytes;
-}
-size_t fp8_ctrl_bytes(const GemmArgs& a) {
-  return 2 * static_cast<size_t>(kMaxKB) * a.BT * 4 + 2 * 2 * kMaxKB * 4 + 512 /*barriers*/ + 2 * 128 * 8 +
-         2 * 2 * 4 * 64 * 4 + 2 * 128 * 8 +
-         (a.route.own ? route_table_bytes(a.E, a.P) : static_cast<size_t>(a.E + 1) * 4) + 64;
 }
 
 template <int MODE, int BT, int NG>
 int launch_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
                cudaStream_t stream) {
-  const size_t smem = 1024 + static_cast<size_t>(a.stages) * fp8_stage_bytes(a) + fp8_ctrl_bytes(a);
+  const size_t smem = 1024 + static_cast<size_t>(a.stages) * fp8_stage_bytes(a.BT) + fp8_ctrl_bytes(a, a.BT);
   if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
   if (cudaFuncSetAttribute(moe_gemm_fp8_kernel<MODE, BT, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
@@ -907,11 +1045,13 @@ void gemm_plan_fp8(GemmArgs* a) {
   while (tc < cols) tc <<= 1;
   a->tmem_cols = tc;
   a->acc_stages = 2;
-  int st = static_cast<int>((kSmemLimit - 1024 - fp8_ctrl_bytes(*a)) / fp8_stage_bytes(*a));
+  int st = static_cast<int>((kSmemLimit - 1024 - fp8_ctrl_bytes(*a, a->BT)) / fp8_stage_bytes(a->BT));
   if (a->orient == 1) {   // tokens on M, 128-token blocks
     a->tmem_cols = 512;
-    st = static_cast<int>((kSmemLimit - 1024 - fp8_tokm_ctrl_bytes(*a)) / (3 * kTileBytes));
+    const size_t room = kSmemLimit - 2048 - mixed_table_bytes(a->E);
+    st = static_cast<int>((room - fp8_tokm_ctrl_bytes(*a)) / (3 * kTileBytes));
     if (st > kXsSlots - 2) st = kXsSlots - 2;
+    a->stages_cold = static_cast<int>((room - fp8_ctrl_bytes(*a, kColdRows)) / fp8_stage_bytes(kColdRows));
   }
   if (st > 10) st = 10;
   if (st < 2) st = 2;
@@ -919,13 +1059,13 @@ void gemm_plan_fp8(GemmArgs* a) {
   if (a->max_split <= 0) a->max_split = 16;
 }
 
-int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs& a, int num_sms,
+int launch_gemm_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_xc, const GemmArgs& a, int num_sms,
                     cudaStream_t stream) {
   if (a.wmode != B200MOE_W_FP8_BLOCK) return B200MOE_ERR_BAD_ARG;
   if (a.K % 128 != 0 || a.N % 128 != 0 || a.K / 128 > kMaxKB) return B200MOE_ERR_UNSUPPORTED;
   if (a.orient == 1 && a.BT == 128)
-    return a.mode == 0 ? launch_fp8_tokm<0>(tm_w, tm_x, a, num_sms, stream)
-                       : launch_fp8_tokm<1>(tm_w, tm_x, a, num_sms, stream);
+    return a.mode == 0 ? launch_fp8_mixed<0>(tm_w, tm_x, tm_xc, a, num_sms, stream)
+                       : launch_fp8_mixed<1>(tm_w, tm_x, tm_xc, a, num_sms, stream);
 #define B200MOE_FP8_CASE(bt, ng)                                                          \
   case bt:                                                                                \
     return a.mode == 0 ? launch_fp8<0, bt, ng>(tm_w, tm_x, a, num_sms, stream)            \

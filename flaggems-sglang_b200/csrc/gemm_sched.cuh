@@ -163,20 +163,24 @@ __device__ __forceinline__ ActParams act_params(const GemmArgs& a) {
   return p;
 }
 
-// Work decomposition for one launch; identical in every thread of every CTA.
-__device__ __forceinline__ Ctrl make_ctrl(const GemmArgs& a, int nblocks, bool may_split) {
+// `nblocks` blocks of `units` tiles each over `ctas` CTAs, evenly: with w waves, ceil(total / w) CTAs do w tiles each.
+__device__ __forceinline__ Ctrl spread_tiles(int nblocks, int units, int split, int ctas, int flags) {
   Ctrl c;
   c.nblocks = nblocks;
-  c.split = 1;
-  if (may_split && !(a.flags & B200MOE_FLAG_NO_SPLIT_K))
-    c.split = pick_split(c.nblocks * a.num_nt, a.kblocks, gridDim.x, a.max_split);
-  c.units_per_block = a.num_nt * c.split;
-  c.total = c.nblocks * c.units_per_block;
-  // spread the tiles evenly: with w waves, ceil(total / w) CTAs do w tiles each
-  int waves = (c.total + gridDim.x - 1) / static_cast<int>(gridDim.x);
+  c.split = split;
+  c.units_per_block = units;
+  c.total = nblocks * units;
+  const int waves = ctas > 0 ? (c.total + ctas - 1) / ctas : 0;
   c.grid_eff = waves > 0 ? (c.total + waves - 1) / waves : 1;
-  if (a.flags & B200MOE_FLAG_NO_GRID_BALANCE) c.grid_eff = gridDim.x;
+  if (flags & B200MOE_FLAG_NO_GRID_BALANCE) c.grid_eff = ctas;
   return c;
+}
+
+// Work decomposition for one launch; identical in every thread of every CTA.
+__device__ __forceinline__ Ctrl make_ctrl(const GemmArgs& a, int nblocks, bool may_split) {
+  int split = 1;
+  if (may_split && !(a.flags & B200MOE_FLAG_NO_SPLIT_K)) split = pick_split(nblocks * a.num_nt, a.kblocks, gridDim.x, a.max_split);
+  return spread_tiles(nblocks, a.num_nt * split, split, gridDim.x, a.flags);
 }
 
 }  // namespace b200moe

@@ -208,15 +208,16 @@ group_quant_fp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* 
   }
 }
 
-// The quantisation for a call whose GEMMs sort the slots themselves (gemm_route.cuh): a warp quantises a run of groups of a
-// token once and stores it for each of the token's slots, where the GEMMs look for the row.  The kernel is a few
+// The quantisation by token: a warp quantises a run of groups once and stores it for each of the token's slots, in the row that
+// the alignment gave it (slot_row) or, where the GEMMs sort the slots themselves (gemm_route.cuh), in the one they
+// look for.  (Quantising the tokens and gathering the bytes: 4096 tokens of 56 groups, top-8, 38 + 67 us.)  At decode the kernel is a few
 // microseconds long, so its loops stay rolled: straight-line code for eight groups and eight slots spent more time being
 // fetched than executed (64 tokens of 56 groups, top-8: 18.5 us; an alignment and one warp per slot: 20).
 constexpr int kQuantRun = 8;      // groups of a run at most; few tokens are dealt out in shorter ones
 template <typename T>
 __global__ void __launch_bounds__(256)
-group_quant_routed_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, const RouteSource route,
-                          int P, int E, int BT, int topk, int M, int K, int run, int ld_scale, uint4* __restrict__ zero,
+group_quant_slots_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, const RouteSource route,
+                          const int* __restrict__ slot_row, int P, int E, int BT, int topk, int M, int K, int run, int ld_scale, uint4* __restrict__ zero,
                           long long zero_chunks) {
   extern __shared__ __align__(16) uint8_t route_smem[];
   __shared__ __align__(16) uint2 s_x[8][kQuantRun][32];
@@ -238,7 +239,7 @@ group_quant_routed_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, floa
   int w = thread >> 5;
   if (w < M * runs) fetch(w);
   for (long long i = thread; i < zero_chunks; i += threads) zero[i] = make_uint4(0, 0, 0, 0);
-  count_slots(route, P, E, BT, t);
+  if (slot_row == nullptr) count_slots(route, P, E, BT, t);
   for (bool first_run = true; w < M * runs; w += threads >> 5, first_run = false) {
     if (!first_run) fetch(w);
     const int tok = w / runs, g0 = (w - tok * runs) * run, n = min(run, groups - g0);
@@ -246,8 +247,9 @@ group_quant_routed_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, floa
     for (int j0 = 0; j0 < topk; j0 += 32) {
       const int nj = min(32, topk - j0);
       int row = -1;             // lane j: padded row of the token's slot j0 + j
+      if (slot_row != nullptr && lane < nj) row = slot_row[tok * topk + j0 + lane];
 #pragma unroll 1
-      for (int j = 0; j < nj; ++j) {
+      for (int j = 0; slot_row == nullptr && j < nj; ++j) {
         const int slot = tok * topk + j0 + j;
         const unsigned e = t.ids[ids_at(slot)];
         const int rank = e == kNoSlot ? -1 : slot_rank(t, slot, e);
@@ -410,28 +412,29 @@ int launch_group_quant_fp8(const void* x, int dtype, void* q, float* scales, con
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
-int launch_group_quant_routed(const void* x, int dtype, void* q, float* scales, const RouteSource& route, int P, int E, int BT,
-                              int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms, cudaStream_t stream,
-                              bool pdl) {
-  const size_t smem = route_table_bytes(E, P);
+int launch_group_quant_slots(const void* x, int dtype, void* q, float* scales, const RouteSource& route, const int* slot_row, int P,
+                             int E, int BT, int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms,
+                             cudaStream_t stream, bool pdl) {
+  const size_t smem = slot_row != nullptr ? 16 : route_table_bytes(E, P);
   if (K % 128 != 0 || zero_bytes % 16 != 0 || route.hist != nullptr) return B200MOE_ERR_UNSUPPORTED;
   if (smem > 30 * 1024) return B200MOE_ERR_TOO_LARGE;
   const int groups = K / 128;
   int run = (M * groups + 16 * num_sms - 1) / (16 * num_sms);
   if (run > kQuantRun) run = kQuantRun;
   int ctas = (M * ((groups + run - 1) / run) + 7) / 8;
-  if (ctas > 2 * num_sms) ctas = 2 * num_sms;
+  const int most = (slot_row != nullptr ? 8 : 2) * num_sms;      // (few where each CTA counts the slots first)
+  if (ctas > most) ctas = most;
   if (ctas < 1) ctas = 1;
   const long long zc = static_cast<long long>(zero_bytes / 16);
-  note_launch("group_quant_routed_kernel");
+  note_launch("group_quant_slots_kernel");
   cudaError_t err;
   if (dtype == B200MOE_DTYPE_BF16)
-    err = launch_kernel(group_quant_routed_kernel<__nv_bfloat16>, dim3(ctas), dim3(256), smem, stream, pdl,
-                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, route, P, E, BT, topk, M, K,
+    err = launch_kernel(group_quant_slots_kernel<__nv_bfloat16>, dim3(ctas), dim3(256), smem, stream, pdl,
+                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E, BT, topk, M, K,
                         run, ld_scale, reinterpret_cast<uint4*>(zero), zc);
   else
-    err = launch_kernel(group_quant_routed_kernel<__half>, dim3(ctas), dim3(256), smem, stream, pdl, reinterpret_cast<const __half*>(x),
-                        reinterpret_cast<uint8_t*>(q), scales, route, P, E, BT, topk, M, K, run, ld_scale,
+    err = launch_kernel(group_quant_slots_kernel<__half>, dim3(ctas), dim3(256), smem, stream, pdl, reinterpret_cast<const __half*>(x),
+                        reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E, BT, topk, M, K, run, ld_scale,
                         reinterpret_cast<uint4*>(zero), zc);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }

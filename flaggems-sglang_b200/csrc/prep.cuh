@@ -18,9 +18,10 @@ int launch_gather_rows(const void* x, void* xs, const int* sorted_ids, const int
 int launch_gather_routed(const void* x, void* xs, const RouteSource& route, int P, int E, int BT, int topk, int row_bytes, void* zero,
                          size_t zero_bytes, int num_sms, cudaStream_t stream, bool pdl);
 
-int launch_group_quant_routed(const void* x, int dtype, void* q, float* scales, const RouteSource& route, int P, int E, int BT,
-                              int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms, cudaStream_t stream,
-                              bool pdl);
+// The quantisation by token (FP8 weights): rows as above, or slot_row[slot] where that is given (-1: none).
+int launch_group_quant_slots(const void* x, int dtype, void* q, float* scales, const RouteSource& route, const int* slot_row, int P,
+                             int E, int BT, int topk, int M, int K, int ld_scale, void* zero, size_t zero_bytes, int num_sms,
+                             cudaStream_t stream, bool pdl);
 
 // Per-token-group (1x128) FP8 quantisation, optionally gathering rows through
 // sorted_ids like launch_gather_rows.  scale_t: store scales group-major.

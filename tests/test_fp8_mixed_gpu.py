@@ -1,0 +1,64 @@
+"""FP8 blocks of 128 in one launch with blocks of at most 16 rows (moe_gemm_fp8_mixed_kernel), against blocks of 16
+alone on the same quantised inputs.
+
+Every product and every per-slice scaling is the same in both; the down projection adds an output's fp32 terms in another
+order or, with pair rows, rounds each to the 16-bit type first (2^-9 of it), so outputs agree to 4e-3 in the 2-norm."""
+import pytest
+import torch
+
+import flaggems_sglang_b200 as F
+from flaggems_sglang_b200 import _lib
+from flaggems_sglang_b200.quant import quantize_fp8_block
+from flaggems_sglang_b200.testing import make_weights
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [1, 15, 16, 17, 127, 128, 129, 0, 300, 2, 255, 257]
+
+
+def _ids(counts, m, k, seed):
+    """[m, k] expert ids with these numbers of slots (the rest is -1), no expert twice in a token where that can be."""
+    slots = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])
+    flat = torch.full((m * k,), -1)
+    flat[: slots.numel()] = slots
+    g = torch.Generator().manual_seed(seed)
+    return flat[torch.randperm(m * k, generator=g)].view(m, k).to(torch.int32)
+
+
+@pytest.mark.parametrize("h,i,counts,kw", [
+    (512, 256, EDGES, {}),
+    (512, 256, EDGES, dict(no_combine=True)),
+    (512, 384, EDGES, dict(apply_router_weight_on_input=True)),
+    (384, 256, EDGES, dict(bias=True, activation="swiglu_oai", swiglu_alpha=1.7, swiglu_limit=7.0)),
+    (512, 256, [9] * 96, {}),                       # nothing but cold blocks
+    (512, 256, [64] * 24, {}),                      # nothing but hot ones
+    (512, 256, [700] + [1] * 250, {}),
+    (2560, 256, EDGES * 3, {}),                     # the down projection stores pair rows
+    (2560, 256, EDGES * 3, dict(bias=True)),
+    (2688, 256, EDGES * 3, dict(dtype=torch.float16)),      # half of a tile's columns past the end
+])
+def test_hot_and_cold_blocks(cuda_device, h, i, counts, kw):
+    d, e, k = cuda_device, len(counts), 4
+    kw = dict(kw)
+    dtype, bias = kw.pop("dtype", torch.bfloat16), kw.pop("bias", False)
+    m = (sum(counts) + k - 1) // k + 3
+    if m * k <= 4 * e:                               # enough slots for blocks of 128
+        m = e + 1
+    ids = _ids(counts, m, k, seed=1).to(d)
+    g = torch.Generator(device=d).manual_seed(2)
+    x = torch.randn(m, h, generator=g, device=d).to(dtype)
+    tw = torch.rand(m, k, generator=g, device=d)
+    w13, w2 = make_weights(h, i, e, device=d, seed=3)
+    (w13, s13), (w2, s2) = quantize_fp8_block(w13), quantize_fp8_block(w2)
+    kw.update(use_fp8_w8a8=True, w13_scale=s13, w2_scale=s2)
+    if bias:
+        kw.update(b13=torch.randn(e, 2 * i, generator=g, device=d) * 0.1, b2=torch.randn(e, h, generator=g, device=d) * 0.1)
+    out = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    names = _lib.launch_stats()[1]
+    assert "moe_gemm_fp8_mixed_kernel<gate/up>" in names and "group_quant_slots_kernel" in names, names
+    ref = F.fused_experts(x, w13, w2, tw, ids, block_tokens=16, **kw)
+    F.check_status()
+    err = ((out.float() - ref.float()).norm() / ref.float().norm()).item()
+    assert torch.isfinite(out).all() and err <= 4e-3, err
+    rows = (out.float() - ref.float()).flatten(0, -2).norm(dim=-1) / ref.float().flatten(0, -2).norm(dim=-1).clamp_min(1e-3)
+    assert rows.max().item() <= 2e-2, rows.max().item()

@@ -52,7 +52,7 @@ def _problem(kind, h, i, e, k, m, dev, variant):
     ("bf16", 1024, 512, 128, 8, 31, "plain"), ("bf16", 1024, 512, 128, 8, 33, "skew"), ("bf16", 520, 264, 64, 4, 70, "twice"),
     ("bf16", 512, 256, 32, 4, 97, "map"), ("fp16", 512, 256, 16, 3, 85, "plain"), ("bf16", 512, 256, 8, 2, 100, "nowhere"),
     ("bf16", 256, 128, 1024, 8, 512, "plain"),
-    ("fp8", 1024, 512, 64, 8, 33, "skew"), ("fp8", 512, 256, 64, 4, 64, "twice"), ("fp8", 512, 256, 64, 4, 80, "map"),
+    ("fp8", 1024, 512, 64, 8, 32, "skew"), ("fp8", 512, 256, 64, 4, 64, "twice"), ("fp8", 512, 256, 64, 4, 61, "map"),
     ("fp8", 512, 256, 256, 12, 85, "plain"), ("fp8", 512, 256, 64, 4, 30, "nowhere"),
     ("int4", 1024, 512, 8, 2, 51, "plain"), ("int4", 640, 384, 16, 4, 33, "twice"), ("int4", 512, 256, 16, 4, 60, "map"),
     ("int4", 512, 256, 8, 2, 100, "nowhere"),
