@@ -697,7 +697,7 @@ bool gemv_eligible(const b200moe_cfg* c, const Layout& L) {
 int run_gemv(const b200moe_cfg* c, const Layout& L, const void* x, const void* w1, const void* w2,
              const b200moe_quant* quant, const float* topk_weights, const void* topk_ids,
              const int32_t* expert_map, const int32_t* hist, const int32_t* topk_indx, const float* gate_scal,
-             uint8_t* ws, void* out, cudaStream_t st, int slot) {
+             uint8_t* ws, void* out, int32_t* status, cudaStream_t st, int slot) {
   if (!gemv_eligible(c, L)) return B200MOE_ERR_UNSUPPORTED;
   const bool w4 = c->wmode == B200MOE_W_INT4_AWQ;
   if (w4 && (quant == nullptr || quant->w1_sz == nullptr || quant->w2_sz == nullptr)) return B200MOE_ERR_BAD_ARG;
@@ -737,6 +737,7 @@ int run_gemv(const b200moe_cfg* c, const Layout& L, const void* x, const void* w
   }
   g.act = ws + L.a2;   // the pairs' activations go where the grouped path keeps GEMM-1's output (cap >= P rows)
   g.out = out;
+  g.status = status;
   if (!gemv_fits(g)) return B200MOE_ERR_UNSUPPORTED;
   const bool pdl = (c->flags & B200MOE_FLAG_NO_PDL) == 0;
   prof_mark(slot, 1, st);
@@ -877,7 +878,7 @@ int b200moe_forward_topk(const b200moe_cfg* cfg, const void* x, const void* w1, 
   launch_log_new_call();
   const int slot = prof_slot();
   prof_mark(slot, 0, st);
-  rc = run_gemv(cfg, L, x, w1, w2, quant, topk_weights, topk_ids, expert_map, nullptr, nullptr, nullptr, ws, out, st,
+  rc = run_gemv(cfg, L, x, w1, w2, quant, topk_weights, topk_ids, expert_map, nullptr, nullptr, nullptr, ws, out, status, st,
                 slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
   const int is64 = (cfg->flags & B200MOE_FLAG_IDS_I64) ? 1 : 0;
@@ -921,7 +922,7 @@ int b200moe_forward_logits(const b200moe_cfg* cfg, const b200moe_router* router,
   rc = launch_route_topk(router, logits, cfg->M, cfg->E, cfg->topk, tw, ids, query_sms(cfg), st,
                          (cfg->flags & B200MOE_FLAG_NO_PDL) == 0);
   if (rc != B200MOE_OK) return rc;
-  rc = run_gemv(cfg, L, x, w1, w2, quant, tw, ids, expert_map, nullptr, nullptr, nullptr, ws, out, st, slot);
+  rc = run_gemv(cfg, L, x, w1, w2, quant, tw, ids, expert_map, nullptr, nullptr, nullptr, ws, out, status, st, slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
   if (L.own) {
     const RouteSource src = topk_source(cfg, ids, 0, expert_map, tw);
@@ -947,7 +948,7 @@ int b200moe_forward_routed(const b200moe_cfg* cfg, const void* x, const void* w1
   launch_log_new_call();
   const int slot = prof_slot();
   prof_mark(slot, 0, st);
-  rc = run_gemv(cfg, L, x, w1, w2, quant, nullptr, nullptr, nullptr, hist, topk_indx, gate_scal, ws, out, st, slot);
+  rc = run_gemv(cfg, L, x, w1, w2, quant, nullptr, nullptr, nullptr, hist, topk_indx, gate_scal, ws, out, status, st, slot);
   if (rc != B200MOE_ERR_UNSUPPORTED) return rc;
   if (L.own && cfg->wmode != B200MOE_W_FP8_BLOCK) {   // (the quantisation looks its rows up by slot)
     RouteSource src = {};

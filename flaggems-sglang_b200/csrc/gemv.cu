@@ -116,8 +116,9 @@ __device__ __forceinline__ void stage_routing(const GemvArgs& a, int* s_e, float
 // U: 256-element chunks of each row that a lane keeps in flight.  4 by default (8 halves the resident
 // CTAs and measured 10 % slower); 5 or 6 when that is the whole row, so that a row of 1280 or 1536
 // elements does not need a second, nearly empty pass.
+// U = 2 where its six CTAs an SM give every column a warp of its own in one wave and three would not (launch_gemv_up).
 template <typename T, int U>
-__global__ void __launch_bounds__(kUpThreads)
+__global__ void __launch_bounds__(kUpThreads, U == 2 ? 6 : 1)
 moe_gemv_up_kernel(const GemvArgs a) {
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   const int P = a.M * a.topk;
@@ -399,6 +400,129 @@ moe_gemv_down_kernel(const GemvArgs a) {
         out[static_cast<size_t>(t) * a.H + h + 1] = from_f32<T>(sum1 * a.routed_scaling);
       }
     }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// The same where a CTA's share of the down weights fits in shared memory (eight pairs of a 2048 x 768 layer: 14 rows of every
+// pair, 172 KB).  It comes as one bulk copy per pair, issued before the wait for the up kernel, all of it in flight at once and
+// without registers (the kernel above holds two thirds of it in flight, and a third round trip remains).  What is left is one
+// pass over shared memory, which wants many warps: 128 / 256 / 512 threads took 24.5 / 20.4 / 19.0 us for both launches.
+// From a graph, weights cold, both launches, us with the kernel above / with this one: 2048 x 768 with 4 pairs 12.4 / 12.7,
+// 6: 17.7 / 16.2, 8: 19.8 / 19.0; 1024 x 512 with 8 11.2 / 11.0; 512 x 256 with 8 14.2 / 6.8; 2048 x 384 with 16 34.2 / 21.6.
+// What bounds it now: its bytes from HBM (75 MB at 2048 x 768: 11.5 us), the routing's round trip in front of the first
+// loads, and the dependent launch between the two.
+constexpr int kShareThreads = 512;
+constexpr int kShareRows = 16;               // rows per CTA at most: one sum each in a lane's registers
+constexpr size_t kShareBytes = 190 * 1024;   // leaves the up kernel three CTAs of up to 10 KB each
+
+__host__ __device__ __forceinline__ int share_rows(int H, int ctas) { return (H + ctas - 1) / ctas; }
+__host__ __device__ __forceinline__ size_t share_bytes(int P, int rows, int I) { return static_cast<size_t>(P) * (rows + 1) * I * 2; }
+
+template <typename T>
+__global__ void __launch_bounds__(kShareThreads)
+moe_gemv_down_share_kernel(const GemvArgs a) {
+  extern __shared__ __align__(128) uint8_t gemv_smem[];
+  __shared__ __align__(8) uint64_t bar[kGemvMaxPairs];
+  __shared__ int s_e[kGemvMaxPairs];
+  __shared__ float s_gam[kGemvMaxPairs];
+  __shared__ float s_val[kGemvMaxPairs][kShareRows];
+  __shared__ volatile int abort_flag;
+  const int P = a.M * a.topk;
+  const int R = share_rows(a.H, gridDim.x);
+  const int h0 = min(a.H, static_cast<int>(blockIdx.x) * R), rows = min(R, a.H - h0);
+  T* s_w = reinterpret_cast<T*>(gemv_smem);                         // [P][rows][I]
+  T* s_act = s_w + static_cast<size_t>(P) * rows * a.I;             // [P][I]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kGemvMaxPairs) mbar_init(smem_u32(&bar[threadIdx.x]), 1);
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  // neither the routing input nor the weights depend on the up kernel
+  stage_routing(a, s_e, s_gam);
+  fence_proxy_async_smem();
+  __syncthreads();
+  const uint32_t bytes = static_cast<uint32_t>(rows) * a.I * 2;
+  if (threadIdx.x < P && s_e[threadIdx.x] >= 0 && rows > 0) {
+    const int p = threadIdx.x;
+    mbar_arrive_expect_tx(smem_u32(&bar[p]), bytes);
+    bulk_copy_g2s(smem_u32(s_w + static_cast<size_t>(p) * rows * a.I),
+                  reinterpret_cast<const T*>(a.w2) + (static_cast<size_t>(s_e[p]) * a.H + h0) * a.I, bytes, smem_u32(&bar[p]));
+  }
+  griddep_wait();
+  griddep_launch_dependents();
+  const uint4* act = reinterpret_cast<const uint4*>(a.act);
+  for (int i = threadIdx.x; i < P * a.I / 8; i += kShareThreads) reinterpret_cast<uint4*>(s_act)[i] = act[i];
+  __syncthreads();
+  // four rows of a pair at a time: their sums are independent, and one exchange adds all four over the lanes
+  bool ok = true;
+  const int groups = (rows + 3) / 4;
+  for (int u = warp; u < P * groups; u += kShareThreads / 32) {
+    const int p = u / groups, r0 = (u - p * groups) * 4;
+    if (s_e[p] < 0) continue;                  // nothing reads its sums
+    if (!mbar_wait(smem_u32(&bar[p]), 0, &abort_flag, DEV_TIMEOUT_PRODUCER)) {
+      ok = false;
+      break;
+    }
+    const T* w[4];
+    float acc[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      w[r] = s_w + (static_cast<size_t>(p) * rows + min(r0 + r, rows - 1)) * a.I;
+      acc[r] = 0.f;
+    }
+#pragma unroll 2
+    for (int k = lane * 8; k < a.I; k += kChunk) {
+      const uint4 av = *reinterpret_cast<const uint4*>(s_act + static_cast<size_t>(p) * a.I + k);
+      float x[8];
+      unpack2<T>(av.x, x[0], x[1]);
+      unpack2<T>(av.y, x[2], x[3]);
+      unpack2<T>(av.z, x[4], x[5]);
+      unpack2<T>(av.w, x[6], x[7]);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint4 wv = *reinterpret_cast<const uint4*>(w[r] + k);
+        const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float lo, hi;
+          unpack2<T>(ww[q], lo, hi);
+          acc[r] = fmaf(hi, x[2 * q + 1], fmaf(lo, x[2 * q], acc[r]));
+        }
+      }
+    }
+    // lanes 0-7 end with row 0, 8-15 with row 1, and so on
+    const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+    const float c0 = (up16 ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, up16 ? acc[0] : acc[2], 16);
+    const float c1 = (up16 ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, up16 ? acc[1] : acc[3], 16);
+    float v = (up8 ? c1 : c0) + __shfl_xor_sync(0xffffffffu, up8 ? c0 : c1, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int r = r0 + (lane >> 3);
+    if ((lane & 7) == 0 && r < rows) s_val[p][r] = v;
+  }
+  if (!ok && lane == 0) atomicCAS(a.status, 0, static_cast<int>(abort_flag));
+  __syncthreads();
+  // a thread adds a token's pairs for one row, in their order
+  const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0, no_combine = (a.flags & B200MOE_FLAG_NO_COMBINE) != 0;
+  T* out = reinterpret_cast<T*>(a.out);
+  for (int i = threadIdx.x; i < a.M * rows; i += kShareThreads) {
+    const int t = i / rows, r = i - t * rows, h = h0 + r;
+    float sum = 0.f;
+    for (int j = 0; j < a.topk; ++j) {
+      const int p = t * a.topk + j, e = s_e[p];
+      float y = 0.f;
+      if (e >= 0) {
+        y = s_val[p][r];
+        if (a.b2 != nullptr) y += __ldg(a.b2 + static_cast<size_t>(e) * a.H + h);
+        if (!w_on_input) y *= s_gam[p];
+        if (a.round_pair) y = to_f32<T>(from_f32<T>(y));
+      }
+      if (no_combine) out[static_cast<size_t>(p) * a.H + h] = from_f32<T>(y);
+      sum += y;
+    }
+    if (!no_combine) out[static_cast<size_t>(t) * a.H + h] = from_f32<T>(sum * a.routed_scaling);
   }
 }
 
@@ -796,19 +920,36 @@ size_t routing_smem() { return kGemvMaxPairs * 12 + 2 * 2 * (kDownThreads / 32) 
 // stays a multiple of the SM count, so every SM streams the same share of the weights
 template <typename K>
 unsigned grid_for(K kernel, size_t smem, int threads, long long items, int num_sms) {
-  int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
+  // the query takes longer than a launch: this thread's last answers are kept (all devices are sm_100a: one answer fits all)
+  struct Known {
+    const void* kernel;
+    size_t smem;
+    int per_sm;
+  };
+  static thread_local Known known[8] = {};
+  const void* id = reinterpret_cast<const void*>(kernel);
+  Known& k = known[(reinterpret_cast<uintptr_t>(id) >> 4) & 7];
+  if (k.kernel != id || k.smem != smem) {
+    int n = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1) n = 1;
+    k = {id, smem, n};
+  }
+  int per_sm = k.per_sm;
   const long long warps_per_cta = threads / 32;
   const long long need_per_sm = (items + warps_per_cta * num_sms - 1) / (warps_per_cta * num_sms);
   if (per_sm > need_per_sm) per_sm = static_cast<int>(need_per_sm < 1 ? 1 : need_per_sm);
   return static_cast<unsigned>(per_sm) * static_cast<unsigned>(num_sms);
 }
 
+// Does the share of the down weights fit?  (The rows are 16-byte pieces for the bulk copy: I is a multiple of 8.)
+bool share_fits(const GemvArgs& a, int num_sms) {
+  const int P = a.M * a.topk, rows = share_rows(a.H, num_sms);
+  return !a.w4 && P <= kGemvMaxPairs && rows <= kShareRows && share_bytes(P, rows, a.I) <= kShareBytes;
+}
 template <typename K>
 int launch_up(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = gemv_up_smem(a);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
   const unsigned grid = grid_for(kernel, smem, kUpThreads, static_cast<long long>(a.M) * a.topk * a.I, num_sms);
   note_launch(a.w4 ? "moe_gemv_w4_up_kernel<gate/up>" : "moe_gemv_up_kernel<gate/up>");
@@ -833,6 +974,18 @@ int launch_down(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, b
                                                                                                     : B200MOE_ERR_CUDA;
 }
 
+template <typename T>
+int launch_share(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
+  const size_t smem = share_bytes(a.M * a.topk, share_rows(a.H, num_sms), a.I);
+  if (cudaFuncSetAttribute(moe_gemv_down_share_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+      cudaSuccess)
+    return B200MOE_ERR_CUDA;
+  note_launch("moe_gemv_down_share_kernel<down>");
+  return launch_kernel(moe_gemv_down_share_kernel<T>, dim3(num_sms), dim3(kShareThreads), smem, stream, pdl, a) == cudaSuccess
+             ? B200MOE_OK
+             : B200MOE_ERR_CUDA;
+}
+
 }  // namespace
 
 size_t gemv_up_smem(const GemvArgs& a) {
@@ -849,6 +1002,13 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_up(moe_gemv_w4_up_kernel, a, num_sms, stream, pdl);
   const int chunks = (a.H + kChunk - 1) / kChunk;
+  // A warp per column in one wave: more columns than the three CTAs an SM of the kernels below seat, up to five.  Just above three the second wave is nearly empty (4096 columns of 2048: 18.5 -> 17.0 us for both launches, 5120:
+  // 17.5 -> 17.25); at 6144 both are even, and with a row that 5 chunks cover the single pass stays ahead (14.25 / 14.6 us).
+  // With four tokens' rows staged six CTAs no longer fit (19.2 / 20.5 us).
+  const long long columns = static_cast<long long>(a.M) * a.topk * a.I, seats = static_cast<long long>(num_sms) * (kUpThreads / 32);
+  if (share_fits(a, num_sms) && a.M <= 2 && chunks != 5 && columns > 3 * seats && columns <= 5 * seats)
+    return a.dtype == B200MOE_DTYPE_BF16 ? launch_up(moe_gemv_up_kernel<__nv_bfloat16, 2>, a, num_sms, stream, pdl)
+                                         : launch_up(moe_gemv_up_kernel<__half, 2>, a, num_sms, stream, pdl);
   const bool bf = a.dtype == B200MOE_DTYPE_BF16;
   if (chunks == 5)
     return bf ? launch_up(moe_gemv_up_kernel<__nv_bfloat16, 5>, a, num_sms, stream, pdl)
@@ -862,6 +1022,8 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
 int launch_gemv_down(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_down(moe_gemv_w4_down_kernel, a, num_sms, stream, pdl);
+  if (share_fits(a, num_sms))
+    return a.dtype == B200MOE_DTYPE_BF16 ? launch_share<__nv_bfloat16>(a, num_sms, stream, pdl) : launch_share<__half>(a, num_sms, stream, pdl);
   return a.dtype == B200MOE_DTYPE_BF16 ? launch_down(moe_gemv_down_kernel<__nv_bfloat16>, a, num_sms, stream, pdl)
                                        : launch_down(moe_gemv_down_kernel<__half>, a, num_sms, stream, pdl);
 }

@@ -41,6 +41,7 @@ struct GemvArgs {
   const void* w2_sz;        // int4: [E, I/128, H]
   void* act;                // scratch [P, I] in the 16-bit type
   void* out;                // [M, H], or [P, H] when nothing is combined
+  int* status;              // device status word
 };
 
 size_t gemv_up_smem(const GemvArgs& a);
