@@ -185,9 +185,11 @@ struct Layout {
   size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, a2, a2_scale, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
 };
 
+double slots_per_expert(const b200moe_cfg* c) { return static_cast<double>(c->M) * c->topk / (c->E > 0 ? c->E : 1); }
+
 int pick_bt(const b200moe_cfg* c) {
   if (c->block_tokens > 0) return c->block_tokens;
-  const double avg = static_cast<double>(c->M) * c->topk / (c->E > 0 ? c->E : 1);
+  const double avg = slots_per_expert(c);
   if (c->wmode == B200MOE_W_FP8_BLOCK) {
     // many-expert FP8 layers route unevenly: hot experts hold several times the average, and every
     // extra block of an expert streams its weights once more from L2, so lean towards larger blocks
@@ -252,10 +254,13 @@ bool route_by_gemm(const b200moe_cfg* c, const Layout& L) {
   return c->wmode != B200MOE_W_INT4_AWQ || gemm_w4_own_ok(c->E, L.P, L.BT);
 }
 
+constexpr double kPairRowsLoad = 8;
+
 int query_sms(const b200moe_cfg* c);
 bool reference_rounds_pairs(int P, int E, int n, int k, int sms);
 
-int make_layout(const b200moe_cfg* c, Layout* L) {
+// `load`: slots per expert of the real load, where the rows of c are a capacity (expert parallelism).
+int make_layout(const b200moe_cfg* c, Layout* L, double load) {
   L->BT = pick_bt(c);
   // FP8: a block of 128 tokens sits on the M side of the MMA; everything else keeps weight rows there
   L->orient = (c->wmode == B200MOE_W_FP8_BLOCK && L->BT == 128) ? 1 : 0;
@@ -306,12 +311,14 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   // pair's row to the 16-bit type (or its rounding is not asked for).
   // (16-bit without the reference's rounding: from four waves of 128 x 256 tiles on; below that the
   // split reduction, which needs the atomics, is what keeps the last wave full)
+  // FP8 below kPairRowsLoad slots per expert sums in fp32 whatever its blocks: few slots meet in a row of the combine
+  // buffer there, and a row rounded per pair would give bits away for nothing that a caller asked for.
   const bool many_tiles = (static_cast<long long>(L->P) / bt_asked) * ((c->H + 255) / 256) >=
                           (fp8 ? 2LL : 4LL) * sms_l;
   const bool pairs_ok16 = (L->pairs2 || L->w4_var) && ((c->flags & B200MOE_FLAG_MIMIC_ROUNDING)
                                             ? reference_rounds_pairs(L->P, c->E, c->H, c->I, sms_l)
                                             : many_tiles);
-  L->pair_rows = ((fp8 && L->BT == 128 && many_tiles) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
+  L->pair_rows = ((fp8 && L->BT == 128 && many_tiles && load >= kPairRowsLoad) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
                  !(c->flags & B200MOE_FLAG_SIMT);
   L->out32 = take(L->pair_rows ? 16 : static_cast<size_t>(L->out_rows > 0 ? L->out_rows : 1) * c->H * 4);
   // Quantising inside the gather repeats the work topk times; beyond a few thousand pairs it pays to
@@ -326,6 +333,7 @@ int make_layout(const b200moe_cfg* c, Layout* L) {
   L->total = off;
   return B200MOE_OK;
 }
+int make_layout(const b200moe_cfg* c, Layout* L) { return make_layout(c, L, slots_per_expert(c)); }
 
 // Would the reference round each (token, expert) row of the down projection to the 16-bit
 // type before the top-k sum?  It does exactly when its grouped matmul does not split the
@@ -1041,17 +1049,16 @@ int check_ep(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep) {
 
 // The local operator's view: every row of every source rank (masked routing entries drop what
 // is not for this rank), activations already quantised.
-b200moe_cfg ep_local_cfg(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep) {
-  b200moe_cfg c = *cfg;
+int ep_local_layout(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, b200moe_cfg* c, Layout* L) {
+  *c = *cfg;
   // token block from the real load (M_global * topk over all experts), not from the row capacity
   b200moe_cfg load = *cfg;
   load.M = ep->m_cap;
-  load.block_tokens = cfg->block_tokens;
-  c.block_tokens = pick_bt(&load);
-  c.M = ep->world * ep->m_cap;
-  c.flags |= B200MOE_FLAG_X_FP8;
-  c.n_global_experts = 0;
-  return c;
+  c->block_tokens = pick_bt(&load);
+  c->M = ep->world * ep->m_cap;
+  c->flags |= B200MOE_FLAG_X_FP8;
+  c->n_global_experts = 0;
+  return make_layout(c, L, slots_per_expert(&load));
 }
 
 }  // namespace
@@ -1063,10 +1070,9 @@ size_t b200moe_ep_heap_bytes(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep) {
 
 size_t b200moe_ep_workspace_bytes(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep) {
   if (check_ep(cfg, ep) != B200MOE_OK) return 0;
-  const b200moe_cfg c = ep_local_cfg(cfg, ep);
+  b200moe_cfg c;
   Layout L;
-  if (make_layout(&c, &L) != B200MOE_OK) return 0;
-  return L.total;
+  return ep_local_layout(cfg, ep, &c, &L) == B200MOE_OK ? L.total : 0;
 }
 
 int b200moe_ep_heap_alloc(size_t bytes, void** heap) {
@@ -1121,9 +1127,9 @@ int b200moe_ep_forward(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, void* c
   if ((phases & ~7) != 0 || phases == 0) return B200MOE_ERR_BAD_ARG;
   for (int r = 0; r < ep->world; ++r)
     if (heaps[r] == nullptr || (reinterpret_cast<uintptr_t>(heaps[r]) & 255) != 0) return B200MOE_ERR_BAD_ARG;
-  const b200moe_cfg c = ep_local_cfg(cfg, ep);
+  b200moe_cfg c;
   Layout L;
-  if ((rc = make_layout(&c, &L)) != B200MOE_OK) return rc;
+  if ((rc = ep_local_layout(cfg, ep, &c, &L)) != B200MOE_OK) return rc;
   if (workspace_bytes < L.total || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return B200MOE_ERR_WORKSPACE;
   const EpHeap H = ep_heap_layout(ep->world, ep->m_cap, cfg->H, cfg->topk, true);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
