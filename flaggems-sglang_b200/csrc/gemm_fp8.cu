@@ -224,7 +224,11 @@ __device__ __forceinline__ void weights_on_m(const CUtensorMap& tm_w, const CUte
     for (int tile = part.cta; tile < c.total; tile += c.grid_eff, ++iter) {
       const TileCoord t = part_tile(tile, part, a, kTileN);
       const int buf = iter & 1;
-      if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) break;
+      if (!mbar_wait(smem_u32(&bar_sempty[buf]), ((iter >> 1) & 1) ^ 1, abort_flag, DEV_TIMEOUT_EPILOGUE)) {
+        // the scales in flight land before the CTA leaves
+        for (int i = 1; i <= 2 && i <= iter; ++i) mbar_wait_brief(smem_u32(&bar_sfull[(iter - i) & 1]), ((iter - i) >> 1) & 1);
+        break;
+      }
       const int nkb = t.kb1 - t.kb0;
       for (int r = 0; r < BT; r += 32) {
         const int slot = rows_slot(a, rt, BT, t.e, t.row0 + r, BT < 32 ? BT : 32), cidx = r + lane;

@@ -502,7 +502,12 @@ moe_gemv_down_share_kernel(const GemvArgs a) {
     const int r = r0 + (lane >> 3);
     if ((lane & 7) == 0 && r < rows) s_val[p][r] = v;
   }
-  if (!ok && lane == 0) atomicCAS(a.status, 0, static_cast<int>(abort_flag));
+  if (!ok && lane == 0) {
+    atomicCAS(a.status, 0, static_cast<int>(abort_flag));
+    // no thread leaves before the barrier below: the copies in flight land first
+    for (int p = 0; p < P; ++p)
+      if (s_e[p] >= 0) mbar_wait_brief(smem_u32(&bar[p]), 0);
+  }
   __syncthreads();
   // a thread adds a token's pairs for one row, in their order
   const bool w_on_input = (a.flags & B200MOE_FLAG_WEIGHT_ON_INPUT) != 0, no_combine = (a.flags & B200MOE_FLAG_NO_COMBINE) != 0;
