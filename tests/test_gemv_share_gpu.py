@@ -25,6 +25,8 @@ def _rel(a, b):
     (2048, 808, 64, 8, 1, torch.float16, SHARE), (264, 136, 16, 2, 1, torch.bfloat16, SHARE),
     (1000, 520, 64, 8, 2, torch.bfloat16, SHARE), (40, 8, 64, 16, 1, torch.float16, SHARE),
     (2400, 520, 64, 4, 3, torch.bfloat16, PLAIN),
+    # the routing triple's counts, 128 experts at a time
+    (264, 136, 129, 16, 1, torch.bfloat16, SHARE), (264, 136, 300, 8, 2, torch.float16, SHARE),
     # up kernel with six CTAs an SM: 3552 < columns <= 5920 and at most two tokens
     (1024, 512, 64, 8, 1, torch.bfloat16, SHARE), (1000, 456, 64, 8, 1, torch.float16, SHARE),
     (776, 296, 64, 8, 2, torch.bfloat16, SHARE), (2048, 736, 64, 8, 1, torch.bfloat16, SHARE),
