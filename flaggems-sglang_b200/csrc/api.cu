@@ -1,6 +1,7 @@
 // C ABI: argument checks, workspace layout, tensor-map encoding and the launch sequence.
 #include <unistd.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -173,7 +174,7 @@ void launch_log_new_call() {
 
 struct Layout {
   int BT, cap, P;
-  bool quant_once; // FP8: quantise each token once, then gather the quantised rows (many pairs per token)
+  bool quant_once; // FP8 from a routing triple: quantise each token once, then gather the quantised rows (many pairs per token)
   bool pair_rows; // the down projection stores one 16-bit row per pair, the output conversion sums them
   bool pairs2;    // 16-bit GEMMs on CTA pairs: rows padded to 32 per expert, tiles of up to `tile_tokens`
   bool w4_var;    // int4 above decode sizes: rows padded to 16 per expert, tiles of up to `tile_tokens`
@@ -300,8 +301,15 @@ int make_layout(const b200moe_cfg* c, Layout* L, double load) {
   L->row_gamma = take(static_cast<size_t>(cap) * 4);
   L->xs = take(static_cast<size_t>(cap) * c->H * L->act_bytes);
   L->xs_scale = take(fp8 ? static_cast<size_t>(cap) * (c->H / 128) * 4 : 0);
-  L->a2 = take(static_cast<size_t>(cap) * c->I * L->act_bytes);
+  // Quantising inside the gather repeats the work topk times; beyond a few thousand pairs it pays to
+  // quantise the M token rows once and gather bytes.  The bytes wait where GEMM-1, which comes after the gather, writes;
+  // only their scales, a thirty-second of them, have room of their own.
+  L->quant_once = fp8 && L->P >= 2048 && c->topk > 1 && !(c->flags & B200MOE_FLAG_X_FP8);
+  const size_t tok_rows = L->quant_once ? c->M : 0;
+  L->a2 = take(std::max(static_cast<size_t>(cap) * c->I * L->act_bytes, tok_rows * c->H));
   L->a2_scale = take(fp8 ? static_cast<size_t>(cap) * (c->I / 128) * 4 : 0);
+  L->xq_tok = L->a2;
+  L->xq_scale = take(tok_rows * (c->H / 128) * 4);
   L->out_rows = (c->flags & B200MOE_FLAG_NO_COMBINE) ? L->P : c->M;   // one fp32 row per pair when nothing is summed
   // Many pairs on 128-token blocks: fp32 atomics into the combine buffer would bound the down
   // projection's tail (every add is a read-modify-write of a row another tile also touches), and
@@ -321,11 +329,6 @@ int make_layout(const b200moe_cfg* c, Layout* L, double load) {
   L->pair_rows = ((fp8 && L->BT == 128 && many_tiles && load >= kPairRowsLoad) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
                  !(c->flags & B200MOE_FLAG_SIMT);
   L->out32 = take(L->pair_rows ? 16 : static_cast<size_t>(L->out_rows > 0 ? L->out_rows : 1) * c->H * 4);
-  // Quantising inside the gather repeats the work topk times; beyond a few thousand pairs it pays to
-  // quantise the M token rows once and gather bytes.
-  L->quant_once = fp8 && L->P >= 2048 && c->topk > 1 && !(c->flags & B200MOE_FLAG_X_FP8);
-  L->xq_tok = take(L->quant_once ? static_cast<size_t>(c->M) * c->H : 0);
-  L->xq_scale = take(L->quant_once ? static_cast<size_t>(c->M) * (c->H / 128) * 4 : 0);
   L->pairs = take(L->pair_rows ? static_cast<size_t>(L->P) * c->H * 2 : 0);
   L->pair_valid = take(L->pair_rows ? align_up(static_cast<size_t>(L->P), 16) : 0);
   L->route_w = take(static_cast<size_t>(L->P > 0 ? L->P : 1) * 4);    // router output when the call starts from logits

@@ -92,6 +92,23 @@ def test_matrix_vector_path_selection(built_lib):
     assert built_lib.b200moe_uses_matrix_vector_path(C.byref(bad)) == _lib.ERR_BAD_ARG
 
 
+def test_quantised_tokens_share_the_activations_room(built_lib):
+    """FP8 calls of many pairs: the quantised token rows that a call from a routing triple gathers wait in the activations'
+    room.  Beyond a call whose rows arrive quantised, the workspace holds their scales, and bytes only where the
+    activations have fewer."""
+    from flaggems_sglang_b200 import _lib
+
+    def ws(m, h, i, e, k, flags=0):
+        cfg = _lib.Cfg(C.sizeof(_lib.Cfg), m, h, i, e, k, 0, _lib.W_FP8_BLOCK, 0, 0, flags, 0, 1.0, 148)
+        return built_lib.b200moe_workspace_bytes(C.byref(cfg))
+
+    for m, h, i, e, k in [(4096, 7168, 2048, 256, 8), (256, 7168, 2048, 256, 8), (1024, 512, 256, 8, 2), (4096, 8192, 128, 4, 2)]:
+        cap = (m * k + e * 127 + 127) // 128 * 128
+        lacking = max(0, m * h - cap * i)
+        more = ws(m, h, i, e, k) - ws(m, h, i, e, k, _lib.FLAG_X_FP8)
+        assert 0 <= more - lacking - m * (h // 128) * 4 <= 2048
+
+
 def test_product_fails_loudly_without_gpu():
     import torch
     import flaggems_sglang_b200 as F

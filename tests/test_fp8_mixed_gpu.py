@@ -9,7 +9,7 @@ import torch
 import flaggems_sglang_b200 as F
 from flaggems_sglang_b200 import _lib
 from flaggems_sglang_b200.quant import quantize_fp8_block
-from flaggems_sglang_b200.testing import make_weights
+from flaggems_sglang_b200.testing import make_tokens, make_weights
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +62,22 @@ def test_hot_and_cold_blocks(cuda_device, h, i, counts, kw):
     assert torch.isfinite(out).all() and err <= 4e-3, err
     rows = (out.float() - ref.float()).flatten(0, -2).norm(dim=-1) / ref.float().flatten(0, -2).norm(dim=-1).clamp_min(1e-3)
     assert rows.max().item() <= 2e-2, rows.max().item()
+
+
+@pytest.mark.parametrize("h,i,e,k,m", [(2048, 256, 16, 8, 640), (4096, 128, 16, 2, 1500)])
+def test_routing_triple_of_many_pairs(cuda_device, h, i, e, k, m):
+    """A call from a routing triple quantises its tokens into the activations' room (the second layer's activations have
+    fewer bytes than its tokens) and gathers them: the same rows as the call from ids, and with pair rows the same bits."""
+    d = cuda_device
+    x, tw, ids = make_tokens(m, h, e, k, device=d, seed=6, skew=True)
+    w13, w2 = make_weights(h, i, e, device=d, seed=7)
+    (w13, s13), (w2, s2) = quantize_fp8_block(w13), quantize_fp8_block(w2)
+    kw = dict(use_fp8_w8a8=True, w13_scale=s13, w2_scale=s2)
+    ref = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    assert "finalize_pairs_kernel" in _lib.launch_stats()[1]
+    order = torch.argsort(ids.flatten().long(), stable=True)
+    triple = (torch.bincount(ids.flatten().long(), minlength=e).int(), order.int(), tw.flatten()[order], k)
+    out = F.fused_experts(x, w13, w2, routing=triple, **kw)
+    assert "gather_rows_kernel" in _lib.launch_stats()[1]
+    F.check_status()
+    assert torch.equal(out, ref)
