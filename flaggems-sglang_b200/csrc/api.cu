@@ -192,12 +192,24 @@ int pick_bt(const b200moe_cfg* c) {
   if (c->block_tokens > 0) return c->block_tokens;
   const double avg = slots_per_expert(c);
   if (c->wmode == B200MOE_W_FP8_BLOCK) {
-    // many-expert FP8 layers route unevenly: hot experts hold several times the average, and every
-    // extra block of an expert streams its weights once more from L2, so lean towards larger blocks
-    // and blocks of 128 take the experts of at most 16 tokens as blocks of 16 anyway (256 experts, zipf-skewed, us,
-    // blocks of 16 or 32 / 128: average 2: 400 / 403, 3.1: 445 / 463, 4.1: 583 / 475, 5.6: 605 / 561, 7.8: 705 / 617)
+    // Blocks of 16 spare the alignment launch and the mixed launch's division of the CTAs, but an expert of more than 16 slots
+    // streams its weights once per block.  What that costs grows with the slots of the call and with an expert's weights,
+    // whatever their number, and crosses at P * H * I = 7e9 to 8e9 where the routing is zipf-skewed (flat, blocks of 16 stay
+    // ahead by 1 to 8 %).  us, blocks of 16 / 128, zipf, flat:
+    //   128 experts of 4096 x 2048: average 6 (6.4e9) 264 / 279, 509 / 544; 8 (8.6e9) 353 / 319, 526 / 551
+    //   64 of 7168 x 2048: 6 (5.6e9) 325 / 345, 451 / 473; 10 (9.4e9) 426 / 392, 474 / 495
+    //   160 of 5120 x 1536: 5 (6.3e9) 250 / 256, 603 / 630; 8 (1.0e10) 328 / 298, 611 / 646
+    //   256 of 7168 x 2048: 2 (7.5e9) 388 / 427, 1475 / 1511; 4 (1.5e10) 552 / 544, 1705 / 1697; 6 760 / 683, 1753 / 1747
+    // Below that, smaller experts turn at an average of 14 to 20, bound by their blocks' tiles:
+    //   128 of 2048 x 768: 8 96 / 109, 129 / 143; 12 106 / 112, 132 / 156; 20 135 / 131, 153 / 179
+    //   64 of 2048 x 1408: 8 96 / 113, 113 / 126; 12 112 / 123, 118 / 149; 20 137 / 133, 142 / 163
+    //   32 of 7168 x 2048: 8 227 / 266, 236 / 245; 12 251 / 278, 239 / 260; 16 283 / 278, 256 / 291
+    // Blocks of 32 were the best nowhere by more than 3 % up to 13.  Layers that fit in L2 were left alone: none is served (one of
+    // 256 experts of 512 x 256 takes 50 / 63 at 4, 56 / 81 at 12).
     if (avg <= 4) return 16;
-    return 128;
+    const double weights = static_cast<double>(c->H) * c->I;
+    const bool beyond_l2 = 3 * c->E * weights > 126e6;
+    return avg <= 13 && beyond_l2 && c->M * weights * c->topk <= 7.5e9 ? 16 : 128;
   }
   // 16-bit and int4: the smaller block until too many experts need a second one.  16 against 32 tokens per block cross at
   // an average of 13 for layers of 8, 64 and 128 experts (us, 16 / 32: 128 experts, average 12.6: 212 / 217, 15: 220 / 218;
@@ -249,9 +261,15 @@ constexpr int kOwnMaxSlots = 4096, kOwnMaxExperts = 1024;
 bool route_by_gemm(const b200moe_cfg* c, const Layout& L) {
   if (c->flags & B200MOE_FLAG_SIMT) return false;
   if (L.pairs2 || L.w4_var || L.BT > 32 || (c->flags & B200MOE_FLAG_X_FP8)) return false;
-  // FP8 beyond 1024 slots: the blocks of hot experts make tiles short beside a scan of the slots (256 experts, zipf-skewed, us
-  // aligned / sorted by the GEMMs: 8 tokens 200 / 191, 200 tokens 656 / 661)
-  if (L.P > (c->wmode == B200MOE_W_FP8_BLOCK ? 1024 : kOwnMaxSlots) || c->E > kOwnMaxExperts) return false;
+  if (L.P > kOwnMaxSlots || c->E > kOwnMaxExperts) return false;
+  // FP8: every slot's row is looked up by a scan too, and hot experts' blocks make tiles short beside theirs.  Aligned / sorted by
+  // the GEMMs, us, zipf and flat, blocks of 16: 128 experts of 2048 x 768, 512 slots 73.5 / 70.9, 126.8 / 120.4; 768:
+  // 80.8 / 81.9, 129.6 / 125.4; 1024: 90.1 / 95.9, 129.4 / 129.6; 160 of 5120 x 1536, 480: 188 / 188, 570 / 568; 960: 281 / 294,
+  // 610 / 614; 64 of 7168 x 2048, 512: 372 / 377, 446 / 452; 832: 484 / 499, 474 / 487; 128 of 4096 x 2048, 1024: 330 / 351, 522 / 520;
+  // 256 of 7168 x 2048, 512: 392 / 392, 1477 / 1473; 1024: 545 / 545, 1697 / 1690.  At four slots per expert or less nothing is lost
+  // up to 1024 (but on 256 experts of 512 x 256, zipf: 34.9 / 42.0).  Beyond, the scans cost up to the whole call again: 128 of
+  // 2048 x 768, 2048 slots: 120 / 164, 138 / 157; 4096: 183 / 363, 184 / 268; 256 of 7168 x 2048, 2304: 915 / 965, 1785 / 1761.
+  if (c->wmode == B200MOE_W_FP8_BLOCK) return L.P <= 640 || (L.P <= 1024 && slots_per_expert(c) <= 4);
   return c->wmode != B200MOE_W_INT4_AWQ || gemm_w4_own_ok(c->E, L.P, L.BT);
 }
 
@@ -1054,9 +1072,11 @@ int check_ep(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep) {
 // is not for this rank), activations already quantised.
 int ep_local_layout(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, b200moe_cfg* c, Layout* L) {
   *c = *cfg;
-  // token block from the real load (M_global * topk over all experts), not from the row capacity
+  // token block of one call over every rank's tokens and experts: the row capacity says nothing of the load, and the sums then
+  // are those of that call
   b200moe_cfg load = *cfg;
-  load.M = ep->m_cap;
+  load.M = ep->world * ep->m_cap;
+  load.E = ep->world * cfg->E;
   c->block_tokens = pick_bt(&load);
   c->M = ep->world * ep->m_cap;
   c->flags |= B200MOE_FLAG_X_FP8;

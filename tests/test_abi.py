@@ -109,6 +109,23 @@ def test_quantised_tokens_share_the_activations_room(built_lib):
         assert 0 <= more - lacking - m * (h // 128) * 4 <= 2048
 
 
+def test_fp8_token_blocks(built_lib):
+    """Blocks of 16 up to four slots per expert, or thirteen while slots times an expert's weights stay below 7.5e9 (layers
+    beyond L2); 128 above.  What a caller asks for stands."""
+    from flaggems_sglang_b200 import _lib
+
+    def block(m, h, i, e, k, asked=0):
+        cfg = _lib.Cfg(C.sizeof(_lib.Cfg), m, h, i, e, k, 0, _lib.W_FP8_BLOCK, 0, 0, 0, asked, 1.0, 148)
+        return built_lib.b200moe_pick_block_tokens(C.byref(cfg))
+
+    assert [block(m, 7168, 2048, 256, 8) for m in (1, 64, 128, 129, 200, 4096)] == [16, 16, 16, 128, 128, 128]
+    assert [block(m, 2048, 768, 128, 8) for m in (64, 65, 208, 209)] == [16, 16, 16, 128]
+    assert [block(m, 7168, 2048, 64, 8) for m in (32, 63, 64)] == [16, 16, 128]
+    assert [block(m, 4096, 7168, 8, 2) for m in (16, 52, 53)] == [16, 16, 128]
+    assert [block(m, 512, 256, 256, 8) for m in (128, 129)] == [16, 128]             # fits in L2
+    assert [block(200, 7168, 2048, 256, 8, bt) for bt in (16, 32, 64, 128)] == [16, 32, 64, 128]
+
+
 def test_product_fails_loudly_without_gpu():
     import torch
     import flaggems_sglang_b200 as F

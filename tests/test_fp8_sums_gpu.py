@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m", [176, 200, 255])      # of 256 experts, top-8: from 1408 slots on the down projection has many tiles
 @pytest.mark.parametrize("entry", ["experts", "block 128", "expert parallel"])
 def test_terms_are_added_in_fp32(cuda_device, m, entry):
-    h, i, e, k, d = 7168, 128, 256, 8, cuda_device
+    h, i, e, k, d = 7168, 2048, 256, 8, cuda_device
     w13, w2 = make_weights(h, i, 1, seed=1)
     (q13, s13), (q2, s2) = quantize_fp8_block(w13), quantize_fp8_block(w2)
     g = torch.Generator().manual_seed(2)
