@@ -140,7 +140,16 @@ __device__ __forceinline__ int block_slots(const RouteSource& r, const RowTables
   const unsigned both = static_cast<unsigned>(e) * 0x10001u;
   for (int i0 = 0; i0 < P && seen < first + rows; i0 += 256) {
     const unsigned hit = ids_equal(t, i0 + lane * 8, both);      // bit q: slot i0 + 32 q + lane
-    for (unsigned rounds = __reduce_or_sync(0xffffffffu, hit); rounds != 0; rounds &= rounds - 1) {
+    // A later block of the expert: pass over 256 slots at once.  (By rounds of 32, with the slots behind the block looked at too, a
+    // zipf-skewed call of 208 tokens on 128 experts of 2048 x 768 took 181 us against 152, of 400 tokens 266 against 207.)
+    if (seen < first) {
+      const int n = __reduce_add_sync(0xffffffffu, __popc(hit));
+      if (seen + n <= first) {
+        seen += n;
+        continue;
+      }
+    }
+    for (unsigned rounds = __reduce_or_sync(0xffffffffu, hit); rounds != 0 && seen < first + rows; rounds &= rounds - 1) {
       const int q = __ffs(rounds) - 1;
       unsigned bits = __ballot_sync(0xffffffffu, (hit >> q) & 1u);
       const int n = __popc(bits);
