@@ -254,23 +254,24 @@ int check_cfg(const b200moe_cfg* c) {
 }
 
 // Calls whose GEMMs sort the slots themselves.  Every CTA counts the slots by itself, 2 to 3 us in front of its first weights
-// against 15 to 20 for the launches of an alignment and a gather.  128 experts, top-8, us with / without them: 8 tokens 90.6 /
-// 80.2, 64: 203 / 188, 200: 209 / 199, 300: 216 / 214.5; int4, 8 experts: 8 tokens 198 / 185, 64: 248 / 230.  Beyond 4096 slots
-// the scan for a tile's slots, which grows with them, would be longer than a tile of a short reduction.
+// against 15 to 20 for the launches of an alignment and a gather; a scan over the slots per tile, and per slot where a
+// kernel moves the rows, grows with their number.  us aligned / sorted by the GEMMs, zipf-skewed and flat routing:
+//   16-bit: 128 experts of 2048 x 768, 512 slots 100 / 87, 203 / 187; 1024: 122 / 114, 206 / 192; 1664: 151 / 152, 210 / 203;
+//     2560: 167 / 174, 218 / 218; 3200: 184 / 207, 222 / 240; 64 of 1280 x 3072, 832: 227 / 226, 252 / 240; 1600: 248 / 264,
+//     258 / 258; 512 of 2048 x 512, 1024: 111 / 108, 446 / 429; 1540: 127 / 135, 486 / 466; 2560: 156 / 189, 509 / 504
+//   FP8: 128 of 2048 x 768, 512: 73 / 70, 126 / 119; 768: 81 / 79, 128 / 123; 1024: 89 / 90, 125 / 127; 1664: 109 / 118, 131 / 139;
+//     160 of 5120 x 1536, 960: 281 / 288, 611 / 606; 256 of 7168 x 2048, 1024: 545 / 551, 1700 / 1710; 2560: 970 / 1003, 1782 / 1766
+//   int4 (the promotion warps wait for their scans): 128 of 2048 x 768, 256: 54 / 51, 98 / 93; 384: 63 / 62, 104 / 104; 768:
+//     84 / 90, 113 / 117; 64 of 2048 x 1408, 320: 82 / 79, 95 / 96; 512: 95 / 96, 96 / 102; 1024: 125 / 131, 119 / 131
+// Layers of experts below 2^16 weights, which no model has, run the tables up to their largest size.
 constexpr int kOwnMaxSlots = 4096, kOwnMaxExperts = 1024;
 bool route_by_gemm(const b200moe_cfg* c, const Layout& L) {
   if (c->flags & B200MOE_FLAG_SIMT) return false;
   if (L.pairs2 || L.w4_var || L.BT > 32 || (c->flags & B200MOE_FLAG_X_FP8)) return false;
-  if (L.P > kOwnMaxSlots || c->E > kOwnMaxExperts) return false;
-  // FP8: every slot's row is looked up by a scan too, and hot experts' blocks make tiles short beside theirs.  Aligned / sorted by
-  // the GEMMs, us, zipf and flat, blocks of 16: 128 experts of 2048 x 768, 512 slots 73.5 / 70.9, 126.8 / 120.4; 768:
-  // 80.8 / 81.9, 129.6 / 125.4; 1024: 90.1 / 95.9, 129.4 / 129.6; 160 of 5120 x 1536, 480: 188 / 188, 570 / 568; 960: 281 / 294,
-  // 610 / 614; 64 of 7168 x 2048, 512: 372 / 377, 446 / 452; 832: 484 / 499, 474 / 487; 128 of 4096 x 2048, 1024: 330 / 351, 522 / 520;
-  // 256 of 7168 x 2048, 512: 392 / 392, 1477 / 1473; 1024: 545 / 545, 1697 / 1690.  At four slots per expert or less nothing is lost
-  // up to 1024 (but on 256 experts of 512 x 256, zipf: 34.9 / 42.0).  Beyond, the scans cost up to the whole call again: 128 of
-  // 2048 x 768, 2048 slots: 120 / 164, 138 / 157; 4096: 183 / 363, 184 / 268; 256 of 7168 x 2048, 2304: 915 / 965, 1785 / 1761.
-  if (c->wmode == B200MOE_W_FP8_BLOCK) return L.P <= 640 || (L.P <= 1024 && slots_per_expert(c) <= 4);
-  return c->wmode != B200MOE_W_INT4_AWQ || gemm_w4_own_ok(c->E, L.P, L.BT);
+  if (c->E > kOwnMaxExperts) return false;
+  if (c->wmode == B200MOE_W_FP8_BLOCK) return L.P <= 1024;
+  if (c->wmode == B200MOE_W_INT4_AWQ) return L.P <= 320 && gemm_w4_own_ok(c->E, L.P, L.BT);
+  return L.P <= (static_cast<long long>(c->H) * c->I < 65536 ? kOwnMaxSlots : 1664);
 }
 
 constexpr double kPairRowsLoad = 8;

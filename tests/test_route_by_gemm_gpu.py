@@ -97,3 +97,25 @@ def test_largest_number_of_slots(cuda_device):
         graph.replay()
         assert _rel(out, F.fused_experts(x2, w13, w2, tw2, ids2, block_tokens=64)) <= 1e-3
     F.check_status()
+
+
+# the last call whose GEMMs sort the slots and the first one that is aligned; half of all slots name one expert, so that its
+# blocks start behind several vectors of 256 slots
+@pytest.mark.parametrize("kind,h,i,e,k,m,most", [
+    ("bf16", 512, 256, 128, 8, 208, 208), ("bf16", 512, 256, 128, 8, 209, 208),
+    ("fp8", 512, 256, 256, 8, 128, 128), ("fp8", 512, 256, 256, 8, 129, 128),
+    ("int4", 512, 256, 64, 8, 40, 40), ("int4", 512, 256, 64, 8, 41, 40),
+])
+@pytest.mark.parametrize("variant", ["plain", "hot"])
+def test_slots_of_a_call(cuda_device, kind, h, i, e, k, m, most, variant):
+    x, w13, w2, tw, ids, kw = _problem(kind, h, i, e, k, m, cuda_device, variant)
+    if variant == "hot":
+        ids[:, :k // 2] = 3
+    if kind == "fp8":
+        kw["block_tokens"] = 16
+    out = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    assert ("align_block_kernel" in _lib.launch_stats()[1]) == (m > most)
+    kw["block_tokens"] = 64
+    aligned = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    F.check_status()
+    assert _rel(out, aligned) <= (2e-3 if kind == "int4" else 1e-3)
