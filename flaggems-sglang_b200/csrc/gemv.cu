@@ -425,8 +425,9 @@ moe_gemv_down_kernel(const GemvArgs a) {
 // pair, 172 KB).  It comes as one bulk copy per pair, issued before the wait for the up kernel, all of it in flight at once and
 // without registers (the kernel above holds two thirds of it in flight, and a third round trip remains).  What is left is one
 // pass over shared memory, which wants many warps: 128 / 256 / 512 threads took 24.5 / 20.4 / 19.0 us for both launches.
-// From a graph, weights cold, both launches, us with the kernel above / with this one: 2048 x 768 with 4 pairs 12.4 / 12.7,
-// 6: 17.7 / 16.2, 8: 19.8 / 19.0; 1024 x 512 with 8 11.2 / 11.0; 512 x 256 with 8 14.2 / 6.8; 2048 x 384 with 16 34.2 / 21.6.
+// From a graph, weights cold, both launches, us with the kernel above / with this one: 2048 x 768 with 1 pair 8.9 / 7.05,
+// 6: 17.9 / 16.4, 8: 19.9 / 19.0; 1024 x 512 with 4 8.7 / 8.0, 8: 11.3 / 11.2; 512 x 256 with 8 14.3 / 6.6; 2048 x 384 with 16
+// 34.2 / 21.6 (share_wins has the calls where the other one is ahead).
 // What bounds it now: its bytes from HBM (75 MB at 2048 x 768: 11.5 us), the routing's round trip in front of the first
 // loads, and the dependent launch between the two.
 constexpr int kShareThreads = 512;
@@ -963,10 +964,31 @@ unsigned grid_for(K kernel, size_t smem, int threads, long long items, int num_s
   return static_cast<unsigned>(per_sm) * static_cast<unsigned>(num_sms);
 }
 
+// Warps that share an output task of the down kernel.  With few output elements (short hidden size) several do, so that every
+// SM still has 16 warps' worth of loads in flight.
+int down_split(const GemvArgs& a, int num_sms) {
+  const long long tasks = static_cast<long long>(a.M) * (a.H / 2);
+  const long long all_warps = static_cast<long long>(num_sms) * (kDownThreads / 32);
+  int split = 1;
+  while (split < 8 && tasks * split * 2 <= all_warps) split *= 2;
+  return split;
+}
+
 // Does the share of the down weights fit?  (The rows are 16-byte pieces for the bulk copy: I is a multiple of 8.)
 bool share_fits(const GemvArgs& a, int num_sms) {
   const int P = a.M * a.topk, rows = share_rows(a.H, num_sms);
   return !a.w4 && P <= kGemvMaxPairs && rows <= kShareRows && share_bytes(P, rows, a.I) <= kShareBytes;
+}
+// ... and is that kernel the faster one?  The other one puts a warp's first eight 256-element slots in flight before it waits, too,
+// and multiplies them from its registers.  With six slots a warp that is all of them, and enough of them (96 KB an SM) to keep HBM
+// busy (both launches from a graph, us, this one / share): 4 pairs of 2048 x 768 12.3 / 12.75, 12 of 1024 x 512 13.1 / 14.2,
+// 3 of 768 x 2048 11.5 / 12.0, 2 of 2048 x 1408 11.9 / 12.3, 3 of 2048 x 1024 12.45 / 12.65, 4 of 2304 x 640 12.9 / 13.3.  With eight
+// slots it goes either way (5 pairs of 2304 x 640 14.2 / 15.7, 4 of 2048 x 1024 15.7 / 14.4), with five too (10 of 1024 x 512
+// 12.3 / 12.9, 3 of 2048 x 768 11.4 / 11.0); with fewer or more, and where a task has one warp, the share kernel is ahead.
+bool share_wins(const GemvArgs& a, int num_sms) {
+  const bool by_pair = (a.flags & B200MOE_FLAG_NO_COMBINE) != 0 || a.round_pair != 0;     // the other one prefetches nothing then
+  const int split = down_split(a, num_sms), slots = a.topk * ((a.I + kChunk - 1) / kChunk);
+  return by_pair || split == 1 || (slots + split - 1) / split != 6;
 }
 template <typename K>
 int launch_up(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
@@ -983,13 +1005,9 @@ int launch_down(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, b
   const size_t smem = gemv_down_smem(a);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
-  // few output elements (short hidden size): several warps share one, so that every SM still has 16
-  // warps' worth of loads in flight
   GemvArgs b = a;
   const long long tasks = static_cast<long long>(a.M) * (a.H / 2);
-  const long long all_warps = static_cast<long long>(num_sms) * (kDownThreads / 32);
-  b.down_split = 1;
-  while (b.down_split < 8 && tasks * b.down_split * 2 <= all_warps) b.down_split *= 2;
+  b.down_split = down_split(a, num_sms);
   const unsigned grid = grid_for(kernel, smem, kDownThreads, tasks * b.down_split, num_sms);
   note_launch(a.w4 ? "moe_gemv_w4_down_kernel<down>" : "moe_gemv_down_kernel<down>");
   return launch_kernel(kernel, dim3(grid), dim3(kDownThreads), smem, stream, pdl, b) == cudaSuccess ? B200MOE_OK
@@ -1044,7 +1062,7 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
 int launch_gemv_down(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_down(moe_gemv_w4_down_kernel, a, num_sms, stream, pdl);
-  if (share_fits(a, num_sms))
+  if (share_fits(a, num_sms) && share_wins(a, num_sms))
     return a.dtype == B200MOE_DTYPE_BF16 ? launch_share<__nv_bfloat16>(a, num_sms, stream, pdl) : launch_share<__half>(a, num_sms, stream, pdl);
   return a.dtype == B200MOE_DTYPE_BF16 ? launch_down(moe_gemv_down_kernel<__nv_bfloat16>, a, num_sms, stream, pdl)
                                        : launch_down(moe_gemv_down_kernel<__half>, a, num_sms, stream, pdl);
