@@ -9,7 +9,9 @@ import torch
 import flaggems_sglang_b200 as F
 from flaggems_sglang_b200 import _lib
 from flaggems_sglang_b200.quant import quantize_fp8_block
-from flaggems_sglang_b200.testing import make_tokens, make_weights
+from flaggems_sglang_b200.testing import make_tokens, make_weights, route, zipf_bias
+from oracle import moe as OM
+from parity import assert_parity
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +83,34 @@ def test_routing_triple_of_many_pairs(cuda_device, h, i, e, k, m):
     assert "gather_rows_kernel" in _lib.launch_stats()[1]
     F.check_status()
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("entry", ["ids", "int64 ids", "logits", "map", "logits and map"])
+@pytest.mark.parametrize("h,i,e,k,m", [(512, 256, 32, 4, 250), (2048, 256, 64, 8, 700)])      # fp32 sums; pair rows
+def test_hot_and_cold_blocks_against_the_oracle(cuda_device, h, i, e, k, m, entry):
+    """The same launch against the fp32 evaluation on the CPU, from every form of the routing that it takes (the router's ids
+    are replaced in place by the rows of the slots)."""
+    d = cuda_device
+    x, _, _ = make_tokens(m, h, e, k, seed=8)
+    logits = torch.randn(m, e, generator=torch.Generator().manual_seed(9)) + zipf_bias(e, 1.1, seed=10)
+    tw, ids = route(logits, k)
+    w13, w2 = make_weights(h, i, e, seed=11)
+    (w13, s13), (w2, s2) = quantize_fp8_block(w13), quantize_fp8_block(w2)
+    counts = torch.bincount(ids.flatten().long(), minlength=e)
+    assert (counts > 128).any() and ((counts > 0) & (counts <= 16)).any(), counts
+    kw = dict(use_fp8_w8a8=True, w13_scale=s13.to(d), w2_scale=s2.to(d))
+    ref_tw = tw
+    if "map" in entry:
+        emap = torch.arange(e, dtype=torch.int32)
+        emap[1::3] = -1
+        kw["expert_map"] = emap.to(d)
+        ref_tw = torch.where(emap[ids.long()] >= 0, tw, torch.zeros_like(tw))
+    if "logits" in entry:
+        out = F.fused_moe(x.to(d), w13.to(d), w2.to(d), logits.to(d), k, **kw)
+    else:
+        ids_in = ids.long() if entry == "int64 ids" else ids
+        out = F.fused_experts(x.to(d), w13.to(d), w2.to(d), tw.to(d), ids_in.to(d), **kw)
+    names = _lib.launch_stats()[1]
+    assert "moe_gemm_fp8_mixed_kernel<gate/up>" in names and ("finalize_pairs_kernel" in names) == (h == 2048), names
+    F.check_status()
+    assert_parity(out, OM.fused_experts_fp8(x, w13, w2, s13, s2, ref_tw, ids), what=f"fp8 mixed {(h, i, e, k, m)} {entry}")

@@ -9,6 +9,8 @@ import torch
 import flaggems_sglang_b200 as F
 from flaggems_sglang_b200 import _lib
 from flaggems_sglang_b200.testing import make_tokens, make_weights
+from oracle import moe as OM
+from parity import assert_parity
 
 pytestmark = pytest.mark.gpu
 SHARE, PLAIN, EARLY = "moe_gemv_down_share_kernel<down>", "moe_gemv_down_kernel<down>", "plain, all loads early"
@@ -63,3 +65,14 @@ def test_share_of_the_down_weights(cuda_device, h, i, e, k, m, dtype, kernel, va
     ref = F.fused_experts(x, w13, w2, tw, ids, block_tokens=16, **kw)
     F.check_status()
     assert torch.isfinite(out).all() and _rel(out, ref) <= 4e-3
+
+
+@pytest.mark.parametrize("h,i,e,k,m,dtype", [(2048, 768, 64, 8, 1, torch.bfloat16), (1000, 456, 64, 8, 2, torch.float16),
+                                             (264, 136, 129, 16, 1, torch.bfloat16)])
+def test_share_of_the_down_weights_against_the_oracle(cuda_device, h, i, e, k, m, dtype):
+    w13, w2 = make_weights(h, i, e, dtype=dtype, seed=5)
+    x, tw, ids = make_tokens(m, h, e, k, dtype=dtype, seed=6)
+    out = F.fused_experts(*(t.to(cuda_device) for t in (x, w13, w2, tw, ids)))
+    assert SHARE in _lib.launch_stats()[1]
+    F.check_status()
+    assert_parity(out, OM.fused_experts(x, w13, w2, tw, ids), what=f"share kernel {(h, i, e, k, m)}")

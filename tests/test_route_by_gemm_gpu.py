@@ -11,6 +11,8 @@ import flaggems_sglang_b200 as F
 from flaggems_sglang_b200 import _lib
 from flaggems_sglang_b200.quant import quantize_awq, quantize_fp8_block, repack_awq_for_kernel
 from flaggems_sglang_b200.testing import make_tokens, make_weights
+from oracle import moe as OM
+from parity import assert_parity
 
 pytestmark = pytest.mark.gpu
 
@@ -119,3 +121,8 @@ def test_slots_of_a_call(cuda_device, kind, h, i, e, k, m, most, variant):
     aligned = F.fused_experts(x, w13, w2, tw, ids, **kw)
     F.check_status()
     assert _rel(out, aligned) <= (2e-3 if kind == "int4" else 1e-3)
+    if m == most and kind != "int4":                 # (int4 decode: tests/test_int4_gpu.py)
+        c = [t.cpu() for t in (x, w13, w2, tw, ids)]
+        ref = OM.fused_experts(*c) if kind == "bf16" else \
+            OM.fused_experts_fp8(*c[:3], kw["w13_scale"].cpu(), kw["w2_scale"].cpu(), *c[3:])
+        assert_parity(out, ref, what=f"sorted by the GEMMs {kind} {variant}")
