@@ -93,13 +93,15 @@ __device__ __forceinline__ GroupSmem group_smem(int* smem, int nwarps, int E) {
   g.scan = g.mine + E;
   return g;
 }
-size_t group_smem_bytes(int nwarps, int E) { return (static_cast<size_t>(nwarps) * E + 4 * static_cast<size_t>(E) + 1 + 40) * sizeof(int); }
+size_t group_smem_bytes(int nwarps, int E) {
+  return (static_cast<size_t>(nwarps) * E + 4 * static_cast<size_t>(E) + 1 + 40) * sizeof(int);
+}
 
 // Core: stable grouping of P slots by expert.  `ids` are expert ids (mapped to local experts when
 // map != nullptr); slots with an id outside [0, E) are dropped.  Each expert's group starts at a
 // multiple of `block`.  place(slot, pos, pre[slot]) records a placement; `pre` (optional, [P]) is a
-// per-slot value fetched alongside the ids; dropped[slot] (optional) becomes -1 for a dropped slot.  Called by every thread of every CTA; the caller ends with
-// cluster_wait() (the CTAs' counts are read by their peers).
+// per-slot value fetched alongside the ids; dropped[slot] (optional) becomes -1 for a dropped slot.  Called by every
+// thread of every CTA; the caller ends with cluster_wait() (the CTAs' counts are read by their peers).
 template <typename Place>
 __device__ __forceinline__ void group_by_expert(const void* ids, int is64, const int* map, int map_len, int P, int E,
                                                 int block, const GroupSmem& g, int nwarps, const float* pre, Place place,

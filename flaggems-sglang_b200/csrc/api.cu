@@ -183,7 +183,8 @@ struct Layout {
   int out_rows;   // rows of the fp32 output buffer: tokens, or pairs when nothing is combined
   int orient;     // GEMM tile orientation that goes with BT
   int act_bytes;  // bytes per activation element fed to the GEMMs
-  size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, a2, a2_scale, out32, pairs, pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
+  size_t meta, blk_off, sorted_ids, expert_ids, num_post, row_gamma, xs, xs_scale, a2, a2_scale, out32, pairs,
+      pair_valid, xq_tok, xq_scale, route_w, route_ids, total;
 };
 
 double slots_per_expert(const b200moe_cfg* c) { return static_cast<double>(c->M) * c->topk / (c->E > 0 ? c->E : 1); }
@@ -195,17 +196,17 @@ int pick_bt(const b200moe_cfg* c) {
     // Blocks of 16 spare the alignment launch and the mixed launch's division of the CTAs, but an expert of more than 16 slots
     // streams its weights once per block.  What that costs grows with the slots of the call and with an expert's weights,
     // whatever their number, and crosses at P * H * I = 7e9 to 8e9 where the routing is zipf-skewed (flat, blocks of 16 stay
-    // ahead by 1 to 8 %).  us, blocks of 16 / 128, zipf, flat:
-    //   128 experts of 4096 x 2048: average 6 (6.4e9) 264 / 279, 509 / 544; 8 (8.6e9) 353 / 319, 526 / 551
-    //   64 of 7168 x 2048: 6 (5.6e9) 325 / 345, 451 / 473; 10 (9.4e9) 426 / 392, 474 / 495
-    //   160 of 5120 x 1536: 5 (6.3e9) 250 / 256, 603 / 630; 8 (1.0e10) 328 / 298, 611 / 646
-    //   256 of 7168 x 2048: 2 (7.5e9) 388 / 427, 1475 / 1511; 4 (1.5e10) 552 / 544, 1705 / 1697; 6 760 / 683, 1753 / 1747
+    // ahead, or within 1.5 % with 256 experts).  us, blocks of 16 / 128, zipf, flat:
+    //   128 experts of 4096 x 2048: average 6 (6.4e9) 265 / 274, 509 / 537; 8 (8.6e9) 327 / 321, 520 / 549
+    //   64 of 7168 x 2048: 6 (5.6e9) 324 / 339, 446 / 469; 10 (9.4e9) 413 / 382, 477 / 491
+    //   160 of 5120 x 1536: 5 (6.3e9) 245 / 257, 601 / 627; 8 (1.0e10) 325 / 295, 609 / 646
+    //   256 of 7168 x 2048: 2 (7.5e9) 392 / 412, 1480 / 1496; 4 (1.5e10) 537 / 529, 1703 / 1678; 6 707 / 637, 1744 / 1724
     // Below that, smaller experts turn at an average of 14 to 20, bound by their blocks' tiles:
-    //   128 of 2048 x 768: 8 96 / 109, 129 / 143; 12 106 / 112, 132 / 156; 20 135 / 131, 153 / 179
-    //   64 of 2048 x 1408: 8 96 / 113, 113 / 126; 12 112 / 123, 118 / 149; 20 137 / 133, 142 / 163
-    //   32 of 7168 x 2048: 8 227 / 266, 236 / 245; 12 251 / 278, 239 / 260; 16 283 / 278, 256 / 291
-    // Blocks of 32 were the best nowhere by more than 3 % up to 13.  Layers that fit in L2 were left alone: none is served (one of
-    // 256 experts of 512 x 256 takes 50 / 63 at 4, 56 / 81 at 12).
+    //   128 of 2048 x 768: 8 91 / 111, 129 / 140; 12 105 / 115, 131 / 155; 20 135 / 130, 151 / 179
+    //   64 of 2048 x 1408: 8 93 / 112, 114 / 129; 12 109 / 122, 117 / 146; 20 137 / 133, 142 / 165
+    //   32 of 7168 x 2048: 8 228 / 260, 234 / 243; 12 245 / 271, 237 / 253; 16 283 / 271, 252 / 283
+    // Blocks of 32 were the best nowhere by more than 3 % up to 13.  Layers that fit in L2 were left alone: none is
+    // served (one of 256 experts of 512 x 256 takes 37 / 49, 49 / 62 at 4 and 47 / 53, 55 / 80 at 12).
     if (avg <= 4) return 16;
     const double weights = static_cast<double>(c->H) * c->I;
     const bool beyond_l2 = 3 * c->E * weights > 126e6;
@@ -260,7 +261,8 @@ int check_cfg(const b200moe_cfg* c) {
 //     2560: 167 / 174, 218 / 218; 3200: 184 / 207, 222 / 240; 64 of 1280 x 3072, 832: 227 / 226, 252 / 240; 1600: 248 / 264,
 //     258 / 258; 512 of 2048 x 512, 1024: 111 / 108, 446 / 429; 1540: 127 / 135, 486 / 466; 2560: 156 / 189, 509 / 504
 //   FP8: 128 of 2048 x 768, 512: 73 / 70, 126 / 119; 768: 81 / 79, 128 / 123; 1024: 89 / 90, 125 / 127; 1664: 109 / 118, 131 / 139;
-//     160 of 5120 x 1536, 960: 281 / 288, 611 / 606; 256 of 7168 x 2048, 1024: 545 / 551, 1700 / 1710; 2560: 970 / 1003, 1782 / 1766
+//     160 of 5120 x 1536, 960: 281 / 288, 611 / 606; 256 of 7168 x 2048, 1024: 545 / 551, 1700 / 1710; 2560: 970 / 1003,
+//     1782 / 1766
 //   int4 (the promotion warps wait for their scans): 128 of 2048 x 768, 256: 54 / 51, 98 / 93; 384: 63 / 62, 104 / 104; 768:
 //     84 / 90, 113 / 117; 64 of 2048 x 1408, 320: 82 / 79, 95 / 96; 512: 95 / 96, 96 / 102; 1024: 125 / 131, 119 / 131
 // Layers of experts below 2^16 weights, which no model has, run the tables up to their largest size.
@@ -345,8 +347,8 @@ int make_layout(const b200moe_cfg* c, Layout* L, double load) {
   const bool pairs_ok16 = (L->pairs2 || L->w4_var) && ((c->flags & B200MOE_FLAG_MIMIC_ROUNDING)
                                             ? reference_rounds_pairs(L->P, c->E, c->H, c->I, sms_l)
                                             : many_tiles);
-  L->pair_rows = ((fp8 && L->BT == 128 && many_tiles && load >= kPairRowsLoad) || pairs_ok16) && !(c->flags & B200MOE_FLAG_NO_COMBINE) &&
-                 !(c->flags & B200MOE_FLAG_SIMT);
+  L->pair_rows = ((fp8 && L->BT == 128 && many_tiles && load >= kPairRowsLoad) || pairs_ok16) &&
+                 !(c->flags & (B200MOE_FLAG_NO_COMBINE | B200MOE_FLAG_SIMT));
   L->out32 = take(L->pair_rows ? 16 : static_cast<size_t>(L->out_rows > 0 ? L->out_rows : 1) * c->H * 4);
   L->pairs = take(L->pair_rows ? static_cast<size_t>(L->P) * c->H * 2 : 0);
   L->pair_valid = take(L->pair_rows ? align_up(static_cast<size_t>(L->P), 16) : 0);
@@ -1217,7 +1219,8 @@ int b200moe_ep_forward(const b200moe_cfg* cfg, const b200moe_ep_cfg* ep, void* c
       po.pairs[r] = h + H.pairs;
       po.pair_valid[r] = h + H.pair_valid;
     }
-    if ((rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, nullptr, nullptr, &po)) != B200MOE_OK) return rc;
+    rc = run_experts(&c, L, me + H.recv_x, w1, w2, &q, ws, nullptr, status, st, slot, nullptr, nullptr, &po);
+    if (rc != B200MOE_OK) return rc;
     uint8_t* hp[kMaxPeers];
     for (int r = 0; r < ep->world; ++r) hp[r] = reinterpret_cast<uint8_t*>(heaps[r]);
     if ((rc = launch_ep_signal(hp, H, kEpFlagDone, ep->world, ep->rank, st, pdl)) != B200MOE_OK) return rc;

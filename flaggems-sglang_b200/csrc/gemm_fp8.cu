@@ -17,8 +17,8 @@
 //           red.global.add.f32 into the combine buffer (K may be split across CTAs).
 // Blocks of 128 tokens run in a launch of their own kind (moe_gemm_fp8_mixed_kernel, below).
 //
-// Warps: TMA producer, MMA issuer (owns tensor memory), four promotion warps per group of up
-// to 64 tokens (one group for blocks of 16/32/64, two for blocks of 128), and a
+// Warps of these kernels: TMA producer, MMA issuer (owns tensor memory), four promotion warps per group of up
+// to 32 tokens (one group for blocks of 16 and 32, two for blocks of 64), and a
 // loader warp that prepares the next tile's per-token tables (output row, routing weight,
 // activation scales by bulk copy, weight scales) in double-buffered shared memory, so that no
 // global-memory latency sits between two tiles of the promotion warps.
@@ -71,7 +71,8 @@ __device__ __forceinline__ void weights_on_m(const CUtensorMap& tm_w, const CUte
   int* s_col_row = reinterpret_cast<int*>(tmem_slot + 4);               // [2][128]
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * 128);     // [2][128]
   float* s_red = s_col_gam + 2 * 128;                                   // [2][NG][4][64]
-  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + 2 * 2 * 4 * 64);   // [2][128] mode 1: base of each token's output row
+  // [2][128] mode 1: base of each token's output row
+  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + 2 * 2 * 4 * 64);
   const RowTables rt = row_tables(s_col_ptr + 2 * 128, a.E);            // own tables, or only the blocks' starts
   int* s_blk_off = rt.blk;                                              // [E+1]
   constexpr int CPT = BT / NG;                                          // token columns per promotion thread
@@ -396,15 +397,15 @@ __device__ __forceinline__ void weights_on_m(const CUtensorMap& tm_w, const CUte
           }
         } else {
 #pragma unroll
-        for (int i = 0; i < CPT; ++i) {
-          const int orow = col_row[i];
-          if (orow >= 0) {
-            const float gam = w_on_input ? 1.0f : col_gam[i];
-            float* out = reinterpret_cast<float*>(col_ptr[i]) + n;   // the token's row, here or on its owner
-            atomicAdd(out, (acc0[i] + b0) * gam);
-            if (second) atomicAdd(out + kTileRows, (acc1[i] + b1) * gam);
+          for (int i = 0; i < CPT; ++i) {
+            const int orow = col_row[i];
+            if (orow >= 0) {
+              const float gam = w_on_input ? 1.0f : col_gam[i];
+              float* out = reinterpret_cast<float*>(col_ptr[i]) + n;   // the token's row, here or on its owner
+              atomicAdd(out, (acc0[i] + b0) * gam);
+              if (second) atomicAdd(out + kTileRows, (acc1[i] + b1) * gam);
+            }
           }
-        }
         }
       }
       // the tables of this tile may now be overwritten
@@ -504,7 +505,8 @@ __device__ __forceinline__ void tokens_on_m(const CUtensorMap& tm_w, const CUten
   int* s_col_row = s_tile + 16;               // [2][128] output row of each token
   float* s_col_gam = reinterpret_cast<float*>(s_col_row + 2 * 128);     // [2][128]
   float* s_red = s_col_gam + 2 * 128;                                   // mode 0: [2][2][128] partial group maxima
-  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + (MODE == 0 ? 2 * 2 * 128 : 0));   // [2][128] mode 1: base of each row's output row
+  // [2][128] mode 1: base of each row's output row
+  unsigned long long* s_col_ptr = reinterpret_cast<unsigned long long*>(s_red + (MODE == 0 ? 2 * 2 * 128 : 0));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -881,12 +883,17 @@ __device__ __forceinline__ void tokens_on_m(const CUtensorMap& tm_w, const CUten
 // HBM, a hot one's is the promotion; one kind after the other, as the experts come, leaves either idle.  So some CTAs
 // take the hot blocks (tokens on M) and the rest the cold ones (weights on M, 16 tokens on N, which also spares the
 // MMAs of 112 padding rows), in proportion to what they cost.  The rows lie in the same blocks of 128 for both.
-// us per call, all blocks with tokens on M / mixed, one board: 130 tokens 583 (blocks of 32) / 475, 300: 745 / 647, 1024: 1265 /
-// 1070, 2048: - / 1650, 4096: 3010 / 2750.
+// us per call in a train, all blocks with tokens on M / mixed, in turn on one board: 130 tokens 556 / 501, 200: 676 / 588,
+// 300: 810 / 676, 1024: 1398 / 1202, 2048: 1966 / 1752, 4096: 3010 / 2795.
 constexpr int kColdRows = 16;
 // Cycles of a 128-wide reduction slice and of a tile's tail, from the CTAs' times at 4096 tokens: hot tiles 65800 (gate/up, 56
-// slices) and 18000 cycles (down, 16), 40000 and 13500 with a quarter of the promotion, cold ones 31800 and 11800.  The
-// cold slices of mode 0 count for more than the 525 measured: 4096 tokens 2800 us with that, 2750 with 600, 2766 with 680.
+// slices) and 18000 cycles (down, 16), 40000 and 13500 with a quarter of the promotion, cold ones 31800 and 11800.
+// A constant for the cold slice is the model's weak point: it is the time of the slice's weights on their way from HBM, 525
+// cycles here, where the launch draws 3 TB/s, and 950 at 200 to 300 tokens, where it draws all there is and both kinds of
+// CTAs wait for it.  Gate/up takes 600 for it (4096 tokens: 2800 us with 525, 2750 with 600, 2766 with 680).  When
+// the last hot and the last cold CTA finish, us, gate/up and down, 256 experts of 7168 x 2048, zipf: 300 tokens 343 / 395
+// and 213 / 200 (at HBM's rate, however they are divided), 1024: 589 / 612 and 363 / 343, 2048: 932 / 915 and 553 / 522,
+// 4096: 1592 / 1576 and 950 / 877.
 template <int MODE>
 struct MixedCost {
   static constexpr float kHotSlice = MODE == 0 ? 970.f : 800.f, kHotTail = MODE == 0 ? 11400.f : 5300.f;
@@ -956,7 +963,8 @@ moe_gemm_fp8_mixed_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   const int units = a.num_nt * split;
   const float slices = static_cast<float>(a.kblocks) / split;
   using Cost = MixedCost<MODE>;
-  const float hot_cost = hot * (slices * Cost::kHotSlice + Cost::kHotTail), cold_cost = cold * (slices * Cost::kColdSlice + Cost::kColdTail);
+  const float hot_cost = hot * (slices * Cost::kHotSlice + Cost::kHotTail);
+  const float cold_cost = cold * (slices * Cost::kColdSlice + Cost::kColdTail);
   int cold_ctas = 0;
   if (cold > 0) {
     cold_ctas = static_cast<int>(grid * cold_cost / (hot_cost + cold_cost) + 0.5f);

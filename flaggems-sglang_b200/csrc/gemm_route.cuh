@@ -175,7 +175,8 @@ __device__ __forceinline__ float rows_weight(const GemmArgs& a, const RowTables&
   const int lane = threadIdx.x & 31;
   if (slot < 0) return 0.f;
   if (!a.route.own) return a.row_gamma[row0 + lane];
-  return a.route.hist != nullptr ? __ldcg(a.route.gate_scal + t.raw[e] + row0 - t.blk[e] * BT + lane) : __ldcg(a.route.weights + slot);
+  if (a.route.hist == nullptr) return __ldcg(a.route.weights + slot);
+  return __ldcg(a.route.gate_scal + t.raw[e] + row0 - t.blk[e] * BT + lane);
 }
 // A warp: number of slots before `slot` that name the same expert e.
 __device__ __forceinline__ int slot_rank(const RowTables& t, int slot, unsigned e) {
@@ -183,7 +184,10 @@ __device__ __forceinline__ int slot_rank(const RowTables& t, int slot, unsigned 
   const unsigned both = e * 0x10001u;
   int n = 0;
 #pragma unroll 1
-  for (int i0 = 0; i0 < slot; i0 += 256) n += __popc(ids_equal(t, i0 + lane * 8, both) & ((1u << ((max(0, min(256, slot - i0 - lane)) + 31) >> 5)) - 1));
+  for (int i0 = 0; i0 < slot; i0 += 256) {
+    const int rounds = (max(0, min(256, slot - i0 - lane)) + 31) >> 5;      // of this lane's slots i0 + 32 q + lane
+    n += __popc(ids_equal(t, i0 + lane * 8, both) & ((1u << rounds) - 1));
+  }
   return __reduce_add_sync(0xffffffffu, n);
 }
 
@@ -215,7 +219,8 @@ struct RowCopier {
     for (int i = 0; i < BT / 4; ++i) {
       const int row = 4 * i + (lane >> 3);
       const uint32_t d = tile + static_cast<uint32_t>(row * 128 + (((lane & 7) ^ (row & 7)) << 4));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src[i] + at : src[i]), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src[i] + at : src[i]), "r"(bytes)
+                   : "memory");
     }
   }
   __device__ __forceinline__ void hand_over(uint32_t bar) const {
@@ -249,7 +254,8 @@ struct RowCopier {
 // The combine buffer is cleared by the kernel before the one that adds to it: `threads` threads of each CTA.
 __device__ __forceinline__ void clear_combine_buffer(const GemmArgs& a, int tid, int threads) {
   uint4* z = reinterpret_cast<uint4*>(a.zero);
-  for (long long i = static_cast<long long>(blockIdx.x) * threads + tid; i < a.zero_chunks; i += static_cast<long long>(gridDim.x) * threads)
+  const long long step = static_cast<long long>(gridDim.x) * threads;
+  for (long long i = static_cast<long long>(blockIdx.x) * threads + tid; i < a.zero_chunks; i += step)
     z[i] = make_uint4(0, 0, 0, 0);
 }
 

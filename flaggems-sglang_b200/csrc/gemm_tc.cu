@@ -247,7 +247,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
               ok = false;
               break;
             }
-            rc.copy(smem_u32(smem + static_cast<size_t>(stage) * stage_bytes) + W_BYTES, static_cast<size_t>(kb) * kStageKBytes, row_bytes);
+            rc.copy(smem_u32(smem + static_cast<size_t>(stage) * stage_bytes) + W_BYTES, static_cast<size_t>(kb) * kStageKBytes,
+                    row_bytes);
             rc.commit(smem_u32(&bar_full[stage]));
             if (++stage == stages) {
               stage = 0;

@@ -435,7 +435,9 @@ constexpr int kShareRows = 16;               // rows per CTA at most: one sum ea
 constexpr size_t kShareBytes = 190 * 1024;   // leaves the up kernel three CTAs of up to 10 KB each
 
 __host__ __device__ __forceinline__ int share_rows(int H, int ctas) { return (H + ctas - 1) / ctas; }
-__host__ __device__ __forceinline__ size_t share_bytes(int P, int rows, int I) { return static_cast<size_t>(P) * (rows + 1) * I * 2; }
+__host__ __device__ __forceinline__ size_t share_bytes(int P, int rows, int I) {
+  return static_cast<size_t>(P) * (rows + 1) * I * 2;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kShareThreads)
@@ -982,9 +984,10 @@ bool share_fits(const GemvArgs& a, int num_sms) {
 // ... and is that kernel the faster one?  The other one puts a warp's first eight 256-element slots in flight before it waits, too,
 // and multiplies them from its registers.  With six slots a warp that is all of them, and enough of them (96 KB an SM) to keep HBM
 // busy (both launches from a graph, us, this one / share): 4 pairs of 2048 x 768 12.3 / 12.75, 12 of 1024 x 512 13.1 / 14.2,
-// 3 of 768 x 2048 11.5 / 12.0, 2 of 2048 x 1408 11.9 / 12.3, 3 of 2048 x 1024 12.45 / 12.65, 4 of 2304 x 640 12.9 / 13.3.  With eight
-// slots it goes either way (5 pairs of 2304 x 640 14.2 / 15.7, 4 of 2048 x 1024 15.7 / 14.4), with five too (10 of 1024 x 512
-// 12.3 / 12.9, 3 of 2048 x 768 11.4 / 11.0); with fewer or more, and where a task has one warp, the share kernel is ahead.
+// 3 of 768 x 2048 11.5 / 12.0, 2 of 2048 x 1408 11.9 / 12.3, 3 of 2048 x 1024 12.45 / 12.65, 4 of 2304 x 640 12.9 / 13.3.
+// With eight slots it goes either way (5 pairs of 2304 x 640 14.2 / 15.7, 4 of 2048 x 1024 15.7 / 14.4), with five too (10
+// of 1024 x 512 12.3 / 12.9, 3 of 2048 x 768 11.4 / 11.0); with fewer or more, and where a task has one warp, the share
+// kernel is ahead.
 bool share_wins(const GemvArgs& a, int num_sms) {
   const bool by_pair = (a.flags & B200MOE_FLAG_NO_COMBINE) != 0 || a.round_pair != 0;     // the other one prefetches nothing then
   const int split = down_split(a, num_sms), slots = a.topk * ((a.I + kChunk - 1) / kChunk);
@@ -993,7 +996,8 @@ bool share_wins(const GemvArgs& a, int num_sms) {
 template <typename K>
 int launch_up(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = gemv_up_smem(a);
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(smem)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
   const unsigned grid = grid_for(kernel, smem, kUpThreads, static_cast<long long>(a.M) * a.topk * a.I, num_sms);
   note_launch(a.w4 ? "moe_gemv_w4_up_kernel<gate/up>" : "moe_gemv_up_kernel<gate/up>");
@@ -1042,7 +1046,8 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_up(moe_gemv_w4_up_kernel, a, num_sms, stream, pdl);
   const int chunks = (a.H + kChunk - 1) / kChunk;
-  // A warp per column in one wave: more columns than the three CTAs an SM of the kernels below seat, up to five.  Just above three the second wave is nearly empty (4096 columns of 2048: 18.5 -> 17.0 us for both launches, 5120:
+  // A warp per column in one wave: more columns than the three CTAs an SM of the kernels below seat, up to five.  Just
+  // above three the second wave is nearly empty (4096 columns of 2048: 18.5 -> 17.0 us for both launches, 5120:
   // 17.5 -> 17.25); at 6144 both are even, and with a row that 5 chunks cover the single pass stays ahead (14.25 / 14.6 us).
   // With four tokens' rows staged six CTAs no longer fit (19.2 / 20.5 us).
   const long long columns = static_cast<long long>(a.M) * a.topk * a.I, seats = static_cast<long long>(num_sms) * (kUpThreads / 32);
@@ -1063,7 +1068,8 @@ int launch_gemv_down(const GemvArgs& a, int num_sms, cudaStream_t stream, bool p
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_down(moe_gemv_w4_down_kernel, a, num_sms, stream, pdl);
   if (share_fits(a, num_sms) && share_wins(a, num_sms))
-    return a.dtype == B200MOE_DTYPE_BF16 ? launch_share<__nv_bfloat16>(a, num_sms, stream, pdl) : launch_share<__half>(a, num_sms, stream, pdl);
+    return a.dtype == B200MOE_DTYPE_BF16 ? launch_share<__nv_bfloat16>(a, num_sms, stream, pdl)
+                                         : launch_share<__half>(a, num_sms, stream, pdl);
   return a.dtype == B200MOE_DTYPE_BF16 ? launch_down(moe_gemv_down_kernel<__nv_bfloat16>, a, num_sms, stream, pdl)
                                        : launch_down(moe_gemv_down_kernel<__half>, a, num_sms, stream, pdl);
 }

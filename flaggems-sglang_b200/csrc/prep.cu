@@ -210,15 +210,15 @@ group_quant_fp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* 
 
 // The quantisation by token: a warp quantises a run of groups once and stores it for each of the token's slots, in the row that
 // the alignment gave it (slot_row) or, where the GEMMs sort the slots themselves (gemm_route.cuh), in the one they
-// look for.  (Quantising the tokens and gathering the bytes: 4096 tokens of 56 groups, top-8, 38 + 67 us.)  At decode the kernel is a few
-// microseconds long, so its loops stay rolled: straight-line code for eight groups and eight slots spent more time being
+// look for.  (Quantising the tokens and gathering the bytes: 4096 tokens of 56 groups, top-8, 38 + 67 us.)  At decode the
+// kernel is a few microseconds long, so its loops stay rolled: straight-line code for eight groups and eight slots spent more time being
 // fetched than executed (64 tokens of 56 groups, top-8: 18.5 us; an alignment and one warp per slot: 20).
 constexpr int kQuantRun = 8;      // groups of a run at most; few tokens are dealt out in shorter ones
 template <typename T>
 __global__ void __launch_bounds__(256)
 group_quant_slots_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, const RouteSource route,
-                          const int* __restrict__ slot_row, int P, int E, int BT, int topk, int M, int K, int run, int ld_scale, uint4* __restrict__ zero,
-                          long long zero_chunks) {
+                         const int* __restrict__ slot_row, int P, int E, int BT, int topk, int M, int K, int run, int ld_scale,
+                         uint4* __restrict__ zero, long long zero_chunks) {
   extern __shared__ __align__(16) uint8_t route_smem[];
   __shared__ __align__(16) uint2 s_x[8][kQuantRun][32];
   const RowTables t = row_tables(route_smem, E);
@@ -430,12 +430,12 @@ int launch_group_quant_slots(const void* x, int dtype, void* q, float* scales, c
   cudaError_t err;
   if (dtype == B200MOE_DTYPE_BF16)
     err = launch_kernel(group_quant_slots_kernel<__nv_bfloat16>, dim3(ctas), dim3(256), smem, stream, pdl,
-                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E, BT, topk, M, K,
-                        run, ld_scale, reinterpret_cast<uint4*>(zero), zc);
+                        reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E,
+                        BT, topk, M, K, run, ld_scale, reinterpret_cast<uint4*>(zero), zc);
   else
-    err = launch_kernel(group_quant_slots_kernel<__half>, dim3(ctas), dim3(256), smem, stream, pdl, reinterpret_cast<const __half*>(x),
-                        reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E, BT, topk, M, K, run, ld_scale,
-                        reinterpret_cast<uint4*>(zero), zc);
+    err = launch_kernel(group_quant_slots_kernel<__half>, dim3(ctas), dim3(256), smem, stream, pdl,
+                        reinterpret_cast<const __half*>(x), reinterpret_cast<uint8_t*>(q), scales, route, slot_row, P, E, BT,
+                        topk, M, K, run, ld_scale, reinterpret_cast<uint4*>(zero), zc);
   return err == cudaSuccess ? B200MOE_OK : B200MOE_ERR_CUDA;
 }
 
