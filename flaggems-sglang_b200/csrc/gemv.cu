@@ -74,16 +74,51 @@ __device__ __forceinline__ void load4_f32(const T* p, float (&v)[4]) {
   unpack2<T>(raw.y, v[2], v[3]);
 }
 
+// A warp: the lane of an expert places its run of sorted rows; 128 experts' counts are fetched at a time.  (Each thread walking
+// the counts by itself, both launches of one token from a graph: 128 experts of 2048 x 768 34.7 us against 23.1, 256 of
+// 512 x 256 36.3 against 13.1.)
+__device__ __forceinline__ void place_sorted_rows(const int* hist, const int* topk_indx, const float* gate_scal, int P, int E,
+                                                  int* s_e, float* s_gam) {
+  const int lane = threadIdx.x & 31;
+  int run = 0;
+  for (int e0 = lane; e0 - lane < E; e0 += 128) {
+    int n[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) n[u] = e0 + 32 * u < E ? max(0, min(P, __ldcg(hist + e0 + 32 * u))) : 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (e0 - lane + 32 * u >= E) break;
+      int end = n[u];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += v;
+      }
+      for (int q = run + end - n[u]; q < min(P, run + end); ++q) {
+        const int slot = __ldcg(topk_indx + q);
+        if (slot >= 0 && slot < P) {
+          s_e[slot] = e0 + 32 * u;
+          s_gam[slot] = __ldcg(gate_scal + q);
+        }
+      }
+      __syncwarp();
+      run += __shfl_sync(0xffffffffu, end, 31);
+    }
+  }
+}
+
 // Local expert and routing weight of every pair, into shared memory (P <= kGemvMaxPairs).  From
 // topk_ids / topk_weights (with an optional global -> local map), or from the routing triple
 // hist[E] / topk_indx[P] / gate_scal[P] (sorted row -> pair slot, weights in sorted order).
 // Called by every thread of the CTA; the caller synchronises before reading the tables.
 // The down kernels call it before they wait for the up kernel: the routing input was complete before that one started, but
 // the reads go to L2, as those of gemm_route.cuh do, so that no line an earlier kernel left in this SM's L1 is taken for it.
+// TRIPLE: the kernel is also launched with a routing triple.
+template <bool TRIPLE = true>
 __device__ __forceinline__ void stage_routing(const GemvArgs& a, int* s_e, float* s_gam) {
   const int P = a.M * a.topk;
   const int p = threadIdx.x;
-  if (a.hist == nullptr) {
+  if (!TRIPLE || a.hist == nullptr) {
     if (p < P) {
       long long id = a.ids_i64 ? __ldcg(reinterpret_cast<const long long*>(a.topk_ids) + p)
                                : static_cast<long long>(__ldcg(reinterpret_cast<const int*>(a.topk_ids) + p));
@@ -95,37 +130,7 @@ __device__ __forceinline__ void stage_routing(const GemvArgs& a, int* s_e, float
   }
   if (p < P) s_e[p] = -1;
   __syncthreads();
-  // The lane of an expert places its run of sorted rows; 128 experts' counts are fetched at a time.  (Each thread walking the
-  // counts by itself, both launches of one token from a graph: 128 experts of 2048 x 768 34.7 us against 23.1, 256 of 512 x 256
-  // 36.3 against 13.1.)
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    int run = 0;
-    for (int e0 = lane; e0 - lane < a.E; e0 += 128) {
-      int n[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) n[u] = e0 + 32 * u < a.E ? max(0, min(P, __ldcg(a.hist + e0 + 32 * u))) : 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (e0 - lane + 32 * u >= a.E) break;
-        int end = n[u];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, end, d);
-          if (lane >= d) end += v;
-        }
-        for (int q = run + end - n[u]; q < min(P, run + end); ++q) {
-          const int slot = __ldcg(a.topk_indx + q);
-          if (slot >= 0 && slot < P) {
-            s_e[slot] = e0 + 32 * u;
-            s_gam[slot] = __ldcg(a.gate_scal + q);
-          }
-        }
-        __syncwarp();
-        run += __shfl_sync(0xffffffffu, end, 31);
-      }
-    }
-  }
+  if (threadIdx.x < 32) place_sorted_rows(a.hist, a.topk_indx, a.gate_scal, P, a.E, s_e, s_gam);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -133,7 +138,8 @@ __device__ __forceinline__ void stage_routing(const GemvArgs& a, int* s_e, float
 // U: 256-element chunks of each row that a lane keeps in flight.  4 by default (8 halves the resident
 // CTAs and measured 10 % slower); 5 or 6 when that is the whole row, so that a row of 1280 or 1536
 // elements does not need a second, nearly empty pass.
-// U = 2 where its six CTAs an SM give every column a warp of its own in one wave and three would not (launch_gemv_up).
+// U = 2 where its six CTAs an SM give every column a warp of its own in one wave and three would not (launch_gemv_up); from ids
+// only, since 40 registers a thread leave none for the placing of a triple's rows.
 template <typename T, int U>
 __global__ void __launch_bounds__(kUpThreads, U == 2 ? 6 : 1)
 moe_gemv_up_kernel(const GemvArgs a) {
@@ -146,7 +152,7 @@ moe_gemv_up_kernel(const GemvArgs a) {
 
   griddep_wait();
   griddep_launch_dependents();
-  stage_routing(a, s_e, s_gam);
+  stage_routing<U != 2>(a, s_e, s_gam);
   const T* x = reinterpret_cast<const T*>(a.x);
   const int quads = a.H >> 2;
   for (int i = threadIdx.x; i < a.M * quads; i += kUpThreads) {
@@ -439,7 +445,9 @@ __host__ __device__ __forceinline__ size_t share_bytes(int P, int rows, int I) {
   return static_cast<size_t>(P) * (rows + 1) * I * 2;
 }
 
-template <typename T>
+// (a form without the routing triple: with the code that places its rows the sums' loop gets other registers, 15.3 us against
+// 14.6 for 1 pair of 2048 x 4096)
+template <typename T, bool TRIPLE>
 __global__ void __launch_bounds__(kShareThreads)
 moe_gemv_down_share_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) uint8_t gemv_smem[];
@@ -460,7 +468,7 @@ moe_gemv_down_share_kernel(const GemvArgs a) {
     fence_mbar_init();
   }
   // neither the routing input nor the weights depend on the up kernel
-  stage_routing(a, s_e, s_gam);
+  stage_routing<TRIPLE>(a, s_e, s_gam);
   fence_proxy_async_smem();
   __syncthreads();
   const uint32_t bytes = static_cast<uint32_t>(rows) * a.I * 2;
@@ -1018,16 +1026,14 @@ int launch_down(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, b
                                                                                                     : B200MOE_ERR_CUDA;
 }
 
-template <typename T>
-int launch_share(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
+template <typename K>
+int launch_share(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = share_bytes(a.M * a.topk, share_rows(a.H, num_sms), a.I);
-  if (cudaFuncSetAttribute(moe_gemv_down_share_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-      cudaSuccess)
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
   note_launch("moe_gemv_down_share_kernel<down>");
-  return launch_kernel(moe_gemv_down_share_kernel<T>, dim3(num_sms), dim3(kShareThreads), smem, stream, pdl, a) == cudaSuccess
-             ? B200MOE_OK
-             : B200MOE_ERR_CUDA;
+  return launch_kernel(kernel, dim3(num_sms), dim3(kShareThreads), smem, stream, pdl, a) == cudaSuccess ? B200MOE_OK
+                                                                                                       : B200MOE_ERR_CUDA;
 }
 
 }  // namespace
@@ -1046,12 +1052,16 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_up(moe_gemv_w4_up_kernel, a, num_sms, stream, pdl);
   const int chunks = (a.H + kChunk - 1) / kChunk;
-  // A warp per column in one wave: more columns than the three CTAs an SM of the kernels below seat, up to five.  Just
-  // above three the second wave is nearly empty (4096 columns of 2048: 18.5 -> 17.0 us for both launches, 5120:
-  // 17.5 -> 17.25); at 6144 both are even, and with a row that 5 chunks cover the single pass stays ahead (14.25 / 14.6 us).
-  // With four tokens' rows staged six CTAs no longer fit (19.2 / 20.5 us).
+  // A warp per column in one wave: more columns than the three CTAs an SM of the kernels below seat, up to five.  Both launches,
+  // us, the kernel below / with six CTAs an SM, columns per seat in front: 2048 elements 3.03 16.6 / 17.8, 3.24 15.6 / 15.0, 3.46
+  // 15.8 / 15.0, 3.9 16.6 / 16.5, 4.3 17.3 / 17.05, 4.76 17.7 / 17.9; 1024 3.03 10.7 / 11.05, 3.24 11.3 / 11.2, 4.3 12.2 / 11.8;
+  // 512 3.46 8.75 / 8.2; 2304 3.46 17.95 / 16.4.  Just above three the second wave is a few columns that are over soon, at five
+  // six CTAs an SM are full as well.  A row that five chunks cover stays ahead in its single pass (1280 4.3 15.15 / 15.65), one that
+  // six cover up to four columns a seat (1536 3.9 15.6 / 17.1, 4.3 15.0 / 14.4).  With four tokens' rows staged six CTAs no
+  // longer fit (19.2 / 20.5).
   const long long columns = static_cast<long long>(a.M) * a.topk * a.I, seats = static_cast<long long>(num_sms) * (kUpThreads / 32);
-  if (share_fits(a, num_sms) && a.M <= 2 && chunks != 5 && columns > 3 * seats && columns <= 5 * seats)
+  if (share_fits(a, num_sms) && a.hist == nullptr && a.M <= 2 && chunks != 5 &&
+      10 * columns > (chunks == 6 ? 40 : 31) * seats && 10 * columns <= 48 * seats)
     return a.dtype == B200MOE_DTYPE_BF16 ? launch_up(moe_gemv_up_kernel<__nv_bfloat16, 2>, a, num_sms, stream, pdl)
                                          : launch_up(moe_gemv_up_kernel<__half, 2>, a, num_sms, stream, pdl);
   const bool bf = a.dtype == B200MOE_DTYPE_BF16;
@@ -1067,9 +1077,14 @@ int launch_gemv_up(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl
 int launch_gemv_down(const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   if (!gemv_fits(a)) return B200MOE_ERR_UNSUPPORTED;
   if (a.w4) return launch_down(moe_gemv_w4_down_kernel, a, num_sms, stream, pdl);
-  if (share_fits(a, num_sms) && share_wins(a, num_sms))
-    return a.dtype == B200MOE_DTYPE_BF16 ? launch_share<__nv_bfloat16>(a, num_sms, stream, pdl)
-                                         : launch_share<__half>(a, num_sms, stream, pdl);
+  if (share_fits(a, num_sms) && share_wins(a, num_sms)) {
+    const bool bf = a.dtype == B200MOE_DTYPE_BF16;
+    if (a.hist != nullptr)
+      return bf ? launch_share(moe_gemv_down_share_kernel<__nv_bfloat16, true>, a, num_sms, stream, pdl)
+                : launch_share(moe_gemv_down_share_kernel<__half, true>, a, num_sms, stream, pdl);
+    return bf ? launch_share(moe_gemv_down_share_kernel<__nv_bfloat16, false>, a, num_sms, stream, pdl)
+              : launch_share(moe_gemv_down_share_kernel<__half, false>, a, num_sms, stream, pdl);
+  }
   return a.dtype == B200MOE_DTYPE_BF16 ? launch_down(moe_gemv_down_kernel<__nv_bfloat16>, a, num_sms, stream, pdl)
                                        : launch_down(moe_gemv_down_kernel<__half>, a, num_sms, stream, pdl);
 }

@@ -32,7 +32,9 @@ def _rel(a, b):
     (2048, 512, 64, 7, 1, torch.bfloat16, SHARE), (2048, 768, 64, 3, 1, torch.bfloat16, SHARE),
     # the routing triple's counts, 128 experts at a time
     (264, 136, 129, 16, 1, torch.bfloat16, SHARE), (264, 136, 300, 8, 2, torch.float16, SHARE),
-    # up kernel with six CTAs an SM: 3552 < columns <= 5920 and at most two tokens
+    # up kernel with six CTAs an SM, or not: 3671 to 5683 columns and at most two tokens take it (rows of six chunks: from 4737)
+    (1000, 464, 64, 8, 1, torch.float16, SHARE), (768, 704, 64, 8, 1, torch.bfloat16, EARLY),
+    (768, 712, 64, 8, 1, torch.bfloat16, EARLY), (1536, 600, 64, 8, 1, torch.bfloat16, SHARE),
     (1024, 512, 64, 8, 1, torch.bfloat16, SHARE), (1000, 456, 64, 8, 1, torch.float16, SHARE),
     (776, 296, 64, 8, 2, torch.bfloat16, SHARE), (2048, 736, 64, 8, 1, torch.bfloat16, SHARE),
 ])
