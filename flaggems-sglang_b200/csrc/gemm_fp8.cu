@@ -893,7 +893,8 @@ constexpr int kColdRows = 16;
 // CTAs wait for it.  Gate/up takes 600 for it (4096 tokens: 2800 us with 525, 2750 with 600, 2766 with 680).  When
 // the last hot and the last cold CTA finish, us, gate/up and down, 256 experts of 7168 x 2048, zipf: 300 tokens 343 / 395
 // and 213 / 200 (at HBM's rate, however they are divided), 1024: 589 / 612 and 363 / 343, 2048: 932 / 915 and 553 / 522,
-// 4096: 1592 / 1576 and 950 / 877.
+// 4096: 1592 / 1576 and 950 / 877.  Tried and slower: hot blocks rated by the groups of 32 rows they promote (3 % over ten
+// layers), and divisions rated by whole tiles on top (3.5 %).
 template <int MODE>
 struct MixedCost {
   static constexpr float kHotSlice = MODE == 0 ? 970.f : 800.f, kHotTail = MODE == 0 ? 11400.f : 5300.f;
@@ -957,7 +958,22 @@ moe_gemm_fp8_mixed_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int hot = s_hot[a.E], cold = s_cold[a.E], grid = gridDim.x;
+  int hot = s_hot[a.E], cold = s_cold[a.E];
+  const int grid = gridDim.x;
+  // A few cold blocks among hot ones that hold little more go with them: around 20 to 25 slots per expert, flat routing, the
+  // division leaves the cold CTAs behind (us, divided / all hot: 64 experts of 2048 x 1408, average 20 163 / 154, 25 175 / 155;
+  // 128 of 2048 x 768, 25 189 / 175; 32 of 7168 x 2048, 20 308 / 294).  Among full hot blocks it gains whatever their number
+  // (256 of 7168 x 2048, zipf, 8192 tokens 4850 / 5080).
+  if (cold * 4 < hot && a.P <= 32 * hot) {
+    __syncthreads();
+    for (int e = threadIdx.x; e <= a.E; e += blockDim.x) {
+      s_hot[e] += s_cold[e];
+      s_cold[e] = 0;
+    }
+    hot += cold;
+    cold = 0;
+    __syncthreads();
+  }
   int split = 1;
   if (MODE == 1 && !(a.flags & B200MOE_FLAG_NO_SPLIT_K)) split = pick_split((hot + cold) * a.num_nt, a.kblocks, grid, a.max_split);
   const int units = a.num_nt * split;
