@@ -35,6 +35,9 @@ def _ids(counts, m, k, seed):
     (512, 256, [9] * 96, {}),                       # nothing but cold blocks
     (512, 256, [64] * 24, {}),                      # nothing but hot ones
     (512, 256, [700] + [1] * 250, {}),
+    (512, 256, [20] * 40 + [3] * 4, {}),            # too few cold blocks for CTAs of their own; one more
+    (512, 256, [20] * 40 + [3] * 10, {}),
+    (2560, 256, [20] * 200 + [16, 1] * 20, {}),
     (2560, 256, EDGES * 3, {}),                     # the down projection stores pair rows
     (2560, 256, EDGES * 3, dict(bias=True)),
     (2688, 256, EDGES * 3, dict(dtype=torch.float16)),      # half of a tile's columns past the end
