@@ -963,8 +963,9 @@ moe_gemm_fp8_mixed_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   // A few cold blocks among hot ones that hold little more go with them: around 20 to 25 slots per expert, flat routing, the
   // division leaves the cold CTAs behind (us, divided / all hot: 64 experts of 2048 x 1408, average 20 163 / 154, 25 175 / 155;
   // 128 of 2048 x 768, 25 189 / 175; 32 of 7168 x 2048, 20 308 / 294).  Among full hot blocks it gains whatever their number
-  // (256 of 7168 x 2048, zipf, 8192 tokens 4850 / 5080).
-  if (cold * 4 < hot && a.P <= 32 * hot) {
+  // (256 of 7168 x 2048, zipf, 8192 tokens 4850 / 5080).  A launch of one CTA cannot be divided: its hot blocks take the cold
+  // ones with them.
+  if ((cold * 4 < hot && a.P <= 32 * hot) || (grid == 1 && hot > 0)) {
     __syncthreads();
     for (int e = threadIdx.x; e <= a.E; e += blockDim.x) {
       s_hot[e] += s_cold[e];

@@ -3,6 +3,8 @@ alone on the same quantised inputs.
 
 Every product and every per-slice scaling is the same in both; the down projection adds an output's fp32 terms in another
 order or, with pair rows, rounds each to the 16-bit type first (2^-9 of it), so outputs agree to 4e-3 in the 2-norm."""
+import importlib
+
 import pytest
 import torch
 
@@ -117,3 +119,34 @@ def test_hot_and_cold_blocks_against_the_oracle(cuda_device, h, i, e, k, m, entr
     assert "moe_gemm_fp8_mixed_kernel<gate/up>" in names and ("finalize_pairs_kernel" in names) == (h == 2048), names
     F.check_status()
     assert_parity(out, OM.fused_experts_fp8(x, w13, w2, s13, s2, ref_tw, ids), what=f"fp8 mixed {(h, i, e, k, m)} {entry}")
+
+
+@pytest.mark.parametrize("sms", [1, 2, 3])
+@pytest.mark.parametrize("counts,h", [(EDGES, 512), ([130, 3, 140, 1, 5, 2, 9, 4], 512), ([9] * 8, 512)])
+def test_few_sms(cuda_device, monkeypatch, sms, counts, h):
+    """A call that is given a few SMs only (the configuration's num_sms): with one, no CTAs can be kept for cold blocks."""
+    fused_moe = importlib.import_module("flaggems_sglang_b200.ops.fused_moe")
+    d, i, e, k = cuda_device, 256, len(counts), 4
+    m = max(4 * e // k + 1, (sum(counts) + k - 1) // k + 3)
+    ids = _ids(counts, m, k, seed=1).to(d)
+    g = torch.Generator(device=d).manual_seed(2)
+    x = torch.randn(m, h, generator=g, device=d).to(torch.bfloat16)
+    tw = torch.rand(m, k, generator=g, device=d)
+    w13, w2 = make_weights(h, i, e, device=d, seed=3)
+    (w13, s13), (w2, s2) = quantize_fp8_block(w13), quantize_fp8_block(w2)
+    kw = dict(use_fp8_w8a8=True, w13_scale=s13, w2_scale=s2, block_tokens=128)
+    ref = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    make_cfg = fused_moe._make_cfg
+
+    def few(*args, **kwargs):
+        cfg = make_cfg(*args, **kwargs)
+        cfg.num_sms = sms
+        return cfg
+
+    monkeypatch.setattr(fused_moe, "_plans", {})
+    monkeypatch.setattr(fused_moe, "_make_cfg", few)
+    out = F.fused_experts(x, w13, w2, tw, ids, **kw)
+    assert "moe_gemm_fp8_mixed_kernel<gate/up>" in _lib.launch_stats()[1]
+    F.check_status()
+    err = ((out.float() - ref.float()).norm() / ref.float().norm()).item()
+    assert torch.isfinite(out).all() and err <= 4e-3, err
