@@ -264,7 +264,8 @@ int launch_ep_dispatch(const EpDispatchArgs& a, int num_sms, cudaStream_t stream
   if (a.world < 1 || a.world > kMaxPeers || a.rank < 0 || a.rank >= a.world || a.topk > 32) return B200MOE_ERR_BAD_ARG;
   if (a.m < 0 || a.m > a.m_cap || a.H % 8 != 0 || (a.fp8_rows && a.H % 128 != 0)) return B200MOE_ERR_BAD_ARG;
   const size_t smem = a.fp8_rows ? ep_stage_bytes(a.H) : 0;
-  if (smem > 200 * 1024) return B200MOE_ERR_TOO_LARGE;
+  constexpr size_t kMaxStage = 200 * 1024;      // (the setting below: see kSmemLimit)
+  if (smem > kMaxStage) return B200MOE_ERR_TOO_LARGE;
   int ctas = a.m_cap;
   if (ctas > num_sms * 8) ctas = num_sms * 8;
   if (ctas < 1) ctas = 1;
@@ -272,12 +273,12 @@ int launch_ep_dispatch(const EpDispatchArgs& a, int num_sms, cudaStream_t stream
   note_launch("ep_dispatch_kernel");
   if (a.dtype == B200MOE_DTYPE_BF16) {
     if (cudaFuncSetAttribute(ep_dispatch_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
+                             static_cast<int>(kMaxStage)) != cudaSuccess)
       return B200MOE_ERR_CUDA;
     err = launch_kernel(ep_dispatch_kernel<__nv_bfloat16>, dim3(ctas), dim3(kDispatchWarps * 32), smem, stream, pdl, a);
   } else {
     if (cudaFuncSetAttribute(ep_dispatch_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
+                             static_cast<int>(kMaxStage)) != cudaSuccess)
       return B200MOE_ERR_CUDA;
     err = launch_kernel(ep_dispatch_kernel<__half>, dim3(ctas), dim3(kDispatchWarps * 32), smem, stream, pdl, a);
   }

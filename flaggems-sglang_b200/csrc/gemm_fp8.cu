@@ -1028,7 +1028,7 @@ int launch_fp8_mixed(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUt
   const size_t smem = 1024 + g.table_off + mixed_table_bytes(a.E);
   if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
   if (cudaFuncSetAttribute(moe_gemm_fp8_mixed_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
+                           static_cast<int>(kSmemLimit)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
   note_launch(MODE == 0 ? "moe_gemm_fp8_mixed_kernel<gate/up>" : "moe_gemm_fp8_mixed_kernel<down>");
   cudaError_t err = launch_kernel(moe_gemm_fp8_mixed_kernel<MODE>, dim3(num_sms), dim3(kThreadsFp8TokM), smem, stream,
@@ -1042,7 +1042,7 @@ int launch_fp8(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const GemmArgs&
   const size_t smem = 1024 + static_cast<size_t>(a.stages) * fp8_stage_bytes(a.BT) + fp8_ctrl_bytes(a, a.BT);
   if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
   if (cudaFuncSetAttribute(moe_gemm_fp8_kernel<MODE, BT, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
+                           static_cast<int>(kSmemLimit)) != cudaSuccess)
     return B200MOE_ERR_CUDA;
   note_launch(MODE == 0 ? "moe_gemm_fp8_kernel<gate/up>" : "moe_gemm_fp8_kernel<down>");
   cudaError_t err = launch_kernel(moe_gemm_fp8_kernel<MODE, BT, NG>, dim3(num_sms), dim3(fp8_threads(NG)), smem,

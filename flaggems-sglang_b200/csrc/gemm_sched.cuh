@@ -9,7 +9,9 @@ constexpr int kTileRows = 128;           // weight rows per MMA (the instruction
 constexpr int kStageKBytes = 128;        // bytes of the reduction dim per stage row (one swizzle atom)
 constexpr int kTileBytes = kTileRows * kStageKBytes;  // 16 KiB
 constexpr int kMaxBT = 256;
-constexpr size_t kSmemLimit = 232448;    // 227 KiB
+// 227 KiB.  A kernel is always allowed the same amount, whatever a call needs: the setting is shared by all host threads,
+// and one that lowered it would make another thread's launch fail.
+constexpr size_t kSmemLimit = 232448;
 
 struct Ctrl {
   int nblocks;

@@ -390,7 +390,7 @@ static int launch_one(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Ge
   const size_t smem = gemm_smem_bytes(a);
   if (smem > kSmemLimit) return B200MOE_ERR_TOO_LARGE;
   cudaError_t err = cudaFuncSetAttribute(moe_gemm_tc_kernel<MODE, T, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+                                         static_cast<int>(kSmemLimit));
   if (err != cudaSuccess) return B200MOE_ERR_CUDA;
   note_launch(MODE == 0 ? "moe_gemm_tc_kernel<gate/up>" : "moe_gemm_tc_kernel<down>");
   err = launch_kernel(moe_gemm_tc_kernel<MODE, T, EXT>, dim3(num_sms), dim3(kTcThreads), smem, stream, a.pdl != 0, tm_w, tm_x,

@@ -1001,12 +1001,17 @@ bool share_wins(const GemvArgs& a, int num_sms) {
   const int split = down_split(a, num_sms), slots = a.topk * ((a.I + kChunk - 1) / kChunk);
   return by_pair || split == 1 || (slots + split - 1) / split != 6;
 }
+// Every kernel may have 48 KB, its static shared memory among them, without being told; above that always the same limit
+// (see kSmemLimit).
+template <typename K>
+bool allow_smem(K kernel, size_t smem, size_t limit) {
+  return smem <= 44 * 1024 ||
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)) == cudaSuccess;
+}
 template <typename K>
 int launch_up(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = gemv_up_smem(a);
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(smem)) != cudaSuccess)
-    return B200MOE_ERR_CUDA;
+  if (!allow_smem(kernel, smem, kSmemLimit)) return B200MOE_ERR_CUDA;
   const unsigned grid = grid_for(kernel, smem, kUpThreads, static_cast<long long>(a.M) * a.topk * a.I, num_sms);
   note_launch(a.w4 ? "moe_gemv_w4_up_kernel<gate/up>" : "moe_gemv_up_kernel<gate/up>");
   return launch_kernel(kernel, dim3(grid), dim3(kUpThreads), smem, stream, pdl, a) == cudaSuccess ? B200MOE_OK
@@ -1015,8 +1020,7 @@ int launch_up(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, boo
 template <typename K>
 int launch_down(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = gemv_down_smem(a);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return B200MOE_ERR_CUDA;
+  if (!allow_smem(kernel, smem, kSmemLimit)) return B200MOE_ERR_CUDA;
   GemvArgs b = a;
   const long long tasks = static_cast<long long>(a.M) * (a.H / 2);
   b.down_split = down_split(a, num_sms);
@@ -1029,8 +1033,7 @@ int launch_down(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, b
 template <typename K>
 int launch_share(K kernel, const GemvArgs& a, int num_sms, cudaStream_t stream, bool pdl) {
   const size_t smem = share_bytes(a.M * a.topk, share_rows(a.H, num_sms), a.I);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return B200MOE_ERR_CUDA;
+  if (!allow_smem(kernel, smem, kShareBytes)) return B200MOE_ERR_CUDA;
   note_launch("moe_gemv_down_share_kernel<down>");
   return launch_kernel(kernel, dim3(num_sms), dim3(kShareThreads), smem, stream, pdl, a) == cudaSuccess ? B200MOE_OK
                                                                                                        : B200MOE_ERR_CUDA;
