@@ -21,7 +21,7 @@ EDGES = [1, 15, 16, 17, 127, 128, 129, 0, 300, 2, 255, 257]
 
 
 def _ids(counts, m, k, seed):
-    """[m, k] expert ids with these numbers of slots (the rest is -1), no expert twice in a token where that can be."""
+    """[m, k] expert ids with these numbers of slots (the rest is -1), in any order: an expert may stand twice in a token."""
     slots = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])
     flat = torch.full((m * k,), -1)
     flat[: slots.numel()] = slots
@@ -39,9 +39,10 @@ def _ids(counts, m, k, seed):
     (512, 256, [700] + [1] * 250, {}),
     (512, 256, [20] * 40 + [3] * 4, {}),            # too few cold blocks for CTAs of their own; one more
     (512, 256, [20] * 40 + [3] * 10, {}),
-    (2560, 256, [20] * 200 + [16, 1] * 20, {}),
-    (2560, 256, EDGES * 3, {}),                     # the down projection stores pair rows
-    (2560, 256, EDGES * 3, dict(bias=True)),
+    (2560, 256, [20] * 200 + [16, 1] * 30, {}),      # pair rows, 35 x 10 tiles; enough cold blocks for CTAs of their own
+    # the down projection stores pair rows (29 full blocks' worth of slots x 11 tiles of columns, from 296 on)
+    (2816, 256, EDGES * 3, {}),
+    (2816, 256, EDGES * 3, dict(bias=True)),
     (2688, 256, EDGES * 3, dict(dtype=torch.float16)),      # half of a tile's columns past the end
 ])
 def test_hot_and_cold_blocks(cuda_device, h, i, counts, kw):
@@ -63,6 +64,7 @@ def test_hot_and_cold_blocks(cuda_device, h, i, counts, kw):
     out = F.fused_experts(x, w13, w2, tw, ids, **kw)
     names = _lib.launch_stats()[1]
     assert "moe_gemm_fp8_mixed_kernel<gate/up>" in names and "group_quant_slots_kernel" in names, names
+    assert ("finalize_pairs_kernel" in names) == (h > 512), names
     ref = F.fused_experts(x, w13, w2, tw, ids, block_tokens=16, **kw)
     F.check_status()
     err = ((out.float() - ref.float()).norm() / ref.float().norm()).item()
