@@ -38,6 +38,7 @@ def test_threads_share_kernels(cuda_device, kind, kernel, layers):
         assert kernel in _lib.launch_stats()[1], _lib.launch_stats()[1]
         calls[-1] = (calls[-1], ref)
     torch.cuda.synchronize()
+    F.release_workspaces()                    # four streams to come, all with room of their own
     calls *= 2
     start = threading.Barrier(len(calls))
 
